@@ -543,6 +543,7 @@ int mdx_close(mdx_ctx *ctx) {
                   d.shk_cl, d.shk_rec, d.shk_mfail, d.pull_atom, d.pull_ref, d.pull_step};
   if (ctx->stream) {
     for (void *p : ptrs) ctx_free(ctx, p);
+    fx_release(ctx);
     cudaStreamSynchronize(ctx->stream);
   }
   ctx->drop_graphs();
@@ -789,6 +790,7 @@ int mdx_upload_topology(mdx_ctx *ctx, const mdx_topo *t) {
   RC(upload(ctx, d.qsite, qsite.data(), n));
   RC(upload(ctx, d.qsitef, qsitef.data(), n));
   ctx->h_q.assign(t->q, t->q + n);
+  RC(fx_update_qscale(ctx));
   ctx->q_dirty = true;
   if (ctx->mixed()) {
     if (ns >= (1 << MDX_SITE_BITS) || d.nop >= (1 << (32 - MDX_SITE_BITS))) {
@@ -1437,7 +1439,7 @@ int mdx_get_path_info(const mdx_ctx *ctx, mdx_path_info *out) {
   out->ewald_force_pass = !mx ? 0 : d.tc_on ? 2 : 1;
   out->ewald_sfac_pass = !mx ? 0 : d.tcs_on ? 2 : 1;
   out->sfac_slices = ctx->furir_init ? sfac_slices(ctx) : 0;
-  out->sfac_ordered = (mx && d.tcs_on) || d.sk_part != nullptr ? 1 : 0;
+  out->sfac_ordered = (mx && d.tcs_on) || d.fx_on || d.sk_part != nullptr ? 1 : 0;
   out->list_mode = ctx->p.rskin > 0.0 ? 1 : 0;
   out->graphs = ctx->use_graphs ? 1 : 0;
   out->nkv = ctx->nkv;
@@ -1560,7 +1562,7 @@ int mdx_set_lambda(mdx_ctx *ctx, double ec, double pw1, double pw2, double bee) 
     cudaStreamSynchronize(ctx->stream);
   }
   if (ctx->mixed()) RC(upload_site_table(ctx));
-  return MDX_OK;
+  return fx_update_qscale(ctx);
 }
 
 int mdx_set_timers(mdx_ctx *ctx, int on) {

@@ -253,6 +253,16 @@ struct DevData {
   unsigned char *tcs_zimg;  // Z image (B operand), per 32-atom chunk
   double *tcs_red;          // partials reduced per M-tile (FP64)
   int tcs_np, tcs_ntm, tcs_nslice, tcs_slice, tcs_items, tcs_gps, tcs_ncg;
+  // FP64 path's fixed-point tensor-core passes (ewald_fx.cu): two-word X, Y
+  // tables and the Z digit images, W digit tiles and their records, integer
+  // S(k) and force sums, the charge scale {qs, 1 / qs}
+  bool fx_on, fx_xys;
+  int4 *fx_xy, *fx_slot;
+  unsigned char *fx_zs, *fx_zf, *fx_tw, *fx_meta;
+  int *fx_scol, *fx_ks, *fx_parts;
+  unsigned long long *fx_acc, *fx_facc;
+  double *fx_qs;
+  int fx_np, fx_ntm, fx_ns, fx_cps, fx_ua, fx_ug, fx_ntile, fx_nsplit;
   int *rf_part;                 // group ranges of the mixed force pass's warps
   int rf_nsplit;                // blocks per atom tile of that pass
   double2 *colrv;               // per column (RXV, RYV) at the current box
@@ -735,6 +745,13 @@ int sfac_slices(const mdx_ctx *ctx);  // slices of the S(k) partial sums
 int tc_force_setup(mdx_ctx *ctx, const std::vector<KCol> &cols, int kmaz);
 int tc_sfac_setup(mdx_ctx *ctx, const std::vector<KCol> &cols);
 int tc_sfac_launch(mdx_ctx *ctx);
+// ewald_fx.cu: the FP64 path's passes in fixed point on the tensor cores
+int fx_setup(mdx_ctx *ctx, const std::vector<KCol> &cols);  // sets dv.fx_on
+void fx_release(mdx_ctx *ctx);
+int fx_update_qscale(mdx_ctx *ctx);
+int fx_tables_launch(mdx_ctx *ctx);
+int fx_sfac_launch(mdx_ctx *ctx);
+int fx_force_launch(mdx_ctx *ctx);
 int tc_zimages_launch(mdx_ctx *ctx);
 int tc_force_launch(mdx_ctx *ctx);
 // Dynamic shared-memory limit of a kernel: process-wide, shared by every

@@ -106,6 +106,8 @@ def estimate_bytes(s: S.System, precision: int) -> int:
     kmax = int(math.ceil((nkv * 3.0 / (2.0 * math.pi)) ** (1.0 / 3.0))) + 2
     rows = 4 * kmax + 3
     per_atom = 1024 + 4 * (cs + cl) + 16 * rows + 4 * s.nbdmax
+    if precision != MDX_MIXED:
+        per_atom += 28 * (2 * kmax + 18)  # the Z digit images of the fixed-point Ewald passes
     slices = max(1, -(-n // 128))
     per_k = 256 + 16 * slices
     return int(n * per_atom + nkv * per_k + (24 << 20))
