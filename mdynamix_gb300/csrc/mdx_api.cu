@@ -539,7 +539,7 @@ int mdx_close(mdx_ctx *ctx) {
                   d.bid, d.brb, d.ibi, d.ara, d.iai, d.titors, d.tft, d.iti, d.br,
                   d.ar, d.tr, d.cols, d.kchunks, d.kgroups, d.kconst, d.rf_part, d.tc_slot, d.tc_w, d.tc_meta, d.tcs_part, d.tcs_cp0, d.tc_zimg, d.tcs_zimg, d.tcs_red, d.sitems, d.tabx, d.tabxf, d.sk, d.sc, d.th,
                   d.rec, d.err, d.shake_iter, d.red, d.scal_scratch, d.nspec_d,
-                  d.red_part, d.red_ctr, d.sk_part, d.snap, d.avsum, d.shk_item,
+                  d.red_part, d.red_ctr, d.sk_part, d.pair_tab, d.snap, d.avsum, d.shk_item,
                   d.shk_cl, d.shk_rec, d.shk_mfail, d.pull_atom, d.pull_ref, d.pull_step};
   if (ctx->stream) {
     for (void *p : ptrs) ctx_free(ctx, p);
@@ -989,6 +989,7 @@ int mdx_set_params(mdx_ctx *ctx, const mdx_params *p) {
   ctx->bozl = p->bozl;
   ctx->furir_init = false;
   set_fix_scales(ctx);
+  RC(pair64_setup(ctx));
   ctx->have_params = true;
   return MDX_OK;
 }

@@ -256,6 +256,7 @@ struct DevData {
   // FP64 path's fixed-point tensor-core passes (ewald_fx.cu): two-word X, Y
   // tables and the Z digit images, W digit tiles and their records, integer
   // S(k) and force sums, the charge scale {qs, 1 / qs}
+  void *pair_tab;  // FP64 pair sweeps: tabulated functions of r^2 (pair64.cu)
   bool fx_on, fx_xys;
   int4 *fx_xy, *fx_slot;
   unsigned char *fx_zs, *fx_zf, *fx_tw, *fx_meta;
@@ -349,6 +350,7 @@ struct mdx_ctx {
         g = nullptr;
       }
   }
+  double pair_tab_alpha = 0.0;  // alpha of dv.pair_tab
   int mbsh = 0, mbln = 0;
   cudaEvent_t snap_ev[MDX_SNAPSHOT_SLOTS] = {};  // completion of mdx_snapshot per slot
   // device timers (mdx_set_timers)
@@ -732,6 +734,9 @@ int export_lists(mdx_ctx *ctx, int32_t *nbs1, int32_t *nbs2, int32_t cap_s,
 int launch_localf(mdx_ctx *ctx, bool split, bool ener = true);
 int pack_lj_tables(mdx_ctx *ctx);  // abf from the FP32 tables
 int launch_forces_long(mdx_ctx *ctx, bool split);
+// pair64.cu
+int pair64_setup(mdx_ctx *ctx);
+int launch_pair64(mdx_ctx *ctx, bool shrt, bool split, bool ener, double *split_buf);
 int launch_wir(mdx_ctx *ctx, int which);  // WIRSS (1) / WIRS (2)
 // ewald.cu
 int host_inifur(mdx_ctx *ctx);

@@ -2,12 +2,7 @@
 //   LOCALF (forces.f:813-998) on the short rows into H,
 //   FORCES (forces.f:1014-1202) on the long rows into G.
 //
-// FP64 path: one warp per owner atom walks its half row (every pair once,
-// as in the reference list); the owner's force is reduced in registers and
-// the partner's goes out with FP64 atomics.  The arithmetic is the
-// reference's, statement by statement.
-//
-// Mixed path: rows are full (both atoms of a pair hold it), so a warp writes
+// The FP64 path's sweeps are in pair64.cu.  Mixed path: rows are full (both atoms of a pair hold it), so a warp writes
 // only its own atom and there is no scattered atomic at all.  Pair geometry
 // comes from 32-bit fixed-point coordinates (x / L * 2^32): the difference of
 // two such integers is exact and wraps to the minimum image by itself, and is
@@ -19,15 +14,12 @@
 #include <cmath>
 
 #include "mdx_internal.cuh"
-#include "pair_math.cuh"
 #include "tune_table.cuh"
 
 namespace {
 
-// Per-pair parameters (forces.f:838-862 / 1040-1066).
+// Per-pair parameters (forces.f:838-862 / 1040-1066) of the mixed sweeps.
 struct PairTables {
-  const double *a6lj, *b12lj, *a6lj0, *b12lj0, *a6_14, *b12_14;
-  const float *a6f, *b12f, *a60f, *b120f, *a614f, *b1214f;
   const float2 *abf;  // (A6, B12) FP32 pairs: [kind][i*nnbt + j], kind 0 inter, 1 intra, 2 1-4
   int nn;             // nnbt^2
 };
@@ -43,182 +35,9 @@ enum {
   P_NSLOT
 };
 
-__device__ __forceinline__ double ewald_erfc_poly(double ttt, double exp2a) {
-  return ((((MDX_A5 * ttt + MDX_A4) * ttt + MDX_A3) * ttt + MDX_A2) * ttt +
-          MDX_A1) * ttt * exp2a;
-}
 __device__ __forceinline__ float ewald_erfc_polyf(float ttt, float exp2a) {
   return (((((float)MDX_A5 * ttt + (float)MDX_A4) * ttt + (float)MDX_A3) * ttt +
            (float)MDX_A2) * ttt + (float)MDX_A1) * ttt * exp2a;
-}
-
-// ---------------------------------------------------------------- FP64 ---
-template <bool SHORT, bool SPLIT, bool ENER>
-__global__ void __launch_bounds__(256) k_pair64(
-    int n, const dbl4 *__restrict__ pos, const int4 *__restrict__ ainfo,
-    const double *__restrict__ qsite, const int *__restrict__ cnt,
-    const int *__restrict__ idx, int cap, PairTables tb, TypeConst tc,
-    PairConst pc, double bx, double by, double bz, CellPbc cp, double *__restrict__ fx,
-    double *__restrict__ fy, double *__restrict__ fz,
-    Dst6 dst, double *__restrict__ split) {
-  __shared__ double s_split[2 * MDX_NTPP + 2 * MDX_NT];
-  if (SPLIT) {
-    for (int k = threadIdx.x; k < 2 * MDX_NTPP + 2 * MDX_NT; k += blockDim.x) s_split[k] = 0.0;
-    __syncthreads();
-  }
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  // ABS(D) > HBOX tests as integer compares of the magnitudes' bit patterns
-  // (the same order as the FP64 compare for finite values; no FP64 issue)
-  const long long hbxb = __double_as_longlong(0.5 * bx), hbyb = __double_as_longlong(0.5 * by);
-  // LOCALF tests DZ against HBOXL (forces.f:871); FORCES against HBOZL
-  const long long hbzb = __double_as_longlong(SHORT ? 0.5 * bx : 0.5 * bz);
-  const long long rc2b = __double_as_longlong(pc.rc2);
-  const bool rae_on = pc.lmdee && pc.raex != 0.0;
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  if (i < n) {
-    const dbl4 pi = pos[i];
-    const int4 ai = ainfo[i];
-    const int ti = ai.x, mi = ai.y, ni = ai.z;
-    const double qsi = qsite[i];
-    const int c = cnt[i];
-    double fix = 0.0, fiy = 0.0, fiz = 0.0;
-    const int *row = idx + (size_t)i * cap;
-    for (int k = lane; k < c; k += 32) {
-      const int v = row[k];
-      const bool is14 = SHORT && v < 0;
-      const int j = v & 0x7fffffff;
-      const dbl4 pj = pos[j];
-      const int4 aj = ainfo[j];
-      const int tj = aj.x, nj = aj.z;
-      const bool same = aj.y == mi;
-      const int mtr = tc.mdx[ti][tj];
-      double QIJ, A6, B12;
-      bool rae = false;  // RAEX shifts this pair's distance (MDEE)
-      const int tix = ni * pc.nnbt + nj;
-      if (same) {
-        if (is14) {
-          QIJ = qsi * qsite[j] * pc.coulf * tc.c14el[ti];
-          A6 = __ldg(&tb.a6_14[tix]) * tc.c14lj[ti];
-          B12 = __ldg(&tb.b12_14[tix]) * tc.c14lj[ti];
-        } else {
-          QIJ = qsi * qsite[j] * pc.coulf;
-          A6 = __ldg(&tb.a6lj0[tix]);
-          B12 = __ldg(&tb.b12lj0[tix]);
-        }
-      } else {
-        QIJ = pi.w * pj.w * pc.coulf;
-        A6 = __ldg(&tb.a6lj[tix]);
-        B12 = __ldg(&tb.b12lj[tix]);
-        rae = rae_on && tc.iee[ti] * tc.iee[tj] == 0;
-      }
-      double DX = pi.x - pj.x, DY = pi.y - pj.y, DZ = pi.z - pj.z;
-      constexpr long long MAG = 0x7fffffffffffffffLL;
-      if (cp.icell == 0) {
-        if ((__double_as_longlong(DX) & MAG) > hbxb) DX = DX - fsign(bx, DX);
-        if ((__double_as_longlong(DZ) & MAG) > hbzb) DZ = DZ - fsign(bz, DZ);
-        if ((__double_as_longlong(DY) & MAG) > hbyb) DY = DY - fsign(by, DY);
-      } else {  // hexagonal / truncated octahedron (forces.f:872-906, 1077-1111)
-        pbc_cell(DX, DY, DZ, cp, SHORT ? cp.hbx : cp.hbz);
-      }
-      const double RR = DX * DX + DY * DY + DZ * DZ;
-      if (!SHORT && __double_as_longlong(RR) > rc2b) continue;  // skin mode: listed beyond RCUT
-      // one reciprocal square root instead of a square root and a division
-      // (within an ulp of DSQRT and 1/R1)
-      const double R1I = rsqrt(RR);
-      const double R1 = RR * R1I;
-      double R1E = R1, R1EI = R1I;
-      if (rae) {
-        R1E = R1 + pc.raex;
-        R1EI = 1. / R1E;
-      }
-      double EE1, EES, FORCE;
-      if (is14 || (same && tc.iee[ti] == 0)) {
-        if (SHORT) {
-          EE1 = QIJ * R1I;
-          FORCE = tc.lmove[ti] ? EE1 * (R1I * R1I) : 0.0;
-        } else {
-          EE1 = QIJ / R1;
-          FORCE = tc.lmove[ti] ? EE1 / (R1 * R1) : 0.0;
-        }
-        EES = EE1;
-      } else if (pc.lmnbl) {
-        EE1 = QIJ * (1.0 / R1E - 0.5 * pc.rff2 * (R1E * R1E) + pc.rff);
-        EES = EE1;
-        if (SHORT) {
-          FORCE = QIJ * (1. / (R1E * R1E * R1E) + pc.rff2);
-          if (ENER) acc[P_VIR] += QIJ * (1.5 * pc.rff2 / (R1E * R1E) - pc.rff);
-        } else {
-          FORCE = QIJ * (1.0 / ((R1E * R1E) * R1) + pc.rff2);
-          if (ENER) acc[P_VIR] += QIJ * (1.5 * pc.rff2 * RR - pc.rff);
-        }
-      } else {
-        const double ALPHAR = pc.alphad * R1;
-        const double TTT = rcp_nr(1.0 + MDX_B1 * ALPHAR);
-        const double EXP2A = exp_neg(ALPHAR * ALPHAR);
-        const double ERFCT = ewald_erfc_poly(TTT, EXP2A);
-        EE1 = QIJ * R1EI;
-        EES = EE1 * ERFCT;
-        FORCE = EE1 * (MDX_TOTPI * pc.alphad * EXP2A + ERFCT * R1EI) * R1I;
-      }
-      if (SPLIT) {
-        if (same) atomicAdd(&s_split[2 * MDX_NTPP + ti], EE1);
-        else atomicAdd(&s_split[mtr], EE1);
-      }
-      if (ENER) acc[P_EES] += EES;
-      if ((__double_as_longlong(B12) << 1) != 0) {  // B12 != 0
-        const double R2I = R1EI * R1EI;
-        const double R6I = R2I * R2I * R2I;
-        double ESR = (A6 + B12 * R6I) * R6I;
-        const double FSR = (6.0 * A6 + 12.0 * B12 * R6I) * R6I * R1EI;
-        FORCE = FORCE + FSR * R1I;
-        if (same) {
-          if (SHORT) {
-            if (tc.lmove[ti]) {
-              if (SPLIT) atomicAdd(&s_split[2 * MDX_NTPP + MDX_NT + ti], ESR);
-              if (ENER) acc[P_VIR] += FSR * R1;
-            } else {
-              ESR = 0.0;
-              FORCE = 0.0;
-            }
-          } else {
-            if (ENER && tc.lmove[ti]) acc[P_VIR] += FSR * R1;
-            if (SPLIT) atomicAdd(&s_split[2 * MDX_NTPP + MDX_NT + ti], ESR);
-          }
-        } else {
-          if (SPLIT) atomicAdd(&s_split[MDX_NTPP + mtr], ESR);
-          if (ENER) acc[P_VIR] += FSR * R1;
-        }
-        if (ENER) acc[P_ESR] += ESR;
-      }
-      const double gxv = FORCE * DX, gyv = FORCE * DY, gzv = FORCE * DZ;
-      if (SHORT || !same || tc.lmove[ti]) {  // FORCE DX^2 as (FORCE DX) DX
-        if (ENER) acc[3] += gxv * DX;
-        if (ENER) acc[4] += gyv * DY;
-        if (ENER) acc[5] += gzv * DZ;
-      }
-      fix += gxv;
-      fiy += gyv;
-      fiz += gzv;
-      atomicAdd(&fx[j], -gxv);
-      atomicAdd(&fy[j], -gyv);
-      atomicAdd(&fz[j], -gzv);
-    }
-    fix = warp_sum(fix);
-    fiy = warp_sum(fiy);
-    fiz = warp_sum(fiz);
-    if (lane == 0 && c > 0) {
-      atomicAdd(&fx[i], fix);
-      atomicAdd(&fy[i], fiy);
-      atomicAdd(&fz[i], fiz);
-    }
-  }
-  if (ENER) block_add<6>(acc, dst);
-  if (SPLIT) {
-    __syncthreads();
-    for (int k = threadIdx.x; k < 2 * MDX_NTPP + 2 * MDX_NT; k += blockDim.x)
-      if (s_split[k] != 0.0) atomicAdd(&split[k], s_split[k]);
-  }
 }
 
 // WIRSS / WIRS: -sum F . (S - COM(molecule)) (forces.f:991-995,
@@ -904,9 +723,7 @@ __global__ void k_fold_split(double *split, mdx_scalars *sc) {
 // whenever the caller asks for the per-type energies.
 
 PairTables tables(const DevData &d) {
-  return PairTables{d.a6lj, d.b12lj, d.a6lj0, d.b12lj0, d.a6_14, d.b12_14,
-                    d.a6f,  d.b12f,  d.a60f,  d.b120f,  d.a614f, d.b1214f,
-                    d.abf,  d.nnbt * d.nnbt};
+  return PairTables{d.abf, d.nnbt * d.nnbt};
 }
 
 __global__ void k_pack_lj(int nn, const float *__restrict__ f, float2 *__restrict__ abf) {
@@ -927,31 +744,14 @@ __global__ void k_pack_lj(int nn, const float *__restrict__ f, float2 *__restric
 int launch_pair(mdx_ctx *ctx, bool shrt, bool split, bool ener) {
   DevData &d = ctx->dv;
   if (ctx->mixed() && !ctx->tune.tpo_short) resolve_tuning(ctx);
-  const int T = 256, WPB = T / 32;
-  const int grid = (d.n + WPB - 1) / WPB;
+  const int T = 256;
   const int *cnt = shrt ? d.ns_cnt : d.nl_cnt;
   const int *idx = shrt ? d.ns_idx : d.nl_idx;
   const int cap = shrt ? d.cap_s : d.cap_l;
   double *split_buf = d.red + 64;
   if (!ctx->mixed()) {
-    double *fx = shrt ? d.hx : d.gx, *fy = shrt ? d.hy : d.gy, *fz = shrt ? d.hz : d.gz;
-    mdx_scalars *sc = d.sc;
-    Dst6 ddst = shrt ? dst6(ctx, grid, 6, &sc->pels2, &sc->pe2, &sc->vir2, &sc->virfx, &sc->virfy, &sc->virfz)
-                     : dst6(ctx, grid, 6, &sc->pels1, &sc->pe1, &sc->vir1, &sc->virx, &sc->viry, &sc->virz);
-#define LP64(S, P)                                                                \
-  if (ener) k_pair64<S, P, true><<<grid, T, 0, ctx->stream>>>(                    \
-      d.n, d.pos, d.ainfo, d.qsite, cnt, idx, cap, tables(d), ctx->tc, ctx->pc,   \
-      ctx->boxl, ctx->boyl, ctx->bozl, cell_pbc(ctx), fx, fy, fz, ddst, split_buf); \
-  else k_pair64<S, P, false><<<grid, T, 0, ctx->stream>>>(                        \
-      d.n, d.pos, d.ainfo, d.qsite, cnt, idx, cap, tables(d), ctx->tc, ctx->pc,   \
-      ctx->boxl, ctx->boyl, ctx->bozl, cell_pbc(ctx), fx, fy, fz, ddst, split_buf)
-    if (shrt) {
-      if (split) { LP64(true, true); } else { LP64(true, false); }
-    } else {
-      if (split) { LP64(false, true); } else { LP64(false, false); }
-    }
-#undef LP64
-    MDX_LAUNCHED(ctx);
+    const int rc = launch_pair64(ctx, shrt, split, ener, split_buf);
+    if (rc) return rc;
   } else {
     unsigned long long *ffix = shrt ? d.hfix : d.gfix;
     unsigned long long *slots = reinterpret_cast<unsigned long long *>(d.red);

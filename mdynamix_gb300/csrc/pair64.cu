@@ -1,0 +1,719 @@
+// pair64.cu -- the FP64 path's real-space sweeps: LOCALF (forces.f:813-998)
+// on the short rows into H, FORCES (forces.f:1014-1202) on the long rows into
+// G.  Half rows (every pair once, as in the reference list); TPO lanes walk an
+// owner's row, the owner's force is summed in registers, the partner's goes
+// out with FP64 atomics.
+//
+// GB300 issues one FP64 warp instruction per 64 cycles on each scheduler, so
+// a sweep's time is its FP64 instruction count: about 84 a pair with the
+// reference's expressions written out (reciprocal square root, exp, erfc
+// polynomial, reciprocal).  The screened Coulomb force and energy are smooth
+// functions of r^2 alone, so k_pair64t takes them from a table (PairPoly): 128
+// bins an octave of r^2, each a polynomial of degree 6 in the position within
+// the bin, whose four leading steps are FP64 FMAs and whose tail (2^-30 of the
+// value) runs in FP32.  Its error, below 2^-54 of the value plus one
+// rounding, is below that of the written-out expressions, whose roundings it
+// replaces.  The bin and the position come from the bits of r^2 by integer
+// operations.  A Coulomb pair then takes 19 FP64 instructions.  Pairs with an
+// LJ term and the few that are not plain Ewald pairs (own molecule, 1-4,
+// shifted by MDEE, r^2 outside the table) are put aside in shared memory, of
+// all owners of a warp, and evaluated 32 at a time, so that no warp issues an
+// expression for a few of its lanes.
+//
+// Measured on a GB300 at 98,304 atoms, against the written-out sweeps (one
+// warp an owner): short rows, forces 0.526 -> 0.20 ms; long rows with energies
+// 4.88 -> 2.40 ms, with energies by type pair 15.3 -> 3.1 ms.  The FP64 pipe is
+// 82-86 % active.  Error of the slow forces against 64 bits unchanged.
+//
+// k_pair64 writes the reference's expressions out for every pair: the
+// reaction field (LMNBL).
+#include <algorithm>
+#include <cmath>
+
+#include "mdx_internal.cuh"
+#include "pair_math.cuh"
+
+namespace {
+
+// LJ tables (forces.f:838-862 / 1040-1066), by LJ type pair.
+struct Lj64 {
+  const double *a6lj, *b12lj, *a6lj0, *b12lj0, *a6_14, *b12_14;
+};
+
+// One bin of a tabulated function of r^2: value = c0 + t (c1 + t (c2 + t (c3 +
+// t tail))), tail = c4 + t (c5 + t c6), t in [-1/2, 1/2) the position in the bin.
+struct __align__(16) PairPoly {
+  double c0, c1, c2, c3;
+  float c4, c5, c6, pad;
+};
+constexpr int PT_OCT0 = -2, PT_NOCT = 12;     // r^2 from 2^-2 to 2^10 A^2
+constexpr int PT_BINS = 128 * PT_NOCT;
+constexpr int PT_BASE = (1023 + PT_OCT0) * 128;  // bin of r^2: its exponent and 7 leading bits
+enum { PT_FORCE = 0, PT_ENER, PT_R2I, PT_R1I, PT_NFN };
+
+// ------------------------------------------------- two-word FP64 numbers --
+// Sums and products of pairs of doubles (Dekker, Numer. Math. 18, 1971): the
+// table's values and coefficients, to about 100 bits.
+struct dd {
+  double h, l;
+};
+__device__ __forceinline__ dd two_sum(double a, double b) {
+  const double s = a + b, t = s - a;
+  return dd{s, (a - (s - t)) + (b - t)};
+}
+__device__ __forceinline__ dd norm(double a, double b) {
+  const double s = a + b;
+  return dd{s, b - (s - a)};
+}
+__device__ __forceinline__ dd operator+(dd a, dd b) {
+  const dd s = two_sum(a.h, b.h);
+  return norm(s.h, s.l + (a.l + b.l));
+}
+__device__ __forceinline__ dd operator-(dd a) { return dd{-a.h, -a.l}; }
+__device__ __forceinline__ dd operator*(dd a, dd b) {
+  const double p = a.h * b.h;
+  return norm(p, fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
+}
+__device__ __forceinline__ dd D(double a) { return dd{a, 0.0}; }
+__device__ dd div(dd a, dd b) {
+  const double q = a.h / b.h;
+  const dd r = a + -(b * D(q));
+  const double q2 = r.h / b.h;
+  const dd r2 = r + -(b * D(q2));
+  const dd s = norm(q, q2);
+  return s + D(r2.h / b.h);
+}
+__device__ dd sqrt_dd(double a) {
+  const double s = sqrt(a);
+  return norm(s, fma(-s, s, a) / (2.0 * s));
+}
+__device__ dd exp_neg_dd(dd y) {  // exp(-y), y >= 0; 0 beyond 600
+  if (y.h > 600.0) return D(0.0);
+  const double n = rint(y.h * 1.4426950408889634);
+  const dd ln2{0.6931471805599453, 2.3190468138462996e-17};
+  dd r = (ln2 * D(n)) + -y;  // exp(-y) = 2^-n exp(r)
+  r.h *= 1.0 / 64;
+  r.l *= 1.0 / 64;
+  dd s = D(1.0);
+  for (int k = 11; k >= 1; --k) s = D(1.0) + div(r * s, D((double)k));
+  for (int k = 0; k < 6; ++k) s = s * s;
+  return dd{ldexp(s.h, -(int)n), ldexp(s.l, -(int)n)};
+}
+
+// The functions at r^2 = x (exact), per unit charge product: FORCE / QIJ and
+// EES / QIJ of forces.f:1149-1157 with its erfc polynomial, 1 / r^2, 1 / r.
+__device__ dd pair_fn(int fn, double x, double alphad) {
+  if (fn == PT_R2I) return div(D(1.0), D(x));
+  const dd r = sqrt_dd(x);
+  if (fn == PT_R1I) return div(D(1.0), r);
+  const dd ar = D(alphad) * r;
+  const dd t = div(D(1.0), D(1.0) + D(MDX_B1) * ar);
+  const dd e = exp_neg_dd(D(alphad) * D(alphad) * D(x));
+  dd p = D(MDX_A5) * t + D(MDX_A4);
+  p = p * t + D(MDX_A3);
+  p = p * t + D(MDX_A2);
+  p = p * t + D(MDX_A1);
+  const dd er = div(p * t * e, r);
+  if (fn == PT_ENER) return er;
+  return div(D(MDX_TOTPI) * D(alphad) * e + er, D(x));
+}
+
+// Thread per (function, bin): values at 7 Chebyshev points of the bin,
+// divided differences, monomial coefficients.
+__global__ void k_pair_table(double alphad, PairPoly *__restrict__ tab) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= PT_NFN * PT_BINS) return;
+  const int fn = id / PT_BINS, bin = id % PT_BINS;
+  const double oct = ldexp(1.0, PT_OCT0 + bin / 128);
+  constexpr int N = 7;
+  double x[N];
+  dd f[N];
+  for (int k = 0; k < N; ++k) {
+    x[k] = rint(0.5 * cospi((2 * k + 1) / (2.0 * N)) * 1073741824.0) / 1073741824.0;
+    f[k] = pair_fn(fn, oct * (1.0 + ((bin % 128) + 0.5 + x[k]) / 128.0), alphad);
+  }
+  for (int o = 1; o < N; ++o)
+    for (int k = N - 1; k >= o; --k) f[k] = div(f[k] + -f[k - 1], D(x[k] - x[k - o]));
+  dd c[N];
+  for (int k = 0; k < N; ++k) c[k] = D(0.0);
+  for (int k = N - 1; k >= 0; --k) {  // c = c (t - x_k) + f_k
+    for (int m = N - 1; m > 0; --m) c[m] = c[m - 1] + -(c[m] * D(x[k]));
+    c[0] = f[k] + -(c[0] * D(x[k]));
+  }
+  PairPoly p;
+  p.c0 = c[0].h + c[0].l;
+  p.c1 = c[1].h + c[1].l;
+  p.c2 = c[2].h + c[2].l;
+  p.c3 = c[3].h + c[3].l;
+  p.c4 = (float)(c[4].h + c[4].l);
+  p.c5 = (float)(c[5].h + c[5].l);
+  p.c6 = (float)(c[6].h + c[6].l);
+  p.pad = 0.f;
+  tab[id] = p;
+}
+
+// FP32 to FP64 by the bits (a conversion instruction issues on the FP64
+// pipe); a zero or denormal comes back as about 2^-127.
+__device__ __forceinline__ double f2d_bits(float f) {
+  const unsigned b = __float_as_uint(f);
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)),
+                          (int)(b << 29));
+}
+
+// Bin and position of r^2.
+struct PtArg {
+  int bin;
+  double t;
+  float tf;
+};
+__device__ __forceinline__ PtArg pt_arg(double rr) {
+  const int hi = __double2hiint(rr), lo = __double2loint(rr);
+  PtArg a;
+  a.bin = (hi >> 13) - PT_BASE;
+  // the 45 bits below the bin's as a number in [1, 2), less 1.5
+  const unsigned m = __funnelshift_l((unsigned)lo, (unsigned)hi, 7) & 0xfffffu;
+  a.t = __hiloint2double((int)(0x3ff00000u | m), lo << 7) - 1.5;
+  a.tf = __uint_as_float(0x3f800000u | (m << 3)) - 1.5f;
+  return a;
+}
+__device__ __forceinline__ double pt_eval(const PairPoly *__restrict__ tab, const PtArg &a) {
+  const PairPoly *p = tab + a.bin;
+  const double2 c01 = __ldg(reinterpret_cast<const double2 *>(p));
+  const double2 c23 = __ldg(reinterpret_cast<const double2 *>(p) + 1);
+  const float4 cf = __ldg(reinterpret_cast<const float4 *>(p) + 2);
+  const double q = f2d_bits(fmaf(fmaf(cf.z, a.tf, cf.y), a.tf, cf.x));
+  return fma(fma(fma(fma(q, a.t, c23.y), a.t, c23.x), a.t, c01.y), a.t, c01.x);
+}
+
+// --------------------------------------------------------------- one lane --
+// Sums of one lane: PELS, PE, VIR and the diagonal virial, the owner's force,
+// and (SPLIT) the energies by type pair: those of one slot are kept and added
+// to the block's shared sums when the slot changes (a row's partners are
+// mostly of one type: an atomic per pair on a few addresses took two thirds
+// of the sweep).  Slot: the type pair, or MDX_NTPP + type for the owner's
+// molecule.
+struct Acc64 {
+  double e[6];
+  double fx, fy, fz;
+  int slot;
+  double see, slj;
+};
+enum { A_EES = 0, A_ESR, A_VIR, A_VX, A_VY, A_VZ };
+constexpr int SPLIT_N = 2 * MDX_NTPP + 2 * MDX_NT;
+// shared layout as the sums' buffer: POTE1, POTL1, PES141, PSR141
+__device__ __forceinline__ int split_ee(int slot) {
+  return slot < MDX_NTPP ? slot : 2 * MDX_NTPP + (slot - MDX_NTPP);
+}
+__device__ __forceinline__ int split_lj(int slot) {
+  return slot < MDX_NTPP ? MDX_NTPP + slot : 2 * MDX_NTPP + MDX_NT + (slot - MDX_NTPP);
+}
+__device__ __forceinline__ void split_flush(Acc64 &a, double *sh) {
+  if (a.slot < 0) return;
+  atomicAdd(&sh[split_ee(a.slot)], a.see);
+  if (a.slj != 0.0) atomicAdd(&sh[split_lj(a.slot)], a.slj);
+}
+__device__ __forceinline__ void split_add(Acc64 &a, int slot, double ee, double lj, double *sh) {
+  if (slot != a.slot) {
+    split_flush(a, sh);
+    a.slot = slot;
+    a.see = a.slj = 0.0;
+  }
+  a.see += ee;
+  a.slj += lj;
+}
+
+struct Env64 {
+  const dbl4 *pos;
+  const int4 *ainfo;
+  const double *qsite;
+  Lj64 lj;
+  double *fx, *fy, *fz;
+  double bx, by, bz;
+  long long hbxb, hbyb, hbzb;  // bits of the half boxes
+  CellPbc cp;
+  bool rae_on;
+};
+
+__device__ __forceinline__ Env64 env64(const dbl4 *pos, const int4 *ainfo, const double *qsite,
+                                       const Lj64 &lj, double *fx, double *fy, double *fz,
+                                       const CellPbc &cp, bool shrt, const PairConst &pc) {
+  // ABS(D) > HBOX tests as integer compares of the magnitudes' bit patterns
+  // (the same order as the FP64 compare for finite values; no FP64 issue).
+  // LOCALF tests DZ against HBOXL (forces.f:871); FORCES against HBOZL
+  return Env64{pos, ainfo, qsite, lj, fx, fy, fz, cp.bx, cp.by, cp.bz,
+               __double_as_longlong(0.5 * cp.bx), __double_as_longlong(0.5 * cp.by),
+               __double_as_longlong(shrt ? 0.5 * cp.bx : 0.5 * cp.bz), cp,
+               pc.lmdee && pc.raex != 0.0};
+}
+
+// Minimum image.  CONV: the whole warp is here, and an axis is shifted behind
+// a vote (the compiler turns a plain condition into an addition for every pair
+// and a select; most warps have no pair across a face).
+template <bool SHORT, bool CONV>
+__device__ __forceinline__ void image64(const Env64 &v, double &DX, double &DY, double &DZ) {
+  constexpr long long MAG = 0x7fffffffffffffffLL;
+  auto some = [](bool c) { return CONV ? __any_sync(0xffffffffu, c) : c; };
+  if (v.cp.icell == 0) {
+    const bool cx = (__double_as_longlong(DX) & MAG) > v.hbxb,
+               cz = (__double_as_longlong(DZ) & MAG) > v.hbzb,
+               cy = (__double_as_longlong(DY) & MAG) > v.hbyb;
+    if (some(cx) && cx) DX = DX - fsign(v.bx, DX);
+    if (some(cz) && cz) DZ = DZ - fsign(v.bz, DZ);
+    if (some(cy) && cy) DY = DY - fsign(v.by, DY);
+  } else {  // hexagonal / truncated octahedron (forces.f:872-906, 1077-1111)
+    pbc_cell(DX, DY, DZ, v.cp, SHORT ? v.cp.hbx : v.cp.hbz);
+  }
+}
+
+// The pair's force onto the partner j and the owner: its register sum (i <
+// 0) or atom i (pairs put aside, of any owner).
+template <bool ENER>
+__device__ __forceinline__ void apply64(const Env64 &v, int i, int j, double F, double DX,
+                                        double DY, double DZ, bool vir, Acc64 &a) {
+  // the partner's force, formed with the sign (a negation would be another
+  // FP64 instruction)
+  const double jx = -F * DX, jy = -F * DY, jz = -F * DZ;
+  if (ENER && vir) {  // FORCE DX^2 as (FORCE DX) DX
+    a.e[A_VX] = fma(-jx, DX, a.e[A_VX]);
+    a.e[A_VY] = fma(-jy, DY, a.e[A_VY]);
+    a.e[A_VZ] = fma(-jz, DZ, a.e[A_VZ]);
+  }
+  if (i < 0) {
+    a.fx -= jx;
+    a.fy -= jy;
+    a.fz -= jz;
+  } else {
+    atomicAdd(&v.fx[i], F * DX);
+    atomicAdd(&v.fy[i], F * DY);
+    atomicAdd(&v.fz[i], F * DZ);
+  }
+  atomicAdd(&v.fx[j], jx);
+  atomicAdd(&v.fy[j], jy);
+  atomicAdd(&v.fz[j], jz);
+}
+
+__device__ __forceinline__ double ewald_erfc_poly(double ttt, double exp2a) {
+  return ((((MDX_A5 * ttt + MDX_A4) * ttt + MDX_A3) * ttt + MDX_A2) * ttt + MDX_A1) * ttt * exp2a;
+}
+
+struct Pair64 {  // force / distance, the vector, whether the pair's virial counts
+  double F, DX, DY, DZ;
+  bool vir, skip;
+};
+
+// One listed pair, the reference's expressions written out (forces.f:868-998 /
+// 1071-1198); e: the row entry (sign bit: 1-4 pair).
+template <bool SHORT, bool SPLIT, bool ENER>
+__device__ __forceinline__ Pair64 pair_general(const Env64 &v, int e, const dbl4 &pi,
+                                               const int4 &ai, double qsi, const TypeConst &tc,
+                                               const PairConst &pc, double *sh, Acc64 &a) {
+  const int ti = ai.x, mi = ai.y, ni = ai.z;
+  const bool is14 = SHORT && e < 0;
+  const int j = e & 0x7fffffff;
+  const dbl4 pj = v.pos[j];
+  const int4 aj = v.ainfo[j];
+  const int tj = aj.x, nj = aj.z;
+  const bool same = aj.y == mi;
+  double QIJ, A6, B12;
+  bool rae = false;  // RAEX shifts this pair's distance (MDEE)
+  const int tix = ni * pc.nnbt + nj;
+  if (same) {
+    if (is14) {
+      QIJ = qsi * v.qsite[j] * pc.coulf * tc.c14el[ti];
+      A6 = __ldg(&v.lj.a6_14[tix]) * tc.c14lj[ti];
+      B12 = __ldg(&v.lj.b12_14[tix]) * tc.c14lj[ti];
+    } else {
+      QIJ = qsi * v.qsite[j] * pc.coulf;
+      A6 = __ldg(&v.lj.a6lj0[tix]);
+      B12 = __ldg(&v.lj.b12lj0[tix]);
+    }
+  } else {
+    QIJ = pi.w * pj.w * pc.coulf;
+    A6 = __ldg(&v.lj.a6lj[tix]);
+    B12 = __ldg(&v.lj.b12lj[tix]);
+    rae = v.rae_on && tc.iee[ti] * tc.iee[tj] == 0;
+  }
+  double DX = pi.x - pj.x, DY = pi.y - pj.y, DZ = pi.z - pj.z;
+  image64<SHORT, false>(v, DX, DY, DZ);
+  const double RR = DX * DX + DY * DY + DZ * DZ;
+  if (!SHORT && __double_as_longlong(RR) > __double_as_longlong(pc.rc2))
+    return Pair64{0.0, DX, DY, DZ, false, true};  // skin mode: listed beyond RCUT
+  // one reciprocal square root instead of a square root and a division
+  // (within an ulp of DSQRT and 1/R1)
+  const double R1I = rsqrt(RR);
+  const double R1 = RR * R1I;
+  double R1E = R1, R1EI = R1I;
+  if (rae) {
+    R1E = R1 + pc.raex;
+    R1EI = 1. / R1E;
+  }
+  double EE1, EES, FORCE, slj = 0.0;
+  if (is14 || (same && tc.iee[ti] == 0)) {
+    if (SHORT) {
+      EE1 = QIJ * R1I;
+      FORCE = tc.lmove[ti] ? EE1 * (R1I * R1I) : 0.0;
+    } else {
+      EE1 = QIJ / R1;
+      FORCE = tc.lmove[ti] ? EE1 / (R1 * R1) : 0.0;
+    }
+    EES = EE1;
+  } else if (pc.lmnbl) {
+    EE1 = QIJ * (1.0 / R1E - 0.5 * pc.rff2 * (R1E * R1E) + pc.rff);
+    EES = EE1;
+    if (SHORT) {
+      FORCE = QIJ * (1. / (R1E * R1E * R1E) + pc.rff2);
+      if (ENER) a.e[A_VIR] += QIJ * (1.5 * pc.rff2 / (R1E * R1E) - pc.rff);
+    } else {
+      FORCE = QIJ * (1.0 / ((R1E * R1E) * R1) + pc.rff2);
+      if (ENER) a.e[A_VIR] += QIJ * (1.5 * pc.rff2 * RR - pc.rff);
+    }
+  } else {
+    const double ALPHAR = pc.alphad * R1;
+    const double TTT = rcp_nr(1.0 + MDX_B1 * ALPHAR);
+    const double EXP2A = exp_neg(ALPHAR * ALPHAR);
+    const double ERFCT = ewald_erfc_poly(TTT, EXP2A);
+    EE1 = QIJ * R1EI;
+    EES = EE1 * ERFCT;
+    FORCE = EE1 * (MDX_TOTPI * pc.alphad * EXP2A + ERFCT * R1EI) * R1I;
+  }
+  if (ENER) a.e[A_EES] += EES;
+  if ((__double_as_longlong(B12) << 1) != 0) {  // B12 != 0
+    const double R2I = R1EI * R1EI;
+    const double R6I = R2I * R2I * R2I;
+    double ESR = (A6 + B12 * R6I) * R6I;
+    const double FSR = (6.0 * A6 + 12.0 * B12 * R6I) * R6I * R1EI;
+    FORCE = FORCE + FSR * R1I;
+    if (same) {
+      if (SHORT) {
+        if (tc.lmove[ti]) {
+          slj = ESR;
+          if (ENER) a.e[A_VIR] += FSR * R1;
+        } else {
+          ESR = 0.0;
+          FORCE = 0.0;
+        }
+      } else {
+        if (ENER && tc.lmove[ti]) a.e[A_VIR] += FSR * R1;
+        slj = ESR;
+      }
+    } else {
+      slj = ESR;
+      if (ENER) a.e[A_VIR] += FSR * R1;
+    }
+    if (ENER) a.e[A_ESR] += ESR;
+  }
+  if (SPLIT) split_add(a, same ? MDX_NTPP + ti : tc.mdx[ti][tj], EE1, slj, sh);
+  return Pair64{FORCE, DX, DY, DZ, SHORT || !same || tc.lmove[ti], false};
+}
+
+// Sums of NV values over groups of W lanes with the additions shared out: the
+// lanes halve the values among them first, then sum what is left (NV = 4, W =
+// 32: 6 additions a lane instead of 20).  Lane W / NV * k of a group holds the
+// total of value k.
+template <int NV, int W>
+__device__ __forceinline__ double lane_sums(double (&v)[NV]) {
+  const int lane = threadIdx.x & 31;
+  int o = W / 2;
+#pragma unroll
+  for (int m = NV / 2; m >= 1; m >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < m; ++k) {
+      const double keep = up ? v[k + m] : v[k], give = up ? v[k] : v[k + m];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  double s = v[0];
+#pragma unroll
+  for (int p = W / (2 * NV); p >= 1; p >>= 1) s += __shfl_xor_sync(0xffffffffu, s, p);
+  return s;
+}
+
+// The owners' forces out, by three lanes of each group of TPO.
+template <int TPO>
+__device__ __forceinline__ void owner_out(const Env64 &v, int i, Acc64 &a, bool any) {
+  double f[4] = {a.fx, a.fy, a.fz, 0.0};
+  const double s = lane_sums<4, TPO>(f);
+  const int l = threadIdx.x & (TPO - 1), k = l / (TPO / 4);
+  if (any && l % (TPO / 4) == 0 && k < 3)
+    atomicAdd(k == 0 ? &v.fx[i] : k == 1 ? &v.fy[i] : &v.fz[i], s);
+  a.fx = a.fy = a.fz = 0.0;
+}
+
+// Block end: energies and virials, energies by type pair.
+template <bool SPLIT, bool ENER>
+__device__ __forceinline__ void sweep_out(Acc64 &a, const Dst6 &dst, double *sh, double *split) {
+  if (SPLIT) {  // one flush a warp where its lanes agree on the slot
+    const int lane = threadIdx.x & 31;
+    const int s0 = __reduce_max_sync(0xffffffffu, a.slot);
+    if (__all_sync(0xffffffffu, a.slot == s0 || a.slot < 0)) {
+      double w[2] = {a.slot < 0 ? 0.0 : a.see, a.slot < 0 ? 0.0 : a.slj};
+      const double t = lane_sums<2, 32>(w);
+      if (s0 >= 0 && (lane & 15) == 0 && t != 0.0)
+        atomicAdd(&sh[lane == 0 ? split_ee(s0) : split_lj(s0)], t);
+    } else {
+      split_flush(a, sh);
+    }
+  }
+  if (ENER) block_add<6>(a.e, dst);
+  if (SPLIT) {
+    __syncthreads();
+    for (int k = threadIdx.x; k < SPLIT_N; k += blockDim.x)
+      if (sh[k] != 0.0) atomicAdd(&split[k], sh[k]);
+  }
+}
+
+__device__ __forceinline__ void acc_zero(Acc64 &a) {
+#pragma unroll
+  for (int k = 0; k < 6; ++k) a.e[k] = 0.0;
+  a.fx = a.fy = a.fz = 0.0;
+  a.slot = -1;
+  a.see = a.slj = 0.0;
+}
+
+// --------------------------------------------------------------- sweeps ---
+template <bool SHORT, bool SPLIT, bool ENER>
+__global__ void __launch_bounds__(256) k_pair64(
+    int n, const dbl4 *__restrict__ pos, const int4 *__restrict__ ainfo,
+    const double *__restrict__ qsite, const int *__restrict__ cnt, const int *__restrict__ idx,
+    int cap, Lj64 lj, TypeConst tc, PairConst pc, CellPbc cp, double *__restrict__ fx,
+    double *__restrict__ fy, double *__restrict__ fz, Dst6 dst, double *__restrict__ split) {
+  __shared__ double s_split[SPLIT ? SPLIT_N : 1];
+  if (SPLIT) {
+    for (int k = threadIdx.x; k < SPLIT_N; k += blockDim.x) s_split[k] = 0.0;
+    __syncthreads();
+  }
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const Env64 v = env64(pos, ainfo, qsite, lj, fx, fy, fz, cp, SHORT, pc);
+  Acc64 a;
+  acc_zero(a);
+  for (int i = blockIdx.x * nw + (threadIdx.x >> 5); i < n; i += gridDim.x * nw) {
+    const dbl4 pi = pos[i];
+    const int4 ai = ainfo[i];
+    const double qsi = qsite[i];
+    const int c = cnt[i];
+    const int *row = idx + (size_t)i * cap;
+    for (int k = lane; k < c; k += 32) {
+      const int e = row[k];
+      const Pair64 p = pair_general<SHORT, SPLIT, ENER>(v, e, pi, ai, qsi, tc, pc, s_split, a);
+      if (!p.skip) apply64<ENER>(v, -1, e & 0x7fffffff, p.F, p.DX, p.DY, p.DZ, p.vir, a);
+    }
+    __syncwarp();
+    owner_out<32>(v, i, a, c > 0);
+  }
+  sweep_out<SPLIT, ENER>(a, dst, s_split, split);
+}
+
+constexpr int PT_WARPS = 8;
+struct LjQueue {  // pairs put aside for their LJ term, per warp
+  double x[64], y[64], z[64], rr[64], f[64];
+  int i[64], j[64], tix[64];
+};
+
+// Ewald sweep from the tables.  eemask: bit t set for IEE(t) = 0.
+template <bool SHORT, bool SPLIT, bool ENER, int TPO>
+__global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64t(
+    int n, const dbl4 *__restrict__ pos, const int4 *__restrict__ ainfo,
+    const double *__restrict__ qsite, const int *__restrict__ cnt, const int *__restrict__ idx,
+    int cap, Lj64 lj, TypeConst tc, PairConst pc, CellPbc cp, unsigned eemask,
+    const PairPoly *__restrict__ tab, double *__restrict__ fx, double *__restrict__ fy,
+    double *__restrict__ fz, Dst6 dst, double *__restrict__ split) {
+  __shared__ double s_split[SPLIT ? SPLIT_N : 1];
+  __shared__ LjQueue s_q[PT_WARPS];
+  __shared__ int2 s_slow[PT_WARPS][64];
+  if (SPLIT) {
+    for (int k = threadIdx.x; k < SPLIT_N; k += blockDim.x) s_split[k] = 0.0;
+    __syncthreads();
+  }
+  constexpr int OPW = 32 / TPO;  // owners of a warp at a time
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  LjQueue &q = s_q[w];
+  int2 *slow = s_slow[w];
+  const Env64 v = env64(pos, ainfo, qsite, lj, fx, fy, fz, cp, SHORT, pc);
+  const unsigned eem = v.rae_on ? eemask : 0u;
+  const long long rc2b = __double_as_longlong(pc.rc2);
+  Acc64 a;
+  acc_zero(a);
+  int nq = 0, nslow = 0;
+  // the last m (<= 32) pairs of the LJ queue: their LJ terms, then forces
+  auto lj_batch = [&](int m) {
+    __syncwarp();
+    if (lane < m) {
+      const int e = nq - m + lane;
+      const double rr = q.rr[e];
+      const int tix = q.tix[e], i = q.i[e], j = q.j[e];
+      const double R2I = pt_eval(tab + PT_R2I * PT_BINS, pt_arg(rr));
+      const double A6 = __ldg(&lj.a6lj[tix]), B12 = __ldg(&lj.b12lj[tix]);
+      const double R6I = R2I * R2I * R2I, T12 = B12 * R6I;
+      const double G = fma(2.0, T12, A6) * R6I;  // FSR R1 / 6
+      const double F = fma(6.0 * R2I, G, q.f[e]);
+      if (ENER || SPLIT) {
+        const double ESR = (A6 + T12) * R6I;
+        if (ENER) {
+          a.e[A_ESR] += ESR;
+          a.e[A_VIR] = fma(6.0, G, a.e[A_VIR]);
+        }
+        if (SPLIT) split_add(a, tc.mdx[ainfo[i].x][ainfo[j].x], 0.0, ESR, s_split);
+      }
+      apply64<ENER>(v, i, j, F, q.x[e], q.y[e], q.z[e], true, a);
+    }
+    nq -= m;
+    __syncwarp();
+  };
+  auto slow_batch = [&](int m) {
+    __syncwarp();
+    if (lane < m) {
+      const int2 s = slow[nslow - m + lane];
+      const Pair64 p = pair_general<SHORT, SPLIT, ENER>(v, s.y, pos[s.x], ainfo[s.x], qsite[s.x],
+                                                        tc, pc, s_split, a);
+      if (!p.skip) apply64<ENER>(v, s.x, s.y & 0x7fffffff, p.F, p.DX, p.DY, p.DZ, p.vir, a);
+    }
+    nslow -= m;
+    __syncwarp();
+  };
+  for (int i0 = (blockIdx.x * PT_WARPS + w) * OPW; i0 < n; i0 += gridDim.x * PT_WARPS * OPW) {
+    const int i = i0 + lane / TPO;
+    const bool own = i < n;
+    const dbl4 pi = pos[own ? i : 0];
+    const int4 ai = ainfo[own ? i : 0];
+    const double qic = pi.w * pc.coulf;
+    const int c = own ? cnt[i] : 0;
+    const int cmax = __reduce_max_sync(0xffffffffu, c);
+    const int *row = idx + (size_t)(own ? i : 0) * cap;
+    const double *b12row = lj.b12lj + ai.z * pc.nnbt;
+    const bool eei = (eem >> ai.x) & 1u;
+    for (int k = lane & (TPO - 1); k - (lane & (TPO - 1)) < cmax; k += TPO) {
+      bool act = k < c;
+      const int e = act ? row[k] : 0;
+      const int j = e & 0x7fffffff;
+      const dbl4 pj = pos[j];
+      const int4 aj = ainfo[j];
+      const bool other = (SHORT && e < 0) || aj.y == ai.y || eei || ((eem >> aj.x) & 1u);
+      double DX = pi.x - pj.x, DY = pi.y - pj.y, DZ = pi.z - pj.z;
+      image64<SHORT, true>(v, DX, DY, DZ);
+      const double RR = DX * DX + DY * DY + DZ * DZ;
+      if (!SHORT && __double_as_longlong(RR) > rc2b) act = false;  // skin mode
+      PtArg p = pt_arg(RR);
+      const bool sl = act && (other || (unsigned)p.bin >= (unsigned)PT_BINS);
+      const bool fast = act && !sl;
+      if (!fast) p.bin = 0;
+      const unsigned ms = __ballot_sync(0xffffffffu, sl);
+      if (ms) {
+        if (sl) slow[nslow + __popc(ms & below)] = make_int2(i, e);
+        nslow += __popc(ms);
+        if (nslow >= 32) slow_batch(32);
+      }
+      const double qq = fast ? qic * pj.w : 0.0;
+      const double F = qq * pt_eval(tab + PT_FORCE * PT_BINS, p);
+      if (ENER) a.e[A_EES] = fma(qq, pt_eval(tab + PT_ENER * PT_BINS, p), a.e[A_EES]);
+      if (SPLIT && fast)
+        split_add(a, tc.mdx[ai.x][aj.x], qq * pt_eval(tab + PT_R1I * PT_BINS, p), 0.0, s_split);
+      const bool lb = fast && (__double_as_longlong(__ldg(&b12row[aj.z])) << 1) != 0;  // B12 != 0
+      if (fast && !lb) apply64<ENER>(v, -1, j, F, DX, DY, DZ, true, a);
+      const unsigned ml = __ballot_sync(0xffffffffu, lb);
+      if (ml) {
+        if (lb) {
+          const int s = nq + __popc(ml & below);
+          q.x[s] = DX;
+          q.y[s] = DY;
+          q.z[s] = DZ;
+          q.rr[s] = RR;
+          q.f[s] = F;
+          q.i[s] = i;
+          q.j[s] = j;
+          q.tix[s] = ai.z * pc.nnbt + aj.z;
+        }
+        nq += __popc(ml);
+        if (nq >= 32) lj_batch(32);
+      }
+    }
+    owner_out<TPO>(v, i, a, c > 0);
+  }
+  if (nq) lj_batch(nq);
+  if (nslow) slow_batch(nslow);
+  sweep_out<SPLIT, ENER>(a, dst, s_split, split);
+}
+
+}  // namespace
+
+// The Ewald tables of the sweeps for the current alpha (FP64 path; set_params).
+int pair64_setup(mdx_ctx *ctx) {
+  DevData &d = ctx->dv;
+  if (ctx->mixed() || ctx->p.alphad <= 0.0 || ctx->p.lmnbl) return MDX_OK;
+  if (d.pair_tab && ctx->pair_tab_alpha == ctx->p.alphad) return MDX_OK;
+  if (!d.pair_tab)
+    MDX_CUDA(ctx_alloc(ctx, &d.pair_tab, sizeof(PairPoly) * PT_NFN * PT_BINS));
+  k_pair_table<<<(PT_NFN * PT_BINS + 63) / 64, 64, 0, ctx->stream>>>(
+      ctx->p.alphad, reinterpret_cast<PairPoly *>(d.pair_tab));
+  MDX_LAUNCHED(ctx);
+  ctx->pair_tab_alpha = ctx->p.alphad;
+  return MDX_OK;
+}
+
+int launch_pair64(mdx_ctx *ctx, bool shrt, bool split, bool ener, double *split_buf) {
+  DevData &d = ctx->dv;
+  const int T = 32 * PT_WARPS;
+  const bool table = d.pair_tab && !ctx->p.lmnbl && ctx->p.alphad > 0.0;
+  // Lanes of an owner: 32 on the long rows.  On the short rows (about 26
+  // entries) fewer lanes make the owner's sums cheaper (short sweep at 98,304
+  // atoms: 8 lanes 0.222 ms, 16 0.234, 32 0.257) as long as the owners still
+  // fill half of the resident lanes (600 atoms: 20, 15, 13 us; 3,000: 21.2,
+  // 20.7, 22.9).  The grid is the 2 resident blocks of a SM, each warp taking
+  // several owners, so that the block sums at the end (a few hundred FP64
+  // instructions) are formed once for all of them (long sweep at 3,000 atoms:
+  // 57 us; 8 blocks a SM 69).
+  int tpo = 32;
+  if (shrt && table)
+    while (tpo > 8 && (size_t)d.n * (tpo / 2) >= (size_t)T * ctx->nsm) tpo /= 2;
+  const int per = T / tpo;  // owners of a block at a time
+  const int grid = std::min((d.n + per - 1) / per, 2 * ctx->nsm);
+  const int *cnt = shrt ? d.ns_cnt : d.nl_cnt;
+  const int *idx = shrt ? d.ns_idx : d.nl_idx;
+  const int cap = shrt ? d.cap_s : d.cap_l;
+  double *fx = shrt ? d.hx : d.gx, *fy = shrt ? d.hy : d.gy, *fz = shrt ? d.hz : d.gz;
+  mdx_scalars *sc = d.sc;
+  const Dst6 dst =
+      shrt ? dst6(ctx, grid, 6, &sc->pels2, &sc->pe2, &sc->vir2, &sc->virfx, &sc->virfy, &sc->virfz)
+           : dst6(ctx, grid, 6, &sc->pels1, &sc->pe1, &sc->vir1, &sc->virx, &sc->viry, &sc->virz);
+  const Lj64 lj{d.a6lj, d.b12lj, d.a6lj0, d.b12lj0, d.a6_14, d.b12_14};
+  unsigned eemask = 0;
+  for (int t = 0; t < ctx->d.ntypes; ++t)
+    if (ctx->tc.iee[t] == 0) eemask |= 1u << t;
+  const PairPoly *tab = reinterpret_cast<const PairPoly *>(d.pair_tab);
+  const CellPbc cp = cell_pbc(ctx);
+#define LP64T(S, P, E, K)                                                                       \
+  k_pair64t<S, P, E, K><<<grid, T, 0, ctx->stream>>>(d.n, d.pos, d.ainfo, d.qsite, cnt, idx, cap, \
+                                                     lj, ctx->tc, ctx->pc, cp, eemask, tab, fx, \
+                                                     fy, fz, dst, split_buf)
+#define LP64(S, P, E)                                                                        \
+  do {                                                                                       \
+    if (!table)                                                                              \
+      k_pair64<S, P, E><<<grid, T, 0, ctx->stream>>>(d.n, d.pos, d.ainfo, d.qsite, cnt, idx, \
+                                                     cap, lj, ctx->tc, ctx->pc, cp, fx, fy,  \
+                                                     fz, dst, split_buf);                    \
+    else if (S && tpo == 8) LP64T(S, P, E, S ? 8 : 32);                                      \
+    else if (S && tpo == 16) LP64T(S, P, E, S ? 16 : 32);                                    \
+    else LP64T(S, P, E, 32);                                                                 \
+  } while (0)
+  if (shrt) {
+    if (split) {
+      if (ener) LP64(true, true, true);
+      else LP64(true, true, false);
+    } else if (ener) {
+      LP64(true, false, true);
+    } else {
+      LP64(true, false, false);
+    }
+  } else if (split) {
+    if (ener) LP64(false, true, true);
+    else LP64(false, true, false);
+  } else {
+    if (ener) LP64(false, false, true);
+    else LP64(false, false, false);
+  }
+#undef LP64
+#undef LP64T
+  MDX_LAUNCHED(ctx);
+  return MDX_OK;
+}
