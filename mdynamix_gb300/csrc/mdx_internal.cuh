@@ -575,6 +575,40 @@ __device__ __forceinline__ float warp_sumf(float v) {
   return v;
 }
 
+// Sums of NV values over groups of W lanes with the additions shared out: the
+// lanes halve the values among them first, then sum what is left (NV = 4, W =
+// 32: 6 additions a lane instead of 20).  Lane W / NV * k of a group holds the
+// total of value k.
+template <int NV, int W>
+__device__ __forceinline__ double lane_sums(double (&v)[NV]) {
+  const int lane = threadIdx.x & 31;
+  int o = W / 2;
+#pragma unroll
+  for (int m = NV / 2; m >= 1; m >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < m; ++k) {
+      const double keep = up ? v[k + m] : v[k], give = up ? v[k] : v[k + m];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  double s = v[0];
+#pragma unroll
+  for (int p = W / (2 * NV); p >= 1; p >>= 1) s += __shfl_xor_sync(0xffffffffu, s, p);
+  return s;
+}
+
+// Energies by type pair of the pair sweeps (POTE1, POTL1, PES141, PSR141 back
+// to back in the sums' buffer): a lane keeps the sums of one slot, the type
+// pair or MDX_NTPP + type for the owner's molecule.
+constexpr int SPLIT_N = 2 * MDX_NTPP + 2 * MDX_NT;
+__device__ __forceinline__ int split_ee(int slot) {
+  return slot < MDX_NTPP ? slot : 2 * MDX_NTPP + (slot - MDX_NTPP);
+}
+__device__ __forceinline__ int split_lj(int slot) {
+  return slot < MDX_NTPP ? MDX_NTPP + slot : 2 * MDX_NTPP + MDX_NT + (slot - MDX_NTPP);
+}
+
 // Block-wide sum of NV doubles added to *dst[k] (null pointers skipped).  All
 // threads of the block must call it.
 //

@@ -87,6 +87,53 @@ constexpr int PAIR32_BLOCKS = 6;  // resident blocks per SM the register cap aim
 constexpr int PAIR32X2_BLOCKS = 4;
 constexpr int PAIR32X2_BLOCKS_SHORT = 6;
 
+// Energies by type pair of the force calls (SPLIT), one slot kept per lane as
+// an FP32 sum with its rounding errors (Knuth's two-sum: as good as the FP64
+// sum of the FP32 terms); added to the block's FP64 sums when the slot
+// changes.  An FP64 shared-memory atomic per pair on a few addresses took 14
+// of the 15 ms of a long sweep at 98,304 atoms.
+struct SplitF {
+  int slot;
+  float eh, el, lh, ll;
+};
+__device__ __forceinline__ void two_add(float &h, float &l, float x) {
+  const float s = h + x, b = s - h;
+  l += (h - (s - b)) + (x - b);
+  h = s;
+}
+__device__ __forceinline__ void split_flush(const SplitF &a, double *sh) {
+  if (a.slot < 0) return;
+  atomicAdd(&sh[split_ee(a.slot)], (double)a.eh + (double)a.el);
+  if (a.lh != 0.f) atomicAdd(&sh[split_lj(a.slot)], (double)a.lh + (double)a.ll);
+}
+__device__ __forceinline__ void split_add(SplitF &a, int slot, float ee, float lj, double *sh) {
+  if (slot != a.slot) {
+    split_flush(a, sh);
+    a.slot = slot;
+    a.eh = a.el = a.lh = a.ll = 0.f;
+  }
+  two_add(a.eh, a.el, ee);
+  two_add(a.lh, a.ll, lj);
+}
+// Block end (every thread): one flush a warp where its lanes agree on the
+// slot; each pair is in two full rows.
+__device__ __forceinline__ void split_out(const SplitF &a, double *sh, double *split) {
+  const int lane = threadIdx.x & 31;
+  const int s0 = __reduce_max_sync(0xffffffffu, a.slot);
+  if (__all_sync(0xffffffffu, a.slot == s0 || a.slot < 0)) {
+    const bool has = a.slot >= 0;
+    double w[2] = {has ? (double)a.eh + (double)a.el : 0.0, has ? (double)a.lh + (double)a.ll : 0.0};
+    const double t = lane_sums<2, 32>(w);
+    if (s0 >= 0 && (lane & 15) == 0 && t != 0.0)
+      atomicAdd(&sh[lane == 0 ? split_ee(s0) : split_lj(s0)], t);
+  } else {
+    split_flush(a, sh);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < SPLIT_N; k += blockDim.x)
+    if (sh[k] != 0.0) atomicAdd(&split[k], 0.5 * sh[k]);
+}
+
 __device__ __forceinline__ float idiff(int a, int b, float s) { return fixdiff(a, b, s); }
 
 // Register cap for occupancy: the sweeps wait on gathered neighbour records,
@@ -103,9 +150,10 @@ __global__ void __launch_bounds__(256, PAIR32_BLOCKS) k_pair32(
     const double *__restrict__ Z, double escale,
     unsigned long long *__restrict__ slots, double *__restrict__ split,
     const int *__restrict__ owner_of, CellF cf) {
-  __shared__ double s_split[2 * MDX_NTPP + 2 * MDX_NT];
+  __shared__ double s_split[SPLIT ? SPLIT_N : 1];
+  SplitF spl{-1, 0.f, 0.f, 0.f, 0.f};
   if (SPLIT) {
-    for (int k = threadIdx.x; k < 2 * MDX_NTPP + 2 * MDX_NT; k += blockDim.x) s_split[k] = 0.0;
+    for (int k = threadIdx.x; k < SPLIT_N; k += blockDim.x) s_split[k] = 0.0;
     __syncthreads();
   }
   // TPO adjacent lanes per owner atom stride its row: short rows (about 50
@@ -214,11 +262,7 @@ __global__ void __launch_bounds__(256, PAIR32_BLOCKS) k_pair32(
           EES = EE1 * ERFCT;
           FORCE = EE1 * ((float)MDX_TOTPI * alphad * EXP2A + ERFCT * R1EI) * R1I;
         }
-        if (SPLIT) {
-          const int mtr = tc.mdx[ti][tj];
-          if (same) atomicAdd(&s_split[2 * MDX_NTPP + ti], (double)EE1);
-          else atomicAdd(&s_split[mtr], (double)EE1);
-        }
+        float slj = 0.f;
         if (ENER) {
           if (same) a[P_EE_SAME] += EE1;
           else a[P_EE_DIFF] += EE1;
@@ -245,15 +289,16 @@ __global__ void __launch_bounds__(256, PAIR32_BLOCKS) k_pair32(
             }
             if (count_esr_split) {
               if (ENER) a[P_ESR_SAME] += ESR;
-              if (SPLIT) atomicAdd(&s_split[2 * MDX_NTPP + MDX_NT + ti], (double)ESR);
+              slj = ESR;
             }
           } else {
             if (ENER) a[P_ESR_DIFF] += ESR;
-            if (SPLIT) atomicAdd(&s_split[MDX_NTPP + tc.mdx[ti][tj]], (double)ESR);
+            slj = ESR;
             if (ENER) a[P_VIR] += FSR * R1;
           }
           if (ENER) a[P_ESR] += ESR;
         }
+        if (SPLIT) split_add(spl, same ? MDX_NTPP + ti : tc.mdx[ti][tj], EE1, slj, s_split);
         if (SHORT || !same || lmovei) {
           if (ENER) a[P_VX] += FORCE * (DX * DX);
           if (ENER) a[P_VY] += FORCE * (DY * DY);
@@ -291,6 +336,7 @@ __global__ void __launch_bounds__(256, PAIR32_BLOCKS) k_pair32(
       if (lane == 0) tot[k] = f2ll_rn(t * fsc.escalef);
     }
   }
+  if (SPLIT) split_out(spl, s_split, split);
   if (!ENER) return;  // forces only: no energy or virial slots
   // block sum of the integer slots, one atomic per slot per block
   __shared__ long long sh[8][P_NSLOT];
@@ -305,16 +351,11 @@ __global__ void __launch_bounds__(256, PAIR32_BLOCKS) k_pair32(
     for (int w = 0; w < nw; ++w) s += sh[w][threadIdx.x];
     if (s != 0) atomicAdd(&slots[threadIdx.x], (unsigned long long)s);
   }
-  if (SPLIT) {
-    __syncthreads();
-    for (int k = threadIdx.x; k < 2 * MDX_NTPP + 2 * MDX_NT; k += blockDim.x)
-      if (s_split[k] != 0.0) atomicAdd(&split[k], 0.5 * s_split[k]);
-  }
 }
 
 // ------------------------------------------------------- mixed, paired ---
-// The common case of the mixed sweeps (Ewald, no energy split by type pair,
-// no MDEE shift): each lane evaluates two row entries per iteration with the
+// The common case of the mixed sweeps (Ewald, no MDEE shift): each lane
+// evaluates two row entries per iteration with the
 // paired FP32 instructions of this GPU (__ffma2_rn / __fmul2_rn /
 // __fadd2_rn: two FP32 operations per issued instruction).  The sweeps are
 // issue-bound, and pairing halves their FP32 instructions.  Entries of the
@@ -353,10 +394,11 @@ struct Acc2 {
 // One entry of the owner's own molecule (forces.f:868-998 / 1071-1198 with
 // SAME set): scaled 1-4 or plain Coulomb for an ion-free site (IEE = 0), the
 // Ewald real-space term otherwise; LJ only where B12 is nonzero.
-template <bool SHORT, bool ENER>
+template <bool SHORT, bool ENER, bool SPLIT>
 __device__ __forceinline__ void pair_same(float DX, float DY, float DZ, bool is14, float QIJ,
                                           float A6, float B12, int eei, int lmovei,
-                                          float alphad, float rc2f, Acc2 &s) {
+                                          float alphad, float rc2f, Acc2 &s, int slot,
+                                          SplitF &spl, double *sh) {
   const float RR = DX * DX + DY * DY + DZ * DZ;
   if (!(SHORT || RR <= rc2f)) return;
   const float R1I = rsqrtf(RR);
@@ -375,6 +417,7 @@ __device__ __forceinline__ void pair_same(float DX, float DY, float DZ, bool is1
     EES = EE1 * ERFCT;
     FORCE = EE1 * ((float)MDX_TOTPI * alphad * EXP2A + ERFCT * R1I) * R1I;
   }
+  float slj = 0.f;
   if (ENER) {
     s.ee.x += EE1;
     s.ee_same += EE1;
@@ -390,12 +433,14 @@ __device__ __forceinline__ void pair_same(float DX, float DY, float DZ, bool is1
       ESR = 0.f;
       FORCE = 0.f;
     }
+    slj = ESR;
     if (ENER) {
       if (lmovei) s.vir.x += FSR * R1;
       s.esr.x += ESR;
       s.esr_same += ESR;
     }
   }
+  if (SPLIT) split_add(spl, slot, EE1, slj, sh);
   if (ENER && (SHORT || lmovei)) {
     s.vx.x += FORCE * (DX * DX);
     s.vy.x += FORCE * (DY * DY);
@@ -431,14 +476,22 @@ __device__ __forceinline__ void slots_out(const float (&a)[P_NSLOT], float escal
   }
 }
 
-template <bool SHORT, bool ENER, int TPO, bool CELL>
-__global__ void __launch_bounds__(256, (SHORT && !ENER) ? PAIR32X2_BLOCKS_SHORT : PAIR32X2_BLOCKS)
+template <bool SHORT, bool SPLIT, bool ENER, int TPO, bool CELL>
+__global__ void __launch_bounds__(256, SPLIT ? 3 : (SHORT && !ENER) ? PAIR32X2_BLOCKS_SHORT
+                                                                    : PAIR32X2_BLOCKS)
 k_pair32x2(
     int n, const int4 *__restrict__ posi, const int4 *__restrict__ posn,
     const float4 *__restrict__ stab, const int *__restrict__ cnt, const int *__restrict__ idx,
     int cap, PairTables tb, TypeConst tc, PairConst pc, float sx, float sy, float sz,
     FixScale fsc, unsigned long long *__restrict__ ffix,
-    unsigned long long *__restrict__ slots, const int *__restrict__ owner_of, CellF cf) {
+    unsigned long long *__restrict__ slots, double *__restrict__ split,
+    const int *__restrict__ owner_of, CellF cf) {
+  __shared__ double s_split[SPLIT ? SPLIT_N : 1];
+  SplitF spl{-1, 0.f, 0.f, 0.f, 0.f};
+  if (SPLIT) {
+    for (int k = threadIdx.x; k < SPLIT_N; k += blockDim.x) s_split[k] = 0.0;
+    __syncthreads();
+  }
   // TPO adjacent lanes per owner atom; lane k0 of an owner takes entries
   // k0 + 2 TPO m and k0 + TPO + 2 TPO m as one pair.  Owner order as in
   // k_pair32.
@@ -499,8 +552,8 @@ k_pair32x2(
           const float A6 = is14 ? ab.x * c14l : ab.x, B12 = is14 ? ab.y * c14l : ab.y;
           const float DX = e ? dxb : dxa, DY = e ? dyb : dya, DZ = e ? dzb : dza;
           if (same) {
-            pair_same<SHORT, ENER>(DX, DY, DZ, is14, QIJ, A6, B12, eei, lmovei, alphad,
-                                   pc.rc2f, s);
+            pair_same<SHORT, ENER, SPLIT>(DX, DY, DZ, is14, QIJ, A6, B12, eei, lmovei, alphad,
+                                          pc.rc2f, s, MDX_NTPP + ti, spl, s_split);
           } else {
             // an inter-molecular entry beside one of the own molecule: the
             // paired arithmetic below with the other half empty
@@ -519,6 +572,7 @@ k_pair32x2(
               const float ESR = (A6 + B12 * R6I) * R6I;
               const float FSR = (6.f * A6 + 12.f * B12 * R6I) * R6I * R1I;
               FORCE = FORCE + FSR * R1I;
+              if (SPLIT) split_add(spl, tc.mdx[ti][__float_as_int(st.w)], EE1, ESR, s_split);
               if (ENER) {
                 s.ees.x += EE1 * ERFCT;
                 s.ee.x += EE1;
@@ -576,6 +630,11 @@ k_pair32x2(
       const float2 R6I = mul2(mul2(R2I, R2I), R2I);
       const float2 FSR = mul2(mul2(fma2(mul2(splat(12.f), B12), R6I, mul2(splat(6.f), A6)), R6I), R1I);
       FORCE = fma2(FSR, R1I, FORCE);
+      if (SPLIT) {
+        const float2 ESR = mul2(fma2(B12, R6I, A6), R6I);
+        if (oka) split_add(spl, tc.mdx[ti][__float_as_int(sa.w)], EE1.x, ESR.x, s_split);
+        if (okb) split_add(spl, tc.mdx[ti][__float_as_int(sb.w)], EE1.y, ESR.y, s_split);
+      }
       if (ENER) {
         const float2 ESR = mul2(fma2(B12, R6I, A6), R6I);
         s.ees = fma2(EE1, ERFCT, s.ees);
@@ -655,6 +714,7 @@ k_pair32x2(
     ffix[n + i] = (unsigned long long)qy;
     ffix[2 * n + i] = (unsigned long long)qz;
   }
+  if (SPLIT) split_out(spl, s_split, split);
   if (!ENER) return;
   float a[P_NSLOT];
   const float ee = s.ee.x + s.ee.y, esr = s.esr.x + s.esr.y;
@@ -766,44 +826,38 @@ int launch_pair(mdx_ctx *ctx, bool shrt, bool split, bool ener) {
       cf = CellF{ctx->p.icell, (float)c.hbx, (float)c.bx, (float)c.by, (float)c.boxy3,
                  (float)(0.5 / (double)0.8660254037844386f)};
     }
-    // threads per owner atom: the context's tuning (the energy-split sweeps
-    // of RECINT keep the defaults)
-    const int tpo = split ? (shrt ? TPO_SHORT_DEFAULT : TPO_LONG_DEFAULT)
-                          : (shrt ? ctx->tune.tpo_short : ctx->tune.tpo_long);
+    // threads per owner atom: the context's tuning
+    const int tpo = shrt ? ctx->tune.tpo_short : ctx->tune.tpo_long;
     const int grid32 = (int)(((long long)tpo * d.n + T - 1) / T);
 #define LP32(S, P, E, K)                                                          \
   k_pair32<S, P, E, K><<<grid32, T, 0, ctx->stream>>>(                            \
       d.n, d.posi, d.cell_pos, d.stab, cnt, idx, cap, tables(d),                 \
       ctx->tc, ctx->pc, (float)sxs, (float)sys, (float)szs, ctx->fix, ffix, d.X,  \
       d.Y, d.Z, escale, slots, split_buf, S ? nullptr : d.cell_list, cf)
-#define LP32X2C(S, E, K, C)                                                       \
-  k_pair32x2<S, E, K, C><<<grid32, T, 0, ctx->stream>>>(                          \
+#define LP32X2C(S, P, E, K, C)                                                    \
+  k_pair32x2<S, P, E, K, C><<<grid32, T, 0, ctx->stream>>>(                       \
       d.n, d.posi, d.cell_pos, d.stab, cnt, idx, cap, tables(d), ctx->tc, ctx->pc, \
-      (float)sxs, (float)sys, (float)szs, ctx->fix, ffix, slots, S ? nullptr : d.cell_list, cf)
-#define LP32X2(S, E, K)                        \
+      (float)sxs, (float)sys, (float)szs, ctx->fix, ffix, slots, split_buf,       \
+      S ? nullptr : d.cell_list, cf)
+#define LP32X2(S, P, E, K)                     \
   do {                                         \
-    if (cf.kind) LP32X2C(S, E, K, true);       \
-    else LP32X2C(S, E, K, false);              \
+    if (cf.kind) LP32X2C(S, P, E, K, true);    \
+    else LP32X2C(S, P, E, K, false);           \
   } while (0)
     // the paired sweeps cover Ewald without MDEE's shifted Coulomb
     const bool paired = !ctx->pc.lmnbl && !ctx->pc.lmdee;
+    // the force calls' energies by type pair come with energies
 #define LP32E(S, K)                            \
   do {                                         \
     if (paired) {                              \
-      if (ener) LP32X2(S, true, K);            \
-      else LP32X2(S, false, K);                \
-    } else if (ener) LP32(S, false, true, K);  \
+      if (split) LP32X2(S, true, true, K);     \
+      else if (ener) LP32X2(S, false, true, K); \
+      else LP32X2(S, false, false, K);         \
+    } else if (split) LP32(S, true, true, K);  \
+    else if (ener) LP32(S, false, true, K);    \
     else LP32(S, false, false, K);             \
   } while (0)
-    if (split) {
-      if (shrt) {
-        if (ener) LP32(true, true, true, TPO_SHORT_DEFAULT);
-        else LP32(true, true, false, TPO_SHORT_DEFAULT);
-      } else {
-        if (ener) LP32(false, true, true, TPO_LONG_DEFAULT);
-        else LP32(false, true, false, TPO_LONG_DEFAULT);
-      }
-    } else if (shrt) {
+    if (shrt) {
       if (tpo == 2) LP32E(true, 2);
       else if (tpo == 8) LP32E(true, 8);
       else LP32E(true, 4);

@@ -199,14 +199,6 @@ struct Acc64 {
   double see, slj;
 };
 enum { A_EES = 0, A_ESR, A_VIR, A_VX, A_VY, A_VZ };
-constexpr int SPLIT_N = 2 * MDX_NTPP + 2 * MDX_NT;
-// shared layout as the sums' buffer: POTE1, POTL1, PES141, PSR141
-__device__ __forceinline__ int split_ee(int slot) {
-  return slot < MDX_NTPP ? slot : 2 * MDX_NTPP + (slot - MDX_NTPP);
-}
-__device__ __forceinline__ int split_lj(int slot) {
-  return slot < MDX_NTPP ? MDX_NTPP + slot : 2 * MDX_NTPP + MDX_NT + (slot - MDX_NTPP);
-}
 __device__ __forceinline__ void split_flush(Acc64 &a, double *sh) {
   if (a.slot < 0) return;
   atomicAdd(&sh[split_ee(a.slot)], a.see);
@@ -404,29 +396,6 @@ __device__ __forceinline__ Pair64 pair_general(const Env64 &v, int e, const dbl4
   }
   if (SPLIT) split_add(a, same ? MDX_NTPP + ti : tc.mdx[ti][tj], EE1, slj, sh);
   return Pair64{FORCE, DX, DY, DZ, SHORT || !same || tc.lmove[ti], false};
-}
-
-// Sums of NV values over groups of W lanes with the additions shared out: the
-// lanes halve the values among them first, then sum what is left (NV = 4, W =
-// 32: 6 additions a lane instead of 20).  Lane W / NV * k of a group holds the
-// total of value k.
-template <int NV, int W>
-__device__ __forceinline__ double lane_sums(double (&v)[NV]) {
-  const int lane = threadIdx.x & 31;
-  int o = W / 2;
-#pragma unroll
-  for (int m = NV / 2; m >= 1; m >>= 1, o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int k = 0; k < m; ++k) {
-      const double keep = up ? v[k + m] : v[k], give = up ? v[k] : v[k + m];
-      v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-    }
-  }
-  double s = v[0];
-#pragma unroll
-  for (int p = W / (2 * NV); p >= 1; p >>= 1) s += __shfl_xor_sync(0xffffffffu, s, p);
-  return s;
 }
 
 // The owners' forces out, by three lanes of each group of TPO.
@@ -696,20 +665,14 @@ int launch_pair64(mdx_ctx *ctx, bool shrt, bool split, bool ener, double *split_
     else if (S && tpo == 16) LP64T(S, P, E, S ? 16 : 32);                                    \
     else LP64T(S, P, E, 32);                                                                 \
   } while (0)
+  // energies by type pair (force calls) come with the energies
   if (shrt) {
-    if (split) {
-      if (ener) LP64(true, true, true);
-      else LP64(true, true, false);
-    } else if (ener) {
-      LP64(true, false, true);
-    } else {
-      LP64(true, false, false);
-    }
-  } else if (split) {
-    if (ener) LP64(false, true, true);
-    else LP64(false, true, false);
+    if (split) LP64(true, true, true);
+    else if (ener) LP64(true, false, true);
+    else LP64(true, false, false);
   } else {
-    if (ener) LP64(false, false, true);
+    if (split) LP64(false, true, true);
+    else if (ener) LP64(false, false, true);
     else LP64(false, false, false);
   }
 #undef LP64

@@ -91,3 +91,38 @@ def test_pair_sweeps_match_oracle(nw, kind):
         for n in ("pote1", "potl1", "pes141", "psr141"):
             x, y = np.array(getattr(a, n)), np.array(getattr(b, n))
             assert np.abs(x - y).max() <= 1e-10 * max(np.abs(y).max(), 1e-9), (routine, n)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nw,kind", [(8, "water"), (203, "water"), (300, "organics"), (300, "ee"),
+                                     (1650, "water")])
+def test_mixed_energies_by_type_pair(nw, kind):
+    """POTE1, POTL1, PES141, PSR141 of the mixed path's force calls (a slot's
+    sums kept per lane) against the FP64 path: rows whose partners change type
+    (ions, organics), own-molecule and 1-4 pairs, the MDEE sweeps.  A term is
+    good to a few 1e-6 (FP32 from 32-bit coordinates); the sums to 1e-4 of the
+    largest, the mixed path's energy bound."""
+    from mdynamix_gb300.abi import MDX_MIXED
+    from mdynamix_gb300.mdx import ForcePath
+    spec = systems.spcfw(n=nw, ions=2, rcut=7.0 if nw < 100 else 8.0)
+    if nw < 100:
+        spec = dataclasses.replace(spec, box=(30.0, 30.0, 30.0))
+    if kind == "organics":
+        spec = systems.organics(nw)
+    if kind == "ee":
+        spec = dataclasses.replace(S.solvation_job("C2H5OH", nw), rcut=8.0)
+    s, st = systems.build(spec)
+    out = []
+    for prec in (MDX_FP64, MDX_MIXED):
+        g = ForcePath(s, precision=prec)
+        if kind == "ee":
+            g.set_lambda(0.5)
+        g.set_state(*st)
+        g.chcnb()
+        g.getcom()
+        out.append(g.allforce())
+        g.close()
+    a, b = out
+    for n in ("pote1", "potl1", "pes141", "psr141"):
+        x, y = np.array(getattr(a, n)), np.array(getattr(b, n))
+        assert np.abs(x - y).max() <= 1e-4 * max(np.abs(x).max(), 1e-9), n
