@@ -14,6 +14,7 @@
 #include <cstring>
 
 #include "mdx_internal.cuh"
+#include "pair_math.cuh"
 
 namespace {
 
@@ -93,55 +94,80 @@ __device__ __forceinline__ void pbc_com(double &x, double &y, double &z, double 
   else pbc_cell(x, y, z, mc.cell);
 }
 
+// Lanes of a molecule in the per-molecule passes: g of a type's molecules
+// share its atoms and join their sums by shuffles.  A thread alone walks a
+// large molecule as one chain of FP64 operations of 64 cycles and more each
+// (lipids of 118 atoms in the bilayer: GETCOM 74 us, SCALING's molecular
+// correction 238 us against 8 and 14 with 32 lanes; a 9-atom solute in 211
+// waters: kick and drift 25 us against 8 with 4 lanes).  Molecules of at most
+// four atoms get four lanes, or one thread (g = 1) once there are enough of
+// them to fill the chip; others eight, 16 or 32.  A block holds molecules of
+// one type.
+struct MolLanes {
+  int nt;
+  int blk[MDX_NT + 1];  // first block of each type
+  int mol0[MDX_NT], nmol[MDX_NT], g[MDX_NT];
+};
+struct MolLane {
+  int m, k, g;  // molecule, lane within it, lanes
+  bool live;
+};
+__device__ __forceinline__ MolLane mol_lane(const MolLanes &L) {
+  int t = 0;
+  while (t + 1 < L.nt && (int)blockIdx.x >= L.blk[t + 1]) ++t;
+  const int idx = ((int)blockIdx.x - L.blk[t]) * blockDim.x + threadIdx.x, g = L.g[t];
+  const int mm = idx / g;
+  const bool live = mm < L.nmol[t];
+  return MolLane{L.mol0[t] + (live ? mm : 0), idx & (g - 1), g, live};
+}
+__device__ __forceinline__ double lanes_sum(double v, int g) {
+  for (int o = g >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // GETCOM (service.f:463-563); with posi set it also refreshes the
 // fixed-point mirror of the wrapped positions (what k_mirror writes for the
 // sweeps), so a short step needs no separate mirror pass.  The FP32 mirror
-// posf only feeds the list build, which refreshes it itself.
-__global__ void k_getcom(int nop, const int *__restrict__ mol_first,
+// posf only feeds the list build, which refreshes it itself.  ibs: 2^32 / box
+// per axis (the fixed-point y word has period 2 BOYL in the hexagonal cell).
+__global__ void k_getcom(MolLanes L, const int *__restrict__ mol_first,
                          const int *__restrict__ mol_nat,
                          const int *__restrict__ mol_type,
                          const double *__restrict__ amass, dbl4 *pos, double *X,
                          double *Y, double *Z, MolConst mc, double bx, double by,
-                         double bz, float4 *__restrict__ posf, int4 *__restrict__ posi,
+                         double bz, double3 ibs, int4 *__restrict__ posi,
                          const int *__restrict__ pinfo) {
-  int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= nop) return;
-  const int f = mol_first[m], na = mol_nat[m];
+  const MolLane ml = mol_lane(L);
+  const int m = ml.m, f = mol_first[m], na = ml.live ? mol_nat[m] : 0;
   const double summ = mc.summas[mol_type[m]];
   double x = 0., y = 0., z = 0.;
-  for (int k = 0; k < na; ++k) {
+  for (int k = ml.k; k < na; k += ml.g) {
     const dbl4 p = pos[f + k];
     const double ms = amass[f + k];
     x = x + ms * p.x;
     y = y + ms * p.y;
     z = z + ms * p.z;
   }
-  x = x / summ;
-  y = y / summ;
-  z = z / summ;
+  x = lanes_sum(x, ml.g) / summ;
+  y = lanes_sum(y, ml.g) / summ;
+  z = lanes_sum(z, ml.g) / summ;
   double xw = x, yw = y, zw = z;
   pbc_com(xw, yw, zw, bx, by, bz, mc);
-  X[m] = xw;
-  Y[m] = yw;
-  Z[m] = zw;
+  if (ml.live && ml.k == 0) {
+    X[m] = xw;
+    Y[m] = yw;
+    Z[m] = zw;
+  }
   // the reference rebuilds every coordinate as (S - X) + Xw (service.f:549-552)
-  // the fixed-point y word has period 2 BOYL in the hexagonal cell
-  const double two32 = 4294967296.0, ibx = 1.0 / bx, ibz = 1.0 / bz;
-  const double iby = mc.cell.icell == 2 ? 0.5 / by : 1.0 / by;
-  for (int k = 0; k < na; ++k) {
+  for (int k = ml.k; k < na; k += ml.g) {
     dbl4 p = pos[f + k];
     p.x = (p.x - x) + xw;
     p.y = (p.y - y) + yw;
     p.z = (p.z - z) + zw;
     pos[f + k] = p;
-    if (posi) {
-      const long long xi = __double2ll_rn(p.x * ibx * two32);
-      const long long yi = __double2ll_rn(p.y * iby * two32);
-      const long long zi = __double2ll_rn(p.z * ibz * two32);
-      posi[f + k] = make_int4((int)(unsigned)(unsigned long long)xi,
-                              (int)(unsigned)(unsigned long long)yi,
-                              (int)(unsigned)(unsigned long long)zi, pinfo[f + k]);
-    }
+    if (posi)
+      posi[f + k] = make_int4(fix32_rn(__dmul_rn(p.x, ibs.x)), fix32_rn(__dmul_rn(p.y, ibs.y)),
+                              fix32_rn(__dmul_rn(p.z, ibs.z)), pinfo[f + k]);
   }
 }
 
@@ -218,13 +244,13 @@ __global__ void k_kick_drift(int n, const int4 *__restrict__ ainfo, MoveConst mv
 
 constexpr int KD_MAXA = 4;  // atoms per molecule of the register path below
 
-// One short step of DOUBLE's inner loop up to the fast forces, thread per
+// One short step of DOUBLE's inner loop up to the fast forces, per
 // molecule: the kick and drift of k_kick_drift for each of its atoms
 // (mdstep.f:383-397), then GETCOM's centre of mass and wrap (service.f:
 // 463-563) and the fixed-point mirror, all in the order the separate
 // kernels use.  hfix (mixed path): the previous short step's fast forces are read
 // as fixed point, so that step needs no fold to FP64.
-__device__ __forceinline__ void kick_drift_com_body(int m, int nop, const int *__restrict__ mol_first,
+__device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int *__restrict__ mol_first,
                                  const int *__restrict__ mol_nat,
                                  const int *__restrict__ mol_type,
                                  const int4 *__restrict__ ainfo, MoveConst mv,
@@ -243,9 +269,9 @@ __device__ __forceinline__ void kick_drift_com_body(int m, int nop, const int *_
   // ibs: 2^32 / box per axis (host-computed: no FP64 division per thread);
   // posi set (mixed path): centre of mass by the reciprocal mass, the
   // fixed-point mirror refreshed, and (posc set) its cell-order copy
-  if (m >= nop) return;
-  const int f = mol_first[m], na = mol_nat[m];
-  if (posi && na <= KD_MAXA) {
+  const int m = ml.m, f = mol_first[m], na = ml.live ? mol_nat[m] : 0;
+  if (ml.g == 1 && posi && na <= KD_MAXA) {
+    if (!ml.live) return;
     // Mixed path, small molecules: the atoms stay in registers between the
     // centre of mass and the wrap, each position is stored once, and the
     // update takes fewer FP64 operations (the two half kicks of one force
@@ -315,44 +341,61 @@ __device__ __forceinline__ void kick_drift_com_body(int m, int nop, const int *_
     }
     return;
   }
+  // lanes of the molecule (or one thread, FP64 path): the reference's
+  // operations per atom; on the mixed path the shorter update of above.  Up
+  // to g atoms stay in registers.
   double x = 0., y = 0., z = 0.;
-  for (int k = 0; k < na; ++k) {
+  const double hk = prev ? 2.0 * htsteb : htsteb, hkf = hk * inv;
+  dbl4 p0;
+  p0.x = p0.y = p0.z = p0.w = 0.0;
+  for (int k = ml.k; k < na; k += ml.g) {
     const int i = f + k;
     dbl4 p = pos[i];
     if (mv.lmove[ainfo[i].x]) {
       double u = vx[i], v = vy[i], w = vz[i];
-      double fx, fy, fz;
-      if (hfix) {
-        fx = (double)(long long)hfix[i] * inv;
-        fy = (double)(long long)hfix[n + i] * inv;
-        fz = (double)(long long)hfix[2 * n + i] * inv;
+      const double mi = massdi[i];
+      if (posi) {
+        if (hfix) {
+          u = fma((double)(long long)hfix[i], hkf, u);
+          v = fma((double)(long long)hfix[n + i], hkf, v);
+          w = fma((double)(long long)hfix[2 * n + i], hkf, w);
+        } else {
+          u = fma(hx[i], hk, u);
+          v = fma(hy[i], hk, v);
+          w = fma(hz[i], hk, w);
+        }
+        const double tm = tsteb * mi;
+        p.x = fma(u, tm, p.x);
+        p.y = fma(v, tm, p.y);
+        p.z = fma(w, tm, p.z);
       } else {
-        fx = hx[i];
-        fy = hy[i];
-        fz = hz[i];
-      }
-      if (prev) {
+        const double fx = hx[i], fy = hy[i], fz = hz[i];
+        if (prev) {
+          u = u + htsteb * fx;
+          v = v + htsteb * fy;
+          w = w + htsteb * fz;
+        }
         u = u + htsteb * fx;
         v = v + htsteb * fy;
         w = w + htsteb * fz;
+        p.x = u * tsteb * mi + p.x;
+        p.y = v * tsteb * mi + p.y;
+        p.z = w * tsteb * mi + p.z;
       }
-      u = u + htsteb * fx;
-      v = v + htsteb * fy;
-      w = w + htsteb * fz;
       vx[i] = u;
       vy[i] = v;
       vz[i] = w;
-      const double mi = massdi[i];
-      p.x = u * tsteb * mi + p.x;
-      p.y = v * tsteb * mi + p.y;
-      p.z = w * tsteb * mi + p.z;
     }
-    pos[i] = p;
+    if (k == ml.k) p0 = p;
+    else pos[i] = p;
     const double ms = amass[i];
     x = x + ms * p.x;
     y = y + ms * p.y;
     z = z + ms * p.z;
   }
+  x = lanes_sum(x, ml.g);
+  y = lanes_sum(y, ml.g);
+  z = lanes_sum(z, ml.g);
   if (posi) {
     const double rs = mc.rsummas[mol_type[m]];
     x = x * rs;
@@ -366,14 +409,19 @@ __device__ __forceinline__ void kick_drift_com_body(int m, int nop, const int *_
   }
   double xw = x, yw = y, zw = z;
   pbc_com(xw, yw, zw, bx, by, bz, mc);
-  X[m] = xw;
-  Y[m] = yw;
-  Z[m] = zw;
-  for (int k = 0; k < na; ++k) {
-    dbl4 p = pos[f + k];
-    p.x = (p.x - x) + xw;
-    p.y = (p.y - y) + yw;
-    p.z = (p.z - z) + zw;
+  if (ml.live && ml.k == 0) {
+    X[m] = xw;
+    Y[m] = yw;
+    Z[m] = zw;
+  }
+  const bool moved = !posi || xw != x || yw != y || zw != z;
+  for (int k = ml.k; k < na; k += ml.g) {
+    dbl4 p = k == ml.k ? p0 : pos[f + k];
+    if (moved) {
+      p.x = (p.x - x) + xw;
+      p.y = (p.y - y) + yw;
+      p.z = (p.z - z) + zw;
+    }
     pos[f + k] = p;
     if (posi) {
       const int4 q = make_int4(fix32_rn(__dmul_rn(p.x, ibs.x)), fix32_rn(__dmul_rn(p.y, ibs.y)),
@@ -384,7 +432,7 @@ __device__ __forceinline__ void kick_drift_com_body(int m, int nop, const int *_
   }
 }
 
-__global__ void k_kick_drift_com(int nop, const int *__restrict__ mol_first,
+__global__ void k_kick_drift_com(MolLanes L, const int *__restrict__ mol_first,
                                  const int *__restrict__ mol_nat,
                                  const int *__restrict__ mol_type,
                                  const int4 *__restrict__ ainfo, MoveConst mv,
@@ -400,7 +448,7 @@ __global__ void k_kick_drift_com(int nop, const int *__restrict__ mol_first,
                                  double bx, double by, double bz, double3 ibs,
                                  int4 *__restrict__ posi, const int *__restrict__ pinfo,
                                  int4 *__restrict__ posc, const int *__restrict__ slot_of) {
-  kick_drift_com_body(blockIdx.x * blockDim.x + threadIdx.x, nop, mol_first, mol_nat, mol_type,
+  kick_drift_com_body(mol_lane(L), mol_first, mol_nat, mol_type,
                       ainfo, mv, mc, htsteb, tsteb, prev, hx, hy, hz, hfix, n, inv, massdi,
                       amass, vx, vy, vz, pos, X, Y, Z, bx, by, bz, ibs, posi, pinfo, posc,
                       slot_of);
@@ -1009,20 +1057,19 @@ __global__ void k_scale_atoms(int n, int mode, const int4 *__restrict__ ainfo,
 }
 
 // SCALING(3) NPT molecular correction (mdstep.f:953-1003): per molecule.
-__global__ void k_com_scale(int nop, const int *__restrict__ mol_first,
+__global__ void k_com_scale(MolLanes L, const int *__restrict__ mol_first,
                             const int *__restrict__ mol_nat,
                             const int *__restrict__ mol_type,
                             const double *__restrict__ amass, MolConst mc,
                             MoveConst mv, const ScalScratch *ss, double *vx,
                             double *vy, double *vz, dbl4 *pos) {
-  int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= nop) return;
-  const int t = mol_type[m];
-  if (!mv.lmove[t]) return;
-  const int f = mol_first[m], na = mol_nat[m];
+  const MolLane ml = mol_lane(L);
+  const int t = mol_type[ml.m];
+  if (!mv.lmove[t]) return;  // a block is of one type
+  const int f = mol_first[ml.m], na = ml.live ? mol_nat[ml.m] : 0;
   const double SUMM = mc.summas[t];
   double XC = 0., YC = 0., ZC = 0., PXC = 0., PYC = 0., PZC = 0.;
-  for (int k = 0; k < na; ++k) {
+  for (int k = ml.k; k < na; k += ml.g) {
     const dbl4 p = pos[f + k];
     const double ms = amass[f + k];
     XC = XC + ms * p.x;
@@ -1032,13 +1079,16 @@ __global__ void k_com_scale(int nop, const int *__restrict__ mol_first,
     PYC = PYC + vy[f + k];
     PZC = PZC + vz[f + k];
   }
-  XC = XC / SUMM;
-  YC = YC / SUMM;
-  ZC = ZC / SUMM;
+  XC = lanes_sum(XC, ml.g) / SUMM;
+  YC = lanes_sum(YC, ml.g) / SUMM;
+  ZC = lanes_sum(ZC, ml.g) / SUMM;
+  PXC = lanes_sum(PXC, ml.g);
+  PYC = lanes_sum(PYC, ml.g);
+  PZC = lanes_sum(PZC, ml.g);
   const double SCV = ss->dxc;
   const double DVX = PXC * SCV, DVY = PYC * SCV, DVZ = PZC * SCV;
   const double DXC = XC * ss->drcx, DYC = YC * ss->drcy, DZC = ZC * ss->drcz;
-  for (int k = 0; k < na; ++k) {
+  for (int k = ml.k; k < na; k += ml.g) {
     const double FAC = amass[f + k] / SUMM;
     vx[f + k] = vx[f + k] - DVX * FAC;
     vy[f + k] = vy[f + k] - DVY * FAC;
@@ -1064,98 +1114,137 @@ struct ShakeConst {
 // bond needs adjusting; constraints that share no atom (e.g. the CH2 and CH3
 // groups of a lipid under SHAKE on bonds to hydrogen) never see each
 // other's updates, so each cluster runs the same sweeps on its own and ends
-// in the same positions bit for bit; the molecule's iteration count is the
-// largest of its clusters'.  Thread per (molecule, cluster); the positions
-// before SHAKE are in fx/fy/fz (written by the leap-frog pass).
-__global__ void k_shake_cluster(int nitem, const int2 *__restrict__ items,
-                                const int2 *__restrict__ clusters,
-                                const int *__restrict__ recs,
-                                const int *__restrict__ mol_first,
-                                const int *__restrict__ mol_type, MoveConst mv,
-                                ShakeConst sk, const int *__restrict__ bib,
-                                const int *__restrict__ bjb,
-                                const double *__restrict__ brb,
-                                const double *__restrict__ massdi, dbl4 *pos,
-                                const double *__restrict__ ox,
-                                const double *__restrict__ oy,
-                                const double *__restrict__ oz, double bx, double by,
-                                double bz, mdx_thermo *th, int *__restrict__ mfail) {
-  const int it = blockIdx.x * blockDim.x + threadIdx.x;
-  if (it >= nitem) return;
-  const int2 item = items[it];
+// in the same positions; the molecule's iteration count is the largest of its
+// clusters'.  The positions before SHAKE are in fx/fy/fz (written by the
+// leap-frog pass).
+//
+// Four lanes take a cluster, lanes 0-2 an axis each: an FP64 instruction
+// costs the same for one lane as for 32, and the sweeps are a chain of them
+// (43 an update by one thread, 18 here).  The warp stays together: a step of
+// the sweeps is taken when any of its clusters needs it.  What does not change
+// over the sweeps is formed once: the old bond vector with its image, 1 / (2
+// (RMA + RMB)), the squared length and its tolerance.  The reciprocal of VDOT
+// is FP32-seeded and refined to FP64.  Rigid SPC/E (3 constraints, 35 sweeps):
+// 200 -> 120 us a step; bilayer (bonds to hydrogen): 261 -> 163.
+constexpr int SHK_T = 64, SHK_KEEP = 8;  // threads; constraints of a cluster kept in shared memory
+
+// Minimum image of this lane's component (lanes 0-2 of each four: x, y, z).
+__device__ __forceinline__ double shk_image(const ShakeConst &sk, int a, double d, double b) {
+  if (sk.cell.icell == 0) {
+    const bool c = (__double_as_longlong(d) & 0x7fffffffffffffffLL) > __double_as_longlong(0.5 * b);
+    if (__any_sync(0xffffffffu, c) && c) d = d - fsign(b, d);
+    return d;
+  }
+  const int l0 = threadIdx.x & 28;
+  double x = __shfl_sync(0xffffffffu, d, l0), y = __shfl_sync(0xffffffffu, d, l0 + 1),
+         z = __shfl_sync(0xffffffffu, d, l0 + 2);
+  pbc_cell(x, y, z, sk.cell);  // mdstep.f:1175, 1186
+  return a == 0 ? x : a == 1 ? y : a == 2 ? z : 0.0;
+}
+
+__global__ void __launch_bounds__(SHK_T) k_shake_cluster(
+    int nitem, const int2 *__restrict__ items, const int2 *__restrict__ clusters,
+    const int *__restrict__ recs, const int *__restrict__ mol_first,
+    const int *__restrict__ mol_type, MoveConst mv, ShakeConst sk, const int *__restrict__ bib,
+    const int *__restrict__ bjb, const double *__restrict__ brb,
+    const double *__restrict__ massdi, dbl4 *pos, const double *__restrict__ ox,
+    const double *__restrict__ oy, const double *__restrict__ oz, double bx, double by, double bz,
+    mdx_thermo *th, int *__restrict__ mfail) {
+  __shared__ double s_d[SHK_KEEP][SHK_T], s_c[SHK_KEEP][SHK_T / 4];
+  constexpr unsigned ALL = 0xffffffffu;
+  const int it = (blockIdx.x * SHK_T + threadIdx.x) >> 2;
+  const int a = threadIdx.x & 3, l0 = threadIdx.x & 28, ax = min(a, 2), gi = threadIdx.x >> 2;
+  const int2 item = items[min(it, nitem - 1)];
   const int m = item.x, t = mol_type[m];
-  if (!(mv.lmove[t] && sk.ishejk[t] > 0)) return;
+  const bool live = it < nitem && mv.lmove[t] && sk.ishejk[t] > 0;
   const int2 cl = clusters[item.y];  // (first record slot, records)
   const int *rr = recs + cl.x;
-  const int f = mol_first[m];
+  const int f = mol_first[m], nc = live ? cl.y : 0;
+  const int ncw = __reduce_max_sync(ALL, nc);
+  const double *o = ax == 0 ? ox : ax == 1 ? oy : oz;
+  const double b = ax == 0 ? bx : ax == 1 ? by : bz;
+  double *px = reinterpret_cast<double *>(pos) + ax;  // stride 4 an atom
+  // the old bond vector and 1 / (2 (RMA + RMB)) of constraint q
+  auto old_bond = [&](int I, int J) {
+    const double d = a < 3 ? o[I] - o[J] : 0.0;
+    return shk_image(sk, a, d, b);
+  };
+  auto inv_mass = [&](int I, int J) { return 1.0 / (2.0 * (massdi[I] + massdi[J])); };
   // MOVING / MOVED flags as bit masks over the molecule's atoms (<= 128)
   unsigned long long moving[2] = {0, 0}, moved[2] = {0, 0};
-  for (int q = 0; q < cl.y; ++q) {
-    const int b = rr[q];
-    const int li = bib[b] - 1, lj = bjb[b] - 1;
-    moved[li >> 6] |= 1ull << (li & 63);
-    moved[lj >> 6] |= 1ull << (lj & 63);
+  for (int q = 0; q < ncw; ++q) {
+    const int r = rr[q < nc ? q : 0];
+    const int li = bib[r] - 1, lj = bjb[r] - 1;
+    if (q < nc) {
+      moved[li >> 6] |= 1ull << (li & 63);
+      moved[lj >> 6] |= 1ull << (lj & 63);
+    }
+    if (q < SHK_KEEP) {
+      s_d[q][threadIdx.x] = old_bond(f + li, f + lj);
+      if (a == 0) s_c[q][gi] = inv_mass(f + li, f + lj);
+    }
   }
+  __syncwarp();
   int ITER = 0;
-  bool DONE = false;
+  bool DONE = !live;
   for (;;) {
-    if (ITER > sk.maxit || DONE) break;
-    DONE = true;
-    for (int q = 0; q < cl.y; ++q) {
-      const int b = rr[q];
-      const int li = bib[b] - 1, lj = bjb[b] - 1;
+    const bool run = !(ITER > sk.maxit || DONE);
+    if (!__any_sync(ALL, run)) break;
+    if (run) DONE = true;
+    for (int q = 0; q < ncw; ++q) {
+      const int r = rr[q < nc ? q : 0];
+      const int li = bib[r] - 1, lj = bjb[r] - 1;
       const bool mvi = (moved[li >> 6] >> (li & 63)) & 1ull;
       const bool mvj = (moved[lj >> 6] >> (lj & 63)) & 1ull;
-      if (!(mvi || mvj)) continue;
+      const bool act = run && q < nc && (mvi || mvj);
+      if (!__any_sync(ALL, act)) continue;
       const int I = f + li, J = f + lj;
-      const double rbb = brb[b];
+      const double rbb = brb[r];
       const double BNDSQ = rbb * rbb;
-      dbl4 pi = pos[I], pj = pos[J];
-      double BXN = pi.x - pj.x, BYN = pi.y - pj.y, BZN = pi.z - pj.z;
-      if (sk.cell.icell == 0) pbc_rect(BXN, BYN, BZN, bx, by, bz, 0.5 * bx, 0.5 * by, 0.5 * bz);
-      else pbc_cell(BXN, BYN, BZN, sk.cell);  // mdstep.f:1175
-      const double BSQ = BXN * BXN + BYN * BYN + BZN * BZN;
+      double pi = px[4 * (size_t)I], pj = px[4 * (size_t)J];
+      const double B = shk_image(sk, a, a < 3 ? pi - pj : 0.0, b);
+      const double DO = q < SHK_KEEP ? s_d[q][threadIdx.x] : old_bond(I, J);
+      double s2[2] = {B * B, B * DO};
+      const double s = lane_sums<2, 4>(s2);  // lanes 0, 1: BSQ; 2, 3: VDOT
+      const double BSQ = __shfl_sync(ALL, s, l0), VDOT = __shfl_sync(ALL, s, l0 + 2);
       const double DIFFSQ = BNDSQ - BSQ;
-      if (fabs(DIFFSQ) > (BNDSQ * sk.tol2)) {
-        double DXN = ox[I] - ox[J], DYN = oy[I] - oy[J], DZN = oz[I] - oz[J];
-        if (sk.cell.icell == 0) pbc_rect(DXN, DYN, DZN, bx, by, bz, 0.5 * bx, 0.5 * by, 0.5 * bz);
-        else pbc_cell(DXN, DYN, DZN, sk.cell);  // mdstep.f:1186
-        const double VDOT = BXN * DXN + BYN * DYN + BZN * DZN;
-        const double RMA = massdi[I], RMB = massdi[J];
-        const double GAB = DIFFSQ / (2.0 * (RMA + RMB) * VDOT);
-        DXN = DXN * GAB;
-        DYN = DYN * GAB;
-        DZN = DZN * GAB;
-        pi.x = pi.x + RMA * DXN;
-        pi.y = pi.y + RMA * DYN;
-        pi.z = pi.z + RMA * DZN;
-        pj.x = pj.x - RMB * DXN;
-        pj.y = pj.y - RMB * DYN;
-        pj.z = pj.z - RMB * DZN;
-        pos[I] = pi;
-        pos[J] = pj;
+      // fabs(DIFFSQ) > BNDSQ tol2 by the bit patterns (the same order)
+      const bool adj = act && (__double_as_longlong(DIFFSQ) & 0x7fffffffffffffffLL) >
+                                  __double_as_longlong(BNDSQ * sk.tol2);
+      if (!__any_sync(ALL, adj)) continue;
+      const double ci = q < SHK_KEEP ? s_c[q][gi] : inv_mass(I, J);
+      const double g = DO * (DIFFSQ * ci * rcp_nr(VDOT));
+      if (adj) {
+        if (a < 3) {
+          px[4 * (size_t)I] = fma(massdi[I], g, pi);
+          px[4 * (size_t)J] = fma(-massdi[J], g, pj);
+        }
         moving[li >> 6] |= 1ull << (li & 63);
         moving[lj >> 6] |= 1ull << (lj & 63);
         DONE = false;
       }
     }
     // MOVED := MOVING restricted to constrained atoms; MOVING := 0
-    moved[0] = moving[0];
-    moved[1] = moving[1];
-    moving[0] = moving[1] = 0;
-    ITER = ITER + 1;
+    if (run) {
+      moved[0] = moving[0];
+      moved[1] = moving[1];
+      moving[0] = moving[1] = 0;
+      ITER = ITER + 1;
+    }
   }
-  atomicMax(&th->shake_iter_max, ITER);
-  if (ITER >= sk.maxit) mfail[m] = 1;
+  if (live && a == 0) {
+    atomicMax(&th->shake_iter_max, ITER);
+    if (ITER >= sk.maxit) mfail[m] = 1;
+  }
 }
 
-// SHEJK's end per molecule (mdstep.f:1240-1275): velocity correction and
-// constraint virial from the displacement SHAKE made, the count of
-// molecules past MAXIT.  Thread per molecule (the virial sums in molecule
-// order).
-__global__ void k_shake_finish(int nop, const int *__restrict__ mol_first,
-                               const int *__restrict__ mol_nat,
-                               const int *__restrict__ mol_type, MoveConst mv,
+// SHEJK's end (mdstep.f:1240-1275): velocity correction and constraint
+// virial from the displacement SHAKE made, the count of molecules past MAXIT.
+// Thread per atom, the virial summed in a fixed order (a thread per molecule
+// took 544 us on lipids of 118 atoms, six FP64 divisions an atom in a row;
+// 17.6 us now).
+__global__ void k_shake_finish(int n, const int4 *__restrict__ ainfo,
+                               const int *__restrict__ mol_first, MoveConst mv,
                                ShakeConst sk, const double *__restrict__ massdi,
                                const dbl4 *__restrict__ pos, double *vx, double *vy,
                                double *vz, const double *__restrict__ ox,
@@ -1165,30 +1254,28 @@ __global__ void k_shake_finish(int nop, const int *__restrict__ mol_first,
                                const double *__restrict__ fz, mdx_thermo *th, int *err,
                                int *__restrict__ mfail, Dst6 vdst) {
   double vir[3] = {0, 0, 0};
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m < nop) {
-    const int t = mol_type[m];
+  const int I = blockIdx.x * blockDim.x + threadIdx.x;
+  if (I < n) {
+    const int4 ai = ainfo[I];
+    const int t = ai.x, m = ai.y;
     if (mv.lmove[t] && sk.ishejk[t] > 0 && sk.nrb[t] > 0) {
-      if (mfail[m]) {
+      if (mfail[m] && mol_first[m] == I) {
         mfail[m] = 0;
         atomicAdd(&th->shake_fail, 1);
         atomicOr(err, DERR_SHAKE);
       }
-      const int f = mol_first[m], na = mol_nat[m];
       const double TS = sk.tstep;
-      for (int k = 0; k < na; ++k) {
-        const int I = f + k;
-        const dbl4 p = pos[I];
-        const double DIX = (p.x - fx[I]) / (massdi[I] * TS);
-        const double DIY = (p.y - fy[I]) / (massdi[I] * TS);
-        const double DIZ = (p.z - fz[I]) / (massdi[I] * TS);
-        vir[0] += DIX * ox[I] / TS;
-        vir[1] += DIY * oy[I] / TS;
-        vir[2] += DIZ * oz[I] / TS;
-        vx[I] = vx[I] + DIX;
-        vy[I] = vy[I] + DIY;
-        vz[I] = vz[I] + DIZ;
-      }
+      const dbl4 p = pos[I];
+      const double mt = massdi[I] * TS;
+      const double DIX = (p.x - fx[I]) / mt;
+      const double DIY = (p.y - fy[I]) / mt;
+      const double DIZ = (p.z - fz[I]) / mt;
+      vir[0] = DIX * ox[I] / TS;
+      vir[1] = DIY * oy[I] / TS;
+      vir[2] = DIZ * oz[I] / TS;
+      vx[I] = vx[I] + DIX;
+      vy[I] = vy[I] + DIY;
+      vz[I] = vz[I] + DIZ;
     }
   }
   block_add<3>(vir, vdst);
@@ -1372,6 +1459,30 @@ __global__ void k_mom_remove(int n, double sumasd, const double *__restrict__ pt
   vz[i] = vz[i] - dvz / massdi[i];
 }
 
+// 2^32 / box per axis, of the fixed-point mirror
+double3 fix_scale3(const mdx_ctx *ctx) {
+  return make_double3(4294967296.0 * (1.0 / ctx->boxl), 4294967296.0 * (1.0 / fix_period_y(ctx)),
+                      4294967296.0 * (1.0 / ctx->bozl));
+}
+
+// Lanes per molecule for the per-molecule passes with threads-wide blocks
+// (copies: systems of one launch, PIMD beads).
+MolLanes mol_lanes(const mdx_ctx *ctx, int threads, int copies = 1) {
+  MolLanes L{};
+  L.nt = ctx->d.ntypes;
+  // one thread a molecule keeps the FP64 pipes busy from about 4 warps a SM
+  // scheduler's worth of small molecules on
+  const bool many = (size_t)ctx->dv.nop * copies >= (size_t)128 * ctx->nsm;
+  for (int t = 0; t < L.nt; ++t) {
+    const int na = ctx->nsits[t];
+    L.mol0[t] = ctx->iaddr[t];
+    L.nmol[t] = ctx->nspec[t];
+    L.g[t] = na <= 4 ? (many || na == 1 ? 1 : 4) : na <= 16 ? 8 : na <= 32 ? 16 : 32;
+    L.blk[t + 1] = L.blk[t] + (L.nmol[t] * L.g[t] + threads - 1) / threads;
+  }
+  return L;
+}
+
 MolConst mol_const(mdx_ctx *ctx) {
   MolConst m{};
   for (int t = 0; t < MDX_NT; ++t) {
@@ -1445,7 +1556,7 @@ struct StageQ {
 };
 
 // DOUBLE-style drift of every bead (no kick before it: htsteb applies to H)
-__global__ void k_kick_drift_com_beads(int nop, const int *__restrict__ mol_first,
+__global__ void k_kick_drift_com_beads(MolLanes L, const int *__restrict__ mol_first,
                                        const int *__restrict__ mol_nat,
                                        const int *__restrict__ mol_type,
                                        const int4 *__restrict__ ainfo, MoveConst mv, MolConst mc,
@@ -1455,7 +1566,7 @@ __global__ void k_kick_drift_com_beads(int nop, const int *__restrict__ mol_firs
                                        double bz, double3 ibs, const int *__restrict__ pinfo,
                                        const BeadMove *__restrict__ beads) {
   const BeadMove &b = beads[blockIdx.y];
-  kick_drift_com_body(blockIdx.x * blockDim.x + threadIdx.x, nop, mol_first, mol_nat, mol_type,
+  kick_drift_com_body(mol_lane(L), mol_first, mol_nat, mol_type,
                       ainfo, mv, mc, htsteb, tsteb, 0, b.f[0][0], b.f[0][1], b.f[0][2], nullptr,
                       n, 0.0, massdi, amass, b.vx, b.vy, b.vz, b.pos, b.X, b.Y, b.Z, bx, by, bz,
                       ibs, b.posi, pinfo, b.posc, b.slot_of);
@@ -1596,8 +1707,9 @@ int launch_scaling(mdx_ctx *ctx, int ial, bool *pending_vscale, const KickSpec *
       if (p.lnpt) {
         RC(q.flush());
         DevData &d = ctx->dv;
-        k_com_scale<<<(d.nop + 127) / 128, 128, 0, ctx->stream>>>(
-            d.nop, d.mol_first, d.mol_nat, d.mol_type, d.amass, mol_const(ctx),
+        const MolLanes L = mol_lanes(ctx, 64);
+        k_com_scale<<<L.blk[L.nt], 64, 0, ctx->stream>>>(
+            L, d.mol_first, d.mol_nat, d.mol_type, d.amass, mol_const(ctx),
             move_const(ctx), scratch(ctx), d.vx, d.vy, d.vz, d.pos);
         MDX_LAUNCHED(ctx);
         q.push(ST_3B);
@@ -1752,9 +1864,10 @@ int launch_sum_forces(mdx_ctx *ctx) {
 int launch_getcom(mdx_ctx *ctx, bool mirror) {
   MDX_TIMER(ctx, MDX_T_MOVE);
   DevData &d = ctx->dv;
-  k_getcom<<<(d.nop + 127) / 128, 128, 0, ctx->stream>>>(
-      d.nop, d.mol_first, d.mol_nat, d.mol_type, d.amass, d.pos, d.X, d.Y, d.Z,
-      mol_const(ctx), ctx->boxl, ctx->boyl, ctx->bozl, nullptr,
+  const MolLanes L = mol_lanes(ctx, 64);
+  k_getcom<<<L.blk[L.nt], 64, 0, ctx->stream>>>(
+      L, d.mol_first, d.mol_nat, d.mol_type, d.amass, d.pos, d.X, d.Y, d.Z,
+      mol_const(ctx), ctx->boxl, ctx->boyl, ctx->bozl, fix_scale3(ctx),
       mirror && ctx->mixed() ? d.posi : nullptr, d.pinfo);
   MDX_LAUNCHED(ctx);
   return mirror ? launch_cell_refresh(ctx) : MDX_OK;
@@ -1807,14 +1920,12 @@ int launch_kick_drift_com(mdx_ctx *ctx, double htsteb, double tsteb, int prev, b
   DevData &d = ctx->dv;
   // a warp per block: the molecules spread over the SMs evenly (this pass
   // waits on its FP64 chains; 0.4 % of the mixed step against 128 threads)
-  k_kick_drift_com<<<(d.nop + 31) / 32, 32, 0, ctx->stream>>>(
-      d.nop, d.mol_first, d.mol_nat, d.mol_type, d.ainfo, move_const(ctx), mol_const(ctx),
+  const MolLanes L = mol_lanes(ctx, 32);
+  k_kick_drift_com<<<L.blk[L.nt], 32, 0, ctx->stream>>>(
+      L, d.mol_first, d.mol_nat, d.mol_type, d.ainfo, move_const(ctx), mol_const(ctx),
       htsteb, tsteb, prev, d.hx, d.hy, d.hz, from_fix ? d.hfix : nullptr, d.n, ctx->fix.inv,
       d.massdi, d.amass, d.vx, d.vy, d.vz, d.pos, d.X, d.Y, d.Z, ctx->boxl, ctx->boyl,
-      ctx->bozl,
-      make_double3(4294967296.0 * (1.0 / ctx->boxl), 4294967296.0 * (1.0 / fix_period_y(ctx)),
-                   4294967296.0 * (1.0 / ctx->bozl)),
-      ctx->mixed() ? d.posi : nullptr, d.pinfo,
+      ctx->bozl, fix_scale3(ctx), ctx->mixed() ? d.posi : nullptr, d.pinfo,
       ctx->mixed() && ctx->have_lists ? d.cell_pos : nullptr, d.slot_of);
   MDX_LAUNCHED(ctx);
   return MDX_OK;
@@ -1905,13 +2016,12 @@ int launch_kick_drift_com_beads(mdx_ctx *c0, int P, const void *table, cudaStrea
                                 double htsteb, double tsteb) {
   MDX_TIMER(c0, MDX_T_MOVE);
   DevData &d = c0->dv;
-  const dim3 grid((d.nop + 127) / 128, P);
+  const MolLanes L = mol_lanes(c0, 128, P);
+  const dim3 grid(L.blk[L.nt], P);
   k_kick_drift_com_beads<<<grid, 128, 0, st>>>(
-      d.nop, d.mol_first, d.mol_nat, d.mol_type, d.ainfo, move_const(c0), mol_const(c0), htsteb,
+      L, d.mol_first, d.mol_nat, d.mol_type, d.ainfo, move_const(c0), mol_const(c0), htsteb,
       tsteb, d.n, d.massdi, d.amass, c0->boxl, c0->boyl, c0->bozl,
-      make_double3(4294967296.0 * (1.0 / c0->boxl), 4294967296.0 * (1.0 / fix_period_y(c0)),
-                   4294967296.0 * (1.0 / c0->bozl)),
-      d.pinfo, static_cast<const BeadMove *>(table));
+      fix_scale3(c0), d.pinfo, static_cast<const BeadMove *>(table));
   MDX_LAUNCHED(c0);
   return MDX_OK;
 }
@@ -1937,16 +2047,16 @@ int launch_leapfrog_shake(mdx_ctx *ctx) {
     sk.tstep = ctx->p.tstep;
     sk.cell = cell_pbc(ctx);
     if (d.shk_nitem > 0) {
-      k_shake_cluster<<<(d.shk_nitem + 63) / 64, 64, 0, ctx->stream>>>(
+      k_shake_cluster<<<(4 * d.shk_nitem + SHK_T - 1) / SHK_T, SHK_T, 0, ctx->stream>>>(
           d.shk_nitem, d.shk_item, d.shk_cl, d.shk_rec, d.mol_first, d.mol_type,
           move_const(ctx), sk, d.bib, d.bjb, d.brb, d.massdi, d.pos, d.ox, d.oy, d.oz,
           ctx->boxl, ctx->boyl, ctx->bozl, d.th, d.shk_mfail);
       MDX_LAUNCHED(ctx);
     }
-    k_shake_finish<<<(d.nop + 63) / 64, 64, 0, ctx->stream>>>(
-        d.nop, d.mol_first, d.mol_nat, d.mol_type, move_const(ctx), sk, d.massdi, d.pos,
+    k_shake_finish<<<(d.n + 127) / 128, 128, 0, ctx->stream>>>(
+        d.n, d.ainfo, d.mol_first, move_const(ctx), sk, d.massdi, d.pos,
         d.vx, d.vy, d.vz, d.ox, d.oy, d.oz, d.fx, d.fy, d.fz, d.th, d.err, d.shk_mfail,
-        dst6(ctx, (d.nop + 63) / 64, 3, &d.th->viran[0], &d.th->viran[1], &d.th->viran[2]));
+        dst6(ctx, (d.n + 127) / 128, 3, &d.th->viran[0], &d.th->viran[1], &d.th->viran[2]));
     MDX_LAUNCHED(ctx);
   }
   return MDX_OK;
