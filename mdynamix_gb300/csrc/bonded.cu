@@ -28,6 +28,7 @@ struct BondOut {
   float sx, sy, sz;   // box / 2^32
   float limx, limy, limz;  // 0.99 x half box: below it no minimum-image shift
   CellPbc cell;            // cell shape (FP64 path: hexagonal / octahedral PBC)
+  bool shared;             // the short sweep adds to the same forces meanwhile
 };
 
 // Fixed-point force term: R = float rounds v * 2^k with FP32 operations only
@@ -119,6 +120,10 @@ __device__ __forceinline__ void avg_add(double *sh, double *gl, int m, int nrec,
 // molecule-local kernel); the same per-term rounding as add_force.
 template <typename R>
 __device__ __forceinline__ void add_force_own(const BondOut &o, int i, R fx, R fy, R fz) {
+  if (o.shared) {
+    add_force<R>(o, i, fx, fy, fz);
+    return;
+  }
   if (o.hfix) {
     o.hfix[i] += (unsigned long long)fix_term<R>(o, fx);
     o.hfix[o.n + i] += (unsigned long long)fix_term<R>(o, fy);
@@ -741,7 +746,7 @@ __global__ void __launch_bounds__(128) k_bonded_all(BondedAll a, const dbl4 *__r
 
 }  // namespace
 
-int launch_bonded(mdx_ctx *ctx, int laver, bool ener) {
+int launch_bonded(mdx_ctx *ctx, int laver, bool ener, bool shared) {
   MDX_TIMER(ctx, MDX_T_BONDED);
   DevData &d = ctx->dv;
   mdx_scalars *sc = d.sc;
@@ -753,7 +758,7 @@ int launch_bonded(mdx_ctx *ctx, int laver, bool ener) {
             nullptr, (float)(ctx->boxl / 4294967296.0),
             (float)(fix_period_y(ctx) / 4294967296.0), (float)(ctx->bozl / 4294967296.0),
             (float)(0.495 * ctx->boxl), (float)(0.495 * ctx->boyl), (float)(0.495 * ctx->bozl),
-            cell_pbc(ctx)};
+            cell_pbc(ctx), shared};
   const int T = 128;
   const double bx = ctx->boxl, by = ctx->boyl, bz = ctx->bozl;
   const int *nspec = d.nspec_d;

@@ -255,9 +255,8 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
                                  const int *__restrict__ mol_type,
                                  const int4 *__restrict__ ainfo, MoveConst mv,
                                  MolConst mc, double htsteb, double tsteb, int prev,
-                                 const double *__restrict__ hx, const double *__restrict__ hy,
-                                 const double *__restrict__ hz,
-                                 const unsigned long long *__restrict__ hfix, int n,
+                                 const double *hx, const double *hy, const double *hz,
+                                 const unsigned long long *hfix, int n,
                                  double inv, const double *__restrict__ massdi,
                                  const double *__restrict__ amass, double *__restrict__ vx,
                                  double *__restrict__ vy, double *__restrict__ vz,
@@ -265,10 +264,13 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
                                  double *__restrict__ Y, double *__restrict__ Z,
                                  double bx, double by, double bz, double3 ibs,
                                  int4 *__restrict__ posi, const int *__restrict__ pinfo,
-                                 int4 *__restrict__ posc, const int *__restrict__ slot_of) {
+                                 int4 *__restrict__ posc, const int *__restrict__ slot_of,
+                                 unsigned long long *zero) {
   // ibs: 2^32 / box per axis (host-computed: no FP64 division per thread);
   // posi set (mixed path): centre of mass by the reciprocal mass, the
-  // fixed-point mirror refreshed, and (posc set) its cell-order copy
+  // fixed-point mirror refreshed, and (posc set) its cell-order copy.
+  // zero set: the atom's fast forces (3 words, stride n: hfix, or hx..hz)
+  // are cleared once read, for an FFORCES whose parts all add to them
   const int m = ml.m, f = mol_first[m], na = ml.live ? mol_nat[m] : 0;
   if (ml.g == 1 && posi && na <= KD_MAXA) {
     if (!ml.live) return;
@@ -305,6 +307,7 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
           p.y = fma(v, tm, p.y);
           p.z = fma(w, tm, p.z);
         }
+        if (zero) zero[i] = zero[n + i] = zero[2 * n + i] = 0ull;
         pr[k] = p;
         const double ms = amass[i];
         x = fma(ms, p.x, x);
@@ -386,6 +389,7 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
       vy[i] = v;
       vz[i] = w;
     }
+    if (zero) zero[i] = zero[n + i] = zero[2 * n + i] = 0ull;
     if (k == ml.k) p0 = p;
     else pos[i] = p;
     const double ms = amass[i];
@@ -437,9 +441,8 @@ __global__ void k_kick_drift_com(MolLanes L, const int *__restrict__ mol_first,
                                  const int *__restrict__ mol_type,
                                  const int4 *__restrict__ ainfo, MoveConst mv,
                                  MolConst mc, double htsteb, double tsteb, int prev,
-                                 const double *__restrict__ hx, const double *__restrict__ hy,
-                                 const double *__restrict__ hz,
-                                 const unsigned long long *__restrict__ hfix, int n,
+                                 const double *hx, const double *hy, const double *hz,
+                                 const unsigned long long *hfix, int n,
                                  double inv, const double *__restrict__ massdi,
                                  const double *__restrict__ amass, double *__restrict__ vx,
                                  double *__restrict__ vy, double *__restrict__ vz,
@@ -447,11 +450,12 @@ __global__ void k_kick_drift_com(MolLanes L, const int *__restrict__ mol_first,
                                  double *__restrict__ Y, double *__restrict__ Z,
                                  double bx, double by, double bz, double3 ibs,
                                  int4 *__restrict__ posi, const int *__restrict__ pinfo,
-                                 int4 *__restrict__ posc, const int *__restrict__ slot_of) {
+                                 int4 *__restrict__ posc, const int *__restrict__ slot_of,
+                                 unsigned long long *zero) {
   kick_drift_com_body(mol_lane(L), mol_first, mol_nat, mol_type,
                       ainfo, mv, mc, htsteb, tsteb, prev, hx, hy, hz, hfix, n, inv, massdi,
                       amass, vx, vy, vz, pos, X, Y, Z, bx, by, bz, ibs, posi, pinfo, posc,
-                      slot_of);
+                      slot_of, zero);
 }
 
 // SULTAN 1.3.1-1.3.2.2 (mdstep.f:89-113): OX = SX, V += TSTEP F,
@@ -1569,7 +1573,7 @@ __global__ void k_kick_drift_com_beads(MolLanes L, const int *__restrict__ mol_f
   kick_drift_com_body(mol_lane(L), mol_first, mol_nat, mol_type,
                       ainfo, mv, mc, htsteb, tsteb, 0, b.f[0][0], b.f[0][1], b.f[0][2], nullptr,
                       n, 0.0, massdi, amass, b.vx, b.vy, b.vz, b.pos, b.X, b.Y, b.Z, bx, by, bz,
-                      ibs, b.posi, pinfo, b.posc, b.slot_of);
+                      ibs, b.posi, pinfo, b.posc, b.slot_of, nullptr);
 }
 
 static KickArgs kick_args(mdx_ctx *ctx, const KickSpec &k) {
@@ -1915,7 +1919,8 @@ int launch_kick_drift(mdx_ctx *ctx, double htsteb, double tsteb, int prev) {
   return MDX_OK;
 }
 
-int launch_kick_drift_com(mdx_ctx *ctx, double htsteb, double tsteb, int prev, bool from_fix) {
+int launch_kick_drift_com(mdx_ctx *ctx, double htsteb, double tsteb, int prev, bool from_fix,
+                          bool zero_fast) {
   MDX_TIMER(ctx, MDX_T_MOVE);
   DevData &d = ctx->dv;
   // a warp per block: the molecules spread over the SMs evenly (this pass
@@ -1926,7 +1931,9 @@ int launch_kick_drift_com(mdx_ctx *ctx, double htsteb, double tsteb, int prev, b
       htsteb, tsteb, prev, d.hx, d.hy, d.hz, from_fix ? d.hfix : nullptr, d.n, ctx->fix.inv,
       d.massdi, d.amass, d.vx, d.vy, d.vz, d.pos, d.X, d.Y, d.Z, ctx->boxl, ctx->boyl,
       ctx->bozl, fix_scale3(ctx), ctx->mixed() ? d.posi : nullptr, d.pinfo,
-      ctx->mixed() && ctx->have_lists ? d.cell_pos : nullptr, d.slot_of);
+      ctx->mixed() && ctx->have_lists ? d.cell_pos : nullptr, d.slot_of,
+      !zero_fast ? nullptr
+      : ctx->mixed() ? d.hfix : reinterpret_cast<unsigned long long *>(d.hx));
   MDX_LAUNCHED(ctx);
   return MDX_OK;
 }

@@ -21,7 +21,7 @@ int launch_leapfrog_shake(mdx_ctx *ctx);
 int launch_vira(mdx_ctx *ctx, int from_viran);
 size_t scal_scratch_bytes();
 // bonded.cu
-int launch_bonded(mdx_ctx *ctx, int laver, bool ener = true);
+int launch_bonded(mdx_ctx *ctx, int laver, bool ener = true, bool shared = false);
 
 namespace {
 
@@ -187,20 +187,42 @@ int require(mdx_ctx *ctx, bool topo, bool par, bool state) {
 }
 
 // ---------------------------------------------------------------- forces
-// ener = false: an intermediate short step of DOUBLE, whose fast energies
-// and virials the next FFORCES zeroes before anything reads them; the pair
-// sweep then computes forces only, and on the mixed path nothing needs
-// zeroing (the short sweep stores every atom's fixed-point force before the
-// bonded terms add to it).  mirrored: GETCOM has just refreshed the FP32 and
-// fixed-point mirrors of the positions.
-int do_fforces(mdx_ctx *ctx, int laver, bool split, bool ener = true, bool mirrored = false,
-               bool fold = true) {
-  if (ener || !ctx->mixed()) RC(launch_zero_fast(ctx));
+// mirrored: GETCOM has just refreshed the FP32 and fixed-point mirrors of the
+// positions.
+int do_fforces(mdx_ctx *ctx, int laver, bool split, bool mirrored = false) {
+  RC(launch_zero_fast(ctx));
   if (ctx->mixed() && !mirrored) RC(launch_mirror_f32(ctx));
-  RC(launch_localf(ctx, split, ener));
-  if (ener) RC(launch_wir(ctx, 1));  // WIRSS from the pair forces, before the bonded terms
-  RC(launch_bonded(ctx, laver, ener));
-  // fold = false: the next step's kick reads the fixed-point forces itself
+  RC(launch_localf(ctx, split));
+  RC(launch_wir(ctx, 1));  // WIRSS from the pair forces, before the bonded terms
+  RC(launch_bonded(ctx, laver));
+  if (ctx->mixed()) RC(launch_fix_to_double(ctx, 1));
+  RC(launch_sclfrc(ctx, 1));
+  return MDX_OK;
+}
+
+// FFORCES of an intermediate short step (forces only, the fast forces cleared
+// by the kick before it): the short sweep and the bonded terms both add, so
+// in a captured step they are two branches of the graph.  Both are bound by
+// latency in small systems (3,000 atoms FP64: 16 and 17 us, 600 mixed: 10 and
+// 12), and the two clearing launches of the FP64 path are gone.
+int do_fforces_mid(mdx_ctx *ctx, bool fold) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  MDX_CUDA(cudaStreamIsCapturing(ctx->stream, &st));
+  const bool fork = st == cudaStreamCaptureStatusActive && ctx->side;
+  if (fork) {
+    MDX_CUDA(cudaEventRecord(ctx->side_ev[0], ctx->stream));
+    MDX_CUDA(cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0));
+    std::swap(ctx->stream, ctx->side);
+    const int rc = launch_bonded(ctx, 0, false, true);
+    std::swap(ctx->stream, ctx->side);
+    MDX_CUDA(cudaEventRecord(ctx->side_ev[1], ctx->side));
+    if (rc) return rc;
+    RC(launch_localf(ctx, false, false, true));
+    MDX_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->side_ev[1], 0));
+  } else {
+    RC(launch_localf(ctx, false, false, true));
+    RC(launch_bonded(ctx, 0, false));
+  }
   if (ctx->mixed() && fold) RC(launch_fix_to_double(ctx, 1));
   RC(launch_sclfrc(ctx, 1));
   return MDX_OK;
@@ -274,16 +296,16 @@ int double_step(mdx_ctx *ctx, int mstep, int slot) {
   for (int s = 1; s <= NFREQ; ++s) {
     // kick, drift, GETCOM and the mirrors; positions then stay put until the
     // next short step
-    RC(launch_kick_drift_com(ctx, HTSTEB, TSTEB, s > 1 ? 1 : 0, keep_fix && s > 1));
+    RC(launch_kick_drift_com(ctx, HTSTEB, TSTEB, s > 1 ? 1 : 0, keep_fix && s > 1, s < NFREQ));
     if (s == NFREQ2) RC(launch_list_update(ctx, mstep));
     if (s == NFREQ) {
       RC(do_slforces(ctx, false, true));
       // the bonded statistics of the step (GETBND..GETTRS form them at every
       // FFORCES, forces.f:113-513) when averages are kept on the device
-      RC(do_fforces(ctx, ctx->averaging ? 1 : 0, false, true, true));
+      RC(do_fforces(ctx, ctx->averaging ? 1 : 0, false, true));
       if (ctx->averaging) RC(launch_acc_bonded(ctx));
     } else {
-      RC(do_fforces(ctx, 0, false, false, true, !keep_fix));
+      RC(do_fforces_mid(ctx, !keep_fix));
     }
   }
   // the two closing half kicks (mdstep.f:405-430) in SCALING(2)'s first GETEMP pass
@@ -327,6 +349,11 @@ int graph_step(mdx_ctx *ctx, int mstep, bool rec, bool dbl) {
   const int g = (list ? 1 : 0) + (rec ? 2 : 0) + (dbl ? 0 : 4);
   if (!ctx->gexec[g]) {
     const int64_t l0 = ctx->launches;
+    if (!ctx->side) {
+      for (auto &e : ctx->side_ev)
+        if (!e) MDX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      MDX_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+    }
     MDX_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     int rc = dbl ? double_step(ctx, mstep, rec ? -1 : -2) : sultan_step(ctx, mstep, rec ? -1 : -2);
     cudaGraph_t graph = nullptr;
@@ -554,6 +581,9 @@ int mdx_close(mdx_ctx *ctx) {
     cudaEventDestroy(sp.b);
   }
   for (auto e : ctx->ev_pool) cudaEventDestroy(e);
+  for (auto e : ctx->side_ev)
+    if (e) cudaEventDestroy(e);
+  if (ctx->side) cudaStreamDestroy(ctx->side);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return MDX_OK;
@@ -1645,5 +1675,5 @@ int api_do_slforces(mdx_ctx *ctx, bool split, bool mirrored) {
   return do_slforces(ctx, split, mirrored);
 }
 int api_do_fforces(mdx_ctx *ctx, int laver, bool split, bool mirrored) {
-  return do_fforces(ctx, laver, split, true, mirrored);
+  return do_fforces(ctx, laver, split, mirrored);
 }

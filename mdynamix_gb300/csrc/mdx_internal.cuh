@@ -351,6 +351,9 @@ struct mdx_ctx {
       }
   }
   double pair_tab_alpha = 0.0;  // alpha of dv.pair_tab
+  // branch of a captured step (bonded terms beside the short sweep)
+  cudaStream_t side = nullptr;
+  cudaEvent_t side_ev[2] = {};
   int mbsh = 0, mbln = 0;
   cudaEvent_t snap_ev[MDX_SNAPSHOT_SLOTS] = {};  // completion of mdx_snapshot per slot
   // device timers (mdx_set_timers)
@@ -765,7 +768,7 @@ bool list_update_every_step(const mdx_ctx *ctx);  // skin mode: the update is in
 int export_lists(mdx_ctx *ctx, int32_t *nbs1, int32_t *nbs2, int32_t cap_s,
                  int32_t *nbl1, int32_t *nbl2, int32_t cap_l);
 // pair.cu
-int launch_localf(mdx_ctx *ctx, bool split, bool ener = true);
+int launch_localf(mdx_ctx *ctx, bool split, bool ener = true, bool add = false);
 int pack_lj_tables(mdx_ctx *ctx);  // abf from the FP32 tables
 int launch_forces_long(mdx_ctx *ctx, bool split);
 // pair64.cu
@@ -822,7 +825,8 @@ int launch_getkin(mdx_ctx *ctx, const double *summd, double *out);  // EKTR, EKR
 int launch_chkmom(mdx_ctx *ctx, double sumasd, double *pt);        // removed momentum
 // DOUBLE's kick + drift + GETCOM + mirrors in one pass (from_fix: fast
 // forces read as fixed point, mixed path)
-int launch_kick_drift_com(mdx_ctx *ctx, double htsteb, double tsteb, int prev, bool from_fix);
+int launch_kick_drift_com(mdx_ctx *ctx, double htsteb, double tsteb, int prev, bool from_fix,
+                          bool zero_fast = false);
 int launch_kick_drift(mdx_ctx *ctx, double htsteb, double tsteb, int prev);
 int launch_record(mdx_ctx *ctx, int slot, int mstep);
 int launch_getemp(mdx_ctx *ctx);

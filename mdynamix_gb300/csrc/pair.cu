@@ -87,6 +87,21 @@ constexpr int PAIR32_BLOCKS = 6;  // resident blocks per SM the register cap aim
 constexpr int PAIR32X2_BLOCKS = 4;
 constexpr int PAIR32X2_BLOCKS_SHORT = 6;
 
+// An owner's fixed-point force out: stored, or (add: FFORCES of an
+// intermediate short step, whose bonded terms run beside the sweep) added.
+__device__ __forceinline__ void owner_store(unsigned long long *__restrict__ f, int n, int i,
+                                            long long x, long long y, long long z, bool add) {
+  if (add) {
+    atomicAdd(&f[i], (unsigned long long)x);
+    atomicAdd(&f[n + i], (unsigned long long)y);
+    atomicAdd(&f[2 * n + i], (unsigned long long)z);
+  } else {
+    f[i] = (unsigned long long)x;
+    f[n + i] = (unsigned long long)y;
+    f[2 * n + i] = (unsigned long long)z;
+  }
+}
+
 // Energies by type pair of the force calls (SPLIT), one slot kept per lane as
 // an FP32 sum with its rounding errors (Knuth's two-sum: as good as the FP64
 // sum of the FP32 terms); added to the block's FP64 sums when the slot
@@ -149,7 +164,7 @@ __global__ void __launch_bounds__(256, PAIR32_BLOCKS) k_pair32(
     const double *__restrict__ X, const double *__restrict__ Y,
     const double *__restrict__ Z, double escale,
     unsigned long long *__restrict__ slots, double *__restrict__ split,
-    const int *__restrict__ owner_of, CellF cf) {
+    const int *__restrict__ owner_of, CellF cf, bool add) {
   __shared__ double s_split[SPLIT ? SPLIT_N : 1];
   SplitF spl{-1, 0.f, 0.f, 0.f, 0.f};
   if (SPLIT) {
@@ -324,11 +339,7 @@ __global__ void __launch_bounds__(256, PAIR32_BLOCKS) k_pair32(
     qy += __shfl_xor_sync(0xffffffffu, qy, o);
     qz += __shfl_xor_sync(0xffffffffu, qz, o);
   }
-  if (i < n && lane % TPO == 0) {
-    ffix[i] = (unsigned long long)qx;
-    ffix[n + i] = (unsigned long long)qy;
-    ffix[2 * n + i] = (unsigned long long)qz;
-  }
+  if (i < n && lane % TPO == 0) owner_store(ffix, n, i, qx, qy, qz, SHORT && !ENER && add);
   if (ENER) {
 #pragma unroll
     for (int k = 0; k < P_WIR; ++k) {
@@ -485,7 +496,7 @@ k_pair32x2(
     int cap, PairTables tb, TypeConst tc, PairConst pc, float sx, float sy, float sz,
     FixScale fsc, unsigned long long *__restrict__ ffix,
     unsigned long long *__restrict__ slots, double *__restrict__ split,
-    const int *__restrict__ owner_of, CellF cf) {
+    const int *__restrict__ owner_of, CellF cf, bool add) {
   __shared__ double s_split[SPLIT ? SPLIT_N : 1];
   SplitF spl{-1, 0.f, 0.f, 0.f, 0.f};
   if (SPLIT) {
@@ -709,11 +720,7 @@ k_pair32x2(
     qy += __shfl_xor_sync(0xffffffffu, qy, o);
     qz += __shfl_xor_sync(0xffffffffu, qz, o);
   }
-  if (i < n && lane % TPO == 0) {
-    ffix[i] = (unsigned long long)qx;
-    ffix[n + i] = (unsigned long long)qy;
-    ffix[2 * n + i] = (unsigned long long)qz;
-  }
+  if (i < n && lane % TPO == 0) owner_store(ffix, n, i, qx, qy, qz, SHORT && !ENER && add);
   if (SPLIT) split_out(spl, s_split, split);
   if (!ENER) return;
   float a[P_NSLOT];
@@ -801,7 +808,7 @@ __global__ void k_pack_lj(int nn, const float *__restrict__ f, float2 *__restric
 // ener = false: forces only (an intermediate short step of DOUBLE, whose fast
 // energies and virials are zeroed again by the next FFORCES before anything
 // reads them, forces.f:36-49).
-int launch_pair(mdx_ctx *ctx, bool shrt, bool split, bool ener) {
+int launch_pair(mdx_ctx *ctx, bool shrt, bool split, bool ener, bool add = false) {
   DevData &d = ctx->dv;
   if (ctx->mixed() && !ctx->tune.tpo_short) resolve_tuning(ctx);
   const int T = 256;
@@ -833,12 +840,12 @@ int launch_pair(mdx_ctx *ctx, bool shrt, bool split, bool ener) {
   k_pair32<S, P, E, K><<<grid32, T, 0, ctx->stream>>>(                            \
       d.n, d.posi, d.cell_pos, d.stab, cnt, idx, cap, tables(d),                 \
       ctx->tc, ctx->pc, (float)sxs, (float)sys, (float)szs, ctx->fix, ffix, d.X,  \
-      d.Y, d.Z, escale, slots, split_buf, S ? nullptr : d.cell_list, cf)
+      d.Y, d.Z, escale, slots, split_buf, S ? nullptr : d.cell_list, cf, add)
 #define LP32X2C(S, P, E, K, C)                                                    \
   k_pair32x2<S, P, E, K, C><<<grid32, T, 0, ctx->stream>>>(                       \
       d.n, d.posi, d.cell_pos, d.stab, cnt, idx, cap, tables(d), ctx->tc, ctx->pc, \
       (float)sxs, (float)sys, (float)szs, ctx->fix, ffix, slots, split_buf,       \
-      S ? nullptr : d.cell_list, cf)
+      S ? nullptr : d.cell_list, cf, add)
 #define LP32X2(S, P, E, K)                     \
   do {                                         \
     if (cf.kind) LP32X2C(S, P, E, K, true);    \
@@ -936,8 +943,8 @@ int pack_lj_tables(mdx_ctx *ctx) {
 }
 
 
-int launch_localf(mdx_ctx *ctx, bool split, bool ener) {
-  MDX_TIMER(ctx, MDX_T_PAIR_SHORT); return launch_pair(ctx, true, split, ener); }
+int launch_localf(mdx_ctx *ctx, bool split, bool ener, bool add) {
+  MDX_TIMER(ctx, MDX_T_PAIR_SHORT); return launch_pair(ctx, true, split, ener, add); }
 int launch_forces_long(mdx_ctx *ctx, bool split) {
   MDX_TIMER(ctx, MDX_T_PAIR_LONG); return launch_pair(ctx, false, split, true); }
 
