@@ -679,8 +679,10 @@ __global__ void k_strbnd(WaterPar w, const dbl4 *__restrict__ pos, double bxl,
 // templated molecule, bond, angle or torsion).  The kinds share no atom
 // unsafely (template molecules are of their own types, the others add with
 // atomics).  In a small system each kind's launch is a few latency-bound
-// microseconds: methanol-like solute in 211 waters 36 us in four launches, 13 in
-// one; bilayer of 22,529 atoms 57 -> 22.
+// microseconds.  The one launch measured 16 us (forces only; solute in 211
+// waters) and 29 us (with energies; bilayer of 22,529 atoms), most of it fetching
+// its code; the solute's step took 11.9 ms / 1600 before, 7.7 after, the
+// bilayer's 9.1 and 9.0.
 enum { BK_MOL = MDX_NT, BK_BOND, BK_ANGLE, BK_TORS, BK_N };  // 0 .. MDX_NT - 1: waters
 struct BondedAll {
   int blk[BK_N + 1];  // first block of each kind (waters by type first)
@@ -762,11 +764,6 @@ int launch_bonded(mdx_ctx *ctx, int laver, bool ener, bool shared) {
   const int T = 128;
   const double bx = ctx->boxl, by = ctx->boyl, bz = ctx->bozl;
   const int *nspec = d.nspec_d;
-  if (laver) {
-    if (d.nrbb) MDX_CUDA(cudaMemsetAsync(d.br, 0, sizeof(double) * 2 * d.nrbb, ctx->stream));
-    if (d.nraa) MDX_CUDA(cudaMemsetAsync(d.ar, 0, sizeof(double) * 2 * d.nraa, ctx->stream));
-    if (d.nrtt) MDX_CUDA(cudaMemsetAsync(d.tr, 0, sizeof(double) * 2 * d.nrtt, ctx->stream));
-  }
   const TorsList tl{d.iti, d.jtj, d.ktk, d.ltl, d.ituk,
                     TorsTab{d.titors, d.tnmul, d.tft, d.trt, d.tft1, d.tft2, d.tft3, d.tft4,
                             d.tft5}};

@@ -37,6 +37,7 @@
 #include <vector>
 
 #include "mdx_internal.cuh"
+#include "ewald_ops.cuh"
 
 namespace {
 
@@ -86,7 +87,8 @@ __global__ void k_tables(int n, int ldn, const dbl4 *__restrict__ pos, double ib
                          double2 *__restrict__ tx, double2 *__restrict__ ty,
                          double2 *__restrict__ tz, float2 *__restrict__ txf,
                          float2 *__restrict__ tyf, float2 *__restrict__ tzf,
-                         const int4 *__restrict__ posi, double hexy) {
+                         const int4 *__restrict__ posi, double hexy, int kp,
+                         unsigned char *__restrict__ zf) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 3 * n) return;
   const int a = t / n, i = t - a * n;
@@ -114,7 +116,9 @@ __global__ void k_tables(int n, int ldn, const dbl4 *__restrict__ pos, double ib
       float s, c;
       sincospif((float)hi * 4.656612873077393e-10f, &s, &c);  // 2^-31
       const float d = (float)lo * 1.4629180792671596e-09f;    // pi 2^-31
-      dst[(size_t)k * ldn] = make_float2(qf * fmaf(-s, d, c), qf * fmaf(c, d, s));
+      const float2 v = make_float2(qf * fmaf(-s, d, c), qf * fmaf(c, d, s));
+      dst[(size_t)k * ldn] = v;
+      if (a == 2 && zf) tc_zimage_store(zf, kp, k, i, v);
     }
     return;
   }
@@ -135,27 +139,15 @@ __global__ void k_tables(int n, int ldn, const dbl4 *__restrict__ pos, double ib
   }
 }
 
-// Write one paired accumulator as S(c, +p) and S(c, -p) (each only if the
-// k-vector exists): slice partial (summed in a fixed order by k_sfac_sum) or
-// atomic.
+// Write one paired accumulator as the slice's partial of S(c, +p) and S(c,
+// -p) (each only if the k-vector exists); k_sfac_sum adds the slices in a
+// fixed order.
 __device__ __forceinline__ void sfac_out(const KCol &col, int p, double A1, double A2,
-                                         double A3, double A4, double2 *part, double2 *sk) {
+                                         double A3, double A4, double2 *part) {
   const int z = kcol_z(col, p);
   const int kp = kcol_k(col, z), km = z > 0 ? kcol_k(col, -z) : -1;
-  const double2 vp = make_double2(A1 - A2, A3 + A4), vm = make_double2(A1 + A2, A4 - A3);
-  if (part) {
-    if (kp >= 0) part[kp] = vp;
-    if (km >= 0) part[km] = vm;
-  } else {
-    if (kp >= 0) {
-      atomicAdd(&sk[kp].x, vp.x);
-      atomicAdd(&sk[kp].y, vp.y);
-    }
-    if (km >= 0) {
-      atomicAdd(&sk[km].x, vm.x);
-      atomicAdd(&sk[km].y, vm.y);
-    }
-  }
+  if (kp >= 0) part[kp] = make_double2(A1 - A2, A3 + A4);
+  if (km >= 0) part[km] = make_double2(A1 + A2, A4 - A3);
 }
 
 // FP64 S(k): thread per chunk (column, CH consecutive p from p0), block.y =
@@ -164,7 +156,7 @@ __global__ void __launch_bounds__(128) k_sfac(
     int n, int nchunk, const Chunk *__restrict__ chunks,
     const KCol *__restrict__ cols, const double2 *__restrict__ tx,
     const double2 *__restrict__ ty, const double2 *__restrict__ tz, int kx, int ky,
-    int kz, double2 *__restrict__ sk, double2 *__restrict__ part, int nkv) {
+    int kz, double2 *__restrict__ part, int nkv) {
   extern __shared__ unsigned char smem_raw[];
   double2 *sx = reinterpret_cast<double2 *>(smem_raw);  // [atom][n]
   double2 *sy = sx + TILE * kx;
@@ -220,10 +212,10 @@ __global__ void __launch_bounds__(128) k_sfac(
     }
   }
   if (ch < nchunk) {
-    double2 *pp = part ? part + (size_t)blockIdx.y * nkv : nullptr;
+    double2 *pp = part + (size_t)blockIdx.y * nkv;
 #pragma unroll
     for (int t = 0; t < CH; ++t)
-      if (t < cc.len) sfac_out(col, cc.nz0 + t, A[t][0], A[t][1], A[t][2], A[t][3], pp, sk);
+      if (t < cc.len) sfac_out(col, cc.nz0 + t, A[t][0], A[t][1], A[t][2], A[t][3], pp);
   }
 }
 
@@ -246,7 +238,7 @@ template <int ZS>
 __global__ void __launch_bounds__(128, 4) k_sfac32(
     int n, int nitem, const SItem *__restrict__ items, const KGroup *__restrict__ groups,
     const KCol *__restrict__ cols, const float2 *__restrict__ tab, int ldn, int kx, int ky,
-    int kz, int slice, double2 *__restrict__ sk, double2 *__restrict__ part, int nkv) {
+    int kz, int slice, double2 *__restrict__ part, int nkv) {
   // tab: the X, Y and Z tables back to back, row r at tab + r * ldn;
   // ZS: the z step of the records, 2 for the octahedron's k-set (a window
   // reads every other z); a template parameter, so that the rectangular
@@ -337,7 +329,7 @@ __global__ void __launch_bounds__(128, 4) k_sfac32(
   if (!active) return;
   const SItem si = items[it];
   const KGroup &G = groups[si.g];
-  double2 *pp = part ? part + (size_t)blockIdx.y * nkv : nullptr;
+  double2 *pp = part + (size_t)blockIdx.y * nkv;
 #pragma unroll
   for (int c = 0; c < KGRP; ++c) {
     const int ci = G.col[c];
@@ -347,19 +339,22 @@ __global__ void __launch_bounds__(128, 4) k_sfac32(
     for (int s = 0; s < SCH; ++s)
       if (si.t0 + s <= G.m)
         sfac_out(col, si.t0 + s, (double)P[c][s].x, (double)Q[c][s].y, (double)P[c][s].y,
-                 (double)Q[c][s].x, pp, sk);
+                 (double)Q[c][s].x, pp);
   }
 }
 
-// S(k) = sum of the slice partials in slice order (deterministic).
 constexpr int SUM_K = 32, SUM_G = 8;  // k-vectors and slice groups of a block
 
 // S(k) = the sum of the slice partials: thread (k, g) adds slices g, g +
 // SUM_G, ... in order, then the groups are added in group order (a fixed
-// order: deterministic); reads are coalesced over k.
+// order: deterministic); reads are coalesced over k.  TERMS: the k's energy
+// and virial terms, W_k and RZV W_k (k_kterms) in the same launch.
+template <bool TERMS>
 __global__ void __launch_bounds__(SUM_K * SUM_G) k_sfac_sum(int nkv, int nslice,
-                                                         const double2 *__restrict__ part,
-                                                         double2 *__restrict__ sk) {
+                                                            const double2 *__restrict__ part,
+                                                            double2 *__restrict__ sk,
+                                                            const double *__restrict__ kc,
+                                                            dbl4 *__restrict__ wk, Dst6 dst) {
   __shared__ double2 sh[SUM_G][SUM_K];
   const int kl = threadIdx.x % SUM_K, g = threadIdx.x / SUM_K;
   const int k = blockIdx.x * SUM_K + kl;
@@ -372,6 +367,7 @@ __global__ void __launch_bounds__(SUM_K * SUM_G) k_sfac_sum(int nkv, int nslice,
     }
   sh[g][kl] = make_double2(x, y);
   __syncthreads();
+  double acc[5] = {0, 0, 0, 0, 0};
   if (g == 0 && k < nkv) {
 #pragma unroll
     for (int q = 1; q < SUM_G; ++q) {
@@ -379,10 +375,14 @@ __global__ void __launch_bounds__(SUM_K * SUM_G) k_sfac_sum(int nkv, int nslice,
       y += sh[q][kl].y;
     }
     sk[k] = make_double2(x, y);
+    if (TERMS) wk[k] = kterm(make_double2(x, y), kc + 5 * (size_t)k, acc);
+  }
+  if (TERMS) {
+    acc[4] = acc[0];
+    block_add<5>(acc, dst);
   }
 }
 
-// Per k: energy and virial terms (forces.f:1316-1331), W_k and RZV W_k.
 // Per-k constants of FURIR that depend on the box and alpha only (forces.f:
 // 1316-1331): AKC, (RXV^2, RYV^2, RZV^2) AKV and RZV, five doubles per k,
 // and the column's (RXV, RYV); rebuilt when the box or alpha changes.
@@ -423,29 +423,17 @@ __global__ void k_kconst(int ncol, const KCol *__restrict__ cols, double bx, dou
 
 // Per k: energy and virial terms (forces.f:1316-1331), W_k and RZV W_k, from
 // S(k) and the per-k constants (the same products as the reference's
-// expressions, in its order).
+// expressions, in its order).  The sums go to QPE, PELS1 and the three virial
+// projections, which take QPE too (forces.f:1333-1336).  For the S(k) that no
+// k_sfac_sum has formed.
 __global__ void k_kterms(int nkv, const double2 *__restrict__ sk,
                          const double *__restrict__ kc, dbl4 *__restrict__ wk, Dst6 dst) {
-  double acc[4] = {0, 0, 0, 0};
+  double acc[5] = {0, 0, 0, 0, 0};
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nkv; k += gridDim.x * blockDim.x) {
-    const double2 S = sk[k];
-    const double SCS = S.x, SSN = S.y;
-    const double *q = kc + 5 * (size_t)k;
-    const double AKC = q[0];
-    const double S2 = SSN * SSN + SCS * SCS;
-    acc[0] += AKC * S2;
-    acc[1] -= q[1] * S2;
-    acc[2] -= q[2] * S2;
-    acc[3] -= q[3] * S2;
-    const double AK2 = 2.0 * AKC;
-    dbl4 W;
-    W.x = AK2 * SCS;
-    W.y = -AK2 * SSN;
-    W.z = q[4] * W.x;
-    W.w = q[4] * W.y;
-    wk[k] = W;
+    wk[k] = kterm(sk[k], kc + 5 * (size_t)k, acc);
   }
-  block_add<4>(acc, dst);
+  acc[4] = acc[0];
+  block_add<5>(acc, dst);
 }
 
 // Paired W per (column, p): P = W(+p) + W(-p), M = W(+p) - W(-p) for U, the
@@ -483,17 +471,6 @@ __global__ void k_wpairs(int ncol, const KCol *__restrict__ cols, const dbl4 *__
       }
     }
   }
-}
-
-// QPE into PELS1 and the three virial projections (forces.f:1333-1336).
-__global__ void k_qpe_fold(mdx_scalars *sc, double *qpe) {
-  const double Q = *qpe;
-  sc->virx = sc->virx + Q;
-  sc->viry = sc->viry + Q;
-  sc->virz = sc->virz + Q;
-  sc->pels1 = sc->pels1 + Q;
-  sc->qpe = Q;
-  *qpe = 0.0;
 }
 
 // Force passes: a block is RF_ATOMS atoms x RF_PARTS column parts (one warp
@@ -842,16 +819,6 @@ __global__ void k_eterms(int n, const dbl4 *__restrict__ pos,
     atomicAdd(&spee[threadIdx.x], spee_sh[threadIdx.x]);
 }
 
-struct SelfEnergy {
-  double spei, speei[MDX_NT];
-};
-
-__global__ void k_eterms_init(mdx_scalars *sc, SelfEnergy se, int ntypes) {
-  sc->spe = se.spei;
-  for (int t = 0; t < MDX_NT; ++t) sc->spee[t] = t < ntypes ? se.speei[t] : 0.0;
-}
-
-
 }  // namespace
 
 std::mutex g_smem_mu;
@@ -1176,14 +1143,10 @@ int sfac_slices(const mdx_ctx *ctx) {
   return ctx->mixed() ? d.sfac_nslice : (d.n + SLICE - 1) / SLICE;
 }
 
-// FURIR's first half (forces.f:1217-1290): the k-set check against the box
-// (INIFUR again past the 5 % window), the phase tables and S(k) of the
-// current positions and charges into d.sk.  *skip: nothing to do (no Ewald,
-// empty k-set or a single molecule).
-int furir_sfac(mdx_ctx *ctx, bool *skip) {
-  DevData &d = ctx->dv;
-  *skip = ctx->p.alphad <= 0.0;
-  if (*skip) return MDX_OK;
+// The k-set check of FURIR against the box (forces.f:1251-1265): INIFUR at the
+// first call and again past the 5 % window.
+int furir_prepare(mdx_ctx *ctx) {
+  if (ctx->p.alphad <= 0.0) return MDX_OK;
   const double FKTX = 1.05, FKTS = 0.95;
   int rc;
   if (!ctx->furir_init) {
@@ -1202,7 +1165,18 @@ int furir_sfac(mdx_ctx *ctx, bool *skip) {
     ctx->bozlo = ctx->bozl;
     if ((rc = host_inifur(ctx))) return rc;
   }
-  *skip = d.nkv == 0 || (ctx->d.ntypes == 1 && ctx->nspec[0] == 1);
+  return MDX_OK;
+}
+
+// FURIR's first half (forces.f:1217-1290): the k-set check, the phase tables
+// and S(k) of the current positions and charges into d.sk.  *skip: nothing to
+// do (no Ewald, empty k-set or a single molecule).  terms: where k_sfac_sum
+// forms S(k), the energy and virial terms and W too.
+int furir_sfac(mdx_ctx *ctx, bool *skip, bool terms) {
+  DevData &d = ctx->dv;
+  int rc = furir_prepare(ctx);
+  if (rc) return rc;
+  *skip = ctx->p.alphad <= 0.0 || d.nkv == 0 || (ctx->d.ntypes == 1 && ctx->nspec[0] == 1);
   if (*skip) return MDX_OK;
   const double ibx = 1.0 / ctx->boxl, iby = 1.0 / ctx->boyl, ibz = 1.0 / ctx->bozl;
   const Chunk *chunks = reinterpret_cast<const Chunk *>(d.kchunks);
@@ -1221,11 +1195,10 @@ int furir_sfac(mdx_ctx *ctx, bool *skip) {
     k_tables<<<(3 * d.n + 255) / 256, 256, 0, ctx->stream>>>(
         d.n, d.ldn, d.pos, ibx, iby, ibz, d.kx, d.ky, d.kz, d.tabx, d.taby, d.tabz,
         d.tabxf, d.tabyf, d.tabzf, mx ? d.posi : nullptr,
-        ctx->p.icell == 2 ? 0.5 * iby : 0.0);
+        ctx->p.icell == 2 ? 0.5 * iby : 0.0, d.tc_kp, mx && d.tc_on ? d.tc_zimg : nullptr);
     MDX_LAUNCHED(ctx);
     if (mx && (rc = tc_zimages_launch(ctx))) return rc;
   }
-  MDX_CUDA(cudaMemsetAsync(d.sk, 0, sizeof(double2) * d.nkv, ctx->stream));
   {
     MDX_TIMER(ctx, MDX_T_EW_SFAC);
     const size_t sh = mx ? 2 * sizeof(float2) * TILE * (d.kx + d.ky + d.kz + SCH * d.zstep)
@@ -1239,18 +1212,21 @@ int furir_sfac(mdx_ctx *ctx, bool *skip) {
         auto kern = d.zstep == 2 ? k_sfac32<2> : k_sfac32<1>;
         kern<<<grid, 128, sh, ctx->stream>>>(
             d.n, d.nsitem, reinterpret_cast<const SItem *>(d.sitems), d.kgroups, d.cols,
-            d.tabxf, d.ldn, d.kx, d.ky, d.kz, d.sfac_slice, d.sk, d.sk_part, d.nkv);
+            d.tabxf, d.ldn, d.kx, d.ky, d.kz, d.sfac_slice, d.sk_part, d.nkv);
       } else {
         grid = dim3((nchunk + 127) / 128, (d.n + SLICE - 1) / SLICE);
         k_sfac<<<grid, 128, sh, ctx->stream>>>(
-            d.n, nchunk, chunks, d.cols, d.tabx, d.taby, d.tabz, d.kx, d.ky, d.kz, d.sk,
-            d.sk_part, d.nkv);
+            d.n, nchunk, chunks, d.cols, d.tabx, d.taby, d.tabz, d.kx, d.ky, d.kz, d.sk_part,
+            d.nkv);
       }
       MDX_LAUNCHED(ctx);
     }
-    if (d.sk_part && !(mx && d.tcs_on)) {
-      k_sfac_sum<<<(d.nkv + SUM_K - 1) / SUM_K, SUM_K * SUM_G, 0, ctx->stream>>>(d.nkv, (int)grid.y,
-                                                                d.sk_part, d.sk);
+    if (!(mx && d.tcs_on)) {
+      const int nb = (d.nkv + SUM_K - 1) / SUM_K;
+      if (terms && (rc = ensure_kconst(ctx))) return rc;
+      auto sum = terms ? k_sfac_sum<true> : k_sfac_sum<false>;
+      sum<<<nb, SUM_K * SUM_G, 0, ctx->stream>>>(d.nkv, (int)grid.y, d.sk_part, d.sk, d.kconst,
+                                                 d.wk, kterm_dst(ctx, nb));
       MDX_LAUNCHED(ctx);
     }
   }
@@ -1284,24 +1260,21 @@ int launch_furir(mdx_ctx *ctx) {
   DevData &d = ctx->dv;
   bool skip = false;
   int rc;
-  if ((rc = furir_sfac(ctx, &skip)) || skip) return rc;
+  if ((rc = furir_sfac(ctx, &skip, true)) || skip) return rc;
   const bool mx = ctx->mixed();
-  double *qpe = d.red + 40;
-  mdx_scalars *sc = d.sc;
   {
     MDX_TIMER(ctx, MDX_T_EW_KTERMS);
     if ((rc = ensure_kconst(ctx))) return rc;
-    const int kb = std::max(1, std::min((d.nkv + 127) / 128, 2 * ctx->nsm));
-    Dst6 dst = dst6(ctx, kb, 4, qpe, &sc->virx, &sc->viry, &sc->virz);
-    k_kterms<<<kb, 128, 0, ctx->stream>>>(d.nkv, d.sk, d.kconst, d.wk, dst);
-    MDX_LAUNCHED(ctx);
+    if (mx && d.tcs_on) {
+      const int kb = std::max(1, std::min((d.nkv + 127) / 128, 2 * ctx->nsm));
+      k_kterms<<<kb, 128, 0, ctx->stream>>>(d.nkv, d.sk, d.kconst, d.wk, kterm_dst(ctx, kb));
+      MDX_LAUNCHED(ctx);
+    }
     if (!(mx && d.tc_on) && !d.fx_on) {
       k_wpairs<<<std::min(d.ncol, 1024), 64, 0, ctx->stream>>>(
           d.ncol, d.cols, d.wk, mx ? nullptr : d.wp64, mx ? d.wkf : nullptr);
       MDX_LAUNCHED(ctx);
     }
-    k_qpe_fold<<<1, 1, 0, ctx->stream>>>(sc, qpe);
-    MDX_LAUNCHED(ctx);
   }
   MDX_TIMER(ctx, MDX_T_EW_FORCE);
   const int rblocks = (d.n + RF_ATOMS - 1) / RF_ATOMS;
@@ -1328,11 +1301,6 @@ int launch_eterms(mdx_ctx *ctx) {
   MDX_TIMER(ctx, MDX_T_ETERMS);
   DevData &d = ctx->dv;
   if (ctx->p.lmnbl) return MDX_OK;
-  SelfEnergy se;
-  se.spei = ctx->spei;
-  for (int t = 0; t < MDX_NT; ++t) se.speei[t] = ctx->speei[t];
-  k_eterms_init<<<1, 1, 0, ctx->stream>>>(d.sc, se, ctx->d.ntypes);
-  MDX_LAUNCHED(ctx);
   mdx_scalars *sc = d.sc;
   Dst6 dst = dst6(ctx, (d.n + 127) / 128, 4, &sc->spe, &sc->virx, &sc->viry, &sc->virz);
   if (ctx->mixed())

@@ -41,6 +41,7 @@
 #include <cmath>
 #include <vector>
 
+#include "ewald_ops.cuh"
 #include "mdx_internal.cuh"
 #include "tc_ptx.cuh"
 
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_fx_sfac(
     int nchunk_all, int cps, int ncol, int np, int kx, int kxy, int ua, int ug,
     const KCol *__restrict__ cols, const int4 *__restrict__ xy,
     const unsigned char *__restrict__ zs, unsigned long long *__restrict__ acc_out,
-    int *__restrict__ err) {
+    int *__restrict__ bad, int *__restrict__ err) {
   extern __shared__ unsigned char dsm_raw[];
   __shared__ __align__(8) unsigned long long xyf[2], zfull[2], af[2], ad[2], gd, rf;
   __shared__ uint32_t tmem_base_sh;
@@ -295,6 +296,10 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_fx_sfac(
   if (warp == 0) {
     tc::tmem_alloc(tc::smem_addr(&tmem_base_sh), 512);
     tc::tmem_relinquish();
+  }
+  if (tid == 32 && blockIdx.x == 0 && blockIdx.y == 0) {  // the flag, for the kernels to come
+    bad[1] = bad[0];
+    bad[0] = 0;
   }
   if (tid == 0) {
     for (int b = 0; b < 2; ++b) {
@@ -480,22 +485,23 @@ __global__ void __launch_bounds__(FX_THREADS, 1) k_fx_sfac(
 }
 
 // S(k) of the k-vectors from the integer sums: block per column, thread per
-// record p (nz = +-z).
+// record p (nz = +-z).  The sums it has read are cleared for the next call.
 __global__ void k_fx_form(int ncol, int np, int ug, const KCol *__restrict__ cols,
-                          const unsigned long long *__restrict__ acc,
-                          const double *__restrict__ qs, const int *__restrict__ bad,
-                          double2 *__restrict__ sk) {
+                          unsigned long long *__restrict__ acc, const double *__restrict__ qs,
+                          const int *__restrict__ bad, double2 *__restrict__ sk) {
   const int c = blockIdx.x;
   if (c >= ncol) return;
   const KCol col = cols[c];
   const double scale = *bad ? __longlong_as_double(0x7ff8000000000000ll) : ldexp(qs[0], -ug);
-  const long long *a = reinterpret_cast<const long long *>(acc) + (size_t)(c >> 6) * np * 128;
+  long long *a = reinterpret_cast<long long *>(acc) + (size_t)(c >> 6) * np * 128;
   const int r = c & 63;
   for (int p = threadIdx.x; p <= col.m; p += blockDim.x) {
     const int z = kcol_z(col, p);
     const long long A1 = a[(size_t)(2 * z) * 128 + r], A3 = a[(size_t)(2 * z + 1) * 128 + r];
     const long long A4 = a[(size_t)(2 * z) * 128 + 64 + r],
                     A2 = a[(size_t)(2 * z + 1) * 128 + 64 + r];
+    a[(size_t)(2 * z) * 128 + r] = a[(size_t)(2 * z + 1) * 128 + r] = 0;
+    a[(size_t)(2 * z) * 128 + 64 + r] = a[(size_t)(2 * z + 1) * 128 + 64 + r] = 0;
     const int kp = kcol_k(col, z), km = z > 0 ? kcol_k(col, -z) : -1;
     if (kp >= 0) sk[kp] = make_double2((double)(A1 - A2) * scale, (double)(A3 + A4) * scale);
     if (km >= 0) sk[km] = make_double2((double)(A1 + A2) * scale, (double)(A4 - A3) * scale);
@@ -513,19 +519,22 @@ __device__ __forceinline__ int exp_above(double x) {  // x < 2^e (0 for x = 0)
   return x > 0.0 ? ilogb(x) + 1 : 0;
 }
 
-// B operand of the F pass, one step: block per tile of FX_TCOL columns.  Row
+// B operand of the F pass, one step, from S(k) and the per-k constants (W = 2
+// AKC conj(S)), and the k-vectors' energy and virial sums: block per tile of
+// FX_TCOL columns.  Row
 // 4 c + t is U.re, U.im, V.re, V.im of column c (V with integer nz weights;
 // 2 PI / BOZL comes with the fold), scaled to the largest U or V entry of the
 // tile by a power of two, as digits in core-matrix order.
 __global__ void __launch_bounds__(256) k_fx_wtiles(
     int kp, const int4 *__restrict__ slot, const int *__restrict__ scol,
-    const int *__restrict__ tks, const KCol *__restrict__ cols, const dbl4 *__restrict__ wk,
-    unsigned char *__restrict__ tw, FxTile *__restrict__ meta) {
+    const int *__restrict__ tks, const KCol *__restrict__ cols,
+    const double2 *__restrict__ sk, const double *__restrict__ kcon,
+    unsigned char *__restrict__ tw, FxTile *__restrict__ meta, Dst6 dst) {
   extern __shared__ double sv[];  // [FX_TN][kp]
   __shared__ double red[2][8], rsum[FX_TN];
   __shared__ int se[2];
   const int tile = blockIdx.x, tid = threadIdx.x;
-  double mx[2] = {0.0, 0.0};
+  double mx[2] = {0.0, 0.0}, acc[5] = {0, 0, 0, 0, 0};
   for (int t = tid; t < FX_TN * (kp / 2); t += blockDim.x) {
     const int z = t % (kp / 2), r = t / (kp / 2), comp = r & 3;
     const int c = scol[tile * FX_TCOL + (r >> 2)];
@@ -534,14 +543,16 @@ __global__ void __launch_bounds__(256) k_fx_wtiles(
       const KCol col = cols[c];
       const int kpl = kcol_k(col, z), kmi = z > 0 ? kcol_k(col, -z) : -1;
       double ar = 0.0, ai = 0.0, br = 0.0, bi = 0.0;
-      if (kpl >= 0) {
-        ar = wk[kpl].x;
-        ai = wk[kpl].y;
-      }
-      if (kmi >= 0) {
-        br = wk[kmi].x;
-        bi = wk[kmi].y;
-      }
+      auto weight = [&](int k, double &wr, double &wi) {
+        const double2 S = sk[k];
+        const double *c5 = kcon + 5 * (size_t)k;
+        const double AK2 = 2.0 * c5[0];
+        wr = AK2 * S.x;
+        wi = -AK2 * S.y;
+        if (comp == 0) kterm_add(acc, c5, S.y * S.y + S.x * S.x);
+      };
+      if (kpl >= 0) weight(kpl, ar, ai);
+      if (kmi >= 0) weight(kmi, br, bi);
       if (comp >= 2) {  // nz W
         ar *= z;
         ai *= z;
@@ -567,7 +578,7 @@ __global__ void __launch_bounds__(256) k_fx_wtiles(
   if (tid < 2) {
     double m = 0.0;
     for (int w = 0; w < 8; ++w) m = fmax(m, red[tid][w]);
-    se[tid] = exp_above(m);
+    se[tid] = max(exp_above(m), -900);  // 2^(FX_BITS - e) stays finite
   }
   if (tid >= 32 && tid < 32 + FX_TN) {  // a row's sum of magnitudes
     double s = 0.0;
@@ -601,11 +612,12 @@ __global__ void __launch_bounds__(256) k_fx_wtiles(
   constexpr int G = FX_SL * FX_TN / 8;
   for (int t = tid; t < FX_TN * (kp / 8); t += blockDim.x) {
     const int r = t % FX_TN, g = t / FX_TN;
-    const int e = se[(r >> 1) & 1];
+    // a power of two: the product is exact
+    const double up = __hiloint2double((1023 + FX_BITS - se[(r >> 1) & 1]) << 20, 0);
     long long w[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-      w[k] = __double2ll_rn(ldexp(sv[r * kp + 8 * g + k], FX_BITS - e)) + FX_BIAS;
+      w[k] = __double2ll_rn(sv[r * kp + 8 * g + k] * up) + FX_BIAS;
     unsigned dg[FX_SL][4];
     fx_digits(w, dg);
 #pragma unroll
@@ -615,6 +627,8 @@ __global__ void __launch_bounds__(256) k_fx_wtiles(
           make_uint4(dg[j][0], dg[j][1], dg[j][2], dg[j][3]);
     }
   }
+  acc[4] = acc[0];
+  block_add<5>(acc, dst);
 }
 
 // F pass: a CTA takes 128 atoms (MMA M) and a range of tiles.  Warp 16 (lane
@@ -968,6 +982,8 @@ int fx_setup(mdx_ctx *ctx, const std::vector<KCol> &cols) {
     ctx->err = "fixed-point Ewald passes: device allocation failed";
     return MDX_ERR_NOMEM;
   }
+  // k_fx_form and k_fx_sfac leave the sums and the flag behind them cleared
+  MDX_CUDA(cudaMemsetAsync(d.fx_acc, 0, accb + 16, ctx->stream));
   d.fx_ks = d.fx_scol + scol.size();
   d.fx_parts = d.fx_ks + ks.size();
   MDX_CUDA(ctx_copy(ctx->stream, d.fx_slot, slot.data(), sizeof(int4) * slot.size(),
@@ -1012,8 +1028,7 @@ int fx_tables_launch(mdx_ctx *ctx) {
     box.ibl[a] = std::fma(-len[a], box.ib[a], 1.0) / len[a];
   }
   const size_t accb = sizeof(long long) * (size_t)d.fx_ntm * d.fx_np * 128;
-  // the sums and, behind them, the flag of a non-finite position
-  MDX_CUDA(cudaMemsetAsync(d.fx_acc, 0, accb + 16, ctx->stream));
+  // behind the sums, the flag of a non-finite position
   int *bad = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(d.fx_acc) + accb);
   k_fx_tables<<<(d.n + 31) / 32, 128, sizeof(int4) * 33 * d.kz, ctx->stream>>>(
       d.n, d.pos, box, d.kx, d.ky, d.kz, d.fx_np, d.fx_np, d.fx_qs, d.fx_xy, d.fx_zs, d.fx_zf, d.fx_facc, bad,
@@ -1025,14 +1040,14 @@ int fx_tables_launch(mdx_ctx *ctx) {
 int fx_sfac_launch(mdx_ctx *ctx) {
   DevData &d = ctx->dv;
   const size_t accb = sizeof(long long) * (size_t)d.fx_ntm * d.fx_np * 128;
-  const int *bad = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(d.fx_acc) + accb);
+  int *bad = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(d.fx_acc) + accb);
   const int kxy = d.kx + d.ky;
   k_fx_sfac<<<dim3(d.fx_ntm, d.fx_ns), FX_THREADS, fx_sfac_smem(d.fx_np, kxy), ctx->stream>>>(
       (d.n + 31) / 32, d.fx_cps, d.ncol, d.fx_np, d.kx, kxy, d.fx_ua, d.fx_ug, d.cols, d.fx_xy,
-      d.fx_zs, d.fx_acc, d.err);
+      d.fx_zs, d.fx_acc, bad, d.err);
   MDX_LAUNCHED(ctx);
   k_fx_form<<<d.ncol, 32, 0, ctx->stream>>>(d.ncol, d.fx_np, d.fx_ug, d.cols, d.fx_acc, d.fx_qs,
-                                            bad, d.sk);
+                                            bad + 1, d.sk);
   MDX_LAUNCHED(ctx);
   return MDX_OK;
 }
@@ -1040,12 +1055,13 @@ int fx_sfac_launch(mdx_ctx *ctx) {
 int fx_force_launch(mdx_ctx *ctx) {
   DevData &d = ctx->dv;
   const size_t accb = sizeof(long long) * (size_t)d.fx_ntm * d.fx_np * 128;
-  const int *bad = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(d.fx_acc) + accb);
+  const int *bad = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(d.fx_acc) + accb) + 1;
   const int kp = d.fx_np, kxy = d.kx + d.ky;
   FxTile *meta = reinterpret_cast<FxTile *>(d.fx_meta);
   int *gexp = reinterpret_cast<int *>(d.fx_facc + 3 * (size_t)d.n);
   k_fx_wtiles<<<d.fx_ntile, 256, sizeof(double) * FX_TN * kp, ctx->stream>>>(
-      kp, d.fx_slot, d.fx_scol, d.fx_ks, d.cols, d.wk, d.fx_tw, meta);
+      kp, d.fx_slot, d.fx_scol, d.fx_ks, d.cols, d.sk, d.kconst, d.fx_tw, meta,
+      kterm_dst(ctx, d.fx_ntile));
   MDX_LAUNCHED(ctx);
   const dim3 grid((d.n + 127) / 128, d.fx_nsplit);
   const size_t sh = fx_force_smem(kp, kxy, d.fx_xys);

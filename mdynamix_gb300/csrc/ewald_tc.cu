@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "mdx_internal.cuh"
+#include "ewald_ops.cuh"
 #include "tc_ptx.cuh"
 
 namespace {
@@ -39,19 +40,6 @@ constexpr int TC_M = 128;          // atoms per CTA of the force pass (MMA M)
 constexpr int TC_N = 128;          // accumulator columns per tile (32 k-columns)
 constexpr int TC_COLS = TC_N / 4;  // k-columns per tile
 constexpr uint32_t TC_POLLS = 1u << 20;  // bounded mbarrier waits
-
-// Force-pass operand layout (128 rows, K-major, unswizzled), K-step major:
-// the 8 K of MMA step s = k / 8 fill 8 KB, [hi | lo] of 4 KB each, and
-// within a part core matrix (r / 8, k / 4) of 128 bytes sits at
-// ((k / 4) % 2) 2048 + (r / 8) 128: LBO (along K) = 2048, SBO (along M/N)
-// = 128.  A tile whose columns need ks steps is then its first ks x 8 KB.
-constexpr uint32_t TC_STEP = 8192;  // bytes of one K step (hi and lo)
-constexpr uint32_t TC_LO = 4096;    // lo part within a step
-constexpr uint32_t TC_LBO = 2048, TC_SBO = 128;
-__host__ __device__ __forceinline__ uint32_t core_off(int r, int k) {  // hi part
-  return (uint32_t)((k >> 3) * TC_STEP + ((k >> 2) & 1) * TC_LBO + (r >> 3) * TC_SBO +
-                    ((r & 7) << 4) + ((k & 3) << 2));
-}
 
 // S-pass operand layout: 32 atoms (K) per chunk, core matrices along K
 // 144 bytes apart (128 + 16 spreads the shared-memory banks), SBO = 8 x 144.
@@ -69,12 +57,12 @@ __host__ __device__ __forceinline__ uint32_t sk_bpart(int np) {  // bytes of one
   return (uint32_t)(np / 8) * SK_SBO;
 }
 
-// Z images of one step: thread per (p, atom), atoms up to ldn (rows past n
-// are zero in the table).  zf: force-pass A operand, per 128-atom tile
-// kp / 8 K steps of [hi | lo]; zs: S-pass B operand, per 32-atom chunk [hi | lo]
-// of np x 32.  Entries with p >= kz stay zero (set once at allocation).
-__global__ void k_zimages(int ldn, int kz, int kp, int np, const float2 *__restrict__ tz,
-                          unsigned char *__restrict__ zf, unsigned char *__restrict__ zs) {
+// Z images of the S pass (the force pass's come with the tables): thread per
+// (p, atom), atoms up to ldn (rows past n are zero in the table).  Per 32-atom
+// chunk [hi | lo] of np x 32.  Entries with p >= kz stay zero (set once at
+// allocation).
+__global__ void k_zimages(int ldn, int kz, int np, const float2 *__restrict__ tz,
+                          unsigned char *__restrict__ zs) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (size_t)kz * ldn) return;
   const int p = (int)(t / ldn), i = (int)(t - (size_t)p * ldn);
@@ -82,23 +70,15 @@ __global__ void k_zimages(int ldn, int kz, int kp, int np, const float2 *__restr
   float ah, al, bh, bl;
   tc::tf32_split(z.x, ah, al);
   tc::tf32_split(z.y, bh, bl);
-  if (zf) {
-    unsigned char *base = zf + (size_t)(i >> 7) * 1024 * kp;
-    const uint32_t o = core_off(i & 127, 2 * p);  // k = 2p and 2p + 1: adjacent
-    *reinterpret_cast<float2 *>(base + o) = make_float2(ah, bh);
-    *reinterpret_cast<float2 *>(base + TC_LO + o) = make_float2(al, bl);
-  }
-  if (zs) {
-    const uint32_t bp = sk_bpart(np);
-    unsigned char *base = zs + (size_t)(i >> 5) * 2 * bp;
-    const int j = i & 31;
-    const uint32_t o0 = sk_off(2 * p, j >> 2) + 4 * (j & 3);
-    const uint32_t o1 = sk_off(2 * p + 1, j >> 2) + 4 * (j & 3);
-    *reinterpret_cast<float *>(base + o0) = ah;
-    *reinterpret_cast<float *>(base + o1) = bh;
-    *reinterpret_cast<float *>(base + bp + o0) = al;
-    *reinterpret_cast<float *>(base + bp + o1) = bl;
-  }
+  const uint32_t bp = sk_bpart(np);
+  unsigned char *base = zs + (size_t)(i >> 5) * 2 * bp;
+  const int j = i & 31;
+  const uint32_t o0 = sk_off(2 * p, j >> 2) + 4 * (j & 3);
+  const uint32_t o1 = sk_off(2 * p + 1, j >> 2) + 4 * (j & 3);
+  *reinterpret_cast<float *>(base + o0) = ah;
+  *reinterpret_cast<float *>(base + o1) = bh;
+  *reinterpret_cast<float *>(base + bp + o0) = al;
+  *reinterpret_cast<float *>(base + bp + o1) = bl;
 }
 
 // B tiles of the force pass, one step: thread per (tile, row r, 4
@@ -765,15 +745,13 @@ static int encode_xy_map(mdx_ctx *ctx, CUtensorMap *m, int box_atoms) {
   return MDX_OK;
 }
 
-// Z images of this step (after the phase tables), for whichever tensor-core
-// pass is on.
+// Z images of this step (after the phase tables) for the S pass when it is on.
 int tc_zimages_launch(mdx_ctx *ctx) {
   DevData &d = ctx->dv;
-  if (!d.tc_on && !d.tcs_on) return MDX_OK;
+  if (!d.tcs_on) return MDX_OK;
   const size_t nth = (size_t)d.kz * d.ldn;
-  k_zimages<<<(unsigned)((nth + 255) / 256), 256, 0, ctx->stream>>>(
-      d.ldn, d.kz, d.tc_kp, d.tcs_np, d.tabzf, d.tc_on ? d.tc_zimg : nullptr,
-      d.tcs_on ? d.tcs_zimg : nullptr);
+  k_zimages<<<(unsigned)((nth + 255) / 256), 256, 0, ctx->stream>>>(d.ldn, d.kz, d.tcs_np,
+                                                                    d.tabzf, d.tcs_zimg);
   MDX_LAUNCHED(ctx);
   return MDX_OK;
 }

@@ -19,26 +19,42 @@
 namespace {
 
 // ------------------------------------------------------------- zeroing ---
-__global__ void k_zero_scalars(mdx_scalars *sc, int which, int molint, int ntypes) {
-  int k = threadIdx.x;
-  if (k < molint) {
+// One block at the start of the force routines (FFORCES which & 1, SLFORCES
+// which & 2): their sums, SPE's self terms (ETERMS, forces.f:1497-1505) and
+// the statistics arrays.
+struct ZeroArgs {
+  mdx_scalars *sc;
+  int which, molint, ntypes, self;
+  double spei, speei[MDX_NT];
+  double *stat[3];
+  int nstat[3];
+};
+__global__ void k_zero_sums(ZeroArgs z) {
+  const int k = threadIdx.x;
+  mdx_scalars *sc = z.sc;
+  if (k < z.molint) {
     sc->pote1[k] = 0.0;
     sc->potl1[k] = 0.0;
   }
-  if (k < ntypes) {
+  if (k < z.ntypes) {
     sc->pes141[k] = 0.0;
     sc->psr141[k] = 0.0;
   }
-  if (k == 0) {
-    if (which == 1) {
-      sc->pels2 = 0.; sc->pint = 0.; sc->pe2 = 0.; sc->virb = 0.; sc->vir2 = 0.;
-      sc->wirss = 0.; sc->virfx = 0.; sc->virfy = 0.; sc->virfz = 0.;
-    } else {
-      sc->wirs = 0.; sc->vir1 = 0.; sc->pe1 = 0.; sc->pels1 = 0.;
-      sc->virx = 0.; sc->viry = 0.; sc->virz = 0.; sc->qpe = 0.;
-      sc->lscfl = 0;
-    }
+  if (k == 0 && (z.which & 1)) {
+    sc->pels2 = 0.; sc->pint = 0.; sc->pe2 = 0.; sc->virb = 0.; sc->vir2 = 0.;
+    sc->wirss = 0.; sc->virfx = 0.; sc->virfy = 0.; sc->virfz = 0.;
   }
+  if (k == 32 && (z.which & 2)) {
+    sc->wirs = 0.; sc->vir1 = 0.; sc->pe1 = 0.; sc->pels1 = 0.;
+    sc->virx = 0.; sc->viry = 0.; sc->virz = 0.; sc->qpe = 0.;
+    sc->lscfl = 0;
+  }
+  if (z.self) {
+    if (k == 64) sc->spe = z.spei;
+    if (k >= 96 && k < 96 + MDX_NT) sc->spee[k - 96] = k - 96 < z.ntypes ? z.speei[k - 96] : 0.0;
+  }
+  for (int a = 0; a < 3; ++a)
+    for (int i = k; i < z.nstat[a]; i += blockDim.x) z.stat[a][i] = 0.0;
 }
 
 __global__ void k_fix_fold(int n, const unsigned long long *__restrict__ f,
@@ -1737,28 +1753,32 @@ int launch_mstep1_rescale(mdx_ctx *ctx) {
   return scale_atoms(ctx, 1);
 }
 
-int launch_zero_fast(mdx_ctx *ctx) {
+// The mixed path's sweeps store every atom's fixed-point force first, so only
+// the FP64 path's force arrays (G and H adjacent) are cleared.
+int launch_zero(mdx_ctx *ctx, int which, int laver) {
   MDX_TIMER(ctx, MDX_T_OTHER);
   DevData &d = ctx->dv;
-  k_zero_scalars<<<1, 64, 0, ctx->stream>>>(d.sc, 1, ctx->p.molint, ctx->d.ntypes);
-  MDX_LAUNCHED(ctx);
-  if (ctx->mixed()) {
-    MDX_CUDA(cudaMemsetAsync(d.hfix, 0, sizeof(unsigned long long) * 3 * d.n, ctx->stream));
-  } else {
-    MDX_CUDA(cudaMemsetAsync(d.hx, 0, sizeof(double) * 3 * d.n, ctx->stream));
+  ZeroArgs z{};
+  z.sc = d.sc;
+  z.which = which;
+  z.molint = ctx->p.molint;
+  z.ntypes = ctx->d.ntypes;
+  z.self = (which & 2) && !ctx->p.lmnbl;
+  z.spei = ctx->spei;
+  for (int t = 0; t < MDX_NT; ++t) z.speei[t] = ctx->speei[t];
+  if (laver) {
+    z.stat[0] = d.br;
+    z.nstat[0] = 2 * d.nrbb;
+    z.stat[1] = d.ar;
+    z.nstat[1] = 2 * d.nraa;
+    z.stat[2] = d.tr;
+    z.nstat[2] = 2 * d.nrtt;
   }
-  return MDX_OK;
-}
-
-int launch_zero_slow(mdx_ctx *ctx) {
-  MDX_TIMER(ctx, MDX_T_OTHER);
-  DevData &d = ctx->dv;
-  k_zero_scalars<<<1, 64, 0, ctx->stream>>>(d.sc, 2, ctx->p.molint, ctx->d.ntypes);
+  k_zero_sums<<<1, 128, 0, ctx->stream>>>(z);
   MDX_LAUNCHED(ctx);
-  if (ctx->mixed()) {
-    MDX_CUDA(cudaMemsetAsync(d.gfix, 0, sizeof(unsigned long long) * 3 * d.n, ctx->stream));
-  } else {
-    MDX_CUDA(cudaMemsetAsync(d.gx, 0, sizeof(double) * 3 * d.n, ctx->stream));
+  if (!ctx->mixed()) {
+    const size_t b = sizeof(double) * 3 * d.n;
+    MDX_CUDA(cudaMemsetAsync(which & 2 ? d.gx : d.hx, 0, which == 3 ? 2 * b : b, ctx->stream));
   }
   return MDX_OK;
 }

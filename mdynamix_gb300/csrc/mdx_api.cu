@@ -189,8 +189,12 @@ int require(mdx_ctx *ctx, bool topo, bool par, bool state) {
 // ---------------------------------------------------------------- forces
 // mirrored: GETCOM has just refreshed the FP32 and fixed-point mirrors of the
 // positions.
+int fforces_parts(mdx_ctx *ctx, int laver, bool split, bool mirrored);
 int do_fforces(mdx_ctx *ctx, int laver, bool split, bool mirrored = false) {
-  RC(launch_zero_fast(ctx));
+  RC(launch_zero(ctx, 1, laver));
+  return fforces_parts(ctx, laver, split, mirrored);
+}
+int fforces_parts(mdx_ctx *ctx, int laver, bool split, bool mirrored) {
   if (ctx->mixed() && !mirrored) RC(launch_mirror_f32(ctx));
   RC(launch_localf(ctx, split));
   RC(launch_wir(ctx, 1));  // WIRSS from the pair forces, before the bonded terms
@@ -228,40 +232,53 @@ int do_fforces_mid(mdx_ctx *ctx, bool fold) {
   return MDX_OK;
 }
 
-int do_slow_parts(mdx_ctx *ctx, bool split, bool mirrored = false) {
+int do_slow_parts(mdx_ctx *ctx, bool split, bool mirrored = false, bool types = true) {
   if (ctx->mixed()) {
     if (!mirrored) RC(launch_mirror_f32(ctx));
-    RC(launch_forces_long(ctx, split));  // stores G first
+    RC(launch_forces_long(ctx, split, types));  // stores G first
     RC(launch_furir(ctx));
     RC(launch_eterms(ctx));
-    RC(launch_fix_to_double(ctx, 2));
+    RC(launch_fold_wirs(ctx));
   } else {
     RC(launch_furir(ctx));
     RC(launch_eterms(ctx));
-    RC(launch_forces_long(ctx, split));
+    RC(launch_forces_long(ctx, split, types));
+    RC(launch_wir(ctx, 2));
   }
   return MDX_OK;
 }
 
-int do_slforces(mdx_ctx *ctx, bool split, bool mirrored = false) {
-  RC(launch_zero_slow(ctx));
-  RC(do_slow_parts(ctx, split, mirrored));
-  RC(launch_wir(ctx, 2));
+int slforces_parts(mdx_ctx *ctx, bool split, bool mirrored, bool types = true) {
+  RC(do_slow_parts(ctx, split, mirrored, types));
   RC(launch_pullback(ctx));
   RC(launch_sclfrc(ctx, 2));
   return MDX_OK;
 }
 
+int do_slforces(mdx_ctx *ctx, bool split, bool mirrored = false) {
+  RC(furir_prepare(ctx));  // SPE's self terms are set with the zeroing
+  RC(launch_zero(ctx, 2));
+  return slforces_parts(ctx, split, mirrored);
+}
+
+// SLFORCES then FFORCES of a step's end (mirrored positions), their sums cleared
+// together; of the energies by type pair FFORCES leaves its own only.
+int do_both(mdx_ctx *ctx, int laver) {
+  RC(furir_prepare(ctx));
+  RC(launch_zero(ctx, 3, laver));
+  RC(slforces_parts(ctx, false, true, false));
+  return fforces_parts(ctx, laver, false, true);
+}
+
 int do_allforce(mdx_ctx *ctx, bool split, bool laver = false) {
-  RC(launch_zero_fast(ctx));
-  RC(launch_zero_slow(ctx));
+  RC(furir_prepare(ctx));
+  RC(launch_zero(ctx, 3, split || laver ? 1 : 0));
   if (ctx->mixed()) RC(launch_mirror_f32(ctx));
   RC(launch_localf(ctx, split));
   RC(launch_wir(ctx, 1));  // WIRSS from the pair forces, before the bonded terms
   RC(launch_bonded(ctx, split || laver ? 1 : 0));
   if (ctx->mixed()) RC(launch_fix_to_double(ctx, 1));
   RC(do_slow_parts(ctx, split));
-  RC(launch_wir(ctx, 2));
   RC(launch_sum_forces(ctx));
   // PULLBACK adds to G after CM_ADDLA has formed F (forces.f:88-95): SULTAN,
   // which moves with F, does not see it -- the reference's order, kept
@@ -299,10 +316,9 @@ int double_step(mdx_ctx *ctx, int mstep, int slot) {
     RC(launch_kick_drift_com(ctx, HTSTEB, TSTEB, s > 1 ? 1 : 0, keep_fix && s > 1, s < NFREQ));
     if (s == NFREQ2) RC(launch_list_update(ctx, mstep));
     if (s == NFREQ) {
-      RC(do_slforces(ctx, false, true));
       // the bonded statistics of the step (GETBND..GETTRS form them at every
       // FFORCES, forces.f:113-513) when averages are kept on the device
-      RC(do_fforces(ctx, ctx->averaging ? 1 : 0, false, true));
+      RC(do_both(ctx, ctx->averaging ? 1 : 0));
       if (ctx->averaging) RC(launch_acc_bonded(ctx));
     } else {
       RC(do_fforces_mid(ctx, !keep_fix));
@@ -1674,6 +1690,7 @@ int api_copy_scalars(mdx_ctx *ctx, mdx_scalars *out) { return copy_scalars(ctx, 
 int api_do_slforces(mdx_ctx *ctx, bool split, bool mirrored) {
   return do_slforces(ctx, split, mirrored);
 }
+int api_do_both(mdx_ctx *ctx, int laver) { return do_both(ctx, laver); }
 int api_do_fforces(mdx_ctx *ctx, int laver, bool split, bool mirrored) {
   return do_fforces(ctx, laver, split, mirrored);
 }

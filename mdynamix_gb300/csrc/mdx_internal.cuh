@@ -770,15 +770,17 @@ int export_lists(mdx_ctx *ctx, int32_t *nbs1, int32_t *nbs2, int32_t cap_s,
 // pair.cu
 int launch_localf(mdx_ctx *ctx, bool split, bool ener = true, bool add = false);
 int pack_lj_tables(mdx_ctx *ctx);  // abf from the FP32 tables
-int launch_forces_long(mdx_ctx *ctx, bool split);
+// types = false: the type pair's energies of a one-type system are not kept
+int launch_forces_long(mdx_ctx *ctx, bool split, bool types = true);
 // pair64.cu
 int pair64_setup(mdx_ctx *ctx);
 int launch_pair64(mdx_ctx *ctx, bool shrt, bool split, bool ener, double *split_buf);
 int launch_wir(mdx_ctx *ctx, int which);  // WIRSS (1) / WIRS (2)
 // ewald.cu
 int host_inifur(mdx_ctx *ctx);
+int furir_prepare(mdx_ctx *ctx);  // k-set check (host), INIFUR when due
 int launch_furir(mdx_ctx *ctx);
-int furir_sfac(mdx_ctx *ctx, bool *skip);  // k-set check, phase tables, S(k) into d.sk
+int furir_sfac(mdx_ctx *ctx, bool *skip, bool terms = false);  // k-set check, phase tables, S(k) into d.sk
 int ensure_kconst(mdx_ctx *ctx);           // per-k constants of the current box
 int launch_eterms(mdx_ctx *ctx);
 int sfac_slices(const mdx_ctx *ctx);  // slices of the S(k) partial sums
@@ -809,13 +811,16 @@ int api_check_err(mdx_ctx *ctx);
 int api_copy_scalars(mdx_ctx *ctx, mdx_scalars *out);
 int api_do_slforces(mdx_ctx *ctx, bool split, bool mirrored = false);
 int api_do_fforces(mdx_ctx *ctx, int laver, bool split, bool mirrored = false);
+int api_do_both(mdx_ctx *ctx, int laver);  // SLFORCES and FFORCES, mirrored positions
 // bonded.cu: running sums of the per-record bonded statistics
 int launch_acc_bonded(mdx_ctx *ctx);
 int bonded_sums_len(const mdx_ctx *ctx);
 // integrate.cu
-int launch_zero_fast(mdx_ctx *ctx);
-int launch_zero_slow(mdx_ctx *ctx);
+// Start of FFORCES (which & 1) and SLFORCES (which & 2): scalars, forces, SPE's
+// self terms, the bonded statistics (laver)
+int launch_zero(mdx_ctx *ctx, int which, int laver = 0);
 int launch_fix_to_double(mdx_ctx *ctx, int which);  // mixed: int64 -> G/H
+int launch_fold_wirs(mdx_ctx *ctx);                 // mixed: int64 -> G, WIRS
 int launch_sclfrc(mdx_ctx *ctx, int nnn);
 int launch_sum_forces(mdx_ctx *ctx);                // F = G + H
 int launch_pullback(mdx_ctx *ctx);                  // PULLBACK into G

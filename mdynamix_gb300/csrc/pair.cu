@@ -57,6 +57,29 @@ __global__ void k_wir(int n, const dbl4 *__restrict__ pos,
   block_add<1>(w, dst);
 }
 
+// End of the mixed path's SLFORCES: G from its fixed-point sums, and WIRS of
+// it in the same pass.
+__global__ void k_fold_wirs(int n, const dbl4 *__restrict__ pos, const int4 *__restrict__ ainfo,
+                            const double *__restrict__ X, const double *__restrict__ Y,
+                            const double *__restrict__ Z,
+                            const unsigned long long *__restrict__ f, double inv,
+                            double *__restrict__ gx, double *__restrict__ gy,
+                            double *__restrict__ gz, Dst6 dst) {
+  double w[1] = {0.0};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const dbl4 p = pos[i];
+    const int m = ainfo[i].y;
+    const double fx = (double)(long long)f[i] * inv;
+    const double fy = (double)(long long)f[n + i] * inv;
+    const double fz = (double)(long long)f[2 * n + i] * inv;
+    gx[i] = fx;
+    gy[i] = fy;
+    gz[i] = fz;
+    w[0] = w[0] - fx * (p.x - X[m]) - fy * (p.y - Y[m]) - fz * (p.z - Z[m]);
+  }
+  block_add<1>(w, dst);
+}
+
 // WIRSS on the mixed path: the short-row sweep has just stored the pair
 // forces as fixed point; the bonded terms have not been added yet.
 __global__ void k_wir_fix(int n, const dbl4 *__restrict__ pos,
@@ -149,6 +172,74 @@ __device__ __forceinline__ void split_out(const SplitF &a, double *sh, double *s
     if (sh[k] != 0.0) atomicAdd(&split[k], 0.5 * sh[k]);
 }
 
+// Where a sweep's integer slots go: the last block to finish folds them into
+// mdx_scalars (full rows count each pair twice, hence the 1/2 on pair sums)
+// and clears them for the next sweep.
+struct SlotFold {
+  unsigned long long *slots;
+  unsigned *ctr;
+  mdx_scalars *sc;
+  double einv;
+  int which, one_type;  // 1 LOCALF, 2 FORCES; one_type: keep the single type pair's energies
+};
+__device__ __forceinline__ void fold_slot(const SlotFold &f, int k) {
+  double v = (double)(long long)atomicExch(&f.slots[k], 0ull) * f.einv;
+  mdx_scalars *sc = f.sc;
+  const bool s = f.which == 1;
+  v *= 0.5;
+  double *dst = nullptr;
+  switch (k) {
+    case P_EES: dst = s ? &sc->pels2 : &sc->pels1; break;
+    case P_ESR: dst = s ? &sc->pe2 : &sc->pe1; break;
+    case P_VIR: dst = s ? &sc->vir2 : &sc->vir1; break;
+    case P_VX: dst = s ? &sc->virfx : &sc->virx; break;
+    case P_VY: dst = s ? &sc->virfy : &sc->viry; break;
+    case P_VZ: dst = s ? &sc->virfz : &sc->virz; break;
+    case P_EE_DIFF: dst = f.one_type ? &sc->pote1[0] : nullptr; break;
+    case P_ESR_DIFF: dst = f.one_type ? &sc->potl1[0] : nullptr; break;
+    case P_EE_SAME: dst = f.one_type ? &sc->pes141[0] : nullptr; break;
+    case P_ESR_SAME: dst = f.one_type ? &sc->psr141[0] : nullptr; break;
+  }
+  if (dst) atomicAdd(dst, v);
+}
+
+// Block sum of a sweep's integer energy/virial slots: warp sums of the lane
+// partials, fixed point, one atomic per slot per block; then the fold.
+__device__ __forceinline__ void slots_out(const float (&a)[P_NSLOT], float escalef,
+                                          const SlotFold &f) {
+  const int lane = threadIdx.x & 31;
+  long long tot[P_WIR];
+#pragma unroll
+  for (int k = 0; k < P_WIR; ++k) {
+    const float t = warp_sumf(a[k]);
+    tot[k] = lane == 0 ? f2ll_rn(t * escalef) : 0;
+  }
+  __shared__ long long sh[8][P_WIR];
+  const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (lane == 0) {
+#pragma unroll
+    for (int k = 0; k < P_WIR; ++k) sh[wid][k] = tot[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < P_WIR) {
+    long long s = 0;
+    for (int w = 0; w < nw; ++w) s += sh[w][threadIdx.x];
+    if (s != 0) atomicAdd(&f.slots[threadIdx.x], (unsigned long long)s);
+    __threadfence();
+  }
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(f.ctr, 1u) == gridDim.x - 1;
+    if (last) *f.ctr = 0u;
+  }
+  __syncthreads();
+  if (last && threadIdx.x < P_WIR) {
+    __threadfence();
+    fold_slot(f, threadIdx.x);
+  }
+}
+
 __device__ __forceinline__ float idiff(int a, int b, float s) { return fixdiff(a, b, s); }
 
 // Register cap for occupancy: the sweeps wait on gathered neighbour records,
@@ -163,7 +254,7 @@ __global__ void __launch_bounds__(256, PAIR32_BLOCKS) k_pair32(
     FixScale fsc, unsigned long long *__restrict__ ffix,
     const double *__restrict__ X, const double *__restrict__ Y,
     const double *__restrict__ Z, double escale,
-    unsigned long long *__restrict__ slots, double *__restrict__ split,
+    SlotFold sf, double *__restrict__ split,
     const int *__restrict__ owner_of, CellF cf, bool add) {
   __shared__ double s_split[SPLIT ? SPLIT_N : 1];
   SplitF spl{-1, 0.f, 0.f, 0.f, 0.f};
@@ -184,9 +275,6 @@ __global__ void __launch_bounds__(256, PAIR32_BLOCKS) k_pair32(
   const int sl = (blockIdx.x * blockDim.x + threadIdx.x) / TPO;
   const int i = owner_of && sl < n ? owner_of[sl] : sl;
   const int k0 = lane % TPO, kstep = TPO;
-  long long tot[P_NSLOT];
-#pragma unroll
-  for (int k = 0; k < P_NSLOT; ++k) tot[k] = 0;
   float a[P_NSLOT];
 #pragma unroll
   for (int k = 0; k < P_NSLOT; ++k) a[k] = 0.f;
@@ -340,28 +428,8 @@ __global__ void __launch_bounds__(256, PAIR32_BLOCKS) k_pair32(
     qz += __shfl_xor_sync(0xffffffffu, qz, o);
   }
   if (i < n && lane % TPO == 0) owner_store(ffix, n, i, qx, qy, qz, SHORT && !ENER && add);
-  if (ENER) {
-#pragma unroll
-    for (int k = 0; k < P_WIR; ++k) {
-      float t = warp_sumf(a[k]);
-      if (lane == 0) tot[k] = f2ll_rn(t * fsc.escalef);
-    }
-  }
   if (SPLIT) split_out(spl, s_split, split);
-  if (!ENER) return;  // forces only: no energy or virial slots
-  // block sum of the integer slots, one atomic per slot per block
-  __shared__ long long sh[8][P_NSLOT];
-  const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < P_NSLOT; ++k) sh[wid][k] = tot[k];
-  }
-  __syncthreads();
-  if (threadIdx.x < P_NSLOT) {
-    long long s = 0;
-    for (int w = 0; w < nw; ++w) s += sh[w][threadIdx.x];
-    if (s != 0) atomicAdd(&slots[threadIdx.x], (unsigned long long)s);
-  }
+  if (ENER) slots_out(a, fsc.escalef, sf);
 }
 
 // ------------------------------------------------------- mixed, paired ---
@@ -462,31 +530,6 @@ __device__ __forceinline__ void pair_same(float DX, float DY, float DZ, bool is1
   s.fz.x += FORCE * DZ;
 }
 
-// Block sum of a sweep's integer energy/virial slots: warp sums of the lane
-// partials, fixed point, one atomic per slot per block.
-__device__ __forceinline__ void slots_out(const float (&a)[P_NSLOT], float escalef,
-                                          unsigned long long *__restrict__ slots) {
-  const int lane = threadIdx.x & 31;
-  long long tot[P_WIR];
-#pragma unroll
-  for (int k = 0; k < P_WIR; ++k) {
-    const float t = warp_sumf(a[k]);
-    tot[k] = lane == 0 ? f2ll_rn(t * escalef) : 0;
-  }
-  __shared__ long long sh[8][P_WIR];
-  const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < P_WIR; ++k) sh[wid][k] = tot[k];
-  }
-  __syncthreads();
-  if (threadIdx.x < P_WIR) {
-    long long s = 0;
-    for (int w = 0; w < nw; ++w) s += sh[w][threadIdx.x];
-    if (s != 0) atomicAdd(&slots[threadIdx.x], (unsigned long long)s);
-  }
-}
-
 template <bool SHORT, bool SPLIT, bool ENER, int TPO, bool CELL>
 __global__ void __launch_bounds__(256, SPLIT ? 3 : (SHORT && !ENER) ? PAIR32X2_BLOCKS_SHORT
                                                                     : PAIR32X2_BLOCKS)
@@ -495,7 +538,7 @@ k_pair32x2(
     const float4 *__restrict__ stab, const int *__restrict__ cnt, const int *__restrict__ idx,
     int cap, PairTables tb, TypeConst tc, PairConst pc, float sx, float sy, float sz,
     FixScale fsc, unsigned long long *__restrict__ ffix,
-    unsigned long long *__restrict__ slots, double *__restrict__ split,
+    SlotFold sf, double *__restrict__ split,
     const int *__restrict__ owner_of, CellF cf, bool add) {
   __shared__ double s_split[SPLIT ? SPLIT_N : 1];
   SplitF spl{-1, 0.f, 0.f, 0.f, 0.f};
@@ -736,36 +779,7 @@ k_pair32x2(
   a[P_ESR_SAME] = s.esr_same;
   a[P_ESR_DIFF] = esr - s.esr_same;
   a[P_WIR] = 0.f;
-  slots_out(a, fsc.escalef, slots);
-}
-
-// Fold the integer slots of a mixed sweep into mdx_scalars (full rows count
-// each pair twice, hence the 1/2 on pair sums).
-__global__ void k_fold_slots(unsigned long long *__restrict__ slots, double einv,
-                             mdx_scalars *__restrict__ sc, int which, int ntypes,
-                             int split) {
-  // thread k folds slot k into its own scalar (the slots' sums are
-  // independent): one conversion deep instead of P_NSLOT in a row
-  const int k = threadIdx.x;
-  if (k >= P_NSLOT) return;
-  double v = (double)(long long)slots[k] * einv;
-  slots[k] = 0ull;
-  if (k < P_WIR) v *= 0.5;
-  double *dst = nullptr;
-  switch (k) {
-    case P_EES: dst = which == 1 ? &sc->pels2 : &sc->pels1; break;
-    case P_ESR: dst = which == 1 ? &sc->pe2 : &sc->pe1; break;
-    case P_VIR: dst = which == 1 ? &sc->vir2 : &sc->vir1; break;
-    case P_VX: dst = which == 1 ? &sc->virfx : &sc->virx; break;
-    case P_VY: dst = which == 1 ? &sc->virfy : &sc->viry; break;
-    case P_VZ: dst = which == 1 ? &sc->virfz : &sc->virz; break;
-    case P_WIR: dst = which == 1 ? &sc->wirss : nullptr; break;
-    case P_EE_DIFF: dst = ntypes == 1 && !split ? &sc->pote1[0] : nullptr; break;
-    case P_ESR_DIFF: dst = ntypes == 1 && !split ? &sc->potl1[0] : nullptr; break;
-    case P_EE_SAME: dst = ntypes == 1 && !split ? &sc->pes141[0] : nullptr; break;
-    case P_ESR_SAME: dst = ntypes == 1 && !split ? &sc->psr141[0] : nullptr; break;
-  }
-  if (dst) *dst += v;
+  slots_out(a, fsc.escalef, sf);
 }
 
 // Copy the split accumulators (POTE1, POTL1, PES141, PSR141) out.
@@ -808,7 +822,7 @@ __global__ void k_pack_lj(int nn, const float *__restrict__ f, float2 *__restric
 // ener = false: forces only (an intermediate short step of DOUBLE, whose fast
 // energies and virials are zeroed again by the next FFORCES before anything
 // reads them, forces.f:36-49).
-int launch_pair(mdx_ctx *ctx, bool shrt, bool split, bool ener, bool add = false) {
+int launch_pair(mdx_ctx *ctx, bool shrt, bool split, bool ener, bool add, bool types) {
   DevData &d = ctx->dv;
   if (ctx->mixed() && !ctx->tune.tpo_short) resolve_tuning(ctx);
   const int T = 256;
@@ -821,7 +835,13 @@ int launch_pair(mdx_ctx *ctx, bool shrt, bool split, bool ener, bool add = false
     if (rc) return rc;
   } else {
     unsigned long long *ffix = shrt ? d.hfix : d.gfix;
-    unsigned long long *slots = reinterpret_cast<unsigned long long *>(d.red);
+    SlotFold sf;
+    sf.slots = reinterpret_cast<unsigned long long *>(d.red) + (shrt ? 0 : 16);
+    sf.ctr = d.red_ctr + 4;
+    sf.sc = d.sc;
+    sf.einv = 1.0 / ctx->fix.escale;
+    sf.which = shrt ? 1 : 2;
+    sf.one_type = ctx->d.ntypes == 1 && !split && types;
     const double sxs = ctx->boxl / 4294967296.0, sys = fix_period_y(ctx) / 4294967296.0,
                  szs = ctx->bozl / 4294967296.0;
     const double escale = ctx->fix.escale;
@@ -834,17 +854,17 @@ int launch_pair(mdx_ctx *ctx, bool shrt, bool split, bool ener, bool add = false
                  (float)(0.5 / (double)0.8660254037844386f)};
     }
     // threads per owner atom: the context's tuning
-    const int tpo = shrt ? ctx->tune.tpo_short : ctx->tune.tpo_long;
+    const int tpo = !shrt ? ctx->tune.tpo_long : split ? TPO_SHORT_DEFAULT : ctx->tune.tpo_short;
     const int grid32 = (int)(((long long)tpo * d.n + T - 1) / T);
 #define LP32(S, P, E, K)                                                          \
   k_pair32<S, P, E, K><<<grid32, T, 0, ctx->stream>>>(                            \
       d.n, d.posi, d.cell_pos, d.stab, cnt, idx, cap, tables(d),                 \
       ctx->tc, ctx->pc, (float)sxs, (float)sys, (float)szs, ctx->fix, ffix, d.X,  \
-      d.Y, d.Z, escale, slots, split_buf, S ? nullptr : d.cell_list, cf, add)
+      d.Y, d.Z, escale, sf, split_buf, S ? nullptr : d.cell_list, cf, add)
 #define LP32X2C(S, P, E, K, C)                                                    \
   k_pair32x2<S, P, E, K, C><<<grid32, T, 0, ctx->stream>>>(                       \
       d.n, d.posi, d.cell_pos, d.stab, cnt, idx, cap, tables(d), ctx->tc, ctx->pc, \
-      (float)sxs, (float)sys, (float)szs, ctx->fix, ffix, slots, split_buf,       \
+      (float)sxs, (float)sys, (float)szs, ctx->fix, ffix, sf, split_buf,       \
       S ? nullptr : d.cell_list, cf, add)
 #define LP32X2(S, P, E, K)                     \
   do {                                         \
@@ -853,19 +873,25 @@ int launch_pair(mdx_ctx *ctx, bool shrt, bool split, bool ener, bool add = false
   } while (0)
     // the paired sweeps cover Ewald without MDEE's shifted Coulomb
     const bool paired = !ctx->pc.lmnbl && !ctx->pc.lmdee;
-    // the force calls' energies by type pair come with energies
-#define LP32E(S, K)                            \
-  do {                                         \
-    if (paired) {                              \
-      if (split) LP32X2(S, true, true, K);     \
-      else if (ener) LP32X2(S, false, true, K); \
-      else LP32X2(S, false, false, K);         \
-    } else if (split) LP32(S, true, true, K);  \
-    else if (ener) LP32(S, false, true, K);    \
-    else LP32(S, false, false, K);             \
+    // The force calls' energies by type pair come with energies.  Their short
+    // sweep takes one entry at a time, by TPO_SHORT_DEFAULT lanes whatever the
+    // tuning: PELS2 of 203 randomly turned waters is 1/450 of the sum of its
+    // terms' magnitudes, FP32 rounding is 3e-6 of it in any order (rms over 24
+    // boxes: 3.5e-6 one at a time, 2.9e-6 paired), so the order is kept.
+#define LP32E(S, K)                              \
+  do {                                           \
+    if (!S && split) {                           \
+      if (paired) LP32X2(false, true, true, K);  \
+      else LP32(false, true, true, K);           \
+    } else if (paired) {                         \
+      if (ener) LP32X2(S, false, true, K);       \
+      else LP32X2(S, false, false, K);           \
+    } else if (ener) LP32(S, false, true, K);    \
+    else LP32(S, false, false, K);               \
   } while (0)
     if (shrt) {
-      if (tpo == 2) LP32E(true, 2);
+      if (split) LP32(true, true, true, TPO_SHORT_DEFAULT);
+      else if (tpo == 2) LP32E(true, 2);
       else if (tpo == 8) LP32E(true, 8);
       else LP32E(true, 4);
     } else {
@@ -879,11 +905,6 @@ int launch_pair(mdx_ctx *ctx, bool shrt, bool split, bool ener, bool add = false
 #undef LP32X2C
 #undef LP32
     MDX_LAUNCHED(ctx);
-    if (ener) {
-      k_fold_slots<<<1, 32, 0, ctx->stream>>>(slots, 1.0 / escale, d.sc, shrt ? 1 : 2,
-                                              ctx->d.ntypes, split ? 1 : 0);
-      MDX_LAUNCHED(ctx);
-    }
   }
   if (split) {
     k_fold_split<<<1, 64, 0, ctx->stream>>>(split_buf, d.sc);
@@ -944,9 +965,20 @@ int pack_lj_tables(mdx_ctx *ctx) {
 
 
 int launch_localf(mdx_ctx *ctx, bool split, bool ener, bool add) {
-  MDX_TIMER(ctx, MDX_T_PAIR_SHORT); return launch_pair(ctx, true, split, ener, add); }
-int launch_forces_long(mdx_ctx *ctx, bool split) {
-  MDX_TIMER(ctx, MDX_T_PAIR_LONG); return launch_pair(ctx, false, split, true); }
+  MDX_TIMER(ctx, MDX_T_PAIR_SHORT); return launch_pair(ctx, true, split, ener, add, true); }
+int launch_forces_long(mdx_ctx *ctx, bool split, bool types) {
+  MDX_TIMER(ctx, MDX_T_PAIR_LONG); return launch_pair(ctx, false, split, true, false, types); }
+
+int launch_fold_wirs(mdx_ctx *ctx) {
+  MDX_TIMER(ctx, MDX_T_OTHER);
+  DevData &d = ctx->dv;
+  const int nb = red_blocks(ctx);
+  k_fold_wirs<<<nb, 256, 0, ctx->stream>>>(d.n, d.pos, d.ainfo, d.X, d.Y, d.Z, d.gfix,
+                                           ctx->fix.inv, d.gx, d.gy, d.gz,
+                                           dst6(ctx, nb, 1, &d.sc->wirs));
+  MDX_LAUNCHED(ctx);
+  return MDX_OK;
+}
 
 int launch_wir(mdx_ctx *ctx, int which) {
   MDX_TIMER(ctx, MDX_T_OTHER);

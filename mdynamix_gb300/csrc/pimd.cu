@@ -313,8 +313,7 @@ int long_step(mdx_pimd *pi, int mstep) {
     RC(fork(pi));
     EACH_BEAD(if (s == NFREQ2) RC(launch_list_update(ctx, mstep));
               if (s == NFREQ) {
-                RC(api_do_slforces(ctx, false, true));
-                RC(api_do_fforces(ctx, 1, false, true));
+                RC(api_do_both(ctx, 1));
               } else {
                 RC(api_do_fforces(ctx, 0, false, true));
               });
