@@ -746,8 +746,19 @@ inline cudaError_t ctx_alloc(mdx_ctx *ctx, void **p, size_t bytes) {
 // (device-to-host reads see their results) and complete on return (host
 // buffers may go away).  The contexts' streams are non-blocking, so a plain
 // cudaMemcpy / cudaMemset on the legacy default stream would race with them.
+//
+// Host memory that no one has written yet has no pages, and a copy into it
+// makes the GPU fault them in one by one: three arrays of 98,304 doubles took
+// 1.5 - 2.4 ms that way, 0.075 ms once their pages were there.  So the host
+// touches the pages first (adding 0: the contents stay as they are).
+inline void touch_pages(void *dst, size_t bytes) {
+  char *p = static_cast<char *>(dst);
+  for (size_t o = 0; o < bytes; o += 4096) __atomic_fetch_add(p + o, 0, __ATOMIC_RELAXED);
+  __atomic_fetch_add(p + bytes - 1, 0, __ATOMIC_RELAXED);
+}
 inline cudaError_t ctx_copy(cudaStream_t s, void *dst, const void *src, size_t bytes,
                             cudaMemcpyKind kind) {
+  if (kind == cudaMemcpyDeviceToHost && bytes >= 65536) touch_pages(dst, bytes);
   cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   return e;
