@@ -67,6 +67,17 @@ __global__ void k_fix_fold(int n, const unsigned long long *__restrict__ f,
   z[i] = (double)(long long)f[2 * n + i] * inv;
 }
 
+__global__ void k_fix_add(int n, unsigned long long *__restrict__ f, double unit,
+                          double *__restrict__ x, double *__restrict__ y,
+                          double *__restrict__ z) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  x[i] = fma((double)(long long)f[i], unit, x[i]);
+  y[i] = fma((double)(long long)f[n + i], unit, y[i]);
+  z[i] = fma((double)(long long)f[2 * n + i], unit, z[i]);
+  f[i] = f[n + i] = f[2 * n + i] = 0ull;
+}
+
 // SCLFRC (service.f:182-287)
 __global__ void k_sclfrc(int n, double fct, const double *__restrict__ massdi,
                          double *x, double *y, double *z, mdx_scalars *sc) {
@@ -272,7 +283,7 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
                                  const int4 *__restrict__ ainfo, MoveConst mv,
                                  MolConst mc, double htsteb, double tsteb, int prev,
                                  const double *hx, const double *hy, const double *hz,
-                                 const unsigned long long *hfix, int n,
+                                 unsigned long long *hfix, int n,
                                  double inv, const double *__restrict__ massdi,
                                  const double *__restrict__ amass, double *__restrict__ vx,
                                  double *__restrict__ vy, double *__restrict__ vz,
@@ -281,12 +292,14 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
                                  double bx, double by, double bz, double3 ibs,
                                  int4 *__restrict__ posi, const int *__restrict__ pinfo,
                                  int4 *__restrict__ posc, const int *__restrict__ slot_of,
-                                 unsigned long long *zero) {
+                                 unsigned long long *zero, const IPosOut ip) {
   // ibs: 2^32 / box per axis (host-computed: no FP64 division per thread);
   // posi set (mixed path): centre of mass by the reciprocal mass, the
   // fixed-point mirror refreshed, and (posc set) its cell-order copy.
   // zero set: the atom's fast forces (3 words, stride n: hfix, or hx..hz)
-  // are cleared once read, for an FFORCES whose parts all add to them
+  // are cleared once read, for an FFORCES whose parts all add to them.
+  // FP64 path: hfix set, the sweep's fixed-point sums to be added to H (unit
+  // inv; cleared once read); ip, where the positions go as integers.
   const int m = ml.m, f = mol_first[m], na = ml.live ? mol_nat[m] : 0;
   if (ml.g == 1 && posi && na <= KD_MAXA) {
     if (!ml.live) return;
@@ -388,7 +401,12 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
         p.y = fma(v, tm, p.y);
         p.z = fma(w, tm, p.z);
       } else {
-        const double fx = hx[i], fy = hy[i], fz = hz[i];
+        double fx = hx[i], fy = hy[i], fz = hz[i];
+        if (hfix) {
+          fx = fma((double)(long long)hfix[i], inv, fx);
+          fy = fma((double)(long long)hfix[n + i], inv, fy);
+          fz = fma((double)(long long)hfix[2 * n + i], inv, fz);
+        }
         if (prev) {
           u = u + htsteb * fx;
           v = v + htsteb * fy;
@@ -405,6 +423,7 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
       vy[i] = v;
       vz[i] = w;
     }
+    if (hfix && !posi) hfix[i] = hfix[n + i] = hfix[2 * n + i] = 0ull;
     if (zero) zero[i] = zero[n + i] = zero[2 * n + i] = 0ull;
     if (k == ml.k) p0 = p;
     else pos[i] = p;
@@ -443,6 +462,7 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
       p.z = (p.z - z) + zw;
     }
     pos[f + k] = p;
+    if (ip.p) ipos_store(ip, f + k, p);
     if (posi) {
       const int4 q = make_int4(fix32_rn(__dmul_rn(p.x, ibs.x)), fix32_rn(__dmul_rn(p.y, ibs.y)),
                                fix32_rn(__dmul_rn(p.z, ibs.z)), pinfo[f + k]);
@@ -458,7 +478,7 @@ __global__ void k_kick_drift_com(MolLanes L, const int *__restrict__ mol_first,
                                  const int4 *__restrict__ ainfo, MoveConst mv,
                                  MolConst mc, double htsteb, double tsteb, int prev,
                                  const double *hx, const double *hy, const double *hz,
-                                 const unsigned long long *hfix, int n,
+                                 unsigned long long *hfix, int n,
                                  double inv, const double *__restrict__ massdi,
                                  const double *__restrict__ amass, double *__restrict__ vx,
                                  double *__restrict__ vy, double *__restrict__ vz,
@@ -467,11 +487,11 @@ __global__ void k_kick_drift_com(MolLanes L, const int *__restrict__ mol_first,
                                  double bx, double by, double bz, double3 ibs,
                                  int4 *__restrict__ posi, const int *__restrict__ pinfo,
                                  int4 *__restrict__ posc, const int *__restrict__ slot_of,
-                                 unsigned long long *zero) {
+                                 unsigned long long *zero, const IPosOut ip) {
   kick_drift_com_body(mol_lane(L), mol_first, mol_nat, mol_type,
                       ainfo, mv, mc, htsteb, tsteb, prev, hx, hy, hz, hfix, n, inv, massdi,
                       amass, vx, vy, vz, pos, X, Y, Z, bx, by, bz, ibs, posi, pinfo, posc,
-                      slot_of, zero);
+                      slot_of, zero, ip);
 }
 
 // SULTAN 1.3.1-1.3.2.2 (mdstep.f:89-113): OX = SX, V += TSTEP F,
@@ -997,6 +1017,7 @@ struct BeadMove {
   double *X, *Y, *Z;
   int4 *posi, *posc;
   const int *slot_of;
+  IPosOut ip;
   double *part;
   unsigned *ctr;
   ScalScratch *ss;
@@ -1589,7 +1610,7 @@ __global__ void k_kick_drift_com_beads(MolLanes L, const int *__restrict__ mol_f
   kick_drift_com_body(mol_lane(L), mol_first, mol_nat, mol_type,
                       ainfo, mv, mc, htsteb, tsteb, 0, b.f[0][0], b.f[0][1], b.f[0][2], nullptr,
                       n, 0.0, massdi, amass, b.vx, b.vy, b.vz, b.pos, b.X, b.Y, b.Z, bx, by, bz,
-                      ibs, b.posi, pinfo, b.posc, b.slot_of, nullptr);
+                      ibs, b.posi, pinfo, b.posc, b.slot_of, nullptr, b.ip);
 }
 
 static KickArgs kick_args(mdx_ctx *ctx, const KickSpec &k) {
@@ -1786,10 +1807,14 @@ int launch_zero(mdx_ctx *ctx, int which, int laver) {
 int launch_fix_to_double(mdx_ctx *ctx, int which) {
   MDX_TIMER(ctx, MDX_T_OTHER);
   DevData &d = ctx->dv;
-  const unsigned long long *f = which == 1 ? d.hfix : d.gfix;
+  unsigned long long *f = which == 1 ? d.hfix : d.gfix;
   double *x = which == 1 ? d.hx : d.gx, *y = which == 1 ? d.hy : d.gy,
          *z = which == 1 ? d.hz : d.gz;
-  k_fix_fold<<<(d.n + 255) / 256, 256, 0, ctx->stream>>>(d.n, f, ctx->fix.inv, x, y, z);
+  if (ctx->mixed())
+    k_fix_fold<<<(d.n + 255) / 256, 256, 0, ctx->stream>>>(d.n, f, ctx->fix.inv, x, y, z);
+  else
+    k_fix_add<<<(d.n + 255) / 256, 256, 0, ctx->stream>>>(d.n, f, px_force_unit(ctx, which), x, y,
+                                                          z);
   MDX_LAUNCHED(ctx);
   return MDX_OK;
 }
@@ -1948,12 +1973,14 @@ int launch_kick_drift_com(mdx_ctx *ctx, double htsteb, double tsteb, int prev, b
   const MolLanes L = mol_lanes(ctx, 32);
   k_kick_drift_com<<<L.blk[L.nt], 32, 0, ctx->stream>>>(
       L, d.mol_first, d.mol_nat, d.mol_type, d.ainfo, move_const(ctx), mol_const(ctx),
-      htsteb, tsteb, prev, d.hx, d.hy, d.hz, from_fix ? d.hfix : nullptr, d.n, ctx->fix.inv,
+      htsteb, tsteb, prev, d.hx, d.hy, d.hz, from_fix ? d.hfix : nullptr, d.n,
+      ctx->mixed() ? ctx->fix.inv : px_force_unit(ctx, 1),
       d.massdi, d.amass, d.vx, d.vy, d.vz, d.pos, d.X, d.Y, d.Z, ctx->boxl, ctx->boyl,
       ctx->bozl, fix_scale3(ctx), ctx->mixed() ? d.posi : nullptr, d.pinfo,
       ctx->mixed() && ctx->have_lists ? d.cell_pos : nullptr, d.slot_of,
       !zero_fast ? nullptr
-      : ctx->mixed() ? d.hfix : reinterpret_cast<unsigned long long *>(d.hx));
+      : ctx->mixed() ? d.hfix : reinterpret_cast<unsigned long long *>(d.hx),
+      ipos_out(ctx));
   MDX_LAUNCHED(ctx);
   return MDX_OK;
 }
@@ -1979,6 +2006,7 @@ void bead_move_fill(mdx_ctx *ctx, void *out) {
   b.posi = ctx->mixed() ? d.posi : nullptr;
   b.posc = ctx->mixed() && ctx->have_lists ? d.cell_pos : nullptr;
   b.slot_of = d.slot_of;
+  b.ip = ipos_out(ctx);
   b.part = d.red_part;
   b.ctr = d.red_ctr;
   b.ss = reinterpret_cast<ScalScratch *>(d.scal_scratch);

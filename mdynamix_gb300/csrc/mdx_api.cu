@@ -195,7 +195,7 @@ int do_fforces(mdx_ctx *ctx, int laver, bool split, bool mirrored = false) {
   return fforces_parts(ctx, laver, split, mirrored);
 }
 int fforces_parts(mdx_ctx *ctx, int laver, bool split, bool mirrored) {
-  if (ctx->mixed() && !mirrored) RC(launch_mirror_f32(ctx));
+  if (!mirrored) RC(ctx->mixed() ? launch_mirror_f32(ctx) : launch_ipos(ctx));
   RC(launch_localf(ctx, split));
   RC(launch_wir(ctx, 1));  // WIRSS from the pair forces, before the bonded terms
   RC(launch_bonded(ctx, laver));
@@ -227,7 +227,7 @@ int do_fforces_mid(mdx_ctx *ctx, bool fold) {
     RC(launch_localf(ctx, false, false, true));
     RC(launch_bonded(ctx, 0, false));
   }
-  if (ctx->mixed() && fold) RC(launch_fix_to_double(ctx, 1));
+  if ((ctx->mixed() || ctx->px_on) && fold) RC(launch_fix_to_double(ctx, 1));
   RC(launch_sclfrc(ctx, 1));
   return MDX_OK;
 }
@@ -240,6 +240,7 @@ int do_slow_parts(mdx_ctx *ctx, bool split, bool mirrored = false, bool types = 
     RC(launch_eterms(ctx));
     RC(launch_fold_wirs(ctx));
   } else {
+    if (!mirrored) RC(launch_ipos(ctx));
     RC(launch_furir(ctx));
     RC(launch_eterms(ctx));
     RC(launch_forces_long(ctx, split, types));
@@ -273,12 +274,12 @@ int do_both(mdx_ctx *ctx, int laver) {
 int do_allforce(mdx_ctx *ctx, bool split, bool laver = false) {
   RC(furir_prepare(ctx));
   RC(launch_zero(ctx, 3, split || laver ? 1 : 0));
-  if (ctx->mixed()) RC(launch_mirror_f32(ctx));
+  RC(ctx->mixed() ? launch_mirror_f32(ctx) : launch_ipos(ctx));
   RC(launch_localf(ctx, split));
   RC(launch_wir(ctx, 1));  // WIRSS from the pair forces, before the bonded terms
   RC(launch_bonded(ctx, split || laver ? 1 : 0));
   if (ctx->mixed()) RC(launch_fix_to_double(ctx, 1));
-  RC(do_slow_parts(ctx, split));
+  RC(do_slow_parts(ctx, split, !ctx->mixed()));
   RC(launch_sum_forces(ctx));
   // PULLBACK adds to G after CM_ADDLA has formed F (forces.f:88-95): SULTAN,
   // which moves with F, does not see it -- the reference's order, kept
@@ -307,9 +308,9 @@ int double_step(mdx_ctx *ctx, int mstep, int slot) {
   RC(launch_scaling(ctx, 1, &pend));
   if (p.lnpt) RC(sync_box_from_device(ctx));
   RC(launch_kick(ctx, 2, HTSTEP, pend));
-  // mixed path, intermediate short steps: the fast forces stay in fixed
-  // point (no fold) unless SCLFRC needs them in FP64
-  const bool keep_fix = ctx->mixed() && !p.lscft;
+  // intermediate short steps: the sweep's forces stay in fixed point (no
+  // fold) unless SCLFRC needs them in FP64
+  const bool keep_fix = (ctx->mixed() || ctx->px_on) && !p.lscft;
   for (int s = 1; s <= NFREQ; ++s) {
     // kick, drift, GETCOM and the mirrors; positions then stay put until the
     // next short step
@@ -544,10 +545,9 @@ int mdx_open(const mdx_dims *dims, mdx_ctx **out) {
     rc = dmalloc(ctx, &ss, scal_scratch_bytes());
     d.scal_scratch = ss;
   }
-  if (!rc && dims->precision == MDX_MIXED) {
-    AL(d.gfix, 3 * n);
-    AL(d.hfix, 3 * n);
-  }
+  AL(d.gfix, 3 * n);
+  AL(d.hfix, 3 * n);
+  if (dims->precision != MDX_MIXED) AL(d.ipos, 4 * n);
 #undef AL
   if (rc) {
     std::string e = ctx->err;
@@ -582,7 +582,7 @@ int mdx_close(mdx_ctx *ctx) {
                   d.bid, d.brb, d.ibi, d.ara, d.iai, d.titors, d.tft, d.iti, d.br,
                   d.ar, d.tr, d.cols, d.kchunks, d.kgroups, d.kconst, d.rf_part, d.tc_slot, d.tc_w, d.tc_meta, d.tcs_part, d.tcs_cp0, d.tc_zimg, d.tcs_zimg, d.tcs_red, d.sitems, d.tabx, d.tabxf, d.sk, d.sc, d.th,
                   d.rec, d.err, d.shake_iter, d.red, d.scal_scratch, d.nspec_d,
-                  d.red_part, d.red_ctr, d.sk_part, d.pair_tab, d.snap, d.avsum, d.shk_item,
+                  d.red_part, d.red_ctr, d.sk_part, d.pair_tab, d.px_tab, d.ipos, d.snap, d.avsum, d.shk_item,
                   d.shk_cl, d.shk_rec, d.shk_mfail, d.pull_atom, d.pull_ref, d.pull_step};
   if (ctx->stream) {
     for (void *p : ptrs) ctx_free(ctx, p);

@@ -185,6 +185,10 @@ struct DevData {
   double *gx, *gy, *gz, *hx, *hy, *hz, *fx, *fy, *fz;
   double *ox, *oy, *oz;
   unsigned long long *gfix, *hfix;  // 3n each, x then y then z
+  // FP64 path, fixed-point pair sweeps (pair64.cu): positions and charges as
+  // 64-bit integers, 4 words an atom, and the tables
+  long long *ipos;
+  void *px_tab;
   // lists
   int cap_s, cap_l;
   int *ns_cnt, *nl_cnt, *ns_idx, *nl_idx;
@@ -354,6 +358,12 @@ struct mdx_ctx {
   // branch of a captured step (bonded terms beside the short sweep)
   cudaStream_t side = nullptr;
   cudaEvent_t side_ev[2] = {};
+  // FP64 path, fixed-point pair sweeps: on, position unit 2^-px_bits A (of the
+  // box when ipos was last written), charge unit 2^(px_eq - 62) e, and the
+  // sweeps' ranges (0 short, 1 long): |d| < 2^px_rho A, r^2 >= 2^px_oct A^2;
+  // px_s: binary scales of the four functions
+  bool px_on = false;
+  int px_bits = 0, px_eq = 0, px_rho[2] = {0, 0}, px_oct[2] = {0, 0}, px_s[2][4] = {};
   int mbsh = 0, mbln = 0;
   cudaEvent_t snap_ev[MDX_SNAPSHOT_SLOTS] = {};  // completion of mdx_snapshot per slot
   // device timers (mdx_set_timers)
@@ -785,6 +795,26 @@ int pack_lj_tables(mdx_ctx *ctx);  // abf from the FP32 tables
 int launch_forces_long(mdx_ctx *ctx, bool split, bool types = true);
 // pair64.cu
 int pair64_setup(mdx_ctx *ctx);
+int launch_ipos(mdx_ctx *ctx);  // ipos from the positions
+// What a kernel that stores positions needs to store ipos too (p null: off).
+struct IPosOut {
+  longlong2 *p;
+  double ps, qs;  // units per A, per e
+};
+IPosOut ipos_out(mdx_ctx *ctx);
+double px_force_unit(const mdx_ctx *ctx, int which);  // of hfix (1), gfix (2), FP64 path
+// A coordinate beyond the range of the units, a NaN or a charge out of range:
+// the charge word is IPOS_BAD, and the sweeps take the atom's pairs in FP64.
+constexpr long long IPOS_BAD = (long long)0x8000000000000000ull;
+#ifdef __CUDACC__
+__device__ __forceinline__ void ipos_store(const IPosOut &o, int i, const dbl4 &p) {
+  constexpr double LIM = 2305843009213693952.0;  // 2^61
+  const double x = p.x * o.ps, y = p.y * o.ps, z = p.z * o.ps, q = p.w * o.qs;
+  const bool ok = fabs(x) < LIM && fabs(y) < LIM && fabs(z) < LIM && fabs(q) <= 2.0 * LIM;
+  o.p[2 * (size_t)i] = make_longlong2(__double2ll_rn(x), __double2ll_rn(y));
+  o.p[2 * (size_t)i + 1] = make_longlong2(__double2ll_rn(z), ok ? __double2ll_rn(q) : IPOS_BAD);
+}
+#endif
 int launch_pair64(mdx_ctx *ctx, bool shrt, bool split, bool ener, double *split_buf);
 int launch_wir(mdx_ctx *ctx, int which);  // WIRSS (1) / WIRS (2)
 // ewald.cu

@@ -57,6 +57,29 @@ __global__ void k_wir(int n, const dbl4 *__restrict__ pos,
   block_add<1>(w, dst);
 }
 
+// WIRSS / WIRS of the FP64 path with fixed-point sweeps: their sums are added
+// to the forces (and cleared for the next sweep) in the same pass.
+__global__ void k_add_wir(int n, const dbl4 *__restrict__ pos, const int4 *__restrict__ ainfo,
+                          const double *__restrict__ X, const double *__restrict__ Y,
+                          const double *__restrict__ Z, unsigned long long *__restrict__ f,
+                          double unit, double *__restrict__ fx, double *__restrict__ fy,
+                          double *__restrict__ fz, Dst6 dst) {
+  double w[1] = {0.0};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const dbl4 p = pos[i];
+    const int m = ainfo[i].y;
+    const double x = fma((double)(long long)f[i], unit, fx[i]);
+    const double y = fma((double)(long long)f[n + i], unit, fy[i]);
+    const double z = fma((double)(long long)f[2 * n + i], unit, fz[i]);
+    f[i] = f[n + i] = f[2 * n + i] = 0ull;
+    fx[i] = x;
+    fy[i] = y;
+    fz[i] = z;
+    w[0] = w[0] - x * (p.x - X[m]) - y * (p.y - Y[m]) - z * (p.z - Z[m]);
+  }
+  block_add<1>(w, dst);
+}
+
 // End of the mixed path's SLFORCES: G from its fixed-point sums, and WIRS of
 // it in the same pass.
 __global__ void k_fold_wirs(int n, const dbl4 *__restrict__ pos, const int4 *__restrict__ ainfo,
@@ -991,9 +1014,17 @@ int launch_wir(mdx_ctx *ctx, int which) {
     MDX_LAUNCHED(ctx);
     return MDX_OK;
   }
-  const double *fx = which == 1 ? d.hx : d.gx, *fy = which == 1 ? d.hy : d.gy,
-               *fz = which == 1 ? d.hz : d.gz;
+  double *fx = which == 1 ? d.hx : d.gx, *fy = which == 1 ? d.hy : d.gy,
+         *fz = which == 1 ? d.hz : d.gz;
   const int nbw = red_blocks(ctx);
+  if (ctx->px_on) {
+    k_add_wir<<<nbw, 256, 0, ctx->stream>>>(d.n, d.pos, d.ainfo, d.X, d.Y, d.Z,
+                                            which == 1 ? d.hfix : d.gfix,
+                                            px_force_unit(ctx, which), fx, fy, fz,
+                                            dst6(ctx, nbw, 1, dst));
+    MDX_LAUNCHED(ctx);
+    return MDX_OK;
+  }
   k_wir<<<nbw, 256, 0, ctx->stream>>>(d.n, d.pos, d.ainfo, d.X, d.Y, d.Z, fx, fy, fz,
                                       dst6(ctx, nbw, 1, dst));
   MDX_LAUNCHED(ctx);

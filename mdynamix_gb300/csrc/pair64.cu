@@ -20,10 +20,15 @@
 // all owners of a warp, and evaluated 32 at a time, so that no warp issues an
 // expression for a few of its lanes.
 //
-// Measured on a GB300 at 98,304 atoms, against the written-out sweeps (one
-// warp an owner): short rows, forces 0.526 -> 0.20 ms; long rows with energies
-// 4.88 -> 2.40 ms, with energies by type pair 15.3 -> 3.1 ms.  The FP64 pipe is
-// 82-86 % active.  Error of the slow forces against 64 bits unchanged.
+// In a rectangular cell k_pair64x does the same in 64-bit integers, which
+// leaves FP64 instructions for the LJ terms and a row's end only.
+//
+// Measured on a GB300 at 98,304 atoms (one warp an owner and everything
+// written out; k_pair64t; k_pair64x): short rows, forces 0.526, 0.20, 0.091 ms;
+// long rows with energies 4.88, 2.40, 1.24 ms, with energies by type pair
+// 15.3, 3.1, 1.5 ms.  k_pair64t's FP64 pipe is 82-86 % active.  Error of the
+// short rows' forces against 128 bits (200 ions; rms, of the rms force): 2.8e-15
+// written out, 4e-16 in integers.
 //
 // k_pair64 writes the reference's expressions out for every pair: the
 // reaction field (LMNBL).
@@ -118,28 +123,39 @@ __device__ dd pair_fn(int fn, double x, double alphad) {
   return div(D(MDX_TOTPI) * D(alphad) * e + er, D(x));
 }
 
-// Thread per (function, bin): values at 7 Chebyshev points of the bin,
-// divided differences, monomial coefficients.
-__global__ void k_pair_table(double alphad, PairPoly *__restrict__ tab) {
-  const int id = blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= PT_NFN * PT_BINS) return;
-  const int fn = id / PT_BINS, bin = id % PT_BINS;
-  const double oct = ldexp(1.0, PT_OCT0 + bin / 128);
-  constexpr int N = 7;
-  double x[N];
-  dd f[N];
-  for (int k = 0; k < N; ++k) {
-    x[k] = rint(0.5 * cospi((2 * k + 1) / (2.0 * N)) * 1073741824.0) / 1073741824.0;
-    f[k] = pair_fn(fn, oct * (1.0 + ((bin % 128) + 0.5 + x[k]) / 128.0), alphad);
+// Coefficients of a function's polynomial in one bin: block of 32 bins x 7
+// Chebyshev points, a thread each for the values, then a thread per bin for
+// the divided differences and the monomial form (true there).
+constexpr int PN = 7, PTB = 32;
+__device__ __forceinline__ double pt_node(int k) {
+  return rint(0.5 * cospi((2 * k + 1) / (2.0 * PN)) * 1073741824.0) / 1073741824.0;
+}
+__device__ bool pt_coef(int fn, int oct0, int nbin, double alphad, dd (&c)[PN]) {
+  __shared__ dd sf[PN][PTB];
+  const int b = threadIdx.x % PTB, node = threadIdx.x / PTB, bin = blockIdx.x * PTB + b;
+  const double oct = ldexp(1.0, oct0 + bin / 128);
+  sf[node][b] = pair_fn(fn, oct * (1.0 + ((bin % 128) + 0.5 + pt_node(node)) / 128.0), alphad);
+  __syncthreads();
+  if (node || bin >= nbin) return false;
+  double x[PN];
+  dd f[PN];
+  for (int k = 0; k < PN; ++k) {
+    x[k] = pt_node(k);
+    f[k] = sf[k][b];
+    c[k] = D(0.0);
   }
-  for (int o = 1; o < N; ++o)
-    for (int k = N - 1; k >= o; --k) f[k] = div(f[k] + -f[k - 1], D(x[k] - x[k - o]));
-  dd c[N];
-  for (int k = 0; k < N; ++k) c[k] = D(0.0);
-  for (int k = N - 1; k >= 0; --k) {  // c = c (t - x_k) + f_k
-    for (int m = N - 1; m > 0; --m) c[m] = c[m - 1] + -(c[m] * D(x[k]));
+  for (int o = 1; o < PN; ++o)
+    for (int k = PN - 1; k >= o; --k) f[k] = div(f[k] + -f[k - 1], D(x[k] - x[k - o]));
+  for (int k = PN - 1; k >= 0; --k) {  // c = c (t - x_k) + f_k
+    for (int m = PN - 1; m > 0; --m) c[m] = c[m - 1] + -(c[m] * D(x[k]));
     c[0] = f[k] + -(c[0] * D(x[k]));
   }
+  return true;
+}
+__global__ void __launch_bounds__(PTB *PN) k_pair_table(double alphad, PairPoly *__restrict__ tab) {
+  dd c[PN];
+  const int bin = blockIdx.x * PTB + threadIdx.x % PTB, fn = blockIdx.y;
+  if (!pt_coef(fn, PT_OCT0, PT_BINS, alphad, c)) return;
   PairPoly p;
   p.c0 = c[0].h + c[0].l;
   p.c1 = c[1].h + c[1].l;
@@ -149,7 +165,7 @@ __global__ void k_pair_table(double alphad, PairPoly *__restrict__ tab) {
   p.c5 = (float)(c[5].h + c[5].l);
   p.c6 = (float)(c[6].h + c[6].l);
   p.pad = 0.f;
-  tab[id] = p;
+  tab[(size_t)fn * PT_BINS + bin] = p;
 }
 
 // FP32 to FP64 by the bits (a conversion instruction issues on the FP64
@@ -604,16 +620,430 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64t(
   sweep_out<SPLIT, ENER>(a, dst, s_split, split);
 }
 
+// ------------------------------------------------- fixed-point sweeps ----
+// The same sweep in 64-bit integers (rectangular cell): a multiplication of
+// two 64-bit numbers is three 32 x 32 + 64 bit multiply-adds, and GB300 issues
+// those 32 times as often as an FP64 instruction, so a Coulomb pair's 19 - 27
+// FP64 instructions become about 200 integer ones in a quarter of the time.
+// Positions are integers of 2^-px_bits A (ipos, written with the positions),
+// their differences are exact, and
+//   d   = difference, minimum image, shifted so that 2^rho A is 2^62
+//   r2  = the upper 64 bits of d.d
+//   t   = position in the bin of r2, 2^-63 units; bins as in PairPoly
+//   F   = polynomial in t, 62 bits at the table's first r^2
+//   G   = F q_i q_j (62 bits), fx = upper 64 bits of G dx, and so on.
+// A product keeps all but its last bit, so a pair's force is good to 2^-54 of
+// the force at the table's start; it is added as an integer, whatever the
+// order.  The LJ term comes from a tabulated 1 / r^2 in 9 FP64 instructions
+// and joins G.  Everything else goes to the FP64 expressions as before, and
+// so do atoms and pairs out of the numbers' range.
+struct __align__(16) PxPoly {
+  long long c0, c1, c2;  // c0, 2 c1, 4 c2
+  int c3, sh;            // 8 c3 in units of 2^(32 - sh)
+  float c4, c5, c6, pad; // 8 times, units of c3
+};
+struct Px {
+  int s, base, nbin, rng;  // left shift of d, first bin's index, bins, range of d (upper word)
+  long long lx, ly, lz, hx, hy, hz;  // box and half box (LOCALF tests DZ against HBOXL)
+  unsigned long long rc2;
+  double uE, uR, uV, uG, iG;  // units of energy, 1 / r, virial; of G, and 1 / that
+  double du;                  // unit of d (A)
+  int s2;                     // 1 / r^2 is 2^-s2 times its table's value
+  const PxPoly *tab;          // PT_NFN x nbin
+};
+
+// v = h 2^32 + l, both signed (|v| < 2^63 - 2^31)
+struct I2 {
+  int h, l;
+};
+__device__ __forceinline__ I2 split2(long long v) {
+  return I2{(int)((v + 0x80000000LL) >> 32), (int)v};
+}
+__device__ __forceinline__ long long cross2(I2 a, I2 b) {
+  return (long long)a.h * b.l + (long long)a.l * b.h;
+}
+// upper 64 bits of a b, to the nearest (|a|, |b| <= 2^62)
+__device__ __forceinline__ long long mulhi2(I2 a, I2 b) {
+  return (long long)a.h * b.h + ((cross2(a, b) + 0x80000000LL) >> 32);
+}
+struct PxArg {
+  int bin;
+  I2 t;
+  float tf;
+};
+__device__ __forceinline__ PxArg px_arg(const Px &x, unsigned long long r2) {
+  const int lz = __clz((int)(r2 >> 32));
+  const unsigned long long m = r2 << (lz & 31);
+  const unsigned mh = (unsigned)(m >> 32);
+  PxArg a;
+  a.bin = x.base - 128 * lz + (int)(mh >> 24);
+  a.t = split2((long long)((m << 7) & 0x7fffffffffffffffull) - 0x4000000000000000LL);
+  a.tf = __uint_as_float(0x3f800000u | ((mh & 0xffffffu) >> 1)) - 1.5f;
+  return a;
+}
+__device__ __forceinline__ long long px_eval(const PxPoly *__restrict__ tab, const PxArg &a) {
+  const PxPoly *p = tab + a.bin;
+  const longlong2 c01 = __ldg(reinterpret_cast<const longlong2 *>(p));
+  const int4 c23 = __ldg(reinterpret_cast<const int4 *>(p) + 1);
+  const float4 cf = __ldg(reinterpret_cast<const float4 *>(p) + 2);
+  const int s3 = c23.z + __float2int_rn(a.tf * fmaf(fmaf(cf.z, a.tf, cf.y), a.tf, cf.x));
+  const long long c2 = (long long)(((unsigned long long)(unsigned)c23.y << 32) | (unsigned)c23.x);
+  const long long s2 = c2 + (((long long)s3 * a.t.h) >> c23.w);
+  const long long s1 = c01.y + mulhi2(split2(s2), a.t);
+  return c01.x + mulhi2(split2(s1), a.t);
+}
+
+struct PxQueue {  // pairs put aside for their LJ term, per warp
+  long long x[64], y[64], z[64], g[64];
+  unsigned long long r2[64];
+  int i[64], j[64], tix[64];
+};
+
+template <bool SHORT, bool SPLIT, bool ENER, int TPO>
+__global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64x(
+    int n, const longlong2 *__restrict__ ipos, const dbl4 *__restrict__ pos,
+    const int4 *__restrict__ ainfo, const double *__restrict__ qsite,
+    const int *__restrict__ cnt, const int *__restrict__ idx, int cap, Lj64 lj, TypeConst tc,
+    PairConst pc, CellPbc cp, unsigned eemask, Px px, double *__restrict__ fx,
+    double *__restrict__ fy, double *__restrict__ fz, unsigned long long *__restrict__ ff,
+    Dst6 dst, double *__restrict__ split) {
+  __shared__ double s_split[SPLIT ? SPLIT_N : 1];
+  __shared__ PxQueue s_q[PT_WARPS];
+  __shared__ int2 s_slow[PT_WARPS][64];
+  if (SPLIT) {
+    for (int k = threadIdx.x; k < SPLIT_N; k += blockDim.x) s_split[k] = 0.0;
+    __syncthreads();
+  }
+  constexpr int OPW = 32 / TPO;  // owners of a warp at a time
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  PxQueue &q = s_q[w];
+  int2 *slow = s_slow[w];
+  const Env64 v = env64(pos, ainfo, qsite, lj, fx, fy, fz, cp, SHORT, pc);
+  const unsigned eem = v.rae_on ? eemask : 0u;
+  Acc64 a;
+  acc_zero(a);
+  long long ie = 0, ivx = 0, ivy = 0, ivz = 0;  // this owner's row
+  int nq = 0, nslow = 0;
+  auto add = [&](int i, long long x, long long y, long long z) {
+    atomicAdd(&ff[i], (unsigned long long)x);
+    atomicAdd(&ff[(size_t)n + i], (unsigned long long)y);
+    atomicAdd(&ff[2 * (size_t)n + i], (unsigned long long)z);
+  };
+  auto virial = [&](long long x, long long y, long long z, I2 dx, I2 dy, I2 dz) {
+    ivx += mulhi2(split2(x), dx);
+    ivy += mulhi2(split2(y), dy);
+    ivz += mulhi2(split2(z), dz);
+  };
+  // the last m (<= 32) pairs of the LJ queue: their LJ terms, then forces
+  auto lj_batch = [&](int m) {
+    __syncwarp();
+    if (lane < m) {
+      const int e = nq - m + lane;
+      const int tix = q.tix[e], i = q.i[e], j = q.j[e];
+      const double r = (double)px_eval(px.tab + PT_R2I * px.nbin, px_arg(px, q.r2[e]));
+      // times 2^-s2 by the exponent
+      const double R2I =
+          __hiloint2double(__double2hiint(r) - (px.s2 << 20), __double2loint(r));
+      const double A6 = __ldg(&lj.a6lj[tix]), B12 = __ldg(&lj.b12lj[tix]);
+      const double R6I = R2I * R2I * R2I, T12 = B12 * R6I;
+      const double G = fma(2.0, T12, A6) * R6I;  // FSR R1 / 6
+      const double FL = R2I * px.iG * G;         // in units of G
+      if (ENER || SPLIT) {
+        const double ESR = (A6 + T12) * R6I;
+        if (ENER) {
+          a.e[A_ESR] += ESR;
+          a.e[A_VIR] = fma(6.0, G, a.e[A_VIR]);
+        }
+        if (SPLIT) split_add(a, tc.mdx[ainfo[i].x][ainfo[j].x], 0.0, ESR, s_split);
+      }
+      // 2^60: the sums of forces stay far below 2^63
+      if ((__double_as_longlong(FL) & 0x7fffffffffffffffLL) < 0x43b0000000000000LL) {
+        const I2 g = split2(q.g[e] + __double2ll_rn(FL));
+        const I2 dx = split2(q.x[e]), dy = split2(q.y[e]), dz = split2(q.z[e]);
+        const long long gx = mulhi2(g, dx), gy = mulhi2(g, dy), gz = mulhi2(g, dz);
+        if (ENER) virial(gx, gy, gz, dx, dy, dz);
+        add(i, gx, gy, gz);
+        add(j, -gx, -gy, -gz);
+      } else {
+        apply64<ENER>(v, i, j, ((double)q.g[e] + FL) * px.uG, (double)q.x[e] * px.du,
+                      (double)q.y[e] * px.du, (double)q.z[e] * px.du, true, a);
+      }
+    }
+    nq -= m;
+    __syncwarp();
+  };
+  auto slow_batch = [&](int m) {
+    __syncwarp();
+    if (lane < m) {
+      const int2 s = slow[nslow - m + lane];
+      const Pair64 p = pair_general<SHORT, SPLIT, ENER>(v, s.y, pos[s.x], ainfo[s.x], qsite[s.x],
+                                                        tc, pc, s_split, a);
+      if (!p.skip) apply64<ENER>(v, s.x, s.y & 0x7fffffff, p.F, p.DX, p.DY, p.DZ, p.vir, a);
+    }
+    nslow -= m;
+    __syncwarp();
+  };
+  auto image = [&](long long &d, long long h, long long l) {
+    const bool c = (unsigned long long)(d + h) > 2ull * (unsigned long long)h;
+    if (__any_sync(0xffffffffu, c) && c) d -= d < 0 ? -l : l;
+  };
+  for (int i0 = (blockIdx.x * PT_WARPS + w) * OPW; i0 < n; i0 += gridDim.x * PT_WARPS * OPW) {
+    const int i = i0 + lane / TPO;
+    const bool own = i < n;
+    const size_t io = 2 * (size_t)(own ? i : 0);
+    const longlong2 pxy = ipos[io], pzq = ipos[io + 1];
+    const int4 ai = ainfo[own ? i : 0];
+    const I2 qi = split2(pzq.y);
+    const int c = own ? cnt[i] : 0;
+    const int cmax = __reduce_max_sync(0xffffffffu, c);
+    const int *row = idx + (size_t)(own ? i : 0) * cap;
+    const double *b12row = lj.b12lj + ai.z * pc.nnbt;
+    const bool eei = ((eem >> ai.x) & 1u) || pzq.y == IPOS_BAD;
+    long long ax = 0, ay = 0, az = 0;
+    for (int k = lane & (TPO - 1); k - (lane & (TPO - 1)) < cmax; k += TPO) {
+      bool act = k < c;
+      const int e = act ? row[k] : 0;
+      const int j = e & 0x7fffffff;
+      const longlong2 jxy = ipos[2 * (size_t)j], jzq = ipos[2 * (size_t)j + 1];
+      const int4 aj = ainfo[j];
+      long long DX = pxy.x - jxy.x, DY = pxy.y - jxy.y, DZ = pzq.x - jzq.x;
+      image(DX, px.hx, px.lx);
+      image(DY, px.hy, px.ly);
+      image(DZ, px.hz, px.lz);
+      const bool in = (unsigned)((int)(DX >> 32) + px.rng) < 2u * (unsigned)px.rng &&
+                      (unsigned)((int)(DY >> 32) + px.rng) < 2u * (unsigned)px.rng &&
+                      (unsigned)((int)(DZ >> 32) + px.rng) < 2u * (unsigned)px.rng;
+      DX <<= px.s;
+      DY <<= px.s;
+      DZ <<= px.s;
+      const I2 dx = split2(DX), dy = split2(DY), dz = split2(DZ);
+      const long long cr = (long long)dx.h * dx.l + (long long)dy.h * dy.l +
+                           (long long)dz.h * dz.l + 0x40000000LL;
+      const unsigned long long r2 =
+          (unsigned long long)((long long)dx.h * dx.h + (long long)dy.h * dy.h +
+                               (long long)dz.h * dz.h + (cr >> 31));
+      PxArg p = px_arg(px, r2);
+      const bool other = (SHORT && e < 0) || aj.y == ai.y || eei || ((eem >> aj.x) & 1u) ||
+                         jzq.y == IPOS_BAD || !in || (unsigned)p.bin >= (unsigned)px.nbin;
+      if (!SHORT && !other && r2 > px.rc2) act = false;  // skin mode
+      const bool sl = act && other, fast = act && !other;
+      if (!fast) p.bin = 0;
+      const unsigned ms = __ballot_sync(0xffffffffu, sl);
+      if (ms) {
+        if (sl) slow[nslow + __popc(ms & below)] = make_int2(i, e);
+        nslow += __popc(ms);
+        if (nslow >= 32) slow_batch(32);
+      }
+      const I2 qq = split2(mulhi2(qi, split2(jzq.y)));
+      const I2 F = split2(px_eval(px.tab + PT_FORCE * px.nbin, p));
+      const long long g = (((long long)F.h * qq.h) << 4) + (cross2(F, qq) >> 28);
+      if (ENER) {
+        const long long E = mulhi2(split2(px_eval(px.tab + PT_ENER * px.nbin, p)), qq);
+        if (fast) ie += E;
+      }
+      if (SPLIT && fast)
+        split_add(a, tc.mdx[ai.x][aj.x],
+                  (double)mulhi2(split2(px_eval(px.tab + PT_R1I * px.nbin, p)), qq) * px.uR, 0.0,
+                  s_split);
+      const bool lb = fast && (__double_as_longlong(__ldg(&b12row[aj.z])) << 1) != 0;  // B12 != 0
+      if (fast && !lb) {
+        const I2 G = split2(g);
+        const long long gx = mulhi2(G, dx), gy = mulhi2(G, dy), gz = mulhi2(G, dz);
+        if (ENER) virial(gx, gy, gz, dx, dy, dz);
+        ax += gx;
+        ay += gy;
+        az += gz;
+        add(j, -gx, -gy, -gz);
+      }
+      const unsigned ml = __ballot_sync(0xffffffffu, lb);
+      if (ml) {
+        if (lb) {
+          const int s = nq + __popc(ml & below);
+          q.x[s] = DX;
+          q.y[s] = DY;
+          q.z[s] = DZ;
+          q.r2[s] = r2;
+          q.g[s] = g;
+          q.i[s] = i;
+          q.j[s] = j;
+          q.tix[s] = ai.z * pc.nnbt + aj.z;
+        }
+        nq += __popc(ml);
+        if (nq >= 32) lj_batch(32);
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < TPO; o <<= 1) {
+      ax += __shfl_xor_sync(0xffffffffu, ax, o);
+      ay += __shfl_xor_sync(0xffffffffu, ay, o);
+      az += __shfl_xor_sync(0xffffffffu, az, o);
+    }
+    if (c > 0 && (lane & (TPO - 1)) < 3) {
+      const int k = lane & (TPO - 1);
+      atomicAdd(&ff[(size_t)k * n + i], (unsigned long long)(k == 0 ? ax : k == 1 ? ay : az));
+    }
+    if (ENER) {  // a row's sums stay below 2^63
+      a.e[A_EES] = fma((double)ie, px.uE, a.e[A_EES]);
+      a.e[A_VX] = fma((double)ivx, px.uV, a.e[A_VX]);
+      a.e[A_VY] = fma((double)ivy, px.uV, a.e[A_VY]);
+      a.e[A_VZ] = fma((double)ivz, px.uV, a.e[A_VZ]);
+      ie = ivx = ivy = ivz = 0;
+    }
+  }
+  if (nq) lj_batch(nq);
+  if (nslow) slow_batch(nslow);
+  if (ENER) {
+    a.e[A_VX] = fma((double)ivx, px.uV, a.e[A_VX]);
+    a.e[A_VY] = fma((double)ivy, px.uV, a.e[A_VY]);
+    a.e[A_VZ] = fma((double)ivz, px.uV, a.e[A_VZ]);
+  }
+  sweep_out<SPLIT, ENER>(a, dst, s_split, split);
+}
+
+struct PxScale {
+  int s[PT_NFN];
+};
+__device__ __forceinline__ long long dd2ll(dd v, int s) {  // v 2^s to the nearest
+  const double h = ldexp(v.h, s), r = rint(h);
+  return (long long)r + __double2ll_rn((h - r) + ldexp(v.l, s));
+}
+__global__ void __launch_bounds__(PTB *PN) k_px_table(int nbin, int oct0, double alphad, PxScale sc,
+                                                     PxPoly *__restrict__ tab) {
+  dd c[PN];
+  const int bin = blockIdx.x * PTB + threadIdx.x % PTB, fn = blockIdx.y;
+  if (!pt_coef(fn, oct0, nbin, alphad, c)) return;
+  const int s = sc.s[fn];
+  PxPoly p;
+  p.c0 = dd2ll(c[0], s);
+  p.c1 = dd2ll(c[1], s + 1);
+  p.c2 = dd2ll(c[2], s + 2);
+  const double c3 = ldexp(c[3].h, s + 3);
+  const int K = min(32, max(0, ilogb(fmax(fabs(c3), 1.0)) + 1 - 30));
+  p.c3 = (int)dd2ll(c[3], s + 3 - K);
+  p.sh = 32 - K;
+  p.c4 = (float)ldexp(c[4].h, s + 3 - K);
+  p.c5 = (float)ldexp(c[5].h, s + 3 - K);
+  p.c6 = (float)ldexp(c[6].h, s + 3 - K);
+  p.pad = 0.f;
+  tab[(size_t)fn * nbin + bin] = p;
+}
+
+__global__ void k_ipos(int n, const dbl4 *__restrict__ pos, IPosOut o) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) ipos_store(o, i, pos[i]);
+}
+
+int px_bins(const mdx_ctx *ctx, int w) { return 128 * (2 * ctx->px_rho[w] - ctx->px_oct[w]); }
+
+// The sweep's constants for the current box (units of ipos as last written).
+Px px_args(const mdx_ctx *ctx, bool shrt) {
+  Px x{};
+  if (!ctx->px_on) return x;
+  const int w = shrt ? 0 : 1, rho = ctx->px_rho[w], B = ctx->px_bits;
+  const int *s = ctx->px_s[w];
+  auto u = [&](double a) { return std::llrint(std::ldexp(a, B)); };
+  x.s = 62 - rho - B;
+  x.rng = 1 << (B + rho - 32);
+  x.nbin = px_bins(ctx, w);
+  // octave of r2: 2 rho + 3 - lz; the upper byte of the mantissa is 128 ..
+  x.base = 128 * (2 * rho + 3 - ctx->px_oct[w]) - 128;
+  x.lx = u(ctx->boxl);
+  x.ly = u(ctx->boyl);
+  x.lz = u(ctx->bozl);
+  x.hx = u(0.5 * ctx->boxl);
+  x.hy = u(0.5 * ctx->boyl);
+  x.hz = shrt ? x.hx : u(0.5 * ctx->bozl);
+  x.rc2 = (unsigned long long)std::ldexp(ctx->pc.rc2, 60 - 2 * rho);
+  const int q2 = 2 * ctx->px_eq;
+  const double cf = ctx->p.coulf;
+  x.uG = std::ldexp(cf, q2 - s[PT_FORCE]);
+  x.iG = 6.0 * std::ldexp(1.0 / cf, s[PT_FORCE] - q2);  // 6: FSR R1 / 6
+  x.du = std::ldexp(1.0, rho - 62);
+  x.uV = std::ldexp(x.uG, 4 + 2 * (rho - 62) + 124);
+  x.uE = std::ldexp(cf, q2 + 4 - s[PT_ENER]);
+  x.uR = std::ldexp(cf, q2 + 4 - s[PT_R1I]);
+  x.s2 = s[PT_R2I];
+  x.tab = reinterpret_cast<const PxPoly *>(ctx->dv.px_tab) + (shrt ? 0 : PT_NFN * px_bins(ctx, 0));
+  return x;
+}
+
 }  // namespace
 
-// The Ewald tables of the sweeps for the current alpha (FP64 path; set_params).
+// Positions beyond 2^61 units are out of range: twice the box to either side.
+// At most 2^-54 A (the sweeps' shifts stay positive), which is below the last
+// bit of an FP64 coordinate beyond 0.25 A.
+IPosOut ipos_out(mdx_ctx *ctx) {
+  if (!ctx->px_on) return IPosOut{nullptr, 0.0, 0.0};
+  const double l = std::max({ctx->boxl, ctx->boyl, ctx->bozl});
+  ctx->px_bits = std::min(54, 61 - (std::ilogb(2.0 * l) + 1));
+  return IPosOut{reinterpret_cast<longlong2 *>(ctx->dv.ipos), std::ldexp(1.0, ctx->px_bits),
+                 std::ldexp(1.0, 62 - ctx->px_eq)};
+}
+int launch_ipos(mdx_ctx *ctx) {
+  if (!ctx->px_on) return MDX_OK;
+  MDX_TIMER(ctx, MDX_T_OTHER);
+  const DevData &d = ctx->dv;
+  k_ipos<<<(d.n + 255) / 256, 256, 0, ctx->stream>>>(d.n, d.pos, ipos_out(ctx));
+  MDX_LAUNCHED(ctx);
+  return MDX_OK;
+}
+// force = coulf F q q d: G has 2^(s - 2 eq), d 2^(62 - rho), their product loses 64 bits
+double px_force_unit(const mdx_ctx *ctx, int which) {
+  if (!ctx->px_on) return 0.0;
+  const int w = which == 1 ? 0 : 1;
+  return std::ldexp(ctx->p.coulf, 2 * ctx->px_eq - ctx->px_s[w][PT_FORCE] + ctx->px_rho[w] + 2);
+}
+
+// The Ewald tables of the sweeps for the current parameters (FP64 path;
+// set_params).  Integers where the cell is rectangular and the cut-offs and
+// charges fit them: the short rows' table from r^2 = 2 A^2, the long rows'
+// from the octave below (0.8 RSHORT)^2; pairs closer by go to the FP64
+// expressions.  A pair's force is good to 2^-54 of the force at its table's
+// start, so the short rows end at 6.6 A: a screened force is down by 2^6
+// there, and the error of an atom's force stays that of its nearest
+// neighbours in FP64.
 int pair64_setup(mdx_ctx *ctx) {
   DevData &d = ctx->dv;
+  ctx->px_on = false;
   if (ctx->mixed() || ctx->p.alphad <= 0.0 || ctx->p.lmnbl) return MDX_OK;
+  double qmax = 0.0;
+  for (double q : ctx->h_q) qmax = std::max(qmax, std::fabs(q));
+  for (double q : ctx->h_charge) qmax = std::max(qmax, std::fabs(q));  // MDEE scales these
+  const double rl = ctx->p.rcut + ctx->p.rskin;
+  auto rho = [](double r) { return std::max(2, std::ilogb(r) + 1); };
+  if (ctx->p.icell == 0 && ctx->p.coulf > 0.0 && qmax > 0.0 && qmax <= 4.0 && rl < 31.0 &&
+      ctx->p.rshort > 2.0 && 1.2 * ctx->p.rshort < 8.0) {
+    ctx->px_eq = std::ilogb(qmax) + (std::ldexp(1.0, std::ilogb(qmax)) < qmax ? 1 : 0);
+    ctx->px_rho[0] = rho(1.2 * ctx->p.rshort);
+    ctx->px_rho[1] = rho(rl);
+    ctx->px_oct[0] = 1;
+    ctx->px_oct[1] = std::max(1, std::ilogb(0.64 * ctx->p.rshort * ctx->p.rshort));
+    const int nb[2] = {px_bins(ctx, 0), px_bins(ctx, 1)};
+    if (!d.px_tab) MDX_CUDA(ctx_alloc(ctx, &d.px_tab, sizeof(PxPoly) * PT_NFN * 2 * 128 * 10));
+    for (int w = 0; w < 2; ++w) {
+      // binary scale of each function: below 2^62 at the first r^2.  Long
+      // rows, forces: 2^60, so that some hundred pairs of one sign still fit
+      const double x = std::ldexp(1.0, ctx->px_oct[w]), r = std::sqrt(x);
+      const double ar = ctx->p.alphad * r, t = 1.0 / (1.0 + MDX_B1 * ar), e = std::exp(-ar * ar);
+      const double er =
+          ((((MDX_A5 * t + MDX_A4) * t + MDX_A3) * t + MDX_A2) * t + MDX_A1) * t * e / r;
+      const double f0[PT_NFN] = {(MDX_TOTPI * ctx->p.alphad * e + er) / x, er, 1.0 / x, 1.0 / r};
+      PxScale sc;
+      for (int f = 0; f < PT_NFN; ++f)
+        sc.s[f] = ctx->px_s[w][f] = (w && f == PT_FORCE ? 60 : 62) - 1 - std::ilogb(1.0001 * f0[f]);
+      k_px_table<<<dim3(nb[w] / PTB, PT_NFN), PTB * PN, 0, ctx->stream>>>(
+          nb[w], ctx->px_oct[w], ctx->p.alphad, sc,
+          reinterpret_cast<PxPoly *>(d.px_tab) + (w ? PT_NFN * nb[0] : 0));
+      MDX_LAUNCHED(ctx);
+    }
+    ctx->px_on = true;
+    return MDX_OK;
+  }
   if (d.pair_tab && ctx->pair_tab_alpha == ctx->p.alphad) return MDX_OK;
   if (!d.pair_tab)
     MDX_CUDA(ctx_alloc(ctx, &d.pair_tab, sizeof(PairPoly) * PT_NFN * PT_BINS));
-  k_pair_table<<<(PT_NFN * PT_BINS + 63) / 64, 64, 0, ctx->stream>>>(
+  k_pair_table<<<dim3(PT_BINS / PTB, PT_NFN), PTB * PN, 0, ctx->stream>>>(
       ctx->p.alphad, reinterpret_cast<PairPoly *>(d.pair_tab));
   MDX_LAUNCHED(ctx);
   ctx->pair_tab_alpha = ctx->p.alphad;
@@ -623,7 +1053,7 @@ int pair64_setup(mdx_ctx *ctx) {
 int launch_pair64(mdx_ctx *ctx, bool shrt, bool split, bool ener, double *split_buf) {
   DevData &d = ctx->dv;
   const int T = 32 * PT_WARPS;
-  const bool table = d.pair_tab && !ctx->p.lmnbl && ctx->p.alphad > 0.0;
+  const bool table = (ctx->px_on || d.pair_tab) && !ctx->p.lmnbl && ctx->p.alphad > 0.0;
   // Lanes of an owner: 32 on the long rows.  On the short rows (about 26
   // entries) fewer lanes make the owner's sums cheaper (short sweep at 98,304
   // atoms: 8 lanes 0.222 ms, 16 0.234, 32 0.257) as long as the owners still
@@ -651,13 +1081,24 @@ int launch_pair64(mdx_ctx *ctx, bool shrt, bool split, bool ener, double *split_
     if (ctx->tc.iee[t] == 0) eemask |= 1u << t;
   const PairPoly *tab = reinterpret_cast<const PairPoly *>(d.pair_tab);
   const CellPbc cp = cell_pbc(ctx);
+  const Px px = px_args(ctx, shrt);
+  unsigned long long *ff = shrt ? d.hfix : d.gfix;
 #define LP64T(S, P, E, K)                                                                       \
   k_pair64t<S, P, E, K><<<grid, T, 0, ctx->stream>>>(d.n, d.pos, d.ainfo, d.qsite, cnt, idx, cap, \
                                                      lj, ctx->tc, ctx->pc, cp, eemask, tab, fx, \
                                                      fy, fz, dst, split_buf)
+#define LP64X(S, P, E, K)                                                                       \
+  k_pair64x<S, P, E, K><<<grid, T, 0, ctx->stream>>>(d.n, reinterpret_cast<longlong2 *>(d.ipos), \
+                                                     d.pos, d.ainfo, d.qsite, cnt, idx, cap, lj, \
+                                                     ctx->tc, ctx->pc, cp, eemask, px, fx, fy,   \
+                                                     fz, ff, dst, split_buf)
 #define LP64(S, P, E)                                                                        \
   do {                                                                                       \
-    if (!table)                                                                              \
+    if (ctx->px_on) {                                                                        \
+      if (S && tpo == 8) LP64X(S, P, E, S ? 8 : 32);                                         \
+      else if (S && tpo == 16) LP64X(S, P, E, S ? 16 : 32);                                  \
+      else LP64X(S, P, E, 32);                                                               \
+    } else if (!table)                                                                              \
       k_pair64<S, P, E><<<grid, T, 0, ctx->stream>>>(d.n, d.pos, d.ainfo, d.qsite, cnt, idx, \
                                                      cap, lj, ctx->tc, ctx->pc, cp, fx, fy,  \
                                                      fz, dst, split_buf);                    \
@@ -677,6 +1118,7 @@ int launch_pair64(mdx_ctx *ctx, bool shrt, bool split, bool ener, double *split_
   }
 #undef LP64
 #undef LP64T
+#undef LP64X
   MDX_LAUNCHED(ctx);
   return MDX_OK;
 }

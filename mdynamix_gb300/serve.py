@@ -108,6 +108,7 @@ def estimate_bytes(s: S.System, precision: int) -> int:
     per_atom = 1024 + 4 * (cs + cl) + 16 * rows + 4 * s.nbdmax
     if precision != MDX_MIXED:
         per_atom += 28 * (2 * kmax + 18)  # the Z digit images of the fixed-point Ewald passes
+        per_atom += 80  # the pair sweeps' integer positions and forces
     slices = max(1, -(-n // 128))
     per_k = 256 + 16 * slices
     return int(n * per_atom + nkv * per_k + (24 << 20))

@@ -126,3 +126,43 @@ def test_mixed_energies_by_type_pair(nw, kind):
     for n in ("pote1", "potl1", "pes141", "psr141"):
         x, y = np.array(getattr(a, n)), np.array(getattr(b, n))
         assert np.abs(x - y).max() <= 1e-4 * max(np.abs(x).max(), 1e-9), n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("box", [(40.0, 40.0, 40.0), (31.0, 45.0, 38.0), (200.0, 60.0, 90.0)])
+def test_fixed_point_pairs(box):
+    """Two ions across the faces of the cell, from 0.3 A (written out; large LJ
+    forces) through the starts and ends of the sweeps' ranges to 12 A, cut at
+    5 A between LOCALF and FORCES.  A pair's force: 2^-53 of the Coulomb force
+    at its sweep's first r^2 (2 and 16 A^2: three roundings of a quarter of
+    that) beside the 2e-14 of its parts; energies alike."""
+    from mdynamix_gb300.mdx import ForcePath
+    # no k-vectors: G is the pair force alone
+    spec = dataclasses.replace(_two_ions().spec, box=box, rshort=5.0, fexp=1e-4)
+    s = S.System(spec)
+    g, o = ForcePath(s, precision=MDX_FP64), oracle.Oracle(s)
+    i = s.inbt[0] - 1
+    rng = np.random.default_rng(3)
+    r = list(np.exp(np.linspace(np.log(0.3), np.log(11.99), 120)))
+    r += [np.sqrt(v) for v in (1.9999999, 2.0, 2.015625, 15.9999, 16.0, 24.999, 25.001, 63.99)]
+    for d in r:
+        u = rng.normal(size=3)
+        u /= np.linalg.norm(u)
+        c = 0.5 * np.array(box) * rng.choice([-1.0, 1.0], 3) + rng.normal(size=3)
+        xy = np.stack([c - 0.5 * d * u, c + 0.5 * d * u], 1)
+        st = tuple(xy) + (np.zeros(2),) * 3
+        for p in (g, o):
+            p.set_state(*st)
+            p.chcnb()
+            p.getcom()
+        for routine, which, r0, names in (("fforces", 1, 2.0, ("pels2", "virfx")),
+                                          ("slforces", 2, 16.0, ("pels1",))):
+            a, b = getattr(g, routine)(), getattr(o, routine)()
+            fa, fb = g.forces(which), o.forces(which)
+            coul = s.coulf * 1.128379169 * s.alphad * np.exp(-(s.alphad * d) ** 2) / d
+            parts = (coul + abs(6 * s.a6lj[i, i]) / d ** 7 + abs(12 * s.b12lj[i, i]) / d ** 13)
+            start = s.coulf / r0
+            tol = 2e-14 * parts + 2.0 ** -53 * start
+            assert np.abs(fa - fb).max() <= tol, (routine, d)
+            assert abs(getattr(a, names[0]) - getattr(b, names[0])) <= (
+                1e-14 * abs(getattr(b, names[0])) + 2.0 ** -53 * start * np.sqrt(r0)), (routine, d)
