@@ -169,6 +169,28 @@ struct MolCut {
   const int4 *ainfo;
 };
 
+// -1 for an excluded bonded pair, 3 for a 1-4 pair, 0 for neither.
+__device__ __forceinline__ int bonded_kind(int i, int j, const int *__restrict__ nnbb,
+                                           const int *__restrict__ inbb, int nbdmax) {
+  const int nb = nnbb[i], jf = j + 1;
+  for (int k = 0; k < nb; ++k) {
+    const int v = inbb[i * nbdmax + k];
+    if (v == jf) return -1;
+    if (v == -jf) return 3;
+  }
+  return 0;
+}
+
+// The prefilter's FP32 constants (formed on the host: an FP64 instruction
+// takes 64 cycles of a scheduler, and every warp is one atom): box, bounds
+// with their margins, cell widths, scales of the fixed-point positions.
+struct BuildF {
+  float bx, by, bz, hx, hy, hz;
+  float rl_hi, rl_lo, s_hi, s_lo, reach;
+  float cx, cy, cz, icx;
+  float sx, sy, sz;
+};
+
 // Exact classification (forces.f:1938-1981): 0 none, 1 short, 2 long,
 // 3 short 1-4, -1 excluded bonded pair.  LMNBL: the molecular cutoff (a
 // template parameter, so the atomic-cutoff build carries none of its code
@@ -200,20 +222,15 @@ __device__ __forceinline__ int classify_exact(
     }
   }
   if (same_mol && rr2 <= 64.0) {
-    int nb = nnbb[i];
-    const int jf = j + 1;
-    for (int k = 0; k < nb; ++k) {
-      int v = inbb[i * nbdmax + k];
-      if (v == jf) return -1;
-      if (v == -jf) return 3;
-    }
+    const int k = bonded_kind(i, j, nnbb, inbb, nbdmax);
+    if (k) return k;
   }
   if (rrm <= short2) return 1;
   if (rrm <= rl2) return 2;
   return 0;
 }
 
-template <int BLK, bool LMNBL>
+template <int BLK, bool LMNBL, bool FULL>
 __global__ void __launch_bounds__(BLK) k_build(
     int n, const dbl4 *__restrict__ pos, const float4 *__restrict__ posf,
     const int4 *__restrict__ ainfo, const int *__restrict__ nnbb,
@@ -223,107 +240,140 @@ __global__ void __launch_bounds__(BLK) k_build(
     double rl2, int cap_s,
     int cap_l, int *__restrict__ ns_cnt, int *__restrict__ nl_cnt,
     int *__restrict__ ns_idx, int *__restrict__ nl_idx, int *__restrict__ err,
-    int *__restrict__ need, int full, const int4 *__restrict__ posi, float sxf, float syf,
-    float szf, dbl4 *__restrict__ pos_ref, const int *__restrict__ gate, MolCut mc) {
-  // posi (mixed path): the prefilter takes the wrapped differences of the
-  // fixed-point positions and the molecule from their packed word, one
+    int *__restrict__ need, const int4 *__restrict__ posi, BuildF c,
+    dbl4 *__restrict__ pos_ref, const int *__restrict__ gate, MolCut mc) {
+  // FULL (mixed path): full rows; the prefilter takes the wrapped differences
+  // of the fixed-point positions and the molecule from their packed word, one
   // 16-byte gather per candidate
+  // A warp per atom, in cell order: the warps of a block read the same runs.
   const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * (BLK / 32) + (threadIdx.x >> 5);
-  if (i >= n || closed(gate)) return;
+  const int slot = blockIdx.x * (BLK / 32) + (threadIdx.x >> 5);
+  if (slot >= n || closed(gate)) return;
+  const int i = cell_list[slot];
   const dbl4 pi = pos[i];
   if (pos_ref && lane == 0) pos_ref[i] = pi;  // skin mode: positions of this build
   const float4 pf = posf[i];
   const int imol = ainfo[i].y;
-  const int4 qi = posi ? posi[i] : make_int4(0, 0, 0, 0);
+  const int4 qi = FULL ? posi[i] : make_int4(0, 0, 0, 0);
   const int c0 = atom_cell[i];
   const int cx0 = c0 % g.nx, cy0 = (c0 / g.nx) % g.ny, cz0 = c0 / (g.nx * g.ny);
-  const float fbx = (float)b.bx, fby = (float)b.by, fbz = (float)b.bz;
-  const float fhx = (float)b.hbx, fhy = (float)b.hby, fhz = (float)b.hbz;
-  const float rl2f_hi = (float)(rl2 * (1.0 + 1e-4)), rl2f_lo = (float)(rl2 * (1.0 - 1e-4));
-  const float s2f_hi = (float)(short2 * (1.0 + 1e-4)), s2f_lo = (float)(short2 * (1.0 - 1e-4));
   int ns = 0, nl = 0;
+  const unsigned lower = (1u << lane) - 1u;
+  int *const lrow = nl_idx + list_slot(i, 0, cap_l, false);
   constexpr int R = CELL_REACH, W = 2 * CELL_REACH + 1;
-  const int ox0 = g.nx >= W ? -R : 0, ox1 = g.nx >= W ? R : g.nx - 1;
   const int oy0 = g.ny >= W ? -R : 0, oy1 = g.ny >= W ? R : g.ny - 1;
   const int oz0 = g.nz >= W ? -R : 0, oz1 = g.nz >= W ? R : g.nz - 1;
   // offsets stay within one period (|o| <= R < W <= n): a conditional wrap,
   // no integer division
   auto wrap = [](int c, int n) { return c < 0 ? c + n : (c >= n ? c - n : c); };
-  auto wrapx = [&](int ox) { return g.nx >= W ? wrap(cx0 + ox, g.nx) : ox; };
-  for (int oz = oz0; oz <= oz1; ++oz)
-    for (int oy = oy0; oy <= oy1; ++oy) {
-      const int cy = g.ny >= W ? wrap(cy0 + oy, g.ny) : oy;
-      const int cz = g.nz >= W ? wrap(cz0 + oz, g.nz) : oz;
-      const int crow = (cz * g.ny + cy) * g.nx;
-      // the row's stencil cells in stencil order, consecutive cells merged
-      // into one run of the cell-sorted arrays (the order of candidates is
-      // unchanged)
-      for (int ox = ox0; ox <= ox1;) {
-        const int cxa = wrapx(ox);
-        int cxb = cxa;
-        while (ox < ox1 && wrapx(ox + 1) == cxb + 1) {
-          ++ox;
-          ++cxb;
+  // Rows of cells out of reach are left out and the others cut to the sphere
+  // (with a margin far above FP32 rounding): of the stencil's (5/2)^3 RL^3
+  // about half is left, and the order of what is left stays as it is.  The
+  // build is bound by issue (82 % active): 98,304 atoms, RL 12 A, 1.78 -> 0.82
+  // ms (mixed), 1.90 -> 0.95 (FP64), of it 0.3 by the cut and the cell order,
+  // 0.3 by the FP64 instructions left out (constants, own-molecule pairs).
+  const bool cut = !LMNBL && b.icell == 0;
+  auto place = [](float x, float L, float h, float cw, int k) {  // in the atom's cell
+    const float u = x + h - k * cw;
+    return u - L * rintf((u - 0.5f * cw) / L);
+  };
+  const float ux = place(pf.x, c.bx, c.hx, c.cx, cx0), uy = place(pf.y, c.by, c.hy, c.cy, cy0),
+              uz = place(pf.z, c.bz, c.hz, c.cz, cz0);
+  // from the atom to the cells at o along one axis (0: scanned whole)
+  auto gap = [&](int o, float u, float cw, int n) {
+    return !cut || n < W || o == 0 ? 0.f : o > 0 ? o * cw - u : u - (o + 1) * cw;
+  };
+  // candidates [s, e) of the cell order
+  auto run = [&](int s, int e) {
+    for (int base = s; base < e; base += 32) {
+      const int k = base + lane;
+      const bool in = k < e;
+      const int4 qj = cell_pos[in ? k : s];
+      int j = -1;
+      bool cand = in && k != slot;
+      if (!FULL) {
+        j = cell_list[in ? k : s];
+        cand = cand && owns(i, j);
+      }
+      const bool same = FULL ? ((unsigned)qj.w >> MDX_SITE_BITS) == ((unsigned)qi.w >> MDX_SITE_BITS)
+                             : qj.w == imol;
+      int kind = 0;
+      if (cut) {
+        float dx, dy, dz;
+        if (FULL) {
+          dx = fixdiff(qi.x, qj.x, c.sx);
+          dy = fixdiff(qi.y, qj.y, c.sy);
+          dz = fixdiff(qi.z, qj.z, c.sz);
+        } else {
+          dx = pf.x - __int_as_float(qj.x);
+          dy = pf.y - __int_as_float(qj.y);
+          dz = pf.z - __int_as_float(qj.z);
+          pbc_rectf(dx, dy, dz, c.bx, c.by, c.bz, c.hx, c.hy, c.hz);
         }
-        ++ox;
-        const int s = cell_start[crow + cxa], e = cell_start[crow + cxb + 1];
-        for (int base = s; base < e; base += 32) {
-          int kind = 0;
-          int j = -1;
-          if (base + lane < e) {
-            j = cell_list[base + lane];
-            const int4 qj = cell_pos[base + lane];  // independent of the load of j
-            if (j != i && (full || owns(i, j))) {
-              const bool same =
-                  posi ? ((unsigned)qj.w >> MDX_SITE_BITS) == ((unsigned)qi.w >> MDX_SITE_BITS)
-                       : qj.w == imol;
-              // the molecular cutoff and the non-rectangular cells: exact test only
-              if (same || LMNBL || b.icell) {
-                kind = classify_exact<LMNBL>(i, j, same, pi, pos[j], b, short2, rl2,
-                                      nnbb, inbb, nbdmax, mc);
-              } else {
-                float dx, dy, dz;
-                if (posi) {
-                  dx = fixdiff(qi.x, qj.x, sxf);
-                  dy = fixdiff(qi.y, qj.y, syf);
-                  dz = fixdiff(qi.z, qj.z, szf);
-                } else {
-                  dx = pf.x - __int_as_float(qj.x);
-                  dy = pf.y - __int_as_float(qj.y);
-                  dz = pf.z - __int_as_float(qj.z);
-                  pbc_rectf(dx, dy, dz, fbx, fby, fbz, fhx, fhy, fhz);
-                }
-                float d2 = dx * dx + dy * dy + dz * dz;
-                if (d2 > rl2f_hi) {
-                  kind = 0;
-                } else if (d2 < rl2f_lo && (d2 < s2f_lo || d2 > s2f_hi)) {
-                  kind = d2 < s2f_lo ? 1 : 2;
-                } else {
-                  kind = classify_exact<LMNBL>(i, j, false, pi, pos[j], b, short2, rl2,
-                                        nnbb, inbb, nbdmax, mc);
-                }
-              }
-            }
+        const float d2 = dx * dx + dy * dy + dz * dz;
+        const bool far = d2 > c.rl_hi, near = d2 < c.s_lo;
+        const bool plain = far || near || (d2 < c.rl_lo && d2 > c.s_hi);
+        if (cand) kind = far ? 0 : near ? 1 : 2;
+        if (cand && (same || !plain)) {  // few
+          if (FULL) j = cell_list[k];
+          if (!plain || fabsf(d2 - 64.f) < 0.02f) {
+            kind = classify_exact<LMNBL>(i, j, same, pi, pos[j], b, short2, rl2, nnbb, inbb,
+                                         nbdmax, mc);
+          } else if (d2 < 64.f) {
+            const int x = bonded_kind(i, j, nnbb, inbb, nbdmax);
+            if (x) kind = x;
           }
-          unsigned ms = __ballot_sync(0xffffffffu, kind == 1 || kind == 3);
-          unsigned ml = __ballot_sync(0xffffffffu, kind == 2);
-          unsigned lower = (1u << lane) - 1u;
-          // full rows (mixed path) hold the neighbour's cell-order slot
-          const int v = full ? base + lane : j;
-          if (kind == 1 || kind == 3) {
-            int k = ns + __popc(ms & lower);
-            if (k < cap_s)
-              ns_idx[list_slot(i, k, cap_s, full)] = v | (kind == 3 ? (int)0x80000000 : 0);
-          } else if (kind == 2) {
-            int k = nl + __popc(ml & lower);
-            if (k < cap_l) nl_idx[list_slot(i, k, cap_l, false)] = v;
-          }
-          ns += __popc(ms);
-          nl += __popc(ml);
         }
+      } else if (cand) {  // the molecular cutoff, other cells: exact test only
+        if (FULL) j = cell_list[k];
+        kind = classify_exact<LMNBL>(i, j, same, pi, pos[j], b, short2, rl2, nnbb, inbb, nbdmax,
+                                     mc);
+      }
+      const int v = FULL ? k : j;  // full rows hold the neighbour's cell-order slot
+      const unsigned ml = __ballot_sync(0xffffffffu, kind == 2);
+      const unsigned ms = __ballot_sync(0xffffffffu, kind == 1 || kind == 3);
+      const int kl = nl + __popc(ml & lower);
+      if (kind == 2 && kl < cap_l) lrow[kl] = v;
+      nl += __popc(ml);
+      if (ms) {
+        const int ks = ns + __popc(ms & lower);
+        if ((kind == 1 || kind == 3) && ks < cap_s)
+          ns_idx[list_slot(i, ks, cap_s, FULL)] = v | (kind == 3 ? (int)0x80000000 : 0);
+        ns += __popc(ms);
       }
     }
+  };
+  for (int oz = oz0; oz <= oz1; ++oz) {
+    const float gz = gap(oz, uz, c.cz, g.nz);
+    const int cz = g.nz >= W ? wrap(cz0 + oz, g.nz) : oz;
+    for (int oy = oy0; oy <= oy1; ++oy) {
+      const float gy = gap(oy, uy, c.cy, g.ny);
+      const float rem = c.reach - gy * gy - gz * gz;
+      if (rem < 0.f) continue;
+      const int cy = g.ny >= W ? wrap(cy0 + oy, g.ny) : oy;
+      const int *cs = cell_start + (size_t)(cz * g.ny + cy) * g.nx;
+      // the row's cells in stencil order: one run of the cell-sorted arrays,
+      // or two where it crosses the cell's face
+      int xa = 0, xb = g.nx - 1;
+      if (g.nx >= W) {
+        int oa = -R, ob = R;
+        if (cut) {
+          const float xr = sqrtf(rem);
+          oa = max(-R, (int)floorf((ux - xr) * c.icx));
+          ob = min(R, (int)floorf((ux + xr) * c.icx));
+        }
+        xa = cx0 + oa;
+        xb = cx0 + ob;
+      }
+      if (xa < 0) {
+        run(cs[xa + g.nx], cs[g.nx]);
+        xa = 0;
+      }
+      const int xe = min(xb, g.nx - 1);
+      run(cs[xa], cs[xe + 1]);
+      if (xb >= g.nx) run(cs[0], cs[xb - g.nx + 1]);
+    }
+  }
   if (lane == 0) {
     ns_cnt[i] = min(ns, cap_s);
     nl_cnt[i] = min(nl, cap_l);
@@ -525,17 +575,27 @@ static int build_lists(mdx_ctx *ctx, const int *gate) {
   int *need = d.shake_iter + 4;  // two ints of scratch after the SHAKE counter
   k_zero_gated<<<1, 32, 0, ctx->stream>>>(need, 2, gate);
   MDX_LAUNCHED(ctx);
+  const double s2 = ctx->p.rshort * ctx->p.rshort, rl2 = rl * rl;
+  BuildF bf{(float)b.bx, (float)b.by, (float)b.bz, (float)b.hbx, (float)b.hby, (float)b.hbz,
+            (float)(rl2 * (1.0 + 1e-4)), (float)(rl2 * (1.0 - 1e-4)), (float)(s2 * (1.0 + 1e-4)),
+            (float)(s2 * (1.0 - 1e-4)), (float)(1.001 * rl2), (float)g.cx, (float)g.cy,
+            (float)g.cz, (float)(1.0 / g.cx), (float)(ctx->boxl / 4294967296.0),
+            (float)(fix_period_y(ctx) / 4294967296.0), (float)(ctx->bozl / 4294967296.0)};
   const int BLK = 256;
-#define KB(L)                                                                              \
-  k_build<BLK, L><<<(d.n + BLK / 32 - 1) / (BLK / 32), BLK, 0, ctx->stream>>>(              \
+#define KB(L, F)                                                                           \
+  k_build<BLK, L, F><<<(d.n + BLK / 32 - 1) / (BLK / 32), BLK, 0, ctx->stream>>>(              \
       d.n, d.pos, d.posf, d.ainfo, d.nnbb, d.inbb, d.nbdmax, b, g, d.atom_cell,            \
       d.cell_start, d.cell_list, d.cell_pos, ctx->p.rshort * ctx->p.rshort, rl * rl,       \
       d.cap_s, d.cap_l, d.ns_cnt, d.nl_cnt, d.ns_idx, d.nl_idx, d.err, need,               \
-      ctx->mixed() ? 1 : 0, ctx->mixed() ? d.posi : nullptr,                               \
-      (float)(ctx->boxl / 4294967296.0), (float)(fix_period_y(ctx) / 4294967296.0),               \
-      (float)(ctx->bozl / 4294967296.0), pos_ref, gate, mol_cut(ctx))
-  if (ctx->p.lmnbl) KB(true);
-  else KB(false);
+      ctx->mixed() ? d.posi : nullptr,                                                     \
+      bf, pos_ref, gate, mol_cut(ctx))
+  if (ctx->mixed()) {
+    if (ctx->p.lmnbl) KB(true, true);
+    else KB(false, true);
+  } else {
+    if (ctx->p.lmnbl) KB(true, false);
+    else KB(false, false);
+  }
 #undef KB
   MDX_LAUNCHED(ctx);
   k_zero_gated<<<1, 32, 0, ctx->stream>>>(&d.sc->mbsh, 2, gate);
