@@ -1064,7 +1064,12 @@ int host_inifur(mdx_ctx *ctx) {
         &per_sm, zstep == 2 ? k_sfac32<2> : k_sfac32<1>, 128, sh));
     const int nib = std::max(1, ((int)items.size() + 127) / 128);
     int ns = std::max(1, std::max(1, per_sm) * nsm / nib);
-    ns = std::min(ns, std::max(1, d.n / 128));  // at least 128 atoms a slice
+    // at least 64 atoms a slice (609 atoms: 128 39 us, 64 31, 32 29, 16 27; but 32
+    // beads of 768 atoms at once: 17.15, 16.96, 17.4, 18.5 ms / 40 steps), or 128
+    // where the partial sums of 64 would not fit mdx_slforces_static's scratch
+    const int n64 = std::max(1, std::min(ns, d.n / 64));
+    const bool fits = (size_t)n64 * d.nkv * sizeof(double2) <= MDX_SK_STATIC_BYTES;
+    ns = fits ? n64 : std::max(1, std::min(ns, d.n / 128));
     d.sfac_slice = (d.n + ns - 1) / ns;
     d.sfac_nslice = (d.n + d.sfac_slice - 1) / d.sfac_slice;
     nslice_max = std::max(nslice_max, (size_t)d.sfac_nslice);
@@ -1256,11 +1261,10 @@ int ensure_kconst(mdx_ctx *ctx) {
   return MDX_OK;
 }
 
-int launch_furir(mdx_ctx *ctx) {
+int furir_first(mdx_ctx *ctx, bool *skip) {
   DevData &d = ctx->dv;
-  bool skip = false;
   int rc;
-  if ((rc = furir_sfac(ctx, &skip, true)) || skip) return rc;
+  if ((rc = furir_sfac(ctx, skip, true)) || *skip) return rc;
   const bool mx = ctx->mixed();
   {
     MDX_TIMER(ctx, MDX_T_EW_KTERMS);
@@ -1277,12 +1281,16 @@ int launch_furir(mdx_ctx *ctx) {
     }
   }
   MDX_TIMER(ctx, MDX_T_EW_FORCE);
-  const int rblocks = (d.n + RF_ATOMS - 1) / RF_ATOMS;
-  if (d.fx_on) {
-    return fx_force_launch(ctx);
-  } else if (mx && d.tc_on) {
-    return tc_force_launch(ctx);
-  } else if (mx) {
+  if (d.fx_on) return fx_force_launch(ctx);
+  return mx && d.tc_on ? tc_operands_launch(ctx) : MDX_OK;
+}
+
+int furir_force(mdx_ctx *ctx) {
+  DevData &d = ctx->dv;
+  MDX_TIMER(ctx, MDX_T_EW_FORCE);
+  if (d.fx_on) return fx_fold_launch(ctx);
+  if (ctx->mixed() && d.tc_on) return tc_force_launch(ctx);
+  if (ctx->mixed()) {
     const size_t shr = sizeof(float2) * RF_BATOMS * d.kz;
     const dim3 grid((d.n + RF_BATOMS - 1) / RF_BATOMS, d.rf_nsplit);
     auto kern = d.zstep == 2 ? k_rforce32<2> : k_rforce32<1>;
@@ -1290,6 +1298,7 @@ int launch_furir(mdx_ctx *ctx) {
         d.n, d.rf_part, d.kgroups, d.cols, d.wkf, d.tabxf, d.ldn, d.kx, d.ky, d.kz, d.colrvf,
         ctx->fix, d.gfix);
   } else {
+    const int rblocks = (d.n + RF_ATOMS - 1) / RF_ATOMS;
     k_rforce64<<<rblocks, RF_ATOMS * RF_PARTS, 0, ctx->stream>>>(
         d.n, d.ncol, d.cols, d.wp64, d.tabx, d.taby, d.tabz, d.colrv, d.gx, d.gy, d.gz);
   }

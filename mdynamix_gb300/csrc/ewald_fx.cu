@@ -1054,8 +1054,6 @@ int fx_sfac_launch(mdx_ctx *ctx) {
 
 int fx_force_launch(mdx_ctx *ctx) {
   DevData &d = ctx->dv;
-  const size_t accb = sizeof(long long) * (size_t)d.fx_ntm * d.fx_np * 128;
-  const int *bad = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(d.fx_acc) + accb) + 1;
   const int kp = d.fx_np, kxy = d.kx + d.ky;
   FxTile *meta = reinterpret_cast<FxTile *>(d.fx_meta);
   int *gexp = reinterpret_cast<int *>(d.fx_facc + 3 * (size_t)d.n);
@@ -1070,6 +1068,14 @@ int fx_force_launch(mdx_ctx *ctx) {
                                               d.fx_slot, d.fx_tw, d.fx_zf, d.fx_xy, d.fx_facc,
                                               gexp, d.err);
   MDX_LAUNCHED(ctx);
+  return MDX_OK;
+}
+// The force pass's sums into G.
+int fx_fold_launch(mdx_ctx *ctx) {
+  DevData &d = ctx->dv;
+  const size_t accb = sizeof(long long) * (size_t)d.fx_ntm * d.fx_np * 128;
+  const int *bad = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(d.fx_acc) + accb) + 1;
+  const int *gexp = reinterpret_cast<int *>(d.fx_facc + 3 * (size_t)d.n);
   const double two = 2.0 * PI_REF;
   k_fx_fold<<<(d.n + 255) / 256, 256, 0, ctx->stream>>>(
       d.n, d.fx_facc, gexp, d.fx_qs, bad, two / ctx->boxl,

@@ -27,8 +27,8 @@ __device__ __forceinline__ dbl4 kterm(double2 S, const double *__restrict__ q,
   return W;
 }
 inline Dst6 kterm_dst(const mdx_ctx *ctx, int nblocks) {
-  mdx_scalars *sc = ctx->dv.sc;
-  return dst6(ctx, nblocks, 5, &sc->pels1, &sc->virx, &sc->viry, &sc->virz, &sc->qpe);
+  double *k = ctx->dv.red + KT0;
+  return dst6(ctx, nblocks, 5, k, k + 1, k + 2, k + 3, k + 4);
 }
 
 // Force-pass operand layout of the mixed tensor-core pass (128 rows, K-major,

@@ -775,14 +775,18 @@ int tc_sfac_launch(mdx_ctx *ctx) {
   return MDX_OK;
 }
 
-// One step's tensor-core force pass: B tiles from W, then the GEMM + fold.
-int tc_force_launch(mdx_ctx *ctx) {
+// One step's tensor-core force pass: B tiles from W; then the GEMM + fold.
+int tc_operands_launch(mdx_ctx *ctx) {
   DevData &d = ctx->dv;
   const int q = d.tc_kp / 4;
   const int nth = d.tc_ntile * TC_N * q;
   k_wtiles<<<(nth + 255) / 256, 256, 0, ctx->stream>>>(d.tc_ntile, d.tc_kp, d.tc_slot, d.cols,
                                                        d.wk, d.colrvf, d.tc_w, d.tc_meta);
   MDX_LAUNCHED(ctx);
+  return MDX_OK;
+}
+int tc_force_launch(mdx_ctx *ctx) {
+  DevData &d = ctx->dv;
   CUtensorMap tm;
   int rc = encode_xy_map(ctx, &tm, TC_M);
   if (rc) return rc;

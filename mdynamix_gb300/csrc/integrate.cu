@@ -28,6 +28,7 @@ struct ZeroArgs {
   double spei, speei[MDX_NT];
   double *stat[3];
   int nstat[3];
+  double *kt;  // the k-vectors' sums
 };
 __global__ void k_zero_sums(ZeroArgs z) {
   const int k = threadIdx.x;
@@ -48,6 +49,7 @@ __global__ void k_zero_sums(ZeroArgs z) {
     sc->wirs = 0.; sc->vir1 = 0.; sc->pe1 = 0.; sc->pels1 = 0.;
     sc->virx = 0.; sc->viry = 0.; sc->virz = 0.; sc->qpe = 0.;
     sc->lscfl = 0;
+    for (int q = 0; q < 5; ++q) z.kt[q] = 0.0;
   }
   if (z.self) {
     if (k == 64) sc->spe = z.spei;
@@ -1785,6 +1787,7 @@ int launch_zero(mdx_ctx *ctx, int which, int laver) {
   z.molint = ctx->p.molint;
   z.ntypes = ctx->d.ntypes;
   z.self = (which & 2) && !ctx->p.lmnbl;
+  z.kt = d.red + KT0;
   z.spei = ctx->spei;
   for (int t = 0; t < MDX_NT; ++t) z.speei[t] = ctx->speei[t];
   if (laver) {

@@ -189,19 +189,15 @@ int require(mdx_ctx *ctx, bool topo, bool par, bool state) {
 // ---------------------------------------------------------------- forces
 // mirrored: GETCOM has just refreshed the FP32 and fixed-point mirrors of the
 // positions.
-int fforces_parts(mdx_ctx *ctx, int laver, bool split, bool mirrored);
+int mirror_positions(mdx_ctx *ctx);
 int do_fforces(mdx_ctx *ctx, int laver, bool split, bool mirrored = false) {
   RC(launch_zero(ctx, 1, laver));
-  return fforces_parts(ctx, laver, split, mirrored);
-}
-int fforces_parts(mdx_ctx *ctx, int laver, bool split, bool mirrored) {
-  if (!mirrored) RC(ctx->mixed() ? launch_mirror_f32(ctx) : launch_ipos(ctx));
+  if (!mirrored) RC(mirror_positions(ctx));
   RC(launch_localf(ctx, split));
   RC(launch_wir(ctx, 1));  // WIRSS from the pair forces, before the bonded terms
   RC(launch_bonded(ctx, laver));
   if (ctx->mixed()) RC(launch_fix_to_double(ctx, 1));
-  RC(launch_sclfrc(ctx, 1));
-  return MDX_OK;
+  return launch_sclfrc(ctx, 1);
 }
 
 // FFORCES of an intermediate short step (forces only, the fast forces cleared
@@ -212,7 +208,7 @@ int fforces_parts(mdx_ctx *ctx, int laver, bool split, bool mirrored) {
 int do_fforces_mid(mdx_ctx *ctx, bool fold) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   MDX_CUDA(cudaStreamIsCapturing(ctx->stream, &st));
-  const bool fork = st == cudaStreamCaptureStatusActive && ctx->side;
+  const bool fork = st == cudaStreamCaptureStatusActive;
   if (fork) {
     MDX_CUDA(cudaEventRecord(ctx->side_ev[0], ctx->stream));
     MDX_CUDA(cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0));
@@ -232,34 +228,72 @@ int do_fforces_mid(mdx_ctx *ctx, bool fold) {
   return MDX_OK;
 }
 
-int do_slow_parts(mdx_ctx *ctx, bool split, bool mirrored = false, bool types = true) {
-  if (ctx->mixed()) {
-    if (!mirrored) RC(launch_mirror_f32(ctx));
-    RC(launch_forces_long(ctx, split, types));  // stores G first
-    RC(launch_furir(ctx));
-    RC(launch_eterms(ctx));
-    RC(launch_fold_wirs(ctx));
+// SLFORCES' parts and, for laver >= 0, FFORCES' (their sums cleared, positions
+// mirrored).  Reciprocal space up to its force pass needs nothing of the pair
+// sweeps, so it runs beside them on the second stream: below some 20,000 atoms
+// neither fills the GPU (3,000 atoms FP64: 75 us beside 96; 609 mixed: 55
+// beside 60).  The mixed force pass adds to G's integers once the long sweep
+// and ETERMS have, the FP64 one at the end.  No fork with the timers on.
+int force_parts_on(mdx_ctx *ctx, bool split, bool types, int laver, bool fork) {
+  const bool mx = ctx->mixed();
+  bool skip = true;
+  auto beside = [&](auto &&f) {
+    std::swap(ctx->stream, ctx->side);
+    ctx->red_slot = 1;
+    const int rc = f();
+    ctx->red_slot = 0;
+    std::swap(ctx->stream, ctx->side);
+    return rc;
+  };
+  if (fork) {
+    MDX_CUDA(cudaEventRecord(ctx->side_ev[0], ctx->stream));
+    MDX_CUDA(cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0));
+    RC(beside([&] { return furir_first(ctx, &skip); }));
   } else {
-    if (!mirrored) RC(launch_ipos(ctx));
-    RC(launch_furir(ctx));
-    RC(launch_eterms(ctx));
-    RC(launch_forces_long(ctx, split, types));
-    RC(launch_wir(ctx, 2));
+    RC(furir_first(ctx, &skip));
   }
-  return MDX_OK;
+  RC(launch_forces_long(ctx, split, types));  // mixed: stores G first
+  RC(launch_eterms(ctx));
+  if (fork) {
+    if (mx && !skip) {
+      MDX_CUDA(cudaEventRecord(ctx->side_ev[2], ctx->stream));
+      MDX_CUDA(cudaStreamWaitEvent(ctx->side, ctx->side_ev[2], 0));
+      RC(beside([&] { return furir_force(ctx); }));
+    }
+    MDX_CUDA(cudaEventRecord(ctx->side_ev[3], ctx->side));
+  }
+  if (laver >= 0) {
+    RC(launch_localf(ctx, split));
+    RC(launch_wir(ctx, 1));  // WIRSS from the pair forces, before the bonded terms
+    RC(launch_bonded(ctx, laver));
+    if (mx) RC(launch_fix_to_double(ctx, 1));
+  }
+  if (fork) MDX_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->side_ev[3], 0));
+  if (!skip && !(fork && mx)) RC(furir_force(ctx));
+  return mx ? launch_fold_wirs(ctx) : launch_wir(ctx, 2);
 }
 
-int slforces_parts(mdx_ctx *ctx, bool split, bool mirrored, bool types = true) {
-  RC(do_slow_parts(ctx, split, mirrored, types));
-  RC(launch_pullback(ctx));
-  RC(launch_sclfrc(ctx, 2));
-  return MDX_OK;
+int force_parts(mdx_ctx *ctx, bool split, bool types, int laver) {
+  const bool fork = !ctx->timing && ctx->p.alphad > 0.0;
+  const int rc = force_parts_on(ctx, split, types, laver, fork);
+  if (rc && fork) {  // whatever was launched beside ends before what comes next
+    cudaEventRecord(ctx->side_ev[3], ctx->side);
+    cudaStreamWaitEvent(ctx->stream, ctx->side_ev[3], 0);
+  }
+  return rc;
+}
+
+int mirror_positions(mdx_ctx *ctx) {
+  return ctx->mixed() ? launch_mirror_f32(ctx) : launch_ipos(ctx);
 }
 
 int do_slforces(mdx_ctx *ctx, bool split, bool mirrored = false) {
   RC(furir_prepare(ctx));  // SPE's self terms are set with the zeroing
   RC(launch_zero(ctx, 2));
-  return slforces_parts(ctx, split, mirrored);
+  if (!mirrored) RC(mirror_positions(ctx));
+  RC(force_parts(ctx, split, true, -1));
+  RC(launch_pullback(ctx));
+  return launch_sclfrc(ctx, 2);
 }
 
 // SLFORCES then FFORCES of a step's end (mirrored positions), their sums cleared
@@ -267,25 +301,23 @@ int do_slforces(mdx_ctx *ctx, bool split, bool mirrored = false) {
 int do_both(mdx_ctx *ctx, int laver) {
   RC(furir_prepare(ctx));
   RC(launch_zero(ctx, 3, laver));
-  RC(slforces_parts(ctx, false, true, false));
-  return fforces_parts(ctx, laver, false, true);
+  RC(force_parts(ctx, false, false, laver));
+  RC(launch_pullback(ctx));
+  RC(launch_sclfrc(ctx, 2));
+  return launch_sclfrc(ctx, 1);
 }
 
 int do_allforce(mdx_ctx *ctx, bool split, bool laver = false) {
+  const int lav = split || laver ? 1 : 0;
   RC(furir_prepare(ctx));
-  RC(launch_zero(ctx, 3, split || laver ? 1 : 0));
-  RC(ctx->mixed() ? launch_mirror_f32(ctx) : launch_ipos(ctx));
-  RC(launch_localf(ctx, split));
-  RC(launch_wir(ctx, 1));  // WIRSS from the pair forces, before the bonded terms
-  RC(launch_bonded(ctx, split || laver ? 1 : 0));
-  if (ctx->mixed()) RC(launch_fix_to_double(ctx, 1));
-  RC(do_slow_parts(ctx, split, !ctx->mixed()));
+  RC(launch_zero(ctx, 3, lav));
+  RC(mirror_positions(ctx));
+  RC(force_parts(ctx, split, true, lav));
   RC(launch_sum_forces(ctx));
   // PULLBACK adds to G after CM_ADDLA has formed F (forces.f:88-95): SULTAN,
   // which moves with F, does not see it -- the reference's order, kept
   RC(launch_pullback(ctx));
-  RC(launch_sclfrc(ctx, 3));
-  return MDX_OK;
+  return launch_sclfrc(ctx, 3);
 }
 
 int sync_box_from_device(mdx_ctx *ctx) {
@@ -366,11 +398,6 @@ int graph_step(mdx_ctx *ctx, int mstep, bool rec, bool dbl) {
   const int g = (list ? 1 : 0) + (rec ? 2 : 0) + (dbl ? 0 : 4);
   if (!ctx->gexec[g]) {
     const int64_t l0 = ctx->launches;
-    if (!ctx->side) {
-      for (auto &e : ctx->side_ev)
-        if (!e) MDX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-      MDX_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
-    }
     MDX_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     int rc = dbl ? double_step(ctx, mstep, rec ? -1 : -2) : sultan_step(ctx, mstep, rec ? -1 : -2);
     cudaGraph_t graph = nullptr;
@@ -489,7 +516,15 @@ int mdx_open(const mdx_dims *dims, mdx_ctx **out) {
     const char *g = getenv("MDX_GRAPHS");
     if (g && g[0] == '0') ctx->use_graphs = false;
   }
-  if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) {
+  bool made = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) == cudaSuccess &&
+              cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) == cudaSuccess;
+  for (auto &e : ctx->side_ev)
+    made = made && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+  if (!made) {
+    for (auto e : ctx->side_ev)
+      if (e) cudaEventDestroy(e);
+    if (ctx->side) cudaStreamDestroy(ctx->side);
+    if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return MDX_ERR_CUDA;
   }
@@ -537,8 +572,8 @@ int mdx_open(const mdx_dims *dims, mdx_ctx **out) {
   AL(d.err, 4);
   AL(d.shake_iter, 32);
   AL(d.red, 512);
-  AL(d.red_part, (size_t)1 << 21);
-  AL(d.red_ctr, 8);
+  AL(d.red_part, ((size_t)1 << 21) + RED_CAP1);
+  AL(d.red_ctr, 16);
   d.red_cap = (size_t)1 << 21;
   if (!rc) {
     unsigned char *ss = nullptr;

@@ -355,9 +355,11 @@ struct mdx_ctx {
       }
   }
   double pair_tab_alpha = 0.0;  // alpha of dv.pair_tab
-  // branch of a captured step (bonded terms beside the short sweep)
+  // second stream of the force routines (bonded terms beside the short sweep,
+  // reciprocal space beside the pair sweeps) and its events
   cudaStream_t side = nullptr;
-  cudaEvent_t side_ev[2] = {};
+  cudaEvent_t side_ev[4] = {};
+  int red_slot = 0;  // 1 while launching on it: its reductions have their own scratch
   // FP64 path, fixed-point pair sweeps: on, position unit 2^-px_bits A (of the
   // box when ipos was last written), charge unit 2^(px_eq - 62) e, and the
   // sweeps' ranges (0 short, 1 long): |d| < 2^px_rho A, r^2 >= 2^px_oct A^2;
@@ -398,6 +400,9 @@ inline double fix_period_y(const mdx_ctx *ctx) {
   return ctx->p.icell == 2 ? 2.0 * ctx->boyl : ctx->boyl;
 }
 
+// Doubles and counters behind the main stream's: the second stream's.
+constexpr size_t RED_CAP1 = (size_t)1 << 19;
+
 // Reduction destinations for a launch of nblocks blocks reducing nv values:
 // deterministic (partials + ordered sum) whenever the partials buffer is
 // large enough.
@@ -405,9 +410,10 @@ inline Dst6 dst6(const mdx_ctx *ctx, size_t nblocks, int nv, double *a,
                  double *b = nullptr, double *c = nullptr, double *d = nullptr,
                  double *e = nullptr, double *f = nullptr) {
   Dst6 r{{a, b, c, d, e, f}, nullptr, nullptr};
-  if (ctx->dv.red_part && nblocks * (size_t)nv <= ctx->dv.red_cap) {
-    r.part = ctx->dv.red_part;
-    r.ctr = ctx->dv.red_ctr;
+  const size_t cap = ctx->red_slot ? RED_CAP1 : ctx->dv.red_cap;
+  if (ctx->dv.red_part && nblocks * (size_t)nv <= cap) {
+    r.part = ctx->dv.red_part + (ctx->red_slot ? ctx->dv.red_cap : 0);
+    r.ctr = ctx->dv.red_ctr + 8 * ctx->red_slot;
   }
   return r;
 }
@@ -820,7 +826,13 @@ int launch_wir(mdx_ctx *ctx, int which);  // WIRSS (1) / WIRS (2)
 // ewald.cu
 int host_inifur(mdx_ctx *ctx);
 int furir_prepare(mdx_ctx *ctx);  // k-set check (host), INIFUR when due
-int launch_furir(mdx_ctx *ctx);
+// FURIR in two parts: up to the force pass's operands (FP64 tensor path: the
+// forces, in its own accumulators), which leaves G and mdx_scalars alone; then
+// the forces into G.  The k-vectors' sums go to d.red + KT0 (wirs_kterms adds
+// them).
+int furir_first(mdx_ctx *ctx, bool *skip);
+int furir_force(mdx_ctx *ctx);
+constexpr int KT0 = 40;
 int furir_sfac(mdx_ctx *ctx, bool *skip, bool terms = false);  // k-set check, phase tables, S(k) into d.sk
 int ensure_kconst(mdx_ctx *ctx);           // per-k constants of the current box
 int launch_eterms(mdx_ctx *ctx);
@@ -837,7 +849,9 @@ int fx_update_qscale(mdx_ctx *ctx);
 int fx_tables_launch(mdx_ctx *ctx);
 int fx_sfac_launch(mdx_ctx *ctx);
 int fx_force_launch(mdx_ctx *ctx);
+int fx_fold_launch(mdx_ctx *ctx);
 int tc_zimages_launch(mdx_ctx *ctx);
+int tc_operands_launch(mdx_ctx *ctx);
 int tc_force_launch(mdx_ctx *ctx);
 // Dynamic shared-memory limit of a kernel: process-wide, shared by every
 // context, so it is only ever raised (under a lock).

@@ -40,13 +40,27 @@ __device__ __forceinline__ float ewald_erfc_polyf(float ttt, float exp2a) {
            (float)MDX_A2) * ttt + (float)MDX_A1) * ttt * exp2a;
 }
 
+// The k-vectors' sums (FURIR, formed beside the sweeps) into PELS1, the virial
+// projections and QPE, by the pass over the finished G.
+__device__ __forceinline__ void add_kterms(const double *__restrict__ kt,
+                                           mdx_scalars *__restrict__ sc) {
+  if (!kt || blockIdx.x != 0 || threadIdx.x != 0) return;
+  sc->pels1 += kt[0];
+  sc->virx += kt[1];
+  sc->viry += kt[2];
+  sc->virz += kt[3];
+  sc->qpe += kt[4];
+}
+
 // WIRSS / WIRS: -sum F . (S - COM(molecule)) (forces.f:991-995,
 // scalar.f:77-82), FP64 path.
 __global__ void k_wir(int n, const dbl4 *__restrict__ pos,
                       const int4 *__restrict__ ainfo, const double *__restrict__ X,
                       const double *__restrict__ Y, const double *__restrict__ Z,
                       const double *__restrict__ fx, const double *__restrict__ fy,
-                      const double *__restrict__ fz, Dst6 dst) {
+                      const double *__restrict__ fz, Dst6 dst, const double *__restrict__ kt,
+                      mdx_scalars *__restrict__ sc) {
+  add_kterms(kt, sc);
   double w[1] = {0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += gridDim.x * blockDim.x) {
@@ -63,7 +77,9 @@ __global__ void k_add_wir(int n, const dbl4 *__restrict__ pos, const int4 *__res
                           const double *__restrict__ X, const double *__restrict__ Y,
                           const double *__restrict__ Z, unsigned long long *__restrict__ f,
                           double unit, double *__restrict__ fx, double *__restrict__ fy,
-                          double *__restrict__ fz, Dst6 dst) {
+                          double *__restrict__ fz, Dst6 dst, const double *__restrict__ kt,
+                          mdx_scalars *__restrict__ sc) {
+  add_kterms(kt, sc);
   double w[1] = {0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const dbl4 p = pos[i];
@@ -87,7 +103,9 @@ __global__ void k_fold_wirs(int n, const dbl4 *__restrict__ pos, const int4 *__r
                             const double *__restrict__ Z,
                             const unsigned long long *__restrict__ f, double inv,
                             double *__restrict__ gx, double *__restrict__ gy,
-                            double *__restrict__ gz, Dst6 dst) {
+                            double *__restrict__ gz, Dst6 dst, const double *__restrict__ kt,
+                            mdx_scalars *__restrict__ sc) {
+  add_kterms(kt, sc);
   double w[1] = {0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const dbl4 p = pos[i];
@@ -998,7 +1016,7 @@ int launch_fold_wirs(mdx_ctx *ctx) {
   const int nb = red_blocks(ctx);
   k_fold_wirs<<<nb, 256, 0, ctx->stream>>>(d.n, d.pos, d.ainfo, d.X, d.Y, d.Z, d.gfix,
                                            ctx->fix.inv, d.gx, d.gy, d.gz,
-                                           dst6(ctx, nb, 1, &d.sc->wirs));
+                                           dst6(ctx, nb, 1, &d.sc->wirs), d.red + KT0, d.sc);
   MDX_LAUNCHED(ctx);
   return MDX_OK;
 }
@@ -1017,16 +1035,17 @@ int launch_wir(mdx_ctx *ctx, int which) {
   double *fx = which == 1 ? d.hx : d.gx, *fy = which == 1 ? d.hy : d.gy,
          *fz = which == 1 ? d.hz : d.gz;
   const int nbw = red_blocks(ctx);
+  const double *kt = which == 2 ? d.red + KT0 : nullptr;
   if (ctx->px_on) {
     k_add_wir<<<nbw, 256, 0, ctx->stream>>>(d.n, d.pos, d.ainfo, d.X, d.Y, d.Z,
                                             which == 1 ? d.hfix : d.gfix,
                                             px_force_unit(ctx, which), fx, fy, fz,
-                                            dst6(ctx, nbw, 1, dst));
+                                            dst6(ctx, nbw, 1, dst), kt, d.sc);
     MDX_LAUNCHED(ctx);
     return MDX_OK;
   }
   k_wir<<<nbw, 256, 0, ctx->stream>>>(d.n, d.pos, d.ainfo, d.X, d.Y, d.Z, fx, fy, fz,
-                                      dst6(ctx, nbw, 1, dst));
+                                      dst6(ctx, nbw, 1, dst), kt, d.sc);
   MDX_LAUNCHED(ctx);
   return MDX_OK;
 }
