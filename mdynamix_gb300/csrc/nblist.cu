@@ -272,7 +272,11 @@ __global__ void __launch_bounds__(BLK) k_build(
   // build is bound by issue (82 % active): 98,304 atoms, RL 12 A, 1.78 -> 0.82
   // ms (mixed), 1.90 -> 0.95 (FP64), of it 0.3 by the cut and the cell order,
   // 0.3 by the FP64 instructions left out (constants, own-molecule pairs).
-  const bool cut = !LMNBL && b.icell == 0;
+  const bool rect = !LMNBL && b.icell == 0;
+  // not for a position many boxes away (or not a number): its place in the
+  // cell is not known in FP32
+  const bool cut = rect && fabsf(pf.x) < 16.f * c.bx && fabsf(pf.y) < 16.f * c.by &&
+                   fabsf(pf.z) < 16.f * c.bz;
   auto place = [](float x, float L, float h, float cw, int k) {  // in the atom's cell
     const float u = x + h - k * cw;
     return u - L * rintf((u - 0.5f * cw) / L);
@@ -298,7 +302,7 @@ __global__ void __launch_bounds__(BLK) k_build(
       const bool same = FULL ? ((unsigned)qj.w >> MDX_SITE_BITS) == ((unsigned)qi.w >> MDX_SITE_BITS)
                              : qj.w == imol;
       int kind = 0;
-      if (cut) {
+      if (rect) {
         float dx, dy, dz;
         if (FULL) {
           dx = fixdiff(qi.x, qj.x, c.sx);
@@ -359,8 +363,8 @@ __global__ void __launch_bounds__(BLK) k_build(
         int oa = -R, ob = R;
         if (cut) {
           const float xr = sqrtf(rem);
-          oa = max(-R, (int)floorf((ux - xr) * c.icx));
-          ob = min(R, (int)floorf((ux + xr) * c.icx));
+          oa = min(max((int)floorf((ux - xr) * c.icx), -R), R);
+          ob = min(max((int)floorf((ux + xr) * c.icx), oa), R);
         }
         xa = cx0 + oa;
         xb = cx0 + ob;

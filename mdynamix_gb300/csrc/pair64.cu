@@ -1016,7 +1016,7 @@ int pair64_setup(mdx_ctx *ctx) {
       ctx->p.rshort > 2.0 && 1.2 * ctx->p.rshort < 8.0) {
     ctx->px_eq = std::ilogb(qmax) + (std::ldexp(1.0, std::ilogb(qmax)) < qmax ? 1 : 0);
     ctx->px_rho[0] = rho(1.2 * ctx->p.rshort);
-    ctx->px_rho[1] = rho(rl);
+    ctx->px_rho[1] = std::max(rho(rl), ctx->px_rho[0]);  // RCUT may lie below RSHORT
     ctx->px_oct[0] = 1;
     ctx->px_oct[1] = std::max(1, std::ilogb(0.64 * ctx->p.rshort * ctx->p.rshort));
     const int nb[2] = {px_bins(ctx, 0), px_bins(ctx, 1)};
