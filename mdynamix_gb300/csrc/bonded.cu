@@ -28,7 +28,6 @@ struct BondOut {
   float sx, sy, sz;   // box / 2^32
   float limx, limy, limz;  // 0.99 x half box: below it no minimum-image shift
   CellPbc cell;            // cell shape (FP64 path: hexagonal / octahedral PBC)
-  bool shared;             // the short sweep adds to the same forces meanwhile
 };
 
 // Fixed-point force term: R = float rounds v * 2^k with FP32 operations only
@@ -100,12 +99,21 @@ __device__ __forceinline__ void vec_r(const dbl4 *pos, const BondOut &o, int a, 
   }
 }
 
+// Square root and its reciprocal.  FP64: from the reciprocal root, a Newton step
+// making the root that of SQRT but for the last bit's rounding, in a third of
+// the instructions of the two.  FP32 keeps the rounded root and division: they
+// cost little there, and stiff bonds show every rounding.
 template <typename R>
-__device__ __forceinline__ R rsqrt_t(R x);
-template <>
-__device__ __forceinline__ double rsqrt_t<double>(double x) { return 1.0 / sqrt(x); }
-template <>
-__device__ __forceinline__ float rsqrt_t<float>(float x) { return 1.0f / sqrtf(x); }
+__device__ __forceinline__ void root(R x, R &s, R &si) {
+  if constexpr (sizeof(R) == sizeof(float)) {
+    s = sqrt(x);
+    si = R(1) / s;
+  } else {
+    const R r = rsqrt(x), a = x * r;
+    s = fma(R(0.5) * r, fma(-a, a, x), a);
+    si = r;
+  }
+}
 
 // Per-record average accumulation into shared arrays (only when averaging).
 __device__ __forceinline__ void avg_add(double *sh, double *gl, int m, int nrec,
@@ -120,10 +128,6 @@ __device__ __forceinline__ void avg_add(double *sh, double *gl, int m, int nrec,
 // molecule-local kernel); the same per-term rounding as add_force.
 template <typename R>
 __device__ __forceinline__ void add_force_own(const BondOut &o, int i, R fx, R fy, R fz) {
-  if (o.shared) {
-    add_force<R>(o, i, fx, fy, fz);
-    return;
-  }
   if (o.hfix) {
     o.hfix[i] += (unsigned long long)fix_term<R>(o, fx);
     o.hfix[o.n + i] += (unsigned long long)fix_term<R>(o, fy);
@@ -150,8 +154,8 @@ __device__ __forceinline__ void bond_term(const dbl4 *__restrict__ pos, int I, i
   vec_r<R>(pos, o, J, I, bx, by, bz, BX, BY, BZ);
   const R REQ = (R)rb[M];
   const R BSQ = BX * BX + BY * BY + BZ * BZ;
-  const R BD = sqrt(BSQ);
-  const R R1I = R(1) / BD;
+  R BD, R1I;
+  root(BSQ, BD, R1I);
   const R BBB = BD - REQ;
   R EBDD, FORB;
   if (bid[M] != 1 || BBB > REQ) {
@@ -196,18 +200,28 @@ __device__ __forceinline__ void angle_term(const dbl4 *__restrict__ pos, int I, 
   vec_r<R>(pos, o, I, J, bx, by, bz, AX, AY, AZ);
   vec_r<R>(pos, o, K, J, bx, by, bz, BX, BY, BZ);
   const R ASQ = AX * AX + AY * AY + AZ * AZ;
-  const R ASQI = R(1) / ASQ;
   const R BSQ = BX * BX + BY * BY + BZ * BZ;
-  const R BSQI = R(1) / BSQ;
-  const R AB = sqrt(ASQ * BSQ);
-  const R ABI = R(1) / AB;
+  R AB, ABI;
+  root(ASQ * BSQ, AB, ABI);
+  R ASQI, BSQI;
+  if constexpr (sizeof(R) == sizeof(float)) {
+    ASQI = R(1) / ASQ;
+    BSQI = R(1) / BSQ;
+  } else {
+    ASQI = BSQ * (ABI * ABI);
+    BSQI = ASQ * (ABI * ABI);
+  }
   R COSA = AX * BX + AY * BY + AZ * BZ;
   COSA = COSA * ABI;
   COSA = fmin(COSA, R(1));
   COSA = fmax(COSA, R(-1));
   const R ALF = acos(COSA);
-  const R SINA = sin(ALF);
-  const R SINAI = R(1) / SINA;
+  // FP64: the sine from the cosine, exact differences, so at least as good as
+  // SIN(ALF) (which a straight angle takes, as the reference)
+  R SINA, SINAI;
+  const R S2 = (R(1) - COSA) * (R(1) + COSA);
+  if (sizeof(R) == sizeof(double) && S2 > R(0)) root(S2, SINA, SINAI);
+  else SINAI = R(1) / sin(ALF);
   const R DALF = ALF - AEQ;
   const R ABC = DALF * FCN;
   const R EANG = ABC * DALF;
@@ -237,7 +251,7 @@ __device__ __forceinline__ void angle_term(const dbl4 *__restrict__ pos, int I, 
   }
 }
 
-template <typename R, bool ENER>
+template <typename R>
 __global__ void k_getbnd(int nrbt, const int *__restrict__ ibi,
                          const int *__restrict__ jbj, const int *__restrict__ ibuk,
                          const int *__restrict__ bid, const double *__restrict__ rb,
@@ -266,7 +280,7 @@ __global__ void k_getbnd(int nrbt, const int *__restrict__ ibi,
       avg_add(sbe, be, M, nrbb, (double)EB * fnspi);
     }
   }
-  if (ENER) block_add<5>(acc, dst);
+  block_add<5>(acc, dst);
   if (laver && nrbb <= 256) {
     __syncthreads();
     for (int k = threadIdx.x; k < nrbb; k += blockDim.x) {
@@ -276,7 +290,7 @@ __global__ void k_getbnd(int nrbt, const int *__restrict__ ibi,
   }
 }
 
-template <typename R, bool ENER>
+template <typename R>
 __global__ void k_getang(int nrat, const int *__restrict__ iai,
                          const int *__restrict__ jaj, const int *__restrict__ kak,
                          const int *__restrict__ iauk, const double *__restrict__ ra,
@@ -304,10 +318,8 @@ __global__ void k_getang(int nrat, const int *__restrict__ iai,
       avg_add(sae, ae, M, nraa, (double)EA * fnspi);
     }
   }
-  if (ENER) {
-    double a4[4] = {acc[0], acc[2], acc[3], acc[4]};
-    block_add<4>(a4, dst);
-  }
+  double a4[4] = {acc[0], acc[2], acc[3], acc[4]};
+  block_add<4>(a4, dst);
   if (laver && nraa <= 256) {
     __syncthreads();
     for (int k = threadIdx.x; k < nraa; k += blockDim.x) {
@@ -320,7 +332,7 @@ __global__ void k_getang(int nrat, const int *__restrict__ iai,
 // Bonds and angles of small molecule types, one thread per molecule: every
 // atom a thread touches belongs to its molecule, so forces are added
 // without atomics (same per-term rounding, so the sums are identical).
-template <typename R, bool ENER>
+template <typename R>
 __global__ void __launch_bounds__(128) k_molbonded(
     int ntpl, const MolTpl *__restrict__ tpl, const int *__restrict__ bid,
     const double *__restrict__ rb, const double *__restrict__ fb,
@@ -383,17 +395,15 @@ __global__ void __launch_bounds__(128) k_molbonded(
       }
     }
   }
-  if (ENER) {
-    double a[5];
-    if (sizeof(R) == sizeof(double)) {
+  double a[5];
+  if (sizeof(R) == sizeof(double)) {
 #pragma unroll
-      for (int k = 0; k < 5; ++k) a[k] = (double)acc[k];
-      block_add<5>(a, dst);
-    } else {  // warp sums in FP32, then the FP64 block sums
+    for (int k = 0; k < 5; ++k) a[k] = (double)acc[k];
+    block_add<5>(a, dst);
+  } else {  // warp sums in FP32, then the FP64 block sums
 #pragma unroll
-      for (int k = 0; k < 5; ++k) a[k] = (double)warp_sumf((float)acc[k]);
-      block_add_core<5, true>(a, dst.p, dst.part, dst.ctr);
-    }
+    for (int k = 0; k < 5; ++k) a[k] = (double)warp_sumf((float)acc[k]);
+    block_add_core<5, true>(a, dst.p, dst.part, dst.ctr);
   }
   if (laver) {
     __syncthreads();
@@ -674,21 +684,23 @@ __global__ void k_strbnd(WaterPar w, const dbl4 *__restrict__ pos, double bxl,
   }
 }
 
-// All intramolecular terms of an FFORCES without statistics in one launch,
-// where there is more than one kind: a block is of one kind (thread per water,
-// templated molecule, bond, angle or torsion).  The kinds share no atom
-// unsafely (template molecules are of their own types, the others add with
-// atomics).  In a small system each kind's launch is a few latency-bound
-// microseconds.  The one launch measured 16 us (forces only; solute in 211
-// waters) and 29 us (with energies; bilayer of 22,529 atoms), most of it fetching
-// its code; the solute's step took 11.9 ms / 1600 before, 7.7 after, the
-// bilayer's 9.1 and 9.0.
+// All intramolecular terms of an FFORCES without statistics in one launch: a
+// block is of one kind (thread per water of STRBND, bond, angle or torsion;
+// of template molecules one term of 128 molecules, mblk).  Forces are added
+// with atomics.  A small system is bound by the longest chain of instructions
+// and by fetching them: an FP64 instruction takes 64 cycles of a scheduler
+// however few warps there are, so a molecule's terms go to different warps,
+// and there is one copy of each term's code.  Forces only, a thread a
+// molecule and a thread a term (with the roots of root()): 3,000 atoms FP64 21.4,
+// 12.5 us; 609 atoms mixed 13.3, 9.6; 98,304 atoms FP64 26.6, 24.6, mixed 13.9,
+// 12.6 (2 us of each are the timer's).
 enum { BK_MOL = MDX_NT, BK_BOND, BK_ANGLE, BK_TORS, BK_N };  // 0 .. MDX_NT - 1: waters
 struct BondedAll {
   int blk[BK_N + 1];  // first block of each kind (waters by type first)
   WaterPar w[MDX_NT];
-  int ntpl, nrbt, nrat, nrrt;
+  int nrbt, nrat, nrrt;
   const MolTpl *tpl;
+  const int2 *mblk;  // template and term (bonds, then angles), first molecule
   const int *bid, *ibi, *jbj, *ibuk, *iai, *jaj, *kak, *iauk;
   const double *rb, *fb, *db, *ro, *ra, *fa;
   TorsList q;
@@ -707,34 +719,41 @@ __global__ void __launch_bounds__(128) k_bonded_all(BondedAll a, const dbl4 *__r
   if (kind < BK_MOL) {
     R len[3], en[3];
     if (N < a.w[kind].nmol) water_term<R>(a.w[kind], N, pos, bx, by, bz, o, acc, len, en);
-  } else if (kind == BK_MOL) {
-    int t = 0;
-    while (t < a.ntpl && N >= a.tpl[t].nmol) {
-      N -= a.tpl[t].nmol;
-      ++t;
+  } else if (kind < BK_TORS) {
+    int I = -1, J = 0, K = 0, M = 0, lmove = 0;
+    bool angle = kind == BK_ANGLE;
+    if (kind == BK_MOL) {
+      const int2 m = a.mblk[(int)blockIdx.x - a.blk[kind]];
+      const MolTpl &T = a.tpl[m.x & 255];
+      const int k = m.x >> 8, g = m.y + threadIdx.x, base = T.first + g * T.nsit;
+      angle = k >= T.nb;
+      if (g < T.nmol) {
+        const int b = angle ? k - T.nb : k;
+        I = base + (angle ? T.ai[b] : T.bi[b]);
+        J = base + (angle ? T.aj[b] : T.bj[b]);
+        K = angle ? base + T.ak[b] : 0;
+        M = angle ? T.am[b] : T.bm[b];
+        lmove = tc.lmove[T.type];
+      }
+    } else if (kind == BK_BOND) {
+      if (N < a.nrbt) {
+        I = a.ibi[N];
+        J = a.jbj[N];
+        M = a.ibuk[N];
+        lmove = tc.lmove[ainfo[I].x];
+      }
+    } else if (N < a.nrat) {
+      I = a.iai[N];
+      J = a.jaj[N];
+      K = a.kak[N];
+      M = a.iauk[N];
+      lmove = tc.lmove[ainfo[I].x];
     }
-    if (t < a.ntpl) {
-      const MolTpl &T = a.tpl[t];
-      const int base = T.first + N * T.nsit, lmove = tc.lmove[T.type];
-      for (int b = 0; b < T.nb; ++b)
-        bond_term<R, true>(pos, base + T.bi[b], base + T.bj[b], T.bm[b], a.bid, a.rb, a.fb, a.db,
-                           a.ro, lmove, bx, by, bz, o, acc, &v, &e);
-      for (int b = 0; b < T.na; ++b)
-        angle_term<R, true>(pos, base + T.ai[b], base + T.aj[b], base + T.ak[b], T.am[b], a.ra,
-                            a.fa, lmove, bx, by, bz, o, acc, &v, &e);
-    }
-  } else if (kind == BK_BOND) {
-    if (N < a.nrbt) {
-      const int I = a.ibi[N];
-      bond_term<R, false>(pos, I, a.jbj[N], a.ibuk[N], a.bid, a.rb, a.fb, a.db, a.ro,
-                          tc.lmove[ainfo[I].x], bx, by, bz, o, acc, &v, &e);
-    }
-  } else if (kind == BK_ANGLE) {
-    if (N < a.nrat) {
-      const int I = a.iai[N];
-      angle_term<R, false>(pos, I, a.jaj[N], a.kak[N], a.iauk[N], a.ra, a.fa,
-                           tc.lmove[ainfo[I].x], bx, by, bz, o, acc, &v, &e);
-    }
+    if (I >= 0 && angle)
+      angle_term<R, false>(pos, I, J, K, M, a.ra, a.fa, lmove, bx, by, bz, o, acc, &v, &e);
+    else if (I >= 0)
+      bond_term<R, false>(pos, I, J, M, a.bid, a.rb, a.fb, a.db, a.ro, lmove, bx, by, bz, o, acc,
+                          &v, &e);
   } else if (N < a.nrrt) {
     double t4[4] = {0, 0, 0, 0};
     tors_term<R>(N, a.q, pos, ainfo, tc, bx, by, bz, o, t4, &v, &e);
@@ -748,7 +767,7 @@ __global__ void __launch_bounds__(128) k_bonded_all(BondedAll a, const dbl4 *__r
 
 }  // namespace
 
-int launch_bonded(mdx_ctx *ctx, int laver, bool ener, bool shared) {
+int launch_bonded(mdx_ctx *ctx, int laver, bool ener) {
   MDX_TIMER(ctx, MDX_T_BONDED);
   DevData &d = ctx->dv;
   mdx_scalars *sc = d.sc;
@@ -760,7 +779,7 @@ int launch_bonded(mdx_ctx *ctx, int laver, bool ener, bool shared) {
             nullptr, (float)(ctx->boxl / 4294967296.0),
             (float)(fix_period_y(ctx) / 4294967296.0), (float)(ctx->bozl / 4294967296.0),
             (float)(0.495 * ctx->boxl), (float)(0.495 * ctx->boyl), (float)(0.495 * ctx->bozl),
-            cell_pbc(ctx), shared};
+            cell_pbc(ctx)};
   const int T = 128;
   const double bx = ctx->boxl, by = ctx->boyl, bz = ctx->bozl;
   const int *nspec = d.nspec_d;
@@ -794,23 +813,23 @@ int launch_bonded(mdx_ctx *ctx, int laver, bool ener, bool shared) {
     w.aadd = w.aaa * w.ro1;
     w.bbdd = w.bbb * w.ro2;
   }
-  if (!laver && nw + (d.ntpl > 0) + (d.nrbt > 0) + (d.nrat > 0) + (d.nrrt > 0) > 1) {
+  if (!laver) {
     BondedAll a{};
     int count[BK_N] = {};
     for (int k = 0; k < nw; ++k) {
       a.w[k] = wp[k];
       count[k] = wp[k].nmol;
     }
-    count[BK_MOL] = d.ntpl > 0 ? d.ntpl_mol : 0;
+    count[BK_MOL] = d.nmblk * T;
     count[BK_BOND] = d.nrbt;
     count[BK_ANGLE] = d.nrat;
     count[BK_TORS] = d.nrrt;
     for (int k = 0; k < BK_N; ++k) a.blk[k + 1] = a.blk[k] + (count[k] + T - 1) / T;
-    a.ntpl = d.ntpl;
     a.nrbt = d.nrbt;
     a.nrat = d.nrat;
     a.nrrt = d.nrrt;
     a.tpl = d.moltpl;
+    a.mblk = d.mblk;
     a.bid = d.bid;
     a.ibi = d.ibi;
     a.jbj = d.jbj;
@@ -827,6 +846,7 @@ int launch_bonded(mdx_ctx *ctx, int laver, bool ener, bool shared) {
     a.fa = d.afa;
     a.q = tl;
     const int nb = a.blk[BK_N];
+    if (nb == 0) return MDX_OK;
     Dst6 dst = dst6(ctx, nb, 5, &sc->pint, &sc->virb, &sc->virfx, &sc->virfy, &sc->virfz);
 #define BA(R, E) \
   k_bonded_all<R, E><<<nb, T, 0, ctx->stream>>>(a, d.pos, d.ainfo, ctx->tc, bx, by, bz, o, dst)
@@ -851,42 +871,42 @@ int launch_bonded(mdx_ctx *ctx, int laver, bool ener, bool shared) {
   if (d.ntpl > 0) {
     const int nb = (d.ntpl_mol + T - 1) / T;
     Dst6 dst = dst6(ctx, nb, 5, &sc->pint, &sc->virb, &sc->virfx, &sc->virfy, &sc->virfz);
-#define GM(R, E)                                                                       \
-  k_molbonded<R, E><<<nb, T, 0, ctx->stream>>>(                                         \
+#define GM(R)                                                                          \
+  k_molbonded<R><<<nb, T, 0, ctx->stream>>>(                                         \
       d.ntpl, d.moltpl, d.bid, d.brb, d.bfb, d.bdb, d.bro, d.ara, d.afa, d.pos, ctx->tc, \
       nspec, bx, by, bz, o, dst, d.nrbb, d.nraa, laver, d.br, d.be, d.ar, d.ae)
     if (mx) {
-      if (ener) GM(float, true); else GM(float, false);
+      GM(float);
     } else {
-      if (ener) GM(double, true); else GM(double, false);
+      GM(double);
     }
 #undef GM
     MDX_LAUNCHED(ctx);
   }
   if (d.nrbt > 0) {
     Dst6 dst = dst6(ctx, (d.nrbt + T - 1) / T, 5, &sc->pint, &sc->virb, &sc->virfx, &sc->virfy, &sc->virfz);
-#define GB(R, E)                                                                       \
-  k_getbnd<R, E><<<(d.nrbt + T - 1) / T, T, 0, ctx->stream>>>(                         \
+#define GB(R)                                                                          \
+  k_getbnd<R><<<(d.nrbt + T - 1) / T, T, 0, ctx->stream>>>(                         \
       d.nrbt, d.ibi, d.jbj, d.ibuk, d.bid, d.brb, d.bfb, d.bdb, d.bro, d.pos, d.ainfo, \
       ctx->tc, nspec, bx, by, bz, o, dst, d.nrbb, laver, d.br, d.be)
     if (mx) {
-      if (ener) GB(float, true); else GB(float, false);
+      GB(float);
     } else {
-      if (ener) GB(double, true); else GB(double, false);
+      GB(double);
     }
 #undef GB
     MDX_LAUNCHED(ctx);
   }
   if (d.nrat > 0) {
     Dst6 dst = dst6(ctx, (d.nrat + T - 1) / T, 4, &sc->pint, &sc->virfx, &sc->virfy, &sc->virfz);
-#define GA(R, E)                                                                       \
-  k_getang<R, E><<<(d.nrat + T - 1) / T, T, 0, ctx->stream>>>(                         \
+#define GA(R)                                                                          \
+  k_getang<R><<<(d.nrat + T - 1) / T, T, 0, ctx->stream>>>(                         \
       d.nrat, d.iai, d.jaj, d.kak, d.iauk, d.ara, d.afa, d.pos, d.ainfo, ctx->tc,      \
       nspec, bx, by, bz, o, dst, d.nraa, laver, d.ar, d.ae)
     if (mx) {
-      if (ener) GA(float, true); else GA(float, false);
+      GA(float);
     } else {
-      if (ener) GA(double, true); else GA(double, false);
+      GA(double);
     }
 #undef GA
     MDX_LAUNCHED(ctx);

@@ -864,6 +864,25 @@ auto fx_force_kernel(int kp, bool xys) {
   return kp > 48 ? (xys ? k_fx_force<true, true> : k_fx_force<false, true>)
                  : (xys ? k_fx_force<true, false> : k_fx_force<false, false>);
 }
+// Points of the circle, scale 2^61, as two-word numbers.  Formed once: on hosts
+// whose long double is done in software the 512 cosines take half a millisecond.
+const std::vector<int> &circle_points() {
+  static const std::vector<int> points = [] {
+    std::vector<int> c(4 * FX_CIRCLE);
+    for (int k = 0; k < FX_CIRCLE; ++k) {
+      const long double th = 6.283185307179586476925286766559005768L * k / FX_CIRCLE;
+      const long double v[2] = {std::cos(th), std::sin(th)};
+      for (int e = 0; e < 2; ++e) {
+        const long long x = std::llrint(v[e] * 2305843009213693952.0L);
+        const int lo = std::max((int)x, -0x7fffffff);  // it can be negated
+        c[4 * k + 2 * e] = lo;
+        c[4 * k + 2 * e + 1] = (int)((x - lo) >> 32);
+      }
+    }
+    return c;
+  }();
+  return points;
+}
 int ceil_log2(int n) {
   int b = 0;
   while ((1ll << b) < n) ++b;
@@ -990,18 +1009,7 @@ int fx_setup(mdx_ctx *ctx, const std::vector<KCol> &cols) {
                     cudaMemcpyHostToDevice));
   MDX_CUDA(ctx_copy(ctx->stream, d.fx_scol, ints.data(), sizeof(int) * ints.size(),
                     cudaMemcpyHostToDevice));
-  // points of the circle, scale 2^61, as two-word numbers (behind the charge scale)
-  std::vector<int> circle(4 * FX_CIRCLE);
-  for (int k = 0; k < FX_CIRCLE; ++k) {
-    const long double th = 6.283185307179586476925286766559005768L * k / FX_CIRCLE;
-    const long double v[2] = {std::cos(th), std::sin(th)};
-    for (int e = 0; e < 2; ++e) {
-      const long long x = std::llrint(v[e] * 2305843009213693952.0L);
-      const int lo = std::max((int)x, -0x7fffffff);  // it can be negated
-      circle[4 * k + 2 * e] = lo;
-      circle[4 * k + 2 * e + 1] = (int)((x - lo) >> 32);
-    }
-  }
+  const std::vector<int> &circle = circle_points();  // behind the charge scale
   MDX_CUDA(ctx_copy(ctx->stream, d.fx_qs + 2, circle.data(), sizeof(int) * circle.size(),
                     cudaMemcpyHostToDevice));
   // chunks past the last atom (a 128-atom tile's end) and the images' rows

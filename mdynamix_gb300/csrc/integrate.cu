@@ -296,22 +296,49 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
                                  int4 *__restrict__ posc, const int *__restrict__ slot_of,
                                  unsigned long long *zero, const IPosOut ip) {
   // ibs: 2^32 / box per axis (host-computed: no FP64 division per thread);
-  // posi set (mixed path): centre of mass by the reciprocal mass, the
-  // fixed-point mirror refreshed, and (posc set) its cell-order copy.
+  // The two half kicks of one force are one, the centre of mass is formed by
+  // the reciprocal mass, coordinates are rebuilt around the wrapped centre
+  // only when it moved: the reference's update up to FP64 rounding, in half
+  // its FP64 instructions.
+  // posi set (mixed path): the fixed-point mirror refreshed, and (posc set) its
+  // cell-order copy.
   // zero set: the atom's fast forces (3 words, stride n: hfix, or hx..hz)
   // are cleared once read, for an FFORCES whose parts all add to them.
   // FP64 path: hfix set, the sweep's fixed-point sums to be added to H (unit
   // inv; cleared once read); ip, where the positions go as integers.
   const int m = ml.m, f = mol_first[m], na = ml.live ? mol_nat[m] : 0;
-  if (ml.g == 1 && posi && na <= KD_MAXA) {
+  // the atom's fast force times the kick factor, added to its velocity
+  const double hk = prev ? 2.0 * htsteb : htsteb, hkf = hk * inv;
+  auto kick = [&](int i, double &u, double &v, double &w) {
+    if (!posi || !hfix) {
+      u = fma(hx[i], hk, u);
+      v = fma(hy[i], hk, v);
+      w = fma(hz[i], hk, w);
+    }
+    if (hfix) {
+      u = fma((double)(long long)hfix[i], hkf, u);
+      v = fma((double)(long long)hfix[n + i], hkf, v);
+      w = fma((double)(long long)hfix[2 * n + i], hkf, w);
+    }
+  };
+  auto clear = [&](int i) {
+    if (hfix && !posi) hfix[i] = hfix[n + i] = hfix[2 * n + i] = 0ull;
+    if (zero) zero[i] = zero[n + i] = zero[2 * n + i] = 0ull;
+  };
+  auto mirror = [&](int i, const dbl4 &p) {
+    pos[i] = p;
+    if (ip.p) ipos_store(ip, i, p);
+    if (posi) {
+      const int4 q = make_int4(fix32_rn(__dmul_rn(p.x, ibs.x)), fix32_rn(__dmul_rn(p.y, ibs.y)),
+                               fix32_rn(__dmul_rn(p.z, ibs.z)), pinfo[i]);
+      posi[i] = q;
+      if (posc) posc[slot_of[i]] = q;
+    }
+  };
+  if (ml.g == 1 && na <= KD_MAXA) {
     if (!ml.live) return;
-    // Mixed path, small molecules: the atoms stay in registers between the
-    // centre of mass and the wrap, each position is stored once, and the
-    // update takes fewer FP64 operations (the two half kicks of one force
-    // as one, 1/2^k folded into the kick factor, the drift factor TSTEB /
-    // m formed once per atom, coordinates rebuilt around the wrapped centre
-    // only when it moved).  The same update up to FP64 rounding.
-    const double hk = prev ? 2.0 * htsteb : htsteb, hkf = hk * inv;
+    // Small molecules: the atoms stay in registers between the centre of mass
+    // and the wrap, each position is stored once.
     dbl4 pr[KD_MAXA];
     double x = 0., y = 0., z = 0.;
 #pragma unroll
@@ -321,15 +348,7 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
         dbl4 p = pos[i];
         if (mv.lmove[ainfo[i].x]) {
           double u = vx[i], v = vy[i], w = vz[i];
-          if (hfix) {
-            u = fma((double)(long long)hfix[i], hkf, u);
-            v = fma((double)(long long)hfix[n + i], hkf, v);
-            w = fma((double)(long long)hfix[2 * n + i], hkf, w);
-          } else {
-            u = fma(hx[i], hk, u);
-            v = fma(hy[i], hk, v);
-            w = fma(hz[i], hk, w);
-          }
+          kick(i, u, v, w);
           vx[i] = u;
           vy[i] = v;
           vz[i] = w;
@@ -338,7 +357,7 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
           p.y = fma(v, tm, p.y);
           p.z = fma(w, tm, p.z);
         }
-        if (zero) zero[i] = zero[n + i] = zero[2 * n + i] = 0ull;
+        clear(i);
         pr[k] = p;
         const double ms = amass[i];
         x = fma(ms, p.x, x);
@@ -365,21 +384,13 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
           p.y = (p.y - y) + yw;
           p.z = (p.z - z) + zw;
         }
-        pos[f + k] = p;
-        const int4 q =
-            make_int4(fix32_rn(__dmul_rn(p.x, ibs.x)), fix32_rn(__dmul_rn(p.y, ibs.y)),
-                      fix32_rn(__dmul_rn(p.z, ibs.z)), pinfo[f + k]);
-        posi[f + k] = q;
-        if (posc) posc[slot_of[f + k]] = q;
+        mirror(f + k, p);
       }
     }
     return;
   }
-  // lanes of the molecule (or one thread, FP64 path): the reference's
-  // operations per atom; on the mixed path the shorter update of above.  Up
-  // to g atoms stay in registers.
+  // lanes of the molecule; up to g atoms stay in registers
   double x = 0., y = 0., z = 0.;
-  const double hk = prev ? 2.0 * htsteb : htsteb, hkf = hk * inv;
   dbl4 p0;
   p0.x = p0.y = p0.z = p0.w = 0.0;
   for (int k = ml.k; k < na; k += ml.g) {
@@ -387,67 +398,30 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
     dbl4 p = pos[i];
     if (mv.lmove[ainfo[i].x]) {
       double u = vx[i], v = vy[i], w = vz[i];
-      const double mi = massdi[i];
-      if (posi) {
-        if (hfix) {
-          u = fma((double)(long long)hfix[i], hkf, u);
-          v = fma((double)(long long)hfix[n + i], hkf, v);
-          w = fma((double)(long long)hfix[2 * n + i], hkf, w);
-        } else {
-          u = fma(hx[i], hk, u);
-          v = fma(hy[i], hk, v);
-          w = fma(hz[i], hk, w);
-        }
-        const double tm = tsteb * mi;
-        p.x = fma(u, tm, p.x);
-        p.y = fma(v, tm, p.y);
-        p.z = fma(w, tm, p.z);
-      } else {
-        double fx = hx[i], fy = hy[i], fz = hz[i];
-        if (hfix) {
-          fx = fma((double)(long long)hfix[i], inv, fx);
-          fy = fma((double)(long long)hfix[n + i], inv, fy);
-          fz = fma((double)(long long)hfix[2 * n + i], inv, fz);
-        }
-        if (prev) {
-          u = u + htsteb * fx;
-          v = v + htsteb * fy;
-          w = w + htsteb * fz;
-        }
-        u = u + htsteb * fx;
-        v = v + htsteb * fy;
-        w = w + htsteb * fz;
-        p.x = u * tsteb * mi + p.x;
-        p.y = v * tsteb * mi + p.y;
-        p.z = w * tsteb * mi + p.z;
-      }
+      kick(i, u, v, w);
+      const double tm = tsteb * massdi[i];
+      p.x = fma(u, tm, p.x);
+      p.y = fma(v, tm, p.y);
+      p.z = fma(w, tm, p.z);
       vx[i] = u;
       vy[i] = v;
       vz[i] = w;
     }
-    if (hfix && !posi) hfix[i] = hfix[n + i] = hfix[2 * n + i] = 0ull;
-    if (zero) zero[i] = zero[n + i] = zero[2 * n + i] = 0ull;
+    clear(i);
     if (k == ml.k) p0 = p;
     else pos[i] = p;
     const double ms = amass[i];
-    x = x + ms * p.x;
-    y = y + ms * p.y;
-    z = z + ms * p.z;
+    x = fma(ms, p.x, x);
+    y = fma(ms, p.y, y);
+    z = fma(ms, p.z, z);
   }
   x = lanes_sum(x, ml.g);
   y = lanes_sum(y, ml.g);
   z = lanes_sum(z, ml.g);
-  if (posi) {
-    const double rs = mc.rsummas[mol_type[m]];
-    x = x * rs;
-    y = y * rs;
-    z = z * rs;
-  } else {
-    const double summ = mc.summas[mol_type[m]];
-    x = x / summ;
-    y = y / summ;
-    z = z / summ;
-  }
+  const double rs = mc.rsummas[mol_type[m]];
+  x = x * rs;
+  y = y * rs;
+  z = z * rs;
   double xw = x, yw = y, zw = z;
   pbc_com(xw, yw, zw, bx, by, bz, mc);
   if (ml.live && ml.k == 0) {
@@ -455,7 +429,7 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
     Y[m] = yw;
     Z[m] = zw;
   }
-  const bool moved = !posi || xw != x || yw != y || zw != z;
+  const bool moved = xw != x || yw != y || zw != z;
   for (int k = ml.k; k < na; k += ml.g) {
     dbl4 p = k == ml.k ? p0 : pos[f + k];
     if (moved) {
@@ -463,14 +437,7 @@ __device__ __forceinline__ void kick_drift_com_body(const MolLane &ml, const int
       p.y = (p.y - y) + yw;
       p.z = (p.z - z) + zw;
     }
-    pos[f + k] = p;
-    if (ip.p) ipos_store(ip, f + k, p);
-    if (posi) {
-      const int4 q = make_int4(fix32_rn(__dmul_rn(p.x, ibs.x)), fix32_rn(__dmul_rn(p.y, ibs.y)),
-                               fix32_rn(__dmul_rn(p.z, ibs.z)), pinfo[f + k]);
-      posi[f + k] = q;
-      if (posc) posc[slot_of[f + k]] = q;
-    }
+    mirror(f + k, p);
   }
 }
 

@@ -21,7 +21,7 @@ int launch_leapfrog_shake(mdx_ctx *ctx);
 int launch_vira(mdx_ctx *ctx, int from_viran);
 size_t scal_scratch_bytes();
 // bonded.cu
-int launch_bonded(mdx_ctx *ctx, int laver, bool ener = true, bool shared = false);
+int launch_bonded(mdx_ctx *ctx, int laver, bool ener = true);
 
 namespace {
 
@@ -213,7 +213,7 @@ int do_fforces_mid(mdx_ctx *ctx, bool fold) {
     MDX_CUDA(cudaEventRecord(ctx->side_ev[0], ctx->stream));
     MDX_CUDA(cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0));
     std::swap(ctx->stream, ctx->side);
-    const int rc = launch_bonded(ctx, 0, false, true);
+    const int rc = launch_bonded(ctx, 0, false);
     std::swap(ctx->stream, ctx->side);
     MDX_CUDA(cudaEventRecord(ctx->side_ev[1], ctx->side));
     if (rc) return rc;
@@ -610,7 +610,7 @@ int mdx_open(const mdx_dims *dims, mdx_ctx **out) {
 int mdx_close(mdx_ctx *ctx) {
   if (!ctx) return MDX_OK;
   DevData &d = ctx->dv;
-  void *ptrs[] = {d.pos, d.posf, d.posi, d.qsitef, d.stab, d.pinfo, d.moltpl, d.vx, d.massdi, d.amass, d.qsite,
+  void *ptrs[] = {d.pos, d.posf, d.posi, d.qsitef, d.stab, d.pinfo, d.moltpl, d.mblk, d.vx, d.massdi, d.amass, d.qsite,
                   d.ainfo, d.nnbb, d.inbb, d.mol_first, d.mol_nat, d.mol_type, d.X,
                   d.gx, d.ox, d.gfix, d.hfix, d.ns_cnt, d.nl_cnt, d.ns_idx, d.nl_idx,
                   d.cell_cnt, d.cell_start, d.cell_list, d.cell_pos, d.slot_of, d.pos_ref, d.atom_cell, d.a6lj, d.a6f, d.abf,
@@ -743,13 +743,27 @@ static int split_bonded(mdx_ctx *ctx, const mdx_topo *t) {
     RC(upload(ctx, d.iauk, am.data(), d.nrat));
   }
   ctx_free(ctx, d.moltpl);
+  ctx_free(ctx, d.mblk);
   d.moltpl = nullptr;
+  d.mblk = nullptr;
+  d.nmblk = 0;
   d.ntpl = (int)use.size();
   d.ntpl_mol = 0;
   for (const MolTpl &m : use) d.ntpl_mol += m.nmol;
   if (d.ntpl) {
     RC(dmalloc(ctx, &d.moltpl, use.size()));
     RC(upload(ctx, d.moltpl, use.data(), use.size()));
+    std::vector<int2> blk;  // angles, the longest, first
+    for (int angle = 1; angle >= 0; --angle)
+      for (size_t t = 0; t < use.size(); ++t)
+        for (int k = angle ? use[t].nb : 0; k < use[t].nb + (angle ? use[t].na : 0); ++k)
+          for (int g = 0; g < use[t].nmol; g += 128)
+            blk.push_back(make_int2((int)t | k << 8, g));
+    d.nmblk = (int)blk.size();
+    if (d.nmblk) {
+      RC(dmalloc(ctx, &d.mblk, blk.size()));
+      RC(upload(ctx, d.mblk, blk.data(), blk.size()));
+    }
   }
   return MDX_OK;
 }

@@ -236,6 +236,8 @@ struct DevData {
   // small molecule types handled per molecule (bonds, angles); the instance
   // lists ibi.. / iai.. then hold only the other types' terms
   MolTpl *moltpl;
+  int2 *mblk;   // k_bonded_all's blocks of template molecules' terms
+  int nmblk;
   int ntpl, ntpl_mol;
   KGroup *kgroups;              // column groups of the mixed force pass
   int ngroup;
@@ -816,7 +818,11 @@ constexpr long long IPOS_BAD = (long long)0x8000000000000000ull;
 __device__ __forceinline__ void ipos_store(const IPosOut &o, int i, const dbl4 &p) {
   constexpr double LIM = 2305843009213693952.0;  // 2^61
   const double x = p.x * o.ps, y = p.y * o.ps, z = p.z * o.ps, q = p.w * o.qs;
-  const bool ok = fabs(x) < LIM && fabs(y) < LIM && fabs(z) < LIM && fabs(q) <= 2.0 * LIM;
+  // compared as integers: an FP64 comparison takes the FP64 pipe
+  auto in = [](double v, double lim) {
+    return (__double_as_longlong(v) & 0x7fffffffffffffffLL) <= __double_as_longlong(lim);
+  };
+  const bool ok = in(x, LIM) && in(y, LIM) && in(z, LIM) && in(q, 2.0 * LIM);
   o.p[2 * (size_t)i] = make_longlong2(__double2ll_rn(x), __double2ll_rn(y));
   o.p[2 * (size_t)i + 1] = make_longlong2(__double2ll_rn(z), ok ? __double2ll_rn(q) : IPOS_BAD);
 }

@@ -1,0 +1,41 @@
+"""Bonded terms, a thread a term (FFORCES without statistics): molecule counts at
+the edges of its blocks, straight angles (CH3CN as built and bent).  FP64 against
+the oracle: a term's force takes some 30 roundings and the sine of a nearly
+straight angle is conditioned like the angle itself: 1e-11 of the largest
+force.  Mixed against FFORCES with statistics, whose threads take a molecule:
+the same FP32 terms, summed as integers, so the same forces."""
+import numpy as np
+import pytest
+
+import oracle
+from mdynamix_gb300 import system as S
+from mdynamix_gb300.abi import MDX_FP64, MDX_MIXED
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", [MDX_FP64, MDX_MIXED])
+@pytest.mark.parametrize("n", [1, 127, 128, 129])
+@pytest.mark.parametrize("jitter", [0.0, 0.03])
+def test_terms_match_oracle(n, jitter, prec):
+    from mdynamix_gb300.mdx import ForcePath
+    box = 14.0 + 9.0 * n ** (1 / 3)
+    spec = S.RunSpec(molecules=[("CH3CN", n), ("SPC-FW", n), ("CH3OH", 2)], box=(box,) * 3,
+                     dt_fs=1.0, nfreq=4, rcut=6.5, rshort=4.0, alpha=2.0, fexp=1.0, ichnb=10,
+                     trtemp=300.0)
+    s = S.System(spec)
+    st = S.make_configuration(s, seed=6, jitter=jitter)
+    g = ForcePath(s, precision=prec)
+    o = oracle.Oracle(s) if prec == MDX_FP64 else None
+    for p in (g, o) if o else (g,):
+        p.set_state(*st)
+        p.chcnb()
+        p.getcom()
+        p.fforces(False)
+    a = g.forces(1)
+    if o:
+        b = o.forces(1)
+        assert np.abs(a - b).max() <= 1e-11 * np.abs(b).max()
+    else:
+        g.fforces(True)
+        assert np.array_equal(a, g.forces(1))
+    g.close()
