@@ -24,9 +24,9 @@
 // leaves FP64 instructions for the LJ terms and a row's end only.
 //
 // Measured on a GB300 at 98,304 atoms (one warp an owner and everything
-// written out; k_pair64t; k_pair64x): short rows, forces 0.526, 0.20, 0.091 ms;
-// long rows with energies 4.88, 2.40, 1.24 ms, with energies by type pair
-// 15.3, 3.1, 1.5 ms.  k_pair64t's FP64 pipe is 82-86 % active.  Error of the
+// written out; k_pair64t; k_pair64x): short rows, forces 0.526, 0.20, 0.090 ms;
+// long rows with energies 4.88, 2.40, 1.09 ms, with energies by type pair
+// 15.3, 3.1, 1.4 ms.  k_pair64t's FP64 pipe is 82-86 % active.  Error of the
 // short rows' forces against 128 bits (200 ions; rms, of the rms force): 2.8e-15
 // written out, 4e-16 in integers.
 //
@@ -54,7 +54,7 @@ struct __align__(16) PairPoly {
 constexpr int PT_OCT0 = -2, PT_NOCT = 12;     // r^2 from 2^-2 to 2^10 A^2
 constexpr int PT_BINS = 128 * PT_NOCT;
 constexpr int PT_BASE = (1023 + PT_OCT0) * 128;  // bin of r^2: its exponent and 7 leading bits
-enum { PT_FORCE = 0, PT_ENER, PT_R2I, PT_R1I, PT_NFN };
+enum { PT_FORCE = 0, PT_ENER, PT_R1I, PT_R2I, PT_NFN };
 
 // ------------------------------------------------- two-word FP64 numbers --
 // Sums and products of pairs of doubles (Dekker, Numer. Math. 18, 1971): the
@@ -681,11 +681,11 @@ __device__ __forceinline__ PxArg px_arg(const Px &x, unsigned long long r2) {
   a.tf = __uint_as_float(0x3f800000u | ((mh & 0xffffffu) >> 1)) - 1.5f;
   return a;
 }
-__device__ __forceinline__ long long px_eval(const PxPoly *__restrict__ tab, const PxArg &a) {
+__device__ __forceinline__ long long px_eval(const PxPoly *tab, const PxArg &a) {
   const PxPoly *p = tab + a.bin;
-  const longlong2 c01 = __ldg(reinterpret_cast<const longlong2 *>(p));
-  const int4 c23 = __ldg(reinterpret_cast<const int4 *>(p) + 1);
-  const float4 cf = __ldg(reinterpret_cast<const float4 *>(p) + 2);
+  const longlong2 c01 = *reinterpret_cast<const longlong2 *>(p);
+  const int4 c23 = *(reinterpret_cast<const int4 *>(p) + 1);
+  const float4 cf = *(reinterpret_cast<const float4 *>(p) + 2);
   const int s3 = c23.z + __float2int_rn(a.tf * fmaf(fmaf(cf.z, a.tf, cf.y), a.tf, cf.x));
   const long long c2 = (long long)(((unsigned long long)(unsigned)c23.y << 32) | (unsigned)c23.x);
   const long long s2 = c2 + (((long long)s3 * a.t.h) >> c23.w);
@@ -693,23 +693,44 @@ __device__ __forceinline__ long long px_eval(const PxPoly *__restrict__ tab, con
   return c01.x + mulhi2(split2(s1), a.t);
 }
 
+// Tables of every pair that a long sweep keeps in shared memory: F, and E with
+// the energies.  32 lanes ask for 32 bins, in L1 a tag each: with the neighbours'
+// records and the atomics that kept L1 88 % busy.  A third table (1 / r, force
+// calls) would leave L1 too little for the records.  98,304 atoms, long rows with
+// energies 1.24 ms from L1, 1.09 from shared memory; with energies by type pair
+// 1.50, 1.39, with all three 2.13.  Only where a warp has several owners: the
+// copy, and the SMs' change to another split of their memory between two
+// kernels of a small system, cost more (3,000 atoms, 20 steps: 6.64 ms without,
+// 7.02 with; the short rows gain 4 % at 98,304 atoms and nothing at 21,003).
+constexpr int px_tables(bool ener) { return ener ? 2 : 1; }
+
 struct PxQueue {  // pairs put aside for their LJ term, per warp
   long long x[64], y[64], z[64], g[64];
   unsigned long long r2[64];
   int i[64], j[64], tix[64];
 };
 
-template <bool SHORT, bool SPLIT, bool ENER, int TPO>
+// TABSH: the tables of every pair in shared memory
+template <bool SHORT, bool SPLIT, bool ENER, int TPO, bool TABSH>
 __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64x(
-    int n, const longlong2 *__restrict__ ipos, const dbl4 *__restrict__ pos,
+    int n, const longlong4_32a *__restrict__ ipos, const dbl4 *__restrict__ pos,
     const int4 *__restrict__ ainfo, const double *__restrict__ qsite,
     const int *__restrict__ cnt, const int *__restrict__ idx, int cap, Lj64 lj, TypeConst tc,
     PairConst pc, CellPbc cp, unsigned eemask, Px px, double *__restrict__ fx,
     double *__restrict__ fy, double *__restrict__ fz, unsigned long long *__restrict__ ff,
     Dst6 dst, double *__restrict__ split) {
+  extern __shared__ __align__(16) unsigned char s_tab[];
   __shared__ double s_split[SPLIT ? SPLIT_N : 1];
   __shared__ PxQueue s_q[PT_WARPS];
   __shared__ int2 s_slow[PT_WARPS][64];
+  if (TABSH) {
+    const int4 *src = reinterpret_cast<const int4 *>(px.tab);
+    int4 *dst = reinterpret_cast<int4 *>(s_tab);
+    for (int k = threadIdx.x; k < px_tables(ENER) * px.nbin * 3; k += blockDim.x)
+      dst[k] = __ldg(src + k);
+    __syncthreads();
+  }
+  const PxPoly *const tab = TABSH ? reinterpret_cast<const PxPoly *>(s_tab) : px.tab;
   if (SPLIT) {
     for (int k = threadIdx.x; k < SPLIT_N; k += blockDim.x) s_split[k] = 0.0;
     __syncthreads();
@@ -791,23 +812,22 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64x(
   for (int i0 = (blockIdx.x * PT_WARPS + w) * OPW; i0 < n; i0 += gridDim.x * PT_WARPS * OPW) {
     const int i = i0 + lane / TPO;
     const bool own = i < n;
-    const size_t io = 2 * (size_t)(own ? i : 0);
-    const longlong2 pxy = ipos[io], pzq = ipos[io + 1];
+    const longlong4_32a ip = ipos[own ? i : 0];
     const int4 ai = ainfo[own ? i : 0];
-    const I2 qi = split2(pzq.y);
+    const I2 qi = split2(ip.w);
     const int c = own ? cnt[i] : 0;
     const int cmax = __reduce_max_sync(0xffffffffu, c);
     const int *row = idx + (size_t)(own ? i : 0) * cap;
     const double *b12row = lj.b12lj + ai.z * pc.nnbt;
-    const bool eei = ((eem >> ai.x) & 1u) || pzq.y == IPOS_BAD;
+    const bool eei = ((eem >> ai.x) & 1u) || ip.w == IPOS_BAD;
     long long ax = 0, ay = 0, az = 0;
     for (int k = lane & (TPO - 1); k - (lane & (TPO - 1)) < cmax; k += TPO) {
       bool act = k < c;
       const int e = act ? row[k] : 0;
       const int j = e & 0x7fffffff;
-      const longlong2 jxy = ipos[2 * (size_t)j], jzq = ipos[2 * (size_t)j + 1];
+      const longlong4_32a jp = ipos[j];
       const int4 aj = ainfo[j];
-      long long DX = pxy.x - jxy.x, DY = pxy.y - jxy.y, DZ = pzq.x - jzq.x;
+      long long DX = ip.x - jp.x, DY = ip.y - jp.y, DZ = ip.z - jp.z;
       image(DX, px.hx, px.lx);
       image(DY, px.hy, px.ly);
       image(DZ, px.hz, px.lz);
@@ -825,7 +845,7 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64x(
                                (long long)dz.h * dz.h + (cr >> 31));
       PxArg p = px_arg(px, r2);
       const bool other = (SHORT && e < 0) || aj.y == ai.y || eei || ((eem >> aj.x) & 1u) ||
-                         jzq.y == IPOS_BAD || !in || (unsigned)p.bin >= (unsigned)px.nbin;
+                         jp.w == IPOS_BAD || !in || (unsigned)p.bin >= (unsigned)px.nbin;
       if (!SHORT && !other && r2 > px.rc2) act = false;  // skin mode
       const bool sl = act && other, fast = act && !other;
       if (!fast) p.bin = 0;
@@ -835,11 +855,11 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64x(
         nslow += __popc(ms);
         if (nslow >= 32) slow_batch(32);
       }
-      const I2 qq = split2(mulhi2(qi, split2(jzq.y)));
-      const I2 F = split2(px_eval(px.tab + PT_FORCE * px.nbin, p));
+      const I2 qq = split2(mulhi2(qi, split2(jp.w)));
+      const I2 F = split2(px_eval(tab + PT_FORCE * px.nbin, p));
       const long long g = (((long long)F.h * qq.h) << 4) + (cross2(F, qq) >> 28);
       if (ENER) {
-        const long long E = mulhi2(split2(px_eval(px.tab + PT_ENER * px.nbin, p)), qq);
+        const long long E = mulhi2(split2(px_eval(tab + PT_ENER * px.nbin, p)), qq);
         if (fast) ie += E;
       }
       if (SPLIT && fast)
@@ -1028,7 +1048,7 @@ int pair64_setup(mdx_ctx *ctx) {
       const double ar = ctx->p.alphad * r, t = 1.0 / (1.0 + MDX_B1 * ar), e = std::exp(-ar * ar);
       const double er =
           ((((MDX_A5 * t + MDX_A4) * t + MDX_A3) * t + MDX_A2) * t + MDX_A1) * t * e / r;
-      const double f0[PT_NFN] = {(MDX_TOTPI * ctx->p.alphad * e + er) / x, er, 1.0 / x, 1.0 / r};
+      const double f0[PT_NFN] = {(MDX_TOTPI * ctx->p.alphad * e + er) / x, er, 1.0 / r, 1.0 / x};
       PxScale sc;
       for (int f = 0; f < PT_NFN; ++f)
         sc.s[f] = ctx->px_s[w][f] = (w && f == PT_FORCE ? 60 : 62) - 1 - std::ilogb(1.0001 * f0[f]);
@@ -1087,11 +1107,22 @@ int launch_pair64(mdx_ctx *ctx, bool shrt, bool split, bool ener, double *split_
   k_pair64t<S, P, E, K><<<grid, T, 0, ctx->stream>>>(d.n, d.pos, d.ainfo, d.qsite, cnt, idx, cap, \
                                                      lj, ctx->tc, ctx->pc, cp, eemask, tab, fx, \
                                                      fy, fz, dst, split_buf)
-#define LP64X(S, P, E, K)                                                                       \
-  k_pair64x<S, P, E, K><<<grid, T, 0, ctx->stream>>>(d.n, reinterpret_cast<longlong2 *>(d.ipos), \
-                                                     d.pos, d.ainfo, d.qsite, cnt, idx, cap, lj, \
-                                                     ctx->tc, ctx->pc, cp, eemask, px, fx, fy,   \
-                                                     fz, ff, dst, split_buf)
+#define LP64XT(S, P, E, K, SH)                                                                   \
+  do {                                                                                           \
+    const size_t sh = SH ? sizeof(PxPoly) * px_tables(E) * px.nbin : 0;                          \
+    if (SH && raise_smem_limit(k_pair64x<S, P, E, K, SH>, sh) != cudaSuccess) {                  \
+      ctx->err = "pair sweep: shared-memory limit";                                              \
+      return MDX_ERR_CUDA;                                                                       \
+    }                                                                                            \
+    k_pair64x<S, P, E, K, SH><<<grid, T, sh, ctx->stream>>>(                                     \
+        d.n, reinterpret_cast<longlong4_32a *>(d.ipos), d.pos, d.ainfo, d.qsite, cnt, idx, cap,  \
+        lj, ctx->tc, ctx->pc, cp, eemask, px, fx, fy, fz, ff, dst, split_buf);                   \
+  } while (0)
+#define LP64X(S, P, E, K)                                                                        \
+  do {                                                                                           \
+    if (!S && d.n >= 4 * PT_WARPS * 2 * ctx->nsm) LP64XT(S, P, E, K, !S);                        \
+    else LP64XT(S, P, E, K, false);                                                              \
+  } while (0)
 #define LP64(S, P, E)                                                                        \
   do {                                                                                       \
     if (ctx->px_on) {                                                                        \
@@ -1119,6 +1150,7 @@ int launch_pair64(mdx_ctx *ctx, bool shrt, bool split, bool ener, double *split_
 #undef LP64
 #undef LP64T
 #undef LP64X
+#undef LP64XT
   MDX_LAUNCHED(ctx);
   return MDX_OK;
 }
