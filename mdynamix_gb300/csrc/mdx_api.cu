@@ -232,23 +232,34 @@ int do_fforces_mid(mdx_ctx *ctx, bool fold) {
 // mirrored).  Reciprocal space up to its force pass needs nothing of the pair
 // sweeps, so it runs beside them on the second stream: below some 20,000 atoms
 // neither fills the GPU (3,000 atoms FP64: 75 us beside 96; 609 mixed: 55
-// beside 60).  The mixed force pass adds to G's integers once the long sweep
-// and ETERMS have, the FP64 one at the end.  No fork with the timers on.
-int force_parts_on(mdx_ctx *ctx, bool split, bool types, int laver, bool fork) {
+// beside 60); FFORCES, which needs neither, on a third.  The mixed force pass adds
+// to G's integers once the long sweep and ETERMS have, the FP64 one at the end.  No fork with the timers on.
+int force_parts_on(mdx_ctx *ctx, bool split, bool types, int laver, bool fork, bool fast2) {
   const bool mx = ctx->mixed();
   bool skip = true;
-  auto beside = [&](auto &&f) {
-    std::swap(ctx->stream, ctx->side);
-    ctx->red_slot = 1;
+  auto on = [&](cudaStream_t &s, int slot, auto &&f) {
+    std::swap(ctx->stream, s);
+    ctx->red_slot = slot;
     const int rc = f();
     ctx->red_slot = 0;
-    std::swap(ctx->stream, ctx->side);
+    std::swap(ctx->stream, s);
     return rc;
+  };
+  auto fast = [&]() -> int {
+    RC(launch_localf(ctx, split));
+    RC(launch_wir(ctx, 1));  // WIRSS from the pair forces, before the bonded terms
+    RC(launch_bonded(ctx, laver));
+    return mx ? launch_fix_to_double(ctx, 1) : MDX_OK;
   };
   if (fork) {
     MDX_CUDA(cudaEventRecord(ctx->side_ev[0], ctx->stream));
     MDX_CUDA(cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0));
-    RC(beside([&] { return furir_first(ctx, &skip); }));
+    RC(on(ctx->side, 1, [&] { return furir_first(ctx, &skip); }));
+    if (fast2) {
+      MDX_CUDA(cudaStreamWaitEvent(ctx->side2, ctx->side_ev[0], 0));
+      RC(on(ctx->side2, 2, fast));
+      MDX_CUDA(cudaEventRecord(ctx->side_ev[4], ctx->side2));
+    }
   } else {
     RC(furir_first(ctx, &skip));
   }
@@ -258,27 +269,31 @@ int force_parts_on(mdx_ctx *ctx, bool split, bool types, int laver, bool fork) {
     if (mx && !skip) {
       MDX_CUDA(cudaEventRecord(ctx->side_ev[2], ctx->stream));
       MDX_CUDA(cudaStreamWaitEvent(ctx->side, ctx->side_ev[2], 0));
-      RC(beside([&] { return furir_force(ctx); }));
+      RC(on(ctx->side, 1, [&] { return furir_force(ctx); }));
     }
     MDX_CUDA(cudaEventRecord(ctx->side_ev[3], ctx->side));
   }
-  if (laver >= 0) {
-    RC(launch_localf(ctx, split));
-    RC(launch_wir(ctx, 1));  // WIRSS from the pair forces, before the bonded terms
-    RC(launch_bonded(ctx, laver));
-    if (mx) RC(launch_fix_to_double(ctx, 1));
-  }
+  if (laver >= 0 && !fast2) RC(fast());
   if (fork) MDX_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->side_ev[3], 0));
   if (!skip && !(fork && mx)) RC(furir_force(ctx));
-  return mx ? launch_fold_wirs(ctx) : launch_wir(ctx, 2);
+  RC(mx ? launch_fold_wirs(ctx) : launch_wir(ctx, 2));
+  if (fast2) MDX_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->side_ev[4], 0));
+  return MDX_OK;
 }
 
-int force_parts(mdx_ctx *ctx, bool split, bool types, int laver) {
+int force_parts(mdx_ctx *ctx, bool split, bool types, int laver, bool alone = true) {
   const bool fork = !ctx->timing && ctx->p.alphad > 0.0;
-  const int rc = force_parts_on(ctx, split, types, laver, fork);
+  // FFORCES beside, but not in one bead of many (20 long steps of 3,000 atoms FP64
+  // 6.68 -> 6.42 ms, bilayer of 22,529 7.25 -> 7.02 / 10, 98,304 FP64 44.8 -> 43.9 /
+  // 10, mixed the same; 32 beads 15.9 -> 16.2); the force calls' energies by type
+  // pair share their scratch between the sweeps
+  const bool fast2 = fork && alone && laver >= 0 && !split;
+  const int rc = force_parts_on(ctx, split, types, laver, fork, fast2);
   if (rc && fork) {  // whatever was launched beside ends before what comes next
     cudaEventRecord(ctx->side_ev[3], ctx->side);
     cudaStreamWaitEvent(ctx->stream, ctx->side_ev[3], 0);
+    cudaEventRecord(ctx->side_ev[4], ctx->side2);
+    cudaStreamWaitEvent(ctx->stream, ctx->side_ev[4], 0);
   }
   return rc;
 }
@@ -298,10 +313,10 @@ int do_slforces(mdx_ctx *ctx, bool split, bool mirrored = false) {
 
 // SLFORCES then FFORCES of a step's end (mirrored positions), their sums cleared
 // together; of the energies by type pair FFORCES leaves its own only.
-int do_both(mdx_ctx *ctx, int laver) {
+int do_both(mdx_ctx *ctx, int laver, bool alone = true) {
   RC(furir_prepare(ctx));
   RC(launch_zero(ctx, 3, laver));
-  RC(force_parts(ctx, false, false, laver));
+  RC(force_parts(ctx, false, false, laver, alone));
   RC(launch_pullback(ctx));
   RC(launch_sclfrc(ctx, 2));
   return launch_sclfrc(ctx, 1);
@@ -517,13 +532,15 @@ int mdx_open(const mdx_dims *dims, mdx_ctx **out) {
     if (g && g[0] == '0') ctx->use_graphs = false;
   }
   bool made = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) == cudaSuccess;
+              cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) == cudaSuccess &&
+              cudaStreamCreateWithFlags(&ctx->side2, cudaStreamNonBlocking) == cudaSuccess;
   for (auto &e : ctx->side_ev)
     made = made && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
   if (!made) {
     for (auto e : ctx->side_ev)
       if (e) cudaEventDestroy(e);
     if (ctx->side) cudaStreamDestroy(ctx->side);
+    if (ctx->side2) cudaStreamDestroy(ctx->side2);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return MDX_ERR_CUDA;
@@ -572,8 +589,8 @@ int mdx_open(const mdx_dims *dims, mdx_ctx **out) {
   AL(d.err, 4);
   AL(d.shake_iter, 32);
   AL(d.red, 512);
-  AL(d.red_part, ((size_t)1 << 21) + RED_CAP1);
-  AL(d.red_ctr, 16);
+  AL(d.red_part, ((size_t)1 << 21) + 2 * RED_CAP1);
+  AL(d.red_ctr, 24);
   d.red_cap = (size_t)1 << 21;
   if (!rc) {
     unsigned char *ss = nullptr;
@@ -635,6 +652,7 @@ int mdx_close(mdx_ctx *ctx) {
   for (auto e : ctx->side_ev)
     if (e) cudaEventDestroy(e);
   if (ctx->side) cudaStreamDestroy(ctx->side);
+  if (ctx->side2) cudaStreamDestroy(ctx->side2);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return MDX_OK;
@@ -1739,7 +1757,7 @@ int api_copy_scalars(mdx_ctx *ctx, mdx_scalars *out) { return copy_scalars(ctx, 
 int api_do_slforces(mdx_ctx *ctx, bool split, bool mirrored) {
   return do_slforces(ctx, split, mirrored);
 }
-int api_do_both(mdx_ctx *ctx, int laver) { return do_both(ctx, laver); }
+int api_do_both(mdx_ctx *ctx, int laver) { return do_both(ctx, laver, false); }
 int api_do_fforces(mdx_ctx *ctx, int laver, bool split, bool mirrored) {
   return do_fforces(ctx, laver, split, mirrored);
 }

@@ -357,11 +357,12 @@ struct mdx_ctx {
       }
   }
   double pair_tab_alpha = 0.0;  // alpha of dv.pair_tab
-  // second stream of the force routines (bonded terms beside the short sweep,
-  // reciprocal space beside the pair sweeps) and its events
-  cudaStream_t side = nullptr;
-  cudaEvent_t side_ev[4] = {};
-  int red_slot = 0;  // 1 while launching on it: its reductions have their own scratch
+  // further streams of the force routines (side: reciprocal space beside the
+  // pair sweeps, bonded terms beside an intermediate short sweep; side2: the fast
+  // forces beside the slow ones) and their events
+  cudaStream_t side = nullptr, side2 = nullptr;
+  cudaEvent_t side_ev[5] = {};
+  int red_slot = 0;  // 1, 2 while launching on them: reduction scratch of their own
   // FP64 path, fixed-point pair sweeps: on, position unit 2^-px_bits A (of the
   // box when ipos was last written), charge unit 2^(px_eq - 62) e, and the
   // sweeps' ranges (0 short, 1 long): |d| < 2^px_rho A, r^2 >= 2^px_oct A^2;
@@ -402,7 +403,7 @@ inline double fix_period_y(const mdx_ctx *ctx) {
   return ctx->p.icell == 2 ? 2.0 * ctx->boyl : ctx->boyl;
 }
 
-// Doubles and counters behind the main stream's: the second stream's.
+// Doubles (and 8 counters) behind the main stream's for each further stream.
 constexpr size_t RED_CAP1 = (size_t)1 << 19;
 
 // Reduction destinations for a launch of nblocks blocks reducing nv values:
@@ -414,7 +415,8 @@ inline Dst6 dst6(const mdx_ctx *ctx, size_t nblocks, int nv, double *a,
   Dst6 r{{a, b, c, d, e, f}, nullptr, nullptr};
   const size_t cap = ctx->red_slot ? RED_CAP1 : ctx->dv.red_cap;
   if (ctx->dv.red_part && nblocks * (size_t)nv <= cap) {
-    r.part = ctx->dv.red_part + (ctx->red_slot ? ctx->dv.red_cap : 0);
+    r.part = ctx->dv.red_part +
+             (ctx->red_slot ? ctx->dv.red_cap + (ctx->red_slot - 1) * RED_CAP1 : 0);
     r.ctr = ctx->dv.red_ctr + 8 * ctx->red_slot;
   }
   return r;
@@ -872,7 +874,7 @@ int api_check_err(mdx_ctx *ctx);
 int api_copy_scalars(mdx_ctx *ctx, mdx_scalars *out);
 int api_do_slforces(mdx_ctx *ctx, bool split, bool mirrored = false);
 int api_do_fforces(mdx_ctx *ctx, int laver, bool split, bool mirrored = false);
-int api_do_both(mdx_ctx *ctx, int laver);  // SLFORCES and FFORCES, mirrored positions
+int api_do_both(mdx_ctx *ctx, int laver);  // SLFORCES and FFORCES of a bead, mirrored positions
 // bonded.cu: running sums of the per-record bonded statistics
 int launch_acc_bonded(mdx_ctx *ctx);
 int bonded_sums_len(const mdx_ctx *ctx);

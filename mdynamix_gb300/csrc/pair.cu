@@ -878,7 +878,7 @@ int launch_pair(mdx_ctx *ctx, bool shrt, bool split, bool ener, bool add, bool t
     unsigned long long *ffix = shrt ? d.hfix : d.gfix;
     SlotFold sf;
     sf.slots = reinterpret_cast<unsigned long long *>(d.red) + (shrt ? 0 : 16);
-    sf.ctr = d.red_ctr + 4;
+    sf.ctr = d.red_ctr + 8 * ctx->red_slot + 4;
     sf.sc = d.sc;
     sf.einv = 1.0 / ctx->fix.escale;
     sf.which = shrt ? 1 : 2;
