@@ -331,8 +331,9 @@ __global__ void k_getang(int nrat, const int *__restrict__ iai,
 
 // Bonds and angles of small molecule types, one thread per molecule: every
 // atom a thread touches belongs to its molecule, so forces are added
-// without atomics (same per-term rounding, so the sums are identical).
-template <typename R>
+// without atomics (same per-term rounding, so the sums are identical).  Without
+// energies (an intermediate short step, whose sweep adds meanwhile) with them.
+template <typename R, bool ENER>
 __global__ void __launch_bounds__(128) k_molbonded(
     int ntpl, const MolTpl *__restrict__ tpl, const int *__restrict__ bid,
     const double *__restrict__ rb, const double *__restrict__ fb,
@@ -377,7 +378,7 @@ __global__ void __launch_bounds__(128) k_molbonded(
     for (int b = 0; b < T.nb; ++b) {
       const int M = T.bm[b];
       R BD, EB;
-      bond_term<R, true, R>(pos, base + T.bi[b], base + T.bj[b], M, bid, rb, fb, db, ro, lmove,
+      bond_term<R, ENER, R>(pos, base + T.bi[b], base + T.bj[b], M, bid, rb, fb, db, ro, lmove,
                          bx, by, bz, o, acc, &BD, &EB);
       if (laver) {
         add(sav[0], br, M, nrbb, (double)BD * fnspi);
@@ -387,7 +388,7 @@ __global__ void __launch_bounds__(128) k_molbonded(
     for (int a = 0; a < T.na; ++a) {
       const int M = T.am[a];
       R ALF, EA;
-      angle_term<R, true, R>(pos, base + T.ai[a], base + T.aj[a], base + T.ak[a], M, ra, fa,
+      angle_term<R, ENER, R>(pos, base + T.ai[a], base + T.aj[a], base + T.ak[a], M, ra, fa,
                           lmove, bx, by, bz, o, acc, &ALF, &EA);
       if (laver) {
         add(sav[2], ar, M, nraa, (double)ALF * fnspi);
@@ -395,15 +396,17 @@ __global__ void __launch_bounds__(128) k_molbonded(
       }
     }
   }
-  double a[5];
-  if (sizeof(R) == sizeof(double)) {
+  if (ENER) {
+    double a[5];
+    if (sizeof(R) == sizeof(double)) {
 #pragma unroll
-    for (int k = 0; k < 5; ++k) a[k] = (double)acc[k];
-    block_add<5>(a, dst);
-  } else {  // warp sums in FP32, then the FP64 block sums
+      for (int k = 0; k < 5; ++k) a[k] = (double)acc[k];
+      block_add<5>(a, dst);
+    } else {  // warp sums in FP32, then the FP64 block sums
 #pragma unroll
-    for (int k = 0; k < 5; ++k) a[k] = (double)warp_sumf((float)acc[k]);
-    block_add_core<5, true>(a, dst.p, dst.part, dst.ctr);
+      for (int k = 0; k < 5; ++k) a[k] = (double)warp_sumf((float)acc[k]);
+      block_add_core<5, true>(a, dst.p, dst.part, dst.ctr);
+    }
   }
   if (laver) {
     __syncthreads();
@@ -430,14 +433,13 @@ struct TorsList {  // torsion instances and their records
   TorsTab t;
 };
 
-// One torsion (GETTRS forces.f:340-505).  acc: PINT VIRFX VIRFY VIRFZ; the
-// angle and energy; false where the term is left out.
+// One torsion (GETTRS forces.f:340-505) in the one launch.  acc: PINT VIRFX VIRFY
+// VIRFZ.
 template <typename R>
-__device__ __forceinline__ bool tors_term(int N, const TorsList &q, const dbl4 *__restrict__ pos,
+__device__ __forceinline__ void tors_term(int N, const TorsList &q, const dbl4 *__restrict__ pos,
                                           const int4 *__restrict__ ainfo, const TypeConst &tc,
                                           double bxl, double byl, double bzl, const BondOut &o,
-                                          double (&acc)[4], R *argp, R *potp) {
-  bool ok = false;
+                                          double (&acc)[4]) {
   const int I = q.iti[N], J = q.jtj[N], K = q.ktk[N], L = q.ltl[N], M = q.ituk[N];
   const int ityp = ainfo[I].x;
   double a0, a1, a2, b0, b1, b2, c0, c1, c2;
@@ -469,7 +471,7 @@ __device__ __forceinline__ bool tors_term(int N, const TorsList &q, const dbl4 *
     if (fabs(si) < R(1.0e-10)) si = copysign(R(1.0e-10), si);
     R POTT = 0, DERI = 0;
     const int it = q.t.itors[M];
-    ok = true;
+    bool ok = true;
     if (it == 0) {
       const R FCN = (R)q.t.ft[M], TEQ = (R)q.t.rt[M];
       const int MUL = q.t.nmul[M];
@@ -506,8 +508,6 @@ __device__ __forceinline__ bool tors_term(int N, const TorsList &q, const dbl4 *
     }
     if (ok) {
       acc[0] = (double)POTT;
-      *argp = arg;
-      *potp = POTT;
       if (tc.lmove[ityp]) {
         const R de1 = DERI / den / si;
         axb = axb / den * co;
@@ -553,22 +553,138 @@ __device__ __forceinline__ bool tors_term(int N, const TorsList &q, const dbl4 *
       }
     }
   }
-  return ok;
 }
 
+// With statistics, and the mixed path's constrained systems (see launch_bonded).
 template <typename R>
-__global__ void k_gettrs(int nrrt, TorsList q, const dbl4 *__restrict__ pos,
+__global__ void k_gettrs(int nrrt, const int *__restrict__ iti,
+                         const int *__restrict__ jtj, const int *__restrict__ ktk,
+                         const int *__restrict__ ltl, const int *__restrict__ ituk,
+                         TorsTab tt, const dbl4 *__restrict__ pos,
                          const int4 *__restrict__ ainfo, TypeConst tc,
                          const int *__restrict__ nspec, double bxl, double byl,
-                         double bzl, BondOut o, Dst6 dst, int laver, double *trv, double *tev) {
+                         double bzl, BondOut o, Dst6 dst, int nrtt, int laver,
+                         double *trv, double *tev) {
   double acc[4] = {0, 0, 0, 0};  // PINT VIRFX VIRFY VIRFZ
   const int N = blockIdx.x * blockDim.x + threadIdx.x;
   if (N < nrrt) {
-    R arg, pot;
-    if (tors_term<R>(N, q, pos, ainfo, tc, bxl, byl, bzl, o, acc, &arg, &pot) && laver) {
-      const double fnspi = 1.0 / (double)nspec[ainfo[q.iti[N]].x];
-      atomicAdd(&trv[q.ituk[N]], fabs((double)arg * fnspi));
-      atomicAdd(&tev[q.ituk[N]], (double)pot * fnspi);
+    const int I = iti[N], J = jtj[N], K = ktk[N], L = ltl[N], M = ituk[N];
+    const int ityp = ainfo[I].x;
+    double a0, a1, a2, b0, b1, b2, c0, c1, c2;
+    vec(pos, J, I, bxl, byl, bzl, a0, a1, a2, o.cell);
+    vec(pos, K, J, bxl, byl, bzl, b0, b1, b2, o.cell);
+    vec(pos, L, K, bxl, byl, bzl, c0, c1, c2, o.cell);
+    const R ax = (R)a0, ay = (R)a1, az = (R)a2;
+    const R bx = (R)b0, by = (R)b1, bz = (R)b2;
+    const R cx = (R)c0, cy = (R)c1, cz = (R)c2;
+    const R ab = ax * bx + ay * by + az * bz;
+    const R bc = bx * cx + by * cy + bz * cz;
+    const R ac = ax * cx + ay * cy + az * cz;
+    const R at = ax * ax + ay * ay + az * az;
+    const R bt = bx * bx + by * by + bz * bz;
+    const R ct = cx * cx + cy * cy + cz * cz;
+    R axb = (at * bt) - (ab * ab);
+    R bxc = (bt * ct) - (bc * bc);
+    const R fnum = (ab * bc) - (ac * bt);
+    R den = axb * bxc;
+    if (den > R(1.0e-10)) {
+      den = sqrt(den);
+      R co = fnum / den;
+      co = fmin(co, R(1));
+      co = fmax(co, R(-1));
+      const R signum = ax * (by * cz - cy * bz) + ay * (bz * cx - cz * bx) + az * (bx * cy - cx * by);
+      const R arg = copysign(acos(co), signum);
+      const R SIN1F = sin(arg);
+      R si = SIN1F;
+      if (fabs(si) < R(1.0e-10)) si = copysign(R(1.0e-10), si);
+      R POTT = 0, DERI = 0;
+      const int it = tt.itors[M];
+      bool ok = true;
+      if (it == 0) {
+        const R FCN = (R)tt.ft[M], TEQ = (R)tt.rt[M];
+        const int MUL = tt.nmul[M];
+        const R EARG = MUL * arg - TEQ;
+        POTT = FCN * (R(1) + cos(EARG));
+        DERI = -FCN * MUL * sin(EARG);
+      } else if (it == 1) {
+        const R FN1 = (R)tt.ft1[M], FN2 = (R)tt.ft2[M], FN3 = (R)tt.ft3[M];
+        const R COS1F = cos(arg);
+        const R COS2F = R(2) * (COS1F * COS1F) - R(1);
+        const R COS3F = COS1F * (R(2) * COS2F - R(1));
+        const R SIN2F = R(2) * SIN1F * COS1F;
+        const R SIN3F = SIN1F * COS2F + SIN2F * COS1F;
+        POTT = FN1 * (R(1) + COS1F) + FN2 * (R(1) - COS2F) + FN3 * (R(1) + COS3F);
+        DERI = -FN1 * SIN1F + R(2) * FN2 * SIN2F - R(3) * FN3 * SIN3F;
+      } else if (it == 5) {
+        const R FN0 = (R)tt.ft[M], FN1 = (R)tt.ft1[M], FN2 = (R)tt.ft2[M], FN3 = (R)tt.ft3[M],
+                FN4 = (R)tt.ft4[M], FN5 = (R)tt.ft5[M], TEQ = (R)tt.rt[M];
+        const R EARG = arg - TEQ;
+        const R COSI = cos(EARG);
+        const R COSI2 = COSI * COSI, COSI3 = COSI * COSI2, COSI4 = COSI * COSI3,
+                COSI5 = COSI * COSI4;
+        const R SINI = sin(EARG);
+        POTT = FN0 + FN1 * COSI + FN2 * COSI2 + FN3 * COSI3 + FN4 * COSI4 + FN5 * COSI5;
+        DERI = -SINI * (FN1 + R(2) * FN2 * COSI + R(3) * FN3 * COSI2 + R(4) * FN4 * COSI3 +
+                        R(5) * FN5 * COSI4);
+      } else if (it == -1) {
+        const R FCN = (R)tt.ft[M], TEQ = (R)tt.rt[M];
+        const R EARG = arg - TEQ;
+        POTT = FCN * (EARG * EARG);
+        DERI = R(2) * FCN * EARG;
+      } else {
+        ok = false;
+      }
+      if (ok) {
+        acc[0] = (double)POTT;
+        if (laver) {
+          const double fnspi = 1.0 / (double)nspec[ityp];
+          atomicAdd(&trv[M], fabs((double)arg * fnspi));
+          atomicAdd(&tev[M], (double)POTT * fnspi);
+        }
+        if (tc.lmove[ityp]) {
+          const R de1 = DERI / den / si;
+          axb = axb / den * co;
+          bxc = bxc / den * co;
+          R dnum, dden;
+          dnum = cx * bt - bx * bc;
+          dden = (ab * bx - ax * bt) * bxc;
+          const R FFI1 = (dnum - dden) * de1;
+          dnum = ((bx - ax) * bc - ab * cx) + (R(2) * ac * bx - cx * bt);
+          dden = axb * (bc * cx - bx * ct) + (ax * bt - at * bx - ab * (bx - ax)) * bxc;
+          const R FFJ1 = (dnum - dden) * de1;
+          dnum = ab * bx - ax * bt;
+          dden = axb * (bt * cx - bc * bx);
+          const R FFL1 = (dnum - dden) * de1;
+          const R FFK1 = -(FFI1 + FFJ1 + FFL1);
+          dnum = cy * bt - by * bc;
+          dden = (ab * by - ay * bt) * bxc;
+          const R FFI2 = (dnum - dden) * de1;
+          dnum = ((by - ay) * bc - ab * cy) + (R(2) * ac * by - cy * bt);
+          dden = axb * (bc * cy - by * ct) + (ay * bt - at * by - ab * (by - ay)) * bxc;
+          const R FFJ2 = (dnum - dden) * de1;
+          dnum = ab * by - ay * bt;
+          dden = axb * (bt * cy - bc * by);
+          const R FFL2 = (dnum - dden) * de1;
+          const R FFK2 = -(FFI2 + FFJ2 + FFL2);
+          dnum = cz * bt - bz * bc;
+          dden = (ab * bz - az * bt) * bxc;
+          const R FFI3 = (dnum - dden) * de1;
+          dnum = ((bz - az) * bc - ab * cz) + (R(2) * ac * bz - cz * bt);
+          dden = axb * (bc * cz - bz * ct) + (az * bt - at * bz - ab * (bz - az)) * bxc;
+          const R FFJ3 = (dnum - dden) * de1;
+          dnum = ab * bz - az * bt;
+          dden = axb * (bt * cz - bc * bz);
+          const R FFL3 = (dnum - dden) * de1;
+          const R FFK3 = -(FFI3 + FFJ3 + FFL3);
+          add_force<R>(o, I, FFI1, FFI2, FFI3);
+          add_force<R>(o, J, FFJ1, FFJ2, FFJ3);
+          add_force<R>(o, K, FFK1, FFK2, FFK3);
+          add_force<R>(o, L, FFL1, FFL2, FFL3);
+          acc[1] = (double)(-(ax + bx) * FFI1 - bx * FFJ1 + cx * FFL1);
+          acc[2] = (double)(-(ay + by) * FFI2 - by * FFJ2 + cy * FFL2);
+          acc[3] = (double)(-(az + bz) * FFI3 - bz * FFJ3 + cz * FFL3);
+        }
+      }
     }
   }
   block_add<4>(acc, dst);
@@ -579,12 +695,12 @@ struct WaterPar {
   double roh1, roh2, rh1h2, aaa, bbb, ccc, eee, fff, ggg, ro1, ro2, aadd, bbdd;
 };
 
-// STRBND of one water (forces.f:560-790).  acc: PINT VIRB VIRFX VIRFY VIRFZ;
-// the three lengths and energies.
+// STRBND of one water (forces.f:560-790) in the one launch.  acc: PINT VIRB VIRFX
+// VIRFY VIRFZ.
 template <typename R>
 __device__ __forceinline__ void water_term(const WaterPar &w, int N, const dbl4 *__restrict__ pos,
                                            double bxl, double byl, double bzl, const BondOut &o,
-                                           double (&acc)[5], R (&len)[3], R (&en)[3]) {
+                                           double (&acc)[5]) {
   const R BBM = (R)(double)1.3f;  // BBMA, a REAL*4 literal (forces.f:566)
   const int I = w.first + 3 * N, J = I + 1, K = I + 2;
   const dbl4 pi = pos[I], pj = pos[J], pk = pos[K];
@@ -626,12 +742,6 @@ __device__ __forceinline__ void water_term(const WaterPar &w, int N, const dbl4 
     WB3 = CCC * SH * SH + GGG * SA * SB;
   }
   acc[0] = (double)WB1 + (double)WB2 + (double)WB3;
-  len[0] = ASS;
-  len[1] = BSS;
-  len[2] = CSS;
-  en[0] = WB1;
-  en[1] = WB2;
-  en[2] = WB3;
   if (w.lmove) {
     if (w.ipt == 2) {
       FB3A = ASS > BBM ? R(-2) * SA * (R)w.aadd * (R)w.ro1 : R(-2) * (R)w.aadd * EXPA * EXPAM;
@@ -668,18 +778,93 @@ template <typename R>
 __global__ void k_strbnd(WaterPar w, const dbl4 *__restrict__ pos, double bxl,
                          double byl, double bzl, BondOut o, Dst6 dst, int laver,
                          double *br, double *be) {
+  const R BBM = (R)(double)1.3f;  // BBMA, a REAL*4 literal (forces.f:566)
   double acc[5] = {0, 0, 0, 0, 0};  // PINT VIRB VIRFX VIRFY VIRFZ
   const int N = blockIdx.x * blockDim.x + threadIdx.x;
-  R len[3] = {0, 0, 0}, en[3] = {0, 0, 0};
-  if (N < w.nmol) water_term<R>(w, N, pos, bxl, byl, bzl, o, acc, len, en);
+  double brs[3] = {0, 0, 0}, bes[3] = {0, 0, 0};
+  if (N < w.nmol) {
+    const int I = w.first + 3 * N, J = I + 1, K = I + 2;
+    const dbl4 pi = pos[I], pj = pos[J], pk = pos[K];
+    double a0 = pj.x - pi.x, a1 = pj.y - pi.y, a2 = pj.z - pi.z;
+    double b0 = pk.x - pi.x, b1 = pk.y - pi.y, b2 = pk.z - pi.z;
+    double c0 = pk.x - pj.x, c1 = pk.y - pj.y, c2 = pk.z - pj.z;
+    if (w.ipt == 2) {  // only the Morse variant applies PBC (forces.f:626-640)
+      if (o.cell.icell == 0) {
+        pbc_rect(a0, a1, a2, bxl, byl, bzl, 0.5 * bxl, 0.5 * byl, 0.5 * bzl);
+        pbc_rect(b0, b1, b2, bxl, byl, bzl, 0.5 * bxl, 0.5 * byl, 0.5 * bzl);
+        pbc_rect(c0, c1, c2, bxl, byl, bzl, 0.5 * bxl, 0.5 * byl, 0.5 * bzl);
+      } else {
+        pbc_cell(a0, a1, a2, o.cell);
+        pbc_cell(b0, b1, b2, o.cell);
+        pbc_cell(c0, c1, c2, o.cell);
+      }
+    }
+    const R AX = (R)a0, AY = (R)a1, AZ = (R)a2, BX = (R)b0, BY = (R)b1, BZ = (R)b2,
+            CX = (R)c0, CY = (R)c1, CZ = (R)c2;
+    const R ASS = sqrt(AX * AX + AY * AY + AZ * AZ);
+    const R BSS = sqrt(BX * BX + BY * BY + BZ * BZ);
+    const R CSS = sqrt(CX * CX + CY * CY + CZ * CZ);
+    const R SA = ASS - (R)w.roh1, SB = BSS - (R)w.roh2, SH = CSS - (R)w.rh1h2;
+    const R AAA = (R)w.aaa, BBB = (R)w.bbb, CCC = (R)w.ccc, EEE = (R)w.eee,
+            FFF = (R)w.fff, GGG = (R)w.ggg;
+    R WB1, WB2, WB3, FB3A, FB3B, FB3C;
+    R EXPA = 0, EXPAM = 0, EXPB = 0, EXPBM = 0;
+    if (w.ipt == 2) {
+      EXPA = exp(-(R)w.ro1 * SA);
+      EXPAM = R(1) - EXPA;
+      EXPB = exp(-(R)w.ro2 * SB);
+      EXPBM = R(1) - EXPB;
+      WB1 = AAA * (EXPAM * EXPAM) + EEE * SA * SH;
+      WB2 = BBB * (EXPBM * EXPBM) + FFF * SB * SH;
+      WB3 = CCC * SH * SH + GGG * SA * SB;
+    } else {
+      WB1 = AAA * SA * SA + EEE * SA * SH;
+      WB2 = BBB * SB * SB + FFF * SB * SH;
+      WB3 = CCC * SH * SH + GGG * SA * SB;
+    }
+    acc[0] = (double)WB1 + (double)WB2 + (double)WB3;
+    if (laver) {
+      const double f = 1.0 / (double)w.nmol;
+      brs[0] = (double)ASS * f; brs[1] = (double)BSS * f; brs[2] = (double)CSS * f;
+      bes[0] = (double)WB1 * f; bes[1] = (double)WB2 * f; bes[2] = (double)WB3 * f;
+    }
+    if (w.lmove) {
+      if (w.ipt == 2) {
+        FB3A = ASS > BBM ? R(-2) * SA * (R)w.aadd * (R)w.ro1 : R(-2) * (R)w.aadd * EXPA * EXPAM;
+        FB3A = FB3A - EEE * SH - GGG * SB;
+        // the reference uses RO(I1) here (forces.f:676)
+        FB3B = BSS > BBM ? R(-2) * SB * (R)w.bbdd * (R)w.ro1 : R(-2) * (R)w.bbdd * EXPB * EXPBM;
+        FB3B = FB3B - FFF * SH - GGG * SA;
+        FB3C = R(-2) * CCC * SH - EEE * SA - FFF * SB;
+      } else {
+        FB3A = R(-2) * AAA * SA - EEE * SH - GGG * SB;
+        FB3B = R(-2) * BBB * SB - FFF * SH - GGG * SA;
+        FB3C = R(-2) * CCC * SH - EEE * SA - FFF * SB;
+      }
+      FB3A = FB3A / ASS;
+      FB3B = FB3B / BSS;
+      FB3C = FB3C / CSS;
+      const R AXX = FB3A * AX, AYY = FB3A * AY, AZZ = FB3A * AZ;
+      const R BXX = FB3B * BX, BYY = FB3B * BY, BZZ = FB3B * BZ;
+      const R CXX = FB3C * CX, CYY = FB3C * CY, CZZ = FB3C * CZ;
+      add_force<R>(o, I, -AXX - BXX, -AYY - BYY, -AZZ - BZZ);
+      add_force<R>(o, J, AXX - CXX, AYY - CYY, AZZ - CZZ);
+      add_force<R>(o, K, BXX + CXX, BYY + CYY, BZZ + CZZ);
+      const R VIX = AX * AXX + BX * BXX + CX * CXX;
+      const R VIY = AY * AYY + BY * BYY + CY * CYY;
+      const R VIZ = AZ * AZZ + BZ * BZZ + CZ * CZZ;
+      acc[1] = (double)VIX + (double)VIY + (double)VIZ;
+      acc[2] = (double)VIX;
+      acc[3] = (double)VIY;
+      acc[4] = (double)VIZ;
+    }
+  }
   block_add<5>(acc, dst);
   if (laver) {
     // second reduction: its own partials region and counter
     Dst6 d6{{&br[w.i1], &br[w.i1 + 1], &br[w.i1 + 2], &be[w.i1], &be[w.i1 + 1], &be[w.i1 + 2]},
             dst.part ? dst.part + (size_t)gridDim.x * 8 : nullptr, dst.ctr ? dst.ctr + 1 : nullptr};
-    const double f = 1.0 / (double)w.nmol;
-    double v6[6] = {(double)len[0] * f, (double)len[1] * f, (double)len[2] * f,
-                    (double)en[0] * f,  (double)en[1] * f,  (double)en[2] * f};
+    double v6[6] = {brs[0], brs[1], brs[2], bes[0], bes[1], bes[2]};
     block_add<6>(v6, d6);
   }
 }
@@ -717,8 +902,7 @@ __global__ void __launch_bounds__(128) k_bonded_all(BondedAll a, const dbl4 *__r
   double acc[5] = {0, 0, 0, 0, 0};  // PINT VIRB VIRFX VIRFY VIRFZ
   R v, e;
   if (kind < BK_MOL) {
-    R len[3], en[3];
-    if (N < a.w[kind].nmol) water_term<R>(a.w[kind], N, pos, bx, by, bz, o, acc, len, en);
+    if (N < a.w[kind].nmol) water_term<R>(a.w[kind], N, pos, bx, by, bz, o, acc);
   } else if (kind < BK_TORS) {
     int I = -1, J = 0, K = 0, M = 0, lmove = 0;
     bool angle = kind == BK_ANGLE;
@@ -756,7 +940,7 @@ __global__ void __launch_bounds__(128) k_bonded_all(BondedAll a, const dbl4 *__r
                           &v, &e);
   } else if (N < a.nrrt) {
     double t4[4] = {0, 0, 0, 0};
-    tors_term<R>(N, a.q, pos, ainfo, tc, bx, by, bz, o, t4, &v, &e);
+    tors_term<R>(N, a.q, pos, ainfo, tc, bx, by, bz, o, t4);
     acc[0] = t4[0];
     acc[2] = t4[1];
     acc[3] = t4[2];
@@ -813,7 +997,17 @@ int launch_bonded(mdx_ctx *ctx, int laver, bool ener) {
     w.aadd = w.aaa * w.ro1;
     w.bbdd = w.bbb * w.ro2;
   }
-  if (!laver) {
+  const int kinds = nw + (d.ntpl > 0) + (d.nrbt > 0) + (d.nrat > 0) + (d.nrrt > 0);
+  bool shake = false;
+  for (int t = 0; t < ctx->d.ntypes; ++t) shake |= ctx->ishejk[t] > 0;
+  // Mixed path: the FP32 terms' last bits depend on the kernel (the contraction
+  // of products and sums), and both stiff random starts and SHAKE's tolerance
+  // make much of a last bit within 20 steps.  Where one launch for all kinds
+  // gains least (template molecules alone: 98,304 atoms 13.9 against 12.6 us;
+  // constrained systems: 57 against 29 us of a 700 us step) the terms stay in
+  // their own kernels.
+  const bool own = mx && ((kinds == 1 && d.ntpl > 0) || (shake && ener));
+  if (!laver && !own) {
     BondedAll a{};
     int count[BK_N] = {};
     for (int k = 0; k < nw; ++k) {
@@ -871,14 +1065,14 @@ int launch_bonded(mdx_ctx *ctx, int laver, bool ener) {
   if (d.ntpl > 0) {
     const int nb = (d.ntpl_mol + T - 1) / T;
     Dst6 dst = dst6(ctx, nb, 5, &sc->pint, &sc->virb, &sc->virfx, &sc->virfy, &sc->virfz);
-#define GM(R)                                                                          \
-  k_molbonded<R><<<nb, T, 0, ctx->stream>>>(                                         \
+#define GM(R, E)                                                                       \
+  k_molbonded<R, E><<<nb, T, 0, ctx->stream>>>(                                         \
       d.ntpl, d.moltpl, d.bid, d.brb, d.bfb, d.bdb, d.bro, d.ara, d.afa, d.pos, ctx->tc, \
       nspec, bx, by, bz, o, dst, d.nrbb, d.nraa, laver, d.br, d.be, d.ar, d.ae)
     if (mx) {
-      GM(float);
+      if (ener) GM(float, true); else GM(float, false);
     } else {
-      GM(double);
+      GM(double, true);
     }
 #undef GM
     MDX_LAUNCHED(ctx);
@@ -915,7 +1109,8 @@ int launch_bonded(mdx_ctx *ctx, int laver, bool ener) {
     Dst6 dst = dst6(ctx, (d.nrrt + T - 1) / T, 4, &sc->pint, &sc->virfx, &sc->virfy, &sc->virfz);
 #define GT(R)                                                                          \
   k_gettrs<R><<<(d.nrrt + T - 1) / T, T, 0, ctx->stream>>>(                            \
-      d.nrrt, tl, d.pos, d.ainfo, ctx->tc, nspec, bx, by, bz, o, dst, laver, d.tr, d.te)
+      d.nrrt, tl.iti, tl.jtj, tl.ktk, tl.ltl, tl.ituk, tl.t, d.pos, d.ainfo, ctx->tc, nspec,  \
+      bx, by, bz, o, dst, d.nrtt, laver, d.tr, d.te)
     if (mx) GT(float); else GT(double);
 #undef GT
     MDX_LAUNCHED(ctx);

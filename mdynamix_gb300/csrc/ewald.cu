@@ -1066,10 +1066,12 @@ int host_inifur(mdx_ctx *ctx) {
     int ns = std::max(1, std::max(1, per_sm) * nsm / nib);
     // at least 64 atoms a slice (609 atoms: 128 39 us, 64 31, 32 29, 16 27; but 32
     // beads of 768 atoms at once: 17.15, 16.96, 17.4, 18.5 ms / 40 steps), or 128
-    // where the partial sums of 64 would not fit mdx_slforces_static's scratch
-    const int n64 = std::max(1, std::min(ns, d.n / 64));
+    // where that leaves a block a SM and a half (nothing to gain: 22,529 atoms 93 us
+    // either way) or the partial sums of 64 would not fit mdx_slforces_static's
+    // scratch
+    const int n64 = std::max(1, std::min(ns, d.n / 64)), n128 = std::max(1, std::min(ns, d.n / 128));
     const bool fits = (size_t)n64 * d.nkv * sizeof(double2) <= MDX_SK_STATIC_BYTES;
-    ns = fits ? n64 : std::max(1, std::min(ns, d.n / 128));
+    ns = fits && 2 * n128 * nib < 3 * nsm ? n64 : n128;
     d.sfac_slice = (d.n + ns - 1) / ns;
     d.sfac_nslice = (d.n + d.sfac_slice - 1) / d.sfac_slice;
     nslice_max = std::max(nslice_max, (size_t)d.sfac_nslice);
