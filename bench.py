@@ -59,15 +59,15 @@ OPS_EW_FROZEN_KATOM = 21
 # `python bench.py --only {fp64,mixed} --steps 2 --warmup 3`
 # (dram__bytes_read.sum + dram__bytes_write.sum of every launch of the
 # group's kernels in one long step, MB).
-# fp64 ewald: k_tables 43.4 + k_sfac 126.0 + k_sfac_sum 51.3 + k_kterms 1.0
-#             + k_wpairs 0.6 + k_rforce64 102.9
-# mixed ewald: k_tables 4.7 + k_zimages 18.0 + k_sfac32 53.7 + k_sfac_sum 32.4
-#              + k_kterms 1.0 + k_wtiles 0.6 + k_rforce_tc 75.4
-# fp64 pair: 9 x 30.7 (short, forces) + 30.7 (short, energies) + 153.1 (long)
-# mixed pair: 9 x 25.9 (short, forces) + 25.9 (short, energies) + 283.2 (long)
+# fp64 ewald: k_fx_tables 164.6 + k_fx_sfac 138.1 + k_fx_form 0.4 + k_fx_wtiles 1.0
+#             + k_fx_force 282.5 + k_fx_fold 4.7
+# mixed ewald: k_tables 27.4 + k_sfac32 52.8 + k_sfac_sum 33.1 + k_wtiles 0.6
+#              + k_rforce_tc 75.4
+# fp64 pair: 9 x 31.1 (short, forces) + 31.1 (short, energies) + 157.6 (long)
+# mixed pair: 9 x 28.3 (short, forces) + 25.9 (short, energies) + 282.8 (long)
 TRAFFIC_MB = {
-    ("fp64", "ewald"): 325.2, ("mixed", "ewald"): 185.8,
-    ("fp64", "pair"): 459.9, ("mixed", "pair"): 542.1,
+    ("fp64", "ewald"): 591.3, ("mixed", "ewald"): 189.3,
+    ("fp64", "pair"): 468.6, ("mixed", "pair"): 563.4,
 }
 
 
@@ -138,12 +138,15 @@ def roofline_of(timers, mbsh, mbln, nfreq, kset, n, peak64, peak32, prec, nsteps
     loops (NFREQ short-list passes + one long-list pass).  Ops per long step
     from the frozen per-unit constants; time from the device timers (CUDA
     events on the launching stream) of the instrumented pass, per long
-    step; peak = measured FMA throughput of the pipe the path computes on."""
+    step; peak = measured FMA throughput of the path's floating-point type.
+    The FP64 path forms most of its products as integers (pair sweeps) and as
+    FP16 digits on the tensor cores (Ewald), so it can exceed its FP64 peak."""
     ms = {k: v[0] / nsteps for k, v in timers.items()}
     nkv, ncol, npair, rows = kset
-    ew_kernels = ("k_tables + k_zimages + k_sfac32 + k_sfac_sum + k_kterms + k_wtiles + "
-                  "k_rforce_tc (TF32 tensor cores)" if prec == "mixed" else
-                  "k_tables + k_sfac + k_sfac_sum + k_kterms + k_wpairs + k_rforce64")
+    ew_kernels = ("k_tables + k_sfac32 + k_sfac_sum + k_wtiles + k_rforce_tc "
+                  "(TF32 tensor cores)" if prec == "mixed" else
+                  "k_fx_tables + k_fx_sfac + k_fx_form + k_fx_wtiles + k_fx_force + "
+                  "k_fx_fold (exact FP16 tensor cores)")
     groups = {
         "ewald": (ms["ew_tables"] + ms["ew_sfac"] + ms["ew_kterms"] + ms["ew_force"],
                   (OPS_EW_PAIR * npair + OPS_EW_COL * ncol + OPS_EW_ROW * rows) * n
