@@ -840,10 +840,6 @@ __global__ void k_fold_split(double *split, mdx_scalars *sc) {
   }
 }
 
-// FP64 path with one molecule type: POTE1 etc. from same/different sums is
-// not available (the FP64 sweep sums totals only), so the split sweep is used
-// whenever the caller asks for the per-type energies.
-
 PairTables tables(const DevData &d) {
   return PairTables{d.abf, d.nnbt * d.nnbt};
 }
