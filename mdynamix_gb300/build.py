@@ -42,8 +42,8 @@ def _stale(obj: str, src: str) -> bool:
     if not os.path.exists(obj):
         return True
     t = os.path.getmtime(obj)
-    deps = [src, os.path.join(CSRC, "mdx_internal.cuh"), os.path.join(CSRC, "tc_ptx.cuh"),
-            os.path.join(ROOT, "include", "mdx_gpu.h"), os.path.abspath(__file__)]
+    deps = [src, os.path.join(ROOT, "include", "mdx_gpu.h"), os.path.abspath(__file__)]
+    deps += [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     return any(os.path.getmtime(d) > t for d in deps)
 
 
