@@ -37,6 +37,7 @@
 
 #include "mdx_internal.cuh"
 #include "pair_math.cuh"
+#include "px_units.h"
 
 namespace {
 
@@ -974,7 +975,7 @@ Px px_args(const mdx_ctx *ctx, bool shrt) {
   x.hx = u(0.5 * ctx->boxl);
   x.hy = u(0.5 * ctx->boyl);
   x.hz = shrt ? x.hx : u(0.5 * ctx->bozl);
-  x.rc2 = (unsigned long long)std::ldexp(ctx->pc.rc2, 60 - 2 * rho);
+  x.rc2 = px_cut2(ctx->pc.rc2, rho);
   const int q2 = 2 * ctx->px_eq;
   const double cf = ctx->p.coulf;
   x.uG = std::ldexp(cf, q2 - s[PT_FORCE]);
