@@ -1044,6 +1044,10 @@ int mdx_upload_topology(mdx_ctx *ctx, const mdx_topo *t) {
   RC(shake_clusters(ctx, t));
   if (ctx->mixed()) RC(upload_site_table(ctx));
   ctx->have_topo = true;
+  if (ctx->have_params) {  // the pair sweeps' units follow the charges
+    ctx->drop_graphs();
+    RC(pair64_setup(ctx));
+  }
   return MDX_OK;
 }
 
