@@ -168,6 +168,14 @@ struct Dst6 {
   unsigned *ctr;
 };
 
+// The tables of the FP64 path's fixed-point pair sweeps, by sweep (0 short rows, 1
+// long): bins, first octave of r^2 (r^2 >= 2^oct0 A^2), binary scales of the four
+// functions.
+struct PxTables {
+  double alphad;
+  int nbin[2], oct0[2], s[2][4];
+};
+
 struct DevData {
   int n, nop, ntypes, nnbt, nbdmax;
   dbl4 *pos;
@@ -364,11 +372,11 @@ struct mdx_ctx {
   cudaEvent_t side_ev[5] = {};
   int red_slot = 0;  // 1, 2 while launching on them: reduction scratch of their own
   // FP64 path, fixed-point pair sweeps: on, position unit 2^-px_bits A (of the
-  // box when ipos was last written), charge unit 2^(px_eq - 62) e, and the
-  // sweeps' ranges (0 short, 1 long): |d| < 2^px_rho A, r^2 >= 2^px_oct A^2;
-  // px_s: binary scales of the four functions
+  // box when ipos was last written), charge unit 2^(px_eq - 62) e, the sweeps'
+  // ranges (0 short, 1 long) |d| < 2^px_rho A, and what dv.px_tab holds
   bool px_on = false;
-  int px_bits = 0, px_eq = 0, px_rho[2] = {0, 0}, px_oct[2] = {0, 0}, px_s[2][4] = {};
+  int px_bits = 0, px_eq = 0, px_rho[2] = {0, 0};
+  PxTables px{};
   int mbsh = 0, mbln = 0;
   cudaEvent_t snap_ev[MDX_SNAPSHOT_SLOTS] = {};  // completion of mdx_snapshot per slot
   // device timers (mdx_set_timers)

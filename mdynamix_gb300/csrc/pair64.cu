@@ -34,6 +34,7 @@
 // reaction field (LMNBL).
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 
 #include "mdx_internal.cuh"
 #include "pair_math.cuh"
@@ -125,48 +126,61 @@ __device__ dd pair_fn(int fn, double x, double alphad) {
 }
 
 // Coefficients of a function's polynomial in one bin: block of 32 bins x 7
-// Chebyshev points, a thread each for the values, then a thread per bin for
-// the divided differences and the monomial form (true there).
+// Chebyshev points.  Thread (point k, bin) forms the value at its point, its
+// divided difference of each order, then coefficient k of the monomial form.
+// An FP64 instruction takes a scheduler 64 cycles, so the chain of two-word
+// divisions is shared by the seven, and one launch makes both sweeps' tables
+// (mdx_set_params with another alpha: 400 us with one thread a bin and a launch a
+// sweep, 157 now; with the same tables 15).
+// Returns coefficient k = threadIdx.x / PTB, all of them left in sh.
 constexpr int PN = 7, PTB = 32;
 __device__ __forceinline__ double pt_node(int k) {
   return rint(0.5 * cospi((2 * k + 1) / (2.0 * PN)) * 1073741824.0) / 1073741824.0;
 }
-__device__ bool pt_coef(int fn, int oct0, int nbin, double alphad, dd (&c)[PN]) {
-  __shared__ dd sf[PN][PTB];
-  const int b = threadIdx.x % PTB, node = threadIdx.x / PTB, bin = blockIdx.x * PTB + b;
-  const double oct = ldexp(1.0, oct0 + bin / 128);
-  sf[node][b] = pair_fn(fn, oct * (1.0 + ((bin % 128) + 0.5 + pt_node(node)) / 128.0), alphad);
+__device__ dd pt_coef(int fn, int block, int oct0, double alphad, dd (&sh)[PN][PTB]) {
+  __shared__ double x[PN];
+  const int b = threadIdx.x % PTB, k = threadIdx.x / PTB, bin = block * PTB + b;
+  const double xk = pt_node(k);
+  if (b == 0) x[k] = xk;
+  dd f = pair_fn(fn, ldexp(1.0, oct0 + bin / 128) * (1.0 + ((bin % 128) + 0.5 + xk) / 128.0),
+                 alphad);
+  for (int o = 1; o < PN; ++o) {
+    sh[k][b] = f;
+    __syncthreads();
+    const dd below = sh[k > 0 ? k - 1 : 0][b];
+    if (k >= o) f = div(f + -below, D(xk - x[k - o]));
+    __syncthreads();
+  }
+  // c_m = c_(m - 1) - c_m x_j, c_0 = f_j - c_0 x_j, j from the last point down
+  __shared__ dd df[PN][PTB];
+  df[k][b] = f;
+  dd c = D(0.0);
+  for (int j = PN - 1; j >= 0; --j) {
+    sh[k][b] = c;
+    __syncthreads();
+    c = (k > 0 ? sh[k - 1][b] : df[j][b]) + -(c * D(x[j]));
+    __syncthreads();
+  }
+  sh[k][b] = c;
   __syncthreads();
-  if (node || bin >= nbin) return false;
-  double x[PN];
-  dd f[PN];
-  for (int k = 0; k < PN; ++k) {
-    x[k] = pt_node(k);
-    f[k] = sf[k][b];
-    c[k] = D(0.0);
-  }
-  for (int o = 1; o < PN; ++o)
-    for (int k = PN - 1; k >= o; --k) f[k] = div(f[k] + -f[k - 1], D(x[k] - x[k - o]));
-  for (int k = PN - 1; k >= 0; --k) {  // c = c (t - x_k) + f_k
-    for (int m = PN - 1; m > 0; --m) c[m] = c[m - 1] + -(c[m] * D(x[k]));
-    c[0] = f[k] + -(c[0] * D(x[k]));
-  }
-  return true;
+  return c;
 }
 __global__ void __launch_bounds__(PTB *PN) k_pair_table(double alphad, PairPoly *__restrict__ tab) {
-  dd c[PN];
-  const int bin = blockIdx.x * PTB + threadIdx.x % PTB, fn = blockIdx.y;
-  if (!pt_coef(fn, PT_OCT0, PT_BINS, alphad, c)) return;
-  PairPoly p;
-  p.c0 = c[0].h + c[0].l;
-  p.c1 = c[1].h + c[1].l;
-  p.c2 = c[2].h + c[2].l;
-  p.c3 = c[3].h + c[3].l;
-  p.c4 = (float)(c[4].h + c[4].l);
-  p.c5 = (float)(c[5].h + c[5].l);
-  p.c6 = (float)(c[6].h + c[6].l);
-  p.pad = 0.f;
-  tab[(size_t)fn * PT_BINS + bin] = p;
+  __shared__ dd sh[PN][PTB];
+  const int bin = blockIdx.x * PTB + threadIdx.x % PTB, fn = blockIdx.y, k = threadIdx.x / PTB;
+  const dd c = pt_coef(fn, blockIdx.x, PT_OCT0, alphad, sh);
+  PairPoly &p = tab[(size_t)fn * PT_BINS + bin];
+  const double v = c.h + c.l;
+  if (k == 0) p.c0 = v;
+  if (k == 1) p.c1 = v;
+  if (k == 2) p.c2 = v;
+  if (k == 3) p.c3 = v;
+  if (k == 4) p.c4 = (float)v;
+  if (k == 5) p.c5 = (float)v;
+  if (k == 6) {
+    p.c6 = (float)v;
+    p.pad = 0.f;
+  }
 }
 
 // FP32 to FP64 by the bits (a conversion instruction issues on the FP64
@@ -922,32 +936,33 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64x(
   sweep_out<SPLIT, ENER>(a, dst, s_split, split);
 }
 
-struct PxScale {
-  int s[PT_NFN];
-};
 __device__ __forceinline__ long long dd2ll(dd v, int s) {  // v 2^s to the nearest
   const double h = ldexp(v.h, s), r = rint(h);
   return (long long)r + __double2ll_rn((h - r) + ldexp(v.l, s));
 }
-__global__ void __launch_bounds__(PTB *PN) k_px_table(int nbin, int oct0, double alphad, PxScale sc,
-                                                     PxPoly *__restrict__ tab) {
-  dd c[PN];
-  const int bin = blockIdx.x * PTB + threadIdx.x % PTB, fn = blockIdx.y;
-  if (!pt_coef(fn, oct0, nbin, alphad, c)) return;
-  const int s = sc.s[fn];
-  PxPoly p;
-  p.c0 = dd2ll(c[0], s);
-  p.c1 = dd2ll(c[1], s + 1);
-  p.c2 = dd2ll(c[2], s + 2);
-  const double c3 = ldexp(c[3].h, s + 3);
+// Block (bins of one sweep, function): the long rows' bins follow the short rows'.
+__global__ void __launch_bounds__(PTB *PN) k_px_table(PxTables x, PxPoly *__restrict__ tab) {
+  __shared__ dd sh[PN][PTB];
+  const int nb0 = x.nbin[0] / PTB, w = (int)blockIdx.x >= nb0, block = blockIdx.x - w * nb0;
+  const int b = threadIdx.x % PTB, k = threadIdx.x / PTB, fn = blockIdx.y, s = x.s[w][fn];
+  const dd c = pt_coef(fn, block, x.oct0[w], x.alphad, sh);
+  PxPoly &p = tab[(w ? PT_NFN * x.nbin[0] : 0) + fn * x.nbin[w] + block * PTB + b];
+  const double c3 = ldexp(sh[3][b].h, s + 3);
   const int K = min(32, max(0, ilogb(fmax(fabs(c3), 1.0)) + 1 - 30));
-  p.c3 = (int)dd2ll(c[3], s + 3 - K);
-  p.sh = 32 - K;
-  p.c4 = (float)ldexp(c[4].h, s + 3 - K);
-  p.c5 = (float)ldexp(c[5].h, s + 3 - K);
-  p.c6 = (float)ldexp(c[6].h, s + 3 - K);
-  p.pad = 0.f;
-  tab[(size_t)fn * nbin + bin] = p;
+  if (k == 0) p.c0 = dd2ll(c, s);
+  if (k == 1) p.c1 = dd2ll(c, s + 1);
+  if (k == 2) p.c2 = dd2ll(c, s + 2);
+  if (k == 3) {
+    p.c3 = (int)dd2ll(c, s + 3 - K);
+    p.sh = 32 - K;
+  }
+  const float v = (float)ldexp(c.h, s + 3 - K);
+  if (k == 4) p.c4 = v;
+  if (k == 5) p.c5 = v;
+  if (k == 6) {
+    p.c6 = v;
+    p.pad = 0.f;
+  }
 }
 
 __global__ void k_ipos(int n, const dbl4 *__restrict__ pos, IPosOut o) {
@@ -955,20 +970,18 @@ __global__ void k_ipos(int n, const dbl4 *__restrict__ pos, IPosOut o) {
   if (i < n) ipos_store(o, i, pos[i]);
 }
 
-int px_bins(const mdx_ctx *ctx, int w) { return 128 * (2 * ctx->px_rho[w] - ctx->px_oct[w]); }
-
 // The sweep's constants for the current box (units of ipos as last written).
 Px px_args(const mdx_ctx *ctx, bool shrt) {
   Px x{};
   if (!ctx->px_on) return x;
   const int w = shrt ? 0 : 1, rho = ctx->px_rho[w], B = ctx->px_bits;
-  const int *s = ctx->px_s[w];
+  const int *s = ctx->px.s[w];
   auto u = [&](double a) { return std::llrint(std::ldexp(a, B)); };
   x.s = 62 - rho - B;
   x.rng = 1 << (B + rho - 32);
-  x.nbin = px_bins(ctx, w);
+  x.nbin = ctx->px.nbin[w];
   // octave of r2: 2 rho + 3 - lz; the upper byte of the mantissa is 128 ..
-  x.base = 128 * (2 * rho + 3 - ctx->px_oct[w]) - 128;
+  x.base = 128 * (2 * rho + 3 - ctx->px.oct0[w]) - 128;
   x.lx = u(ctx->boxl);
   x.ly = u(ctx->boyl);
   x.lz = u(ctx->bozl);
@@ -985,7 +998,7 @@ Px px_args(const mdx_ctx *ctx, bool shrt) {
   x.uE = std::ldexp(cf, q2 + 4 - s[PT_ENER]);
   x.uR = std::ldexp(cf, q2 + 4 - s[PT_R1I]);
   x.s2 = s[PT_R2I];
-  x.tab = reinterpret_cast<const PxPoly *>(ctx->dv.px_tab) + (shrt ? 0 : PT_NFN * px_bins(ctx, 0));
+  x.tab = reinterpret_cast<const PxPoly *>(ctx->dv.px_tab) + (shrt ? 0 : PT_NFN * ctx->px.nbin[0]);
   return x;
 }
 
@@ -1013,7 +1026,7 @@ int launch_ipos(mdx_ctx *ctx) {
 double px_force_unit(const mdx_ctx *ctx, int which) {
   if (!ctx->px_on) return 0.0;
   const int w = which == 1 ? 0 : 1;
-  return std::ldexp(ctx->p.coulf, 2 * ctx->px_eq - ctx->px_s[w][PT_FORCE] + ctx->px_rho[w] + 2);
+  return std::ldexp(ctx->p.coulf, 2 * ctx->px_eq - ctx->px.s[w][PT_FORCE] + ctx->px_rho[w] + 2);
 }
 
 // The Ewald tables of the sweeps for the current parameters (FP64 path;
@@ -1038,25 +1051,30 @@ int pair64_setup(mdx_ctx *ctx) {
     ctx->px_eq = std::ilogb(qmax) + (std::ldexp(1.0, std::ilogb(qmax)) < qmax ? 1 : 0);
     ctx->px_rho[0] = rho(1.2 * ctx->p.rshort);
     ctx->px_rho[1] = std::max(rho(rl), ctx->px_rho[0]);  // RCUT may lie below RSHORT
-    ctx->px_oct[0] = 1;
-    ctx->px_oct[1] = std::max(1, std::ilogb(0.64 * ctx->p.rshort * ctx->p.rshort));
-    const int nb[2] = {px_bins(ctx, 0), px_bins(ctx, 1)};
-    if (!d.px_tab) MDX_CUDA(ctx_alloc(ctx, &d.px_tab, sizeof(PxPoly) * PT_NFN * 2 * 128 * 10));
+    PxTables x{};
+    x.alphad = ctx->p.alphad;
+    x.oct0[0] = 1;
+    x.oct0[1] = std::max(1, std::ilogb(0.64 * ctx->p.rshort * ctx->p.rshort));
     for (int w = 0; w < 2; ++w) {
+      x.nbin[w] = 128 * (2 * ctx->px_rho[w] - x.oct0[w]);
       // binary scale of each function: below 2^62 at the first r^2.  Long
       // rows, forces: 2^60, so that some hundred pairs of one sign still fit
-      const double x = std::ldexp(1.0, ctx->px_oct[w]), r = std::sqrt(x);
+      const double x2 = std::ldexp(1.0, x.oct0[w]), r = std::sqrt(x2);
       const double ar = ctx->p.alphad * r, t = 1.0 / (1.0 + MDX_B1 * ar), e = std::exp(-ar * ar);
       const double er =
           ((((MDX_A5 * t + MDX_A4) * t + MDX_A3) * t + MDX_A2) * t + MDX_A1) * t * e / r;
-      const double f0[PT_NFN] = {(MDX_TOTPI * ctx->p.alphad * e + er) / x, er, 1.0 / r, 1.0 / x};
-      PxScale sc;
+      const double f0[PT_NFN] = {(MDX_TOTPI * ctx->p.alphad * e + er) / x2, er, 1.0 / r, 1.0 / x2};
       for (int f = 0; f < PT_NFN; ++f)
-        sc.s[f] = ctx->px_s[w][f] = (w && f == PT_FORCE ? 60 : 62) - 1 - std::ilogb(1.0001 * f0[f]);
-      k_px_table<<<dim3(nb[w] / PTB, PT_NFN), PTB * PN, 0, ctx->stream>>>(
-          nb[w], ctx->px_oct[w], ctx->p.alphad, sc,
-          reinterpret_cast<PxPoly *>(d.px_tab) + (w ? PT_NFN * nb[0] : 0));
+        x.s[w][f] = (w && f == PT_FORCE ? 60 : 62) - 1 - std::ilogb(1.0001 * f0[f]);
+    }
+    // Formed again only when something they depend on has changed: a caller that
+    // sets thermostats or time steps between segments keeps them.
+    if (!d.px_tab) MDX_CUDA(ctx_alloc(ctx, &d.px_tab, sizeof(PxPoly) * PT_NFN * 2 * 128 * 10));
+    if (std::memcmp(&ctx->px, &x, sizeof x) != 0) {
+      k_px_table<<<dim3((x.nbin[0] + x.nbin[1]) / PTB, PT_NFN), PTB * PN, 0, ctx->stream>>>(
+          x, reinterpret_cast<PxPoly *>(d.px_tab));
       MDX_LAUNCHED(ctx);
+      ctx->px = x;
     }
     ctx->px_on = true;
     return MDX_OK;

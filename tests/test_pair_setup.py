@@ -4,6 +4,7 @@ not depend on an order, so contexts that run the same sweeps in the same units
 agree to the last bit: no tolerance."""
 import copy
 import ctypes as C
+import dataclasses
 
 import numpy as np
 import pytest
@@ -77,3 +78,24 @@ def test_parameters_before_topology():
     assert _same(a, _evaluate(p, st))
     g.close()
     p.close()
+
+
+def test_tables_are_made_when_they_change():
+    """The same parameters again launch nothing; another alpha or RSHORT and back
+    gives what a context with them from the start gives."""
+    from mdynamix_gb300.mdx import ForcePath
+    s = _ions(150, 30.0, fexp=4.0)
+    st = S.make_configuration(s, seed=4, jitter=0.05)
+    g = ForcePath(s, precision=MDX_FP64)
+    a = _evaluate(g, st)
+    n = g.launches
+    g.set_params(g.packed.params)
+    assert g.launches == n
+    assert _same(a, _evaluate(g, st))
+    for change in (dict(alpha=3.0), dict(rshort=6.5), dict(rcut=8.5), {}):
+        t = S.System(dataclasses.replace(s.spec, **change))
+        f = ForcePath(t, precision=MDX_FP64)
+        g.set_params(f.packed.params)
+        assert _same(_evaluate(f, st), _evaluate(g, st)), change
+        f.close()
+    g.close()
