@@ -329,12 +329,17 @@ int mdx_pool_usage(size_t *used_bytes, size_t *reserved_bytes);
 /* Which kernels the context runs, for reports next to measured numbers (no
  * counterpart in the reference).  Valid once the k-set exists.
  *  ewald_force_pass: 0 FP64 CUDA cores; 1 FP32 CUDA cores; 2 TF32 tensor
- *                    cores, three products per operand pair.
+ *                    cores, three products per operand pair; 3 (FP64 path)
+ *                    fixed point, FP16 digits on the tensor cores.
  *  ewald_sfac_pass:  0 FP64 per slice, slices summed in FP64; 1 FP32 FMAs
  *                    per slice, slices summed in FP64; 2 TF32 tensor cores
- *                    with FP32 partials of 1024 atoms summed in FP64.
- *  sfac_ordered:     1 when slice partials are summed in slice order (the
- *                    reciprocal sums are then reproducible run to run).
+ *                    with FP32 partials of 1024 atoms summed in FP64; 3 (FP64
+ *                    path) fixed point on the tensor cores, slices summed as
+ *                    64-bit integers.
+ *  sfac_slices:      atom slices of the S(k) pass.
+ *  sfac_ordered:     1 when slice partials are summed in slice order or as
+ *                    integers (the reciprocal sums are then reproducible run
+ *                    to run).
  *  list_mode:        0 the reference's (CHCNB every ICHNB long steps);
  *                    1 Verlet skin. */
 typedef struct {

@@ -1554,9 +1554,9 @@ int mdx_get_path_info(const mdx_ctx *ctx, mdx_path_info *out) {
   const DevData &d = ctx->dv;
   const bool mx = ctx->mixed();
   out->precision = ctx->d.precision;
-  out->ewald_force_pass = !mx ? 0 : d.tc_on ? 2 : 1;
-  out->ewald_sfac_pass = !mx ? 0 : d.tcs_on ? 2 : 1;
-  out->sfac_slices = ctx->furir_init ? sfac_slices(ctx) : 0;
+  out->ewald_force_pass = !mx ? (d.fx_on ? 3 : 0) : d.tc_on ? 2 : 1;
+  out->ewald_sfac_pass = !mx ? (d.fx_on ? 3 : 0) : d.tcs_on ? 2 : 1;
+  out->sfac_slices = !ctx->furir_init ? 0 : d.fx_on ? d.fx_ns : sfac_slices(ctx);
   out->sfac_ordered = (mx && d.tcs_on) || d.fx_on || d.sk_part != nullptr ? 1 : 0;
   out->list_mode = ctx->p.rskin > 0.0 ? 1 : 0;
   out->graphs = ctx->use_graphs ? 1 : 0;
