@@ -837,6 +837,7 @@ int host_inifur(mdx_ctx *ctx) {
   const int icell = ctx->p.icell;
   DevData &d = ctx->dv;
   ctx->drop_graphs();  // k-set buffers are reallocated below
+  ctx->furir_init = false;  // the caller's, once all of it has succeeded
   const double alphad = ctx->p.alphad;
   const double ALP2 = alphad * alphad;
   const double CUTK2 = 4.0 * ALP2 * ctx->p.fexp;
@@ -1079,7 +1080,7 @@ int host_inifur(mdx_ctx *ctx) {
   if (d.fx_on) {  // the FP64 tables stay unused
     ctx_free(ctx, d.tabx);
     d.tabx = d.taby = d.tabz = nullptr;
-  } else if (realloc_tables || (!ctx->mixed() && !d.tabx)) {
+  } else if (realloc_tables || !(ctx->mixed() ? (void *)d.tabxf : (void *)d.tabx)) {
     ctx_free(ctx, d.tabx);
     ctx_free(ctx, d.tabxf);
     d.tabx = d.taby = d.tabz = nullptr;
@@ -1100,6 +1101,7 @@ int host_inifur(mdx_ctx *ctx) {
   }
   ctx_free(ctx, d.sk);
   ctx_free(ctx, d.kconst);
+  d.sk = nullptr;
   d.kconst = nullptr;
   ctx->kc_box[0] = -1.0;  // per-k constants rebuilt at the next FURIR
   const size_t nk = (size_t)std::max(1, nkv);
@@ -1157,11 +1159,11 @@ int furir_prepare(mdx_ctx *ctx) {
   const double FKTX = 1.05, FKTS = 0.95;
   int rc;
   if (!ctx->furir_init) {
-    ctx->furir_init = true;
     ctx->boxlo = ctx->boxl;
     ctx->boylo = ctx->boyl;
     ctx->bozlo = ctx->bozl;
     if ((rc = host_inifur(ctx))) return rc;
+    ctx->furir_init = true;
   }
   const double DBX = ctx->boxl / ctx->boxlo, DBY = ctx->boyl / ctx->boylo,
                DBZ = ctx->bozl / ctx->bozlo;
@@ -1171,6 +1173,7 @@ int furir_prepare(mdx_ctx *ctx) {
     ctx->boylo = ctx->boyl;
     ctx->bozlo = ctx->bozl;
     if ((rc = host_inifur(ctx))) return rc;
+    ctx->furir_init = true;
   }
   return MDX_OK;
 }

@@ -922,7 +922,8 @@ void fx_release(mdx_ctx *ctx) {
 // Sizes, tables and buffers for a k-set (INIFUR).  The passes need K = 2 kz
 // <= 64 (exact class sums, tensor memory) and their operands in shared
 // memory: |nz| up to 31 and about 60 X and Y rows; other k-sets keep the
-// FP64-pipe passes.  Returns MDX_OK with d.fx_on telling which.
+// FP64-pipe passes, and so does a system whose images the device has no room for.
+// Returns MDX_OK with d.fx_on telling which.
 int fx_setup(mdx_ctx *ctx, const std::vector<KCol> &cols) {
   DevData &d = ctx->dv;
   fx_release(ctx);
@@ -997,9 +998,9 @@ int fx_setup(mdx_ctx *ctx, const std::vector<KCol> &cols) {
       ctx_alloc(ctx, &d.fx_acc, accb + 16) != cudaSuccess ||
       ctx_alloc(ctx, &d.fx_facc, sizeof(long long) * 3 * d.n + 16) != cudaSuccess ||
       ctx_alloc(ctx, &d.fx_qs, 2 * sizeof(double) + FX_CIRCLE * sizeof(int4)) != cudaSuccess) {
-    cudaGetLastError();
-    ctx->err = "fixed-point Ewald passes: device allocation failed";
-    return MDX_ERR_NOMEM;
+    // no room for the images (some 2 KB an atom): the FP64-pipe passes
+    fx_release(ctx);
+    return MDX_OK;
   }
   // k_fx_form and k_fx_sfac leave the sums and the flag behind them cleared
   MDX_CUDA(cudaMemsetAsync(d.fx_acc, 0, accb + 16, ctx->stream));

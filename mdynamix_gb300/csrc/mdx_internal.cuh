@@ -377,6 +377,7 @@ struct mdx_ctx {
   bool px_on = false;
   int px_bits = 0, px_eq = 0, px_rho[2] = {0, 0};
   PxTables px{};
+  int fail_alloc = 0;  // mdx_probe_fail_alloc: this many ctx_alloc calls from now, one fails
   int mbsh = 0, mbln = 0;
   cudaEvent_t snap_ev[MDX_SNAPSHOT_SLOTS] = {};  // completion of mdx_snapshot per slot
   // device timers (mdx_set_timers)
@@ -766,8 +767,10 @@ __device__ __forceinline__ void fix_addf(unsigned long long *a, float v,
 // allocation is followed by a sync of the context's own stream, so host-side
 // copies into it may follow at once.
 inline cudaError_t ctx_alloc(mdx_ctx *ctx, void **p, size_t bytes) {
+  if (ctx->fail_alloc > 0 && --ctx->fail_alloc == 0) return cudaErrorMemoryAllocation;
   cudaError_t e = cudaMallocAsync(p, bytes, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  else cudaGetLastError();  // reported here, not by the next launch's check
   return e;
 }
 // Copy on a context's stream and wait: ordered after the stream's kernels

@@ -101,6 +101,14 @@ extern "C" int mdx_probe_pair_math(int n, const double *y, const double *d, doub
   return rc;
 }
 
+// The k-th device allocation of a context's set-up routines from now on is
+// answered with "out of memory" (0: none), so that tests reach what follows.
+extern "C" int mdx_probe_fail_alloc(mdx_ctx *ctx, int k) {
+  if (!ctx || k < 0) return MDX_ERR_ARG;
+  ctx->fail_alloc = k;
+  return MDX_OK;
+}
+
 extern "C" int mdx_probe_fma_peak(int fp64, double *tflops) {
   if (!tflops) return MDX_ERR_ARG;
   *tflops = fp64 ? run<double>(1 << 12) : run<float>(1 << 16);
