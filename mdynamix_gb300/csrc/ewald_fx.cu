@@ -39,6 +39,7 @@
 // at 3,000 (4.2e-15).
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "ewald_ops.cuh"
@@ -894,28 +895,27 @@ int ceil_log2(int n) {
 // The charge scale (a power of two above every |q|) for the tables, kept on
 // the device so that captured graphs see the current one: after the topology
 // upload and every RECINT.
-int fx_update_qscale(mdx_ctx *ctx) {
-  DevData &d = ctx->dv;
-  if (!d.fx_qs) return MDX_OK;
+static void fx_qscale(const mdx_ctx *ctx, double (&qs)[2]) {
   double m = 0.0;
   for (double q : ctx->h_q) m = std::max(m, std::fabs(q));
   int e = 0;
   if (m > 0.0) std::frexp(m, &e);  // m < 2^e
-  const double qs[2] = {std::ldexp(1.0, e), std::ldexp(1.0, -e)};
-  MDX_CUDA(ctx_copy(ctx->stream, d.fx_qs, qs, sizeof qs, cudaMemcpyHostToDevice));
+  qs[0] = std::ldexp(1.0, e);
+  qs[1] = std::ldexp(1.0, -e);
+}
+int fx_update_qscale(mdx_ctx *ctx) {
+  if (!ctx->dv.fx_qs) return MDX_OK;
+  double qs[2];
+  fx_qscale(ctx, qs);
+  MDX_CUDA(ctx_copy(ctx->stream, ctx->dv.fx_qs, qs, sizeof qs, cudaMemcpyHostToDevice));
   return MDX_OK;
 }
 
 void fx_release(mdx_ctx *ctx) {
   DevData &d = ctx->dv;
-  void **p[] = {(void **)&d.fx_xy,   (void **)&d.fx_zs,   (void **)&d.fx_zf,
-                (void **)&d.fx_tw,   (void **)&d.fx_meta, (void **)&d.fx_slot,
-                (void **)&d.fx_scol, (void **)&d.fx_acc,  (void **)&d.fx_facc,
-                (void **)&d.fx_qs};
-  for (void **q : p) {
-    ctx_free(ctx, *q);
-    *q = nullptr;
-  }
+  ctx_free(ctx, d.fx_buf);
+  d.fx_buf = nullptr;
+  d.fx_qs = nullptr;
   d.fx_on = false;
 }
 
@@ -984,47 +984,64 @@ int fx_setup(mdx_ctx *ctx, const std::vector<KCol> &cols) {
   const size_t zfb = (size_t)natile * (kp / 16) * FX_SL * 4096;
   const size_t xyb = sizeof(int4) * (size_t)natile * 4 * kxy * FX_ROW;
   const size_t accb = sizeof(long long) * (size_t)d.fx_ntm * np * 128;
-  std::vector<int> ints;
-  ints.insert(ints.end(), scol.begin(), scol.end());
-  ints.insert(ints.end(), ks.begin(), ks.end());
-  ints.insert(ints.end(), parts.begin(), parts.end());
-  if (ctx_alloc(ctx, &d.fx_xy, xyb) != cudaSuccess ||
-      ctx_alloc(ctx, &d.fx_zs, zsb) != cudaSuccess ||
-      ctx_alloc(ctx, &d.fx_zf, zfb) != cudaSuccess ||
-      ctx_alloc(ctx, &d.fx_tw, (size_t)ntile * (kp / 16) * FX_SL * FX_TN * 32) != cudaSuccess ||
-      ctx_alloc(ctx, &d.fx_meta, sizeof(FxTile) * ntile) != cudaSuccess ||
-      ctx_alloc(ctx, &d.fx_slot, sizeof(int4) * slot.size()) != cudaSuccess ||
-      ctx_alloc(ctx, &d.fx_scol, sizeof(int) * ints.size()) != cudaSuccess ||
-      ctx_alloc(ctx, &d.fx_acc, accb + 16) != cudaSuccess ||
-      ctx_alloc(ctx, &d.fx_facc, sizeof(long long) * 3 * d.n + 16) != cudaSuccess ||
-      ctx_alloc(ctx, &d.fx_qs, 2 * sizeof(double) + FX_CIRCLE * sizeof(int4)) != cudaSuccess) {
-    // no room for the images (some 2 KB an atom): the FP64-pipe passes
-    fx_release(ctx);
+  // One allocation, one upload and one clearing: an INIFUR of a small box is a few
+  // dozen microseconds, and each allocation or copy waits for the stream.
+  size_t len = 0;
+  auto part = [&](size_t bytes) {
+    const size_t o = len;
+    len = (len + bytes + 255) & ~(size_t)255;
+    return o;
+  };
+  // uploaded: charge scale and circle points, column slots, columns, K steps, ranges
+  const size_t oqs = part(2 * sizeof(double) + FX_CIRCLE * sizeof(int4)),
+               oslot = part(sizeof(int4) * slot.size()), oscol = part(sizeof(int) * scol.size()),
+               oks = part(sizeof(int) * ks.size()), oparts = part(sizeof(int) * parts.size());
+  const size_t up = len;
+  // cleared: the sums and the flag behind them, which k_fx_form and k_fx_sfac leave
+  // cleared; chunks past the last atom (a 128-atom tile's end) and the images' rows
+  // past 2 kz, which stay zero
+  const size_t oacc = part(accb + 16), oxy = part(xyb), ozs = part(zsb), ozf = part(zfb);
+  const size_t clear = len;
+  const size_t otw = part((size_t)ntile * (kp / 16) * FX_SL * FX_TN * 32),
+               ometa = part(sizeof(FxTile) * ntile),
+               ofacc = part(sizeof(long long) * 3 * d.n + 16);
+  if (ctx_alloc(ctx, &d.fx_buf, len) != cudaSuccess) {
+    d.fx_buf = nullptr;  // no room for the images (some 2 KB an atom): the FP64-pipe passes
     return MDX_OK;
   }
-  // k_fx_form and k_fx_sfac leave the sums and the flag behind them cleared
-  MDX_CUDA(cudaMemsetAsync(d.fx_acc, 0, accb + 16, ctx->stream));
-  d.fx_ks = d.fx_scol + scol.size();
-  d.fx_parts = d.fx_ks + ks.size();
-  MDX_CUDA(ctx_copy(ctx->stream, d.fx_slot, slot.data(), sizeof(int4) * slot.size(),
-                    cudaMemcpyHostToDevice));
-  MDX_CUDA(ctx_copy(ctx->stream, d.fx_scol, ints.data(), sizeof(int) * ints.size(),
-                    cudaMemcpyHostToDevice));
-  const std::vector<int> &circle = circle_points();  // behind the charge scale
-  MDX_CUDA(ctx_copy(ctx->stream, d.fx_qs + 2, circle.data(), sizeof(int) * circle.size(),
-                    cudaMemcpyHostToDevice));
-  // chunks past the last atom (a 128-atom tile's end) and the images' rows
-  // past 2 kz stay zero
-  MDX_CUDA(cudaMemsetAsync(d.fx_xy, 0, xyb, ctx->stream));
-  MDX_CUDA(cudaMemsetAsync(d.fx_zs, 0, zsb, ctx->stream));
-  MDX_CUDA(cudaMemsetAsync(d.fx_zf, 0, zfb, ctx->stream));
+  unsigned char *const buf = d.fx_buf;
+  d.fx_qs = reinterpret_cast<double *>(buf + oqs);
+  d.fx_slot = reinterpret_cast<int4 *>(buf + oslot);
+  d.fx_scol = reinterpret_cast<int *>(buf + oscol);
+  d.fx_ks = reinterpret_cast<int *>(buf + oks);
+  d.fx_parts = reinterpret_cast<int *>(buf + oparts);
+  d.fx_acc = reinterpret_cast<unsigned long long *>(buf + oacc);
+  d.fx_xy = reinterpret_cast<int4 *>(buf + oxy);
+  d.fx_zs = buf + ozs;
+  d.fx_zf = buf + ozf;
+  d.fx_tw = buf + otw;
+  d.fx_meta = buf + ometa;
+  d.fx_facc = reinterpret_cast<unsigned long long *>(buf + ofacc);
+  std::vector<unsigned char> host(up);
+  auto put = [&](size_t o, const void *p, size_t bytes) { std::memcpy(host.data() + o, p, bytes); };
+  const std::vector<int> &circle = circle_points();
+  double qs[2];
+  fx_qscale(ctx, qs);
+  put(oqs, qs, sizeof qs);
+  put(oqs + sizeof qs, circle.data(), sizeof(int) * circle.size());
+  put(oslot, slot.data(), sizeof(int4) * slot.size());
+  put(oscol, scol.data(), sizeof(int) * scol.size());
+  put(oks, ks.data(), sizeof(int) * ks.size());
+  put(oparts, parts.data(), sizeof(int) * parts.size());
+  MDX_CUDA(cudaMemsetAsync(buf + up, 0, clear - up, ctx->stream));
+  MDX_CUDA(ctx_copy(ctx->stream, buf, host.data(), up, cudaMemcpyHostToDevice));
   MDX_CUDA(raise_smem_limit(k_fx_sfac, fx_sfac_smem(np, kxy)));
   const size_t fsm = fx_force_smem(kp, kxy, d.fx_xys);
   MDX_CUDA(raise_smem_limit(fx_force_kernel(kp, d.fx_xys), fsm));
   d.fx_np = np;
   d.fx_ntile = ntile;
   d.fx_on = true;
-  return fx_update_qscale(ctx);
+  return MDX_OK;
 }
 
 // Phase tables, operand images and S(k) of the current positions.

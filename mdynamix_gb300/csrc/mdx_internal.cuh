@@ -272,6 +272,7 @@ struct DevData {
   // S(k) and force sums, the charge scale {qs, 1 / qs}
   void *pair_tab;  // FP64 pair sweeps: tabulated functions of r^2 (pair64.cu)
   bool fx_on, fx_xys;
+  unsigned char *fx_buf;  // holds all of them
   int4 *fx_xy, *fx_slot;
   unsigned char *fx_zs, *fx_zf, *fx_tw, *fx_meta;
   int *fx_scol, *fx_ks, *fx_parts;

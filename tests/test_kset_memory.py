@@ -49,3 +49,27 @@ def test_refused_allocations(prec):
         g.close()
     assert "refused" in outcomes and outcomes[-1] == "ok"  # past the last allocation
     assert prec == MDX_MIXED or "ok, FP64 pipe" in outcomes
+
+
+def test_fixed_point_passes_cost_one_allocation(monkeypatch):
+    """INIFUR with the fixed-point passes allocates no more often than with the
+    FP64-pipe passes (an allocation waits for the stream).  Counted with the hook:
+    the first allocation whose refusal changes nothing is one too many."""
+    from mdynamix_gb300.mdx import ForcePath, MdxError
+    s, st = systems.build(systems.spcfw(n=216))
+    count = {}
+    for tc, passes in (("0", 0), ("1", 3)):
+        monkeypatch.setenv("MDX_EWALD_TC", tc)
+        for k in range(1, 60):
+            g = ForcePath(s, precision=MDX_FP64)
+            assert g.L.mdx_probe_fail_alloc(g.h, k) == 0
+            try:
+                g.inifur()
+                done = g.path_info()["ewald_force_pass"] == passes
+            except MdxError:
+                done = False
+            g.close()
+            if done:
+                break
+        count[tc] = k - 1
+    assert 0 < count["1"] <= count["0"]
