@@ -589,9 +589,10 @@ int mdx_open(const mdx_dims *dims, mdx_ctx **out) {
   AL(d.err, 4);
   AL(d.shake_iter, 32);
   AL(d.red, 512);
-  AL(d.red_part, ((size_t)1 << 21) + 2 * RED_CAP1);
-  AL(d.red_ctr, 24);
   d.red_cap = (size_t)1 << 21;
+  d.red_cap1 = std::max<size_t>((size_t)1 << 15, 5 * ((size_t)ctx->d.nkv_max / 32 + 1)) + n;
+  AL(d.red_part, d.red_cap + 2 * d.red_cap1);
+  AL(d.red_ctr, 24);
   if (!rc) {
     unsigned char *ss = nullptr;
     rc = dmalloc(ctx, &ss, scal_scratch_bytes());

@@ -296,7 +296,10 @@ struct DevData {
   int *nspec_d;        // NSPEC per type
   double *red_part;    // per-block partials of the deterministic reductions
   unsigned *red_ctr;
-  size_t red_cap;      // doubles in red_part
+  // doubles in red_part: the main stream's, and (with 8 counters each) behind them
+  // those of each further stream, whose largest sums are the bonded terms' (5 a
+  // block of 128, below one an atom) and the k-vectors' (5 a block of 32)
+  size_t red_cap, red_cap1;
   double2 *sk_part;    // per-slice S(k) partials (deterministic slice sum)
   double *snap;        // mdx_snapshot: positions unpacked for the copy out (3n)
   double *avsum;       // mdx_set_averaging: running sums of the bonded statistics
@@ -413,9 +416,6 @@ inline double fix_period_y(const mdx_ctx *ctx) {
   return ctx->p.icell == 2 ? 2.0 * ctx->boyl : ctx->boyl;
 }
 
-// Doubles (and 8 counters) behind the main stream's for each further stream.
-constexpr size_t RED_CAP1 = (size_t)1 << 19;
-
 // Reduction destinations for a launch of nblocks blocks reducing nv values:
 // deterministic (partials + ordered sum) whenever the partials buffer is
 // large enough.
@@ -423,10 +423,10 @@ inline Dst6 dst6(const mdx_ctx *ctx, size_t nblocks, int nv, double *a,
                  double *b = nullptr, double *c = nullptr, double *d = nullptr,
                  double *e = nullptr, double *f = nullptr) {
   Dst6 r{{a, b, c, d, e, f}, nullptr, nullptr};
-  const size_t cap = ctx->red_slot ? RED_CAP1 : ctx->dv.red_cap;
+  const size_t cap = ctx->red_slot ? ctx->dv.red_cap1 : ctx->dv.red_cap;
   if (ctx->dv.red_part && nblocks * (size_t)nv <= cap) {
     r.part = ctx->dv.red_part +
-             (ctx->red_slot ? ctx->dv.red_cap + (ctx->red_slot - 1) * RED_CAP1 : 0);
+             (ctx->red_slot ? ctx->dv.red_cap + (ctx->red_slot - 1) * ctx->dv.red_cap1 : 0);
     r.ctr = ctx->dv.red_ctr + 8 * ctx->red_slot;
   }
   return r;

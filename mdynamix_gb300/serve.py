@@ -109,9 +109,13 @@ def estimate_bytes(s: S.System, precision: int) -> int:
     if precision != MDX_MIXED:
         per_atom += 28 * (2 * kmax + 18)  # the Z digit images of the fixed-point Ewald passes
         per_atom += 80  # the pair sweeps' integer positions and forces
-    slices = max(1, -(-n // 128))
-    per_k = 256 + 16 * slices
-    return int(n * per_atom + nkv * per_k + (24 << 20))
+    # S(k) partial sums: atom slices of 128, or of 64 where those sums stay
+    # within mdx_slforces_static's scratch (MDX_SK_STATIC_BYTES)
+    part = 16 * nkv * max(1, -(-n // 128))
+    if precision == MDX_MIXED:
+        part = max(part, min(4 << 20, 2 * part))
+    # 16 MiB of reduction scratch; graphs and streams are outside the pool
+    return int(n * per_atom + 256 * nkv + part + (24 << 20))
 
 
 class _Running:

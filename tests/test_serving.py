@@ -133,3 +133,34 @@ def test_same_result_alone_and_in_the_mix(precision, tol):
         y = together[name]
         err = np.abs(x - y).max() / np.abs(x).max()
         assert err <= tol, (name, err)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [MDX_FP64, MDX_MIXED])
+@pytest.mark.parametrize("nwater", [200, 2000])
+def test_estimate_covers_a_context(nwater, precision):
+    """Admission counts a context's device memory by its sizes: what it takes from
+    the pool in a segment with a move stays a tenth below."""
+    import ctypes as C
+    import time
+    from mdynamix_gb300.mdx import ForcePath, load
+
+    def used():
+        u, r = C.c_size_t(), C.c_size_t()
+        assert load().mdx_pool_usage(C.byref(u), C.byref(r)) == 0
+        return u.value
+
+    s = S.System(S.solvation_job("C2H5OH", nwater))
+    st = S.make_configuration(s, seed=3, jitter=0.03)
+    before = used()
+    g = ForcePath(s, precision=precision)
+    g.set_lambda(0.5)
+    g.set_state(*st)
+    g.enqueue_double(2, 0, True)
+    while not g.poll():
+        time.sleep(0.01)
+    g.ee_delta(0.5, 0.25)
+    g.sync()
+    took = used() - before
+    g.close()
+    assert took <= 0.9 * serve.estimate_bytes(s, precision)
