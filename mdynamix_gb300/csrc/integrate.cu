@@ -1218,9 +1218,11 @@ __global__ void __launch_bounds__(SHK_T) k_shake_cluster(
       const double s = lane_sums<2, 4>(s2);  // lanes 0, 1: BSQ; 2, 3: VDOT
       const double BSQ = __shfl_sync(ALL, s, l0), VDOT = __shfl_sync(ALL, s, l0 + 2);
       const double DIFFSQ = BNDSQ - BSQ;
-      // fabs(DIFFSQ) > BNDSQ tol2 by the bit patterns (the same order)
-      const bool adj = act && (__double_as_longlong(DIFFSQ) & 0x7fffffffffffffffLL) >
-                                  __double_as_longlong(BNDSQ * sk.tol2);
+      // fabs(DIFFSQ) > BNDSQ tol2 by the bit patterns: the same order up to
+      // infinity, and no adjustment of a bond that is not a number
+      const long long diff = __double_as_longlong(DIFFSQ) & 0x7fffffffffffffffLL;
+      const bool adj = act && diff > __double_as_longlong(BNDSQ * sk.tol2) &&
+                       diff <= 0x7ff0000000000000LL;
       if (!__any_sync(ALL, adj)) continue;
       const double ci = q < SHK_KEEP ? s_c[q][gi] : inv_mass(I, J);
       const double g = DO * (DIFFSQ * ci * rcp_nr(VDOT));
