@@ -111,6 +111,8 @@ __device__ __forceinline__ void root(R x, R &s, R &si) {
   } else {
     const R r = rsqrt(x), a = x * r;
     s = fma(R(0.5) * r, fma(-a, a, x), a);
+    // 0 and infinity are their own roots (0 times infinity above)
+    if ((unsigned long long)__double_as_longlong(x) - 1 >= 0x7fefffffffffffffull) s = x;
     si = r;
   }
 }
