@@ -12,28 +12,32 @@
 // Both contractions are those of ewald_tc.cu,
 //   S:  D[(e, c)][2z + e'] = sum_j T_j(c)_e Z_j(z)_e',  T = X Y
 //   F:  D[j][4c + t]       = sum_k Z_j[k] W[4c + t][k],  k = 2z + e,
-// done exactly on integers (the splitting of Ozaki, Ogita, Oishi and Rump,
-// Numer. Algorithms 59, 2012): each operand, 55 fractional bits, is cut into
+// done on integers (the splitting of Ozaki, Ogita, Oishi and Rump, Numer.
+// Algorithms 59, 2012): each operand, 55 fractional bits, is cut into
 // 7 signed 8-bit digits d_0 .. d_6 (base 256, d_0 the leading one), exact in
 // FP16.  A product of two digits has 14 bits, so an FP32 accumulator in
 // tensor memory holds the sum of up to 1024 of them exactly.  The products of
 // equal weight (class s = i + j, weight 2^(-14 - 8 s)) share an accumulator;
 // the 28 products with s <= 6 are kept, the rest is below 2^-53 of the
-// operands' range.  One MMA multiplies digit A_i with the digits B_0 ..
-// B_(6-i) side by side along N: they fall on the accumulators i .. 6, which
-// lie side by side too, so A_i is read once and not 7 - i times.
+// operands' range.  F sums at most 64 (s + 1) products of a class and is exact.
+// S drains its accumulators every 192 atoms, s + 1 products each: exact for s <=
+// 4, and for 5 and 6 (weights 2^-54, 2^-62) unless nearly all of 192 atoms have
+// digits near +-128 of one sign throughout, which then costs a few 2^-54 of one
+// atom.  One MMA multiplies digit A_i with the digits B_0 .. B_(6-i) side by
+// side along N: they fall on the accumulators i .. 6, which lie side by side
+// too, so A_i is read once and not 7 - i times.
 //
-// S's accumulators are added to 64-bit integers every 256 atoms; T is formed
+// S's accumulators are added to 64-bit integers every 192 atoms; T is formed
 // in integers (complex product of two-word numbers: 12 wide multiply-adds
 // and a few adds against 4 FP64 instructions of 64 cycles).  F's classes are
 // put together into a 64-bit U, and Im(T U), Im(T V) weighted with nx, ny are
-// again integer.  All sums are exact or rounded once to a fixed unit, so the
-// results do not depend on the order of anything.
+// again integer.  All sums are exact or rounded in one fixed order to a
+// fixed unit, so the results do not depend on the order of anything else.
 //
 // Measured on a GB300 against the FP64-pipe passes of ewald.cu, per
-// evaluation: 98,304 atoms, 16,700 k-vectors: tables 0.060 ms (0.098), S(k)
-// 0.55 (7.7), forces 0.87 (12.8); 21,003 atoms, 3,576 k-vectors: S(k) 0.052
-// (0.76), forces 0.099 (0.73); 609 atoms, 510 k-vectors: 0.015 (0.73), 0.025
+// evaluation: 98,304 atoms, 16,700 k-vectors: tables 0.056 ms (0.098), S(k)
+// 0.58 (7.7), forces 0.91 (12.8); 21,003 atoms, 3,576 k-vectors: S(k) 0.056
+// (0.76), forces 0.113 (0.73); 609 atoms, 510 k-vectors: 0.015 (0.73), 0.025
 // (0.045).  Error of the slow forces against phases and sums of more than 64
 // bits, RMS relative: 5.3e-15 at 98,304 atoms (FP64 pipe: 6.8e-15), 3.6e-15
 // at 3,000 (4.2e-15).
@@ -54,7 +58,11 @@ constexpr int FX_BITS = 8 * FX_SL - 1;   // fractional bits of an operand
 constexpr int FX_ROW = 33;               // int4 per X / Y row of a 32-atom chunk (one of padding)
 constexpr uint32_t FX_POLLS = 1u << 20;  // bounded mbarrier waits
 constexpr size_t FX_SMEM_MAX = 227 * 1024;
-constexpr int FX_DRAIN = 8;              // chunks (of 32 atoms) per S accumulation
+// Chunks (of 32 atoms) per S accumulation: 32 x 6 x 5 products of class 4 stay
+// below 2^24.  With 8 chunks they do not, and atoms of like phase lost 2^-46 of an
+// atom an accumulation; with 4 every class is exact (S(k) of 98,304 atoms: 8
+// chunks 0.562 ms, 6 0.576, 4 0.597).
+constexpr int FX_DRAIN = 6;
 constexpr int FX_TCOL = 8;               // k-columns of an F tile
 constexpr int FX_TN = 4 * FX_TCOL;       // its rows (U.re, U.im, V.re, V.im)
 constexpr int FX_GEN_WARPS = 16;

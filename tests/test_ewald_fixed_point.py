@@ -97,3 +97,52 @@ def test_fixed_point_ewald_reports_non_finite_positions(monkeypatch):
     assert not np.isfinite(g.forces(2)).any()
     g.set_state(*st)   # and back
     assert g.slforces().qpe == ref.qpe
+
+
+@pytest.mark.gpu
+def test_coherent_phases():
+    """S(k) of atoms whose phases and charges are alike, the most that the digit
+    sums can be asked to hold: 17,536 atoms of one sign in a row, and as many of the
+    other with the same z spread among neutral ones, so that the two halves fill the
+    sums to different heights and cancel.  The only k-vector is (0, 0, 1).
+
+    Charges of 39 bits and the images' 55-bit phases are exact, so S(k) is 0 but for
+    the rounding of each block's sum to the unit 2^-46 of 40,960 atoms: half a unit
+    from at most 200 blocks, in either component."""
+    import copy
+    from mdynamix_gb300.mdx import ForcePath
+    rng = np.random.default_rng(7)
+    box, dense, n = (600.0, 600.0, 1500.0), 17536, 40960
+    cutk = 1.5 * 2.0 * np.pi / box[2]
+    s = S.System(S.RunSpec(molecules=[("Na+", n)], box=box, dt_fs=2.0, nfreq=1, rcut=25.0,
+                           rshort=4.0, alpha=0.35 * 25.0, fexp=cutk ** 2 / (4 * 0.35 ** 2),
+                           ichnb=10, trtemp=300.0))
+    s = copy.copy(s)
+
+    def digits(count, m):  # 0.d0 d1 .. in signed base 256 with d0 .. from 116 to 127
+        d = rng.integers(116, 128, (count, m)).astype(float)
+        return (d * 2.0 ** (-7.0 - 8.0 * np.arange(m))).sum(axis=1)
+
+    q = digits(dense, 5)
+    z = np.arccos(digits(dense, 6)) * box[2] / (2 * 3.1415926536) * rng.choice([-1.0, 1.0], dense)
+    grid = rng.permutation(207 * 207)[:n]
+    x, y = ((grid // 207 + 0.5) / 207 - 0.5) * box[0], ((grid % 207 + 0.5) / 207 - 0.5) * box[1]
+    qs, zs = np.zeros(n), rng.uniform(-80.0, 80.0, n)
+    qs[:dense], zs[:dense] = q, z
+    other = (dense + np.arange(n - dense))[np.arange(n - dense) % 4 != 3][:dense]
+    zs[other] = z
+    s.site_charge = np.array([1.0])
+    sums = []
+    for sign in (0.0, -1.0):
+        qs[other] = sign * q
+        s.q = qs.copy()
+        g = ForcePath(s, precision=MDX_FP64)
+        g.set_state(x, y, zs, *[np.zeros(n)] * 3)
+        g.chcnb()
+        sc = g.slforces()
+        assert sc.nkv == 1 and g.path_info()["ewald_sfac_pass"] == 3
+        sums.append(sc.qpe)
+        g.close()
+    one = np.hypot((q * np.cos(2 * 3.1415926536 / box[2] * z)).sum(),
+                   (q * np.sin(2 * 3.1415926536 / box[2] * z)).sum())
+    assert np.sqrt(sums[1] / sums[0]) * one <= 200 * 2.0 ** -47 * np.sqrt(2.0)
