@@ -139,8 +139,11 @@ def roofline_of(timers, mbsh, mbln, nfreq, kset, n, peak64, peak32, prec, nsteps
     from the frozen per-unit constants; time from the device timers (CUDA
     events on the launching stream) of the instrumented pass, per long
     step; peak = measured FMA throughput of the path's floating-point type.
-    The FP64 path forms most of its products as integers (pair sweeps) and as
-    FP16 digits on the tensor cores (Ewald), so it can exceed its FP64 peak."""
+    The FP64 path forms its products as integers (pair sweeps, bound by integer
+    issue and L1) and as FP16 digits on the tensor cores (Ewald, bound by making
+    the digits), off the FP64 pipe: its ratio to the FP64 peak says what the
+    pipe would have allowed, not how far it is from a floor, so it goes by
+    another name and there is no fraction."""
     ms = {k: v[0] / nsteps for k, v in timers.items()}
     nkv, ncol, npair, rows = kset
     ew_kernels = ("k_tables + k_sfac32 + k_sfac_sum + k_wtiles + k_rforce_tc "
@@ -165,14 +168,18 @@ def roofline_of(timers, mbsh, mbln, nfreq, kset, n, peak64, peak32, prec, nsteps
                  "traffic": (TRAFFIC_MB.get((prec, g)) or 0) * 1e6, "kernels": v[2]}
              for g, v in groups.items()}
     frozen = OPS_EW_FROZEN_KATOM * nkv * n + OPS_EW_K * nkv if top == "ewald" else ops
-    return {"bound": "fp64" if prec == "fp64" else "fp32", "achieved": achieved, "peak": peak,
-            "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
+    ratio = achieved / peak if peak else None
+    ratio_frozen = frozen / (t_ms * 1e-3) / 1e12 / peak if peak else None
+    fp64 = prec == "fp64"
+    return {"bound": ("integer issue" if top == "pair" else "digit operands") if fp64 else "fp32",
+            "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+            "frac": None if fp64 else ratio, "over_fp64_pipe": ratio if fp64 else None,
             "traffic": tr * 1e6 if tr is not None else None,
             "kernel": f"{top}: {kernels}", "ms_per_long_step": t_ms, "share_of_step": share,
             "ops_per_long_step": ops,
             "frozen": {"ops_per_long_step": frozen,
                        "achieved": frozen / (t_ms * 1e-3) / 1e12,
-                       "frac": frozen / (t_ms * 1e-3) / 1e12 / peak if peak else None},
+                       "frac": None if fp64 else ratio_frozen},
             "groups": other,
             "peak_source": "measured in-run FMA probe (mdx_probe_fma_peak, of measured)"}
 
@@ -740,7 +747,8 @@ def main():
 
     def roof_short(x):
         return {"bound": x["bound"], "achieved": x["achieved"], "peak": x["peak"],
-                "unit": x["unit"], "frac": x["frac"], "traffic": x["traffic"],
+                "unit": x["unit"], "frac": x["frac"], "over_fp64_pipe": x["over_fp64_pipe"],
+                "traffic": x["traffic"],
                 "kernel": x["kernel"].split(":")[0] + " group",
                 "frac_frozen_ops": x["frozen"]["frac"], "ms_per_step": x["ms_per_long_step"],
                 "share": x["share_of_step"]}
