@@ -388,9 +388,11 @@ int mdx_pending_cuda_error(void);
  * The address is cached per device for the process: do not cudaDeviceReset
  * between calls.  With the mixed path's tensor-core S(k) pass on
  * (MDX_EWALD_TC=2) the pass needs no slice scratch and the size limit does
- * not apply.  Calls whose kernels overlap on the device (other
- * contexts, other streams or threads) share the scratch and race: serialise
- * them. */
+ * not apply.  On the FP64 path the limit applies whichever Ewald passes run (it
+ * is that of the FP64-pipe passes, slices of 512 atoms), although the
+ * fixed-point passes (mdx_path_info.ewald_sfac_pass 3) leave the scratch alone.
+ * Other calls whose kernels overlap on the device (other contexts, other
+ * streams or threads) share the scratch and race: serialise them. */
 #define MDX_SK_STATIC_BYTES (4u << 20)
 int mdx_slforces_static(mdx_ctx *ctx, mdx_scalars *out);
 

@@ -1004,10 +1004,10 @@ int launch_bonded(mdx_ctx *ctx, int laver, bool ener) {
   for (int t = 0; t < ctx->d.ntypes; ++t) shake |= ctx->ishejk[t] > 0;
   // Mixed path: the FP32 terms' last bits depend on the kernel (the contraction
   // of products and sums), and both stiff random starts and SHAKE's tolerance
-  // make much of a last bit within 20 steps.  Where one launch for all kinds
-  // gains least (template molecules alone: 98,304 atoms 13.9 against 12.6 us;
-  // constrained systems: 57 against 29 us of a 700 us step) the terms stay in
-  // their own kernels.
+  // make much of a last bit within 20 steps.  For reproducibility, not speed,
+  // template molecules alone (98,304 atoms: 13.9 us, one launch for all kinds
+  // 12.6) and constrained systems (57 us of a 700 us step against 29) keep the
+  // kernels, and with them the bits, that their trajectories have had.
   const bool own = mx && ((kinds == 1 && d.ntpl > 0) || (shake && ener));
   if (!laver && !own) {
     BondedAll a{};

@@ -15,13 +15,18 @@
 //  - the partial sums (slices x k-vectors x 16 bytes) must fit in
 //    MDX_SK_STATIC_BYTES, else MDX_ERR_UNSUPPORTED (not checked, and the
 //    scratch not used, when the mixed path's tensor-core S(k) pass is on:
-//    that pass keeps its partials in buffers of the k-set);
+//    that pass keeps its partials in buffers of the k-set).  The FP64 path
+//    keeps this limit whichever passes run, so that a program's sizes do not
+//    depend on the switch between them: it is that of the FP64-pipe passes,
+//    in slices of 512 atoms; the fixed-point passes sum S(k) in integers of the
+//    k-set's own and leave the scratch alone;
 //  - device timers must be off (they create events), else MDX_ERR_STATE.
 // Nothing in the static scratch has to start at zero: every (slice, k)
 // partial is written by the S(k) kernel before k_sfac_sum reads it.
-// The scratch is one per device and per process: two calls whose kernels
-// overlap on the device (two contexts on two streams, two host threads) race
-// on it and corrupt each other's S(k).  Serialise such calls.
+// The scratch is one per device and per process: two calls that use it (all but
+// those of the passes named above) and whose kernels overlap on the device (two
+// contexts on two streams, two host threads) race on it and corrupt each other's
+// S(k).  Serialise such calls.
 // Set-up: the first call on a device looks up the scratch's device address
 // with cudaGetSymbolAddress, with that device current; make that first call
 // before any stream capture that is to contain later calls.  Under CUDA's

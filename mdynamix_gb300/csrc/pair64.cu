@@ -651,7 +651,11 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64t(
 // the force at the table's start; it is added as an integer, whatever the
 // order.  The LJ term comes from a tabulated 1 / r^2 in 9 FP64 instructions
 // and joins G.  Everything else goes to the FP64 expressions as before, and
-// so do atoms and pairs out of the numbers' range.
+// so do atoms and pairs out of the numbers' range.  The unit is one for a sweep, so
+// a distant pair's force, alone, has fewer significant bits than an FP64 number;
+// an atom's slow force does not show it, in a gas either, because the rounding of
+// its reciprocal part is larger (two waters 10 A apart: 2.5e-13 of the force,
+// written out 2.3e-13).
 struct __align__(16) PxPoly {
   long long c0, c1, c2;  // c0, 2 c1, 4 c2
   int c3, sh;            // 8 c3 in units of 2^(32 - sh)
