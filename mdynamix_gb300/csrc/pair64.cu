@@ -25,8 +25,8 @@
 //
 // Measured on a GB300 at 98,304 atoms (one warp an owner and everything
 // written out; k_pair64t; k_pair64x): short rows, forces 0.526, 0.20, 0.090 ms;
-// long rows with energies 4.88, 2.40, 1.09 ms, with energies by type pair
-// 15.3, 3.1, 1.4 ms.  k_pair64t's FP64 pipe is 82-86 % active.  Error of the
+// long rows with energies 4.88, 2.40, 1.15 ms, with energies by type pair
+// 15.3, 3.1, 1.43 ms.  k_pair64t's FP64 pipe is 82-86 % active.  Error of the
 // short rows' forces against 128 bits (200 ions; rms, of the rms force): 2.8e-15
 // written out, 4e-16 in integers.
 //
@@ -685,6 +685,35 @@ __device__ __forceinline__ long long cross2(I2 a, I2 b) {
 __device__ __forceinline__ long long mulhi2(I2 a, I2 b) {
   return (long long)a.h * b.h + ((cross2(a, b) + 0x80000000LL) >> 32);
 }
+// a a / 2^62 from its crossed product c = h l + 2^28, to the nearest
+__device__ __forceinline__ long long sq_cross(I2 a) {
+  return (long long)a.h * a.l + 0x10000000LL;
+}
+__device__ __forceinline__ long long sq4(I2 a, long long c) {
+  return ((long long)a.h * a.h << 2) + (c >> 29);
+}
+// A lane's sum of products a b / 2^64 (|a b| < 2^122), kept to 24 bits below that
+// unit: the high products and the crossed ones apart.  Energies and virials are sums
+// of terms that nearly cancel and one unit holds for the closest pair and the most
+// distant one, so a pair's term rounded to the unit shows in the sum: 1,500 ions,
+// long rows from 4.5 to 12 A, in 2^-53 of the root of the terms' squares, the virial
+// 152 off rounded pair by pair, 10 so, 5 written out in FP64; the energy from 6.6 A on
+// 41, 6, 3.  Costs 0.04 to 0.06 ms of the long sweep at 98,304 atoms.
+struct Sum2 {
+  long long h = 0, c = 0;
+  __device__ __forceinline__ void add(I2 a, I2 b) {
+    h += (long long)a.h * b.h;
+    c += cross2(a, b) >> 8;
+  }
+  // whole units out, to the nearest (a floor would be the same way in every row);
+  // the rest stays for the next row
+  __device__ __forceinline__ double take() {
+    const long long k = (c + 0x800000LL) >> 24, u = h + k;
+    c -= k << 24;
+    h = 0;
+    return (double)u;
+  }
+};
 struct PxArg {
   int bin;
   I2 t;
@@ -717,10 +746,11 @@ __device__ __forceinline__ long long px_eval(const PxPoly *tab, const PxArg &a) 
 // records and the atomics that kept L1 88 % busy.  A third table (1 / r, force
 // calls) would leave L1 too little for the records.  98,304 atoms, long rows with
 // energies 1.24 ms from L1, 1.09 from shared memory; with energies by type pair
-// 1.50, 1.39, with all three 2.13.  Only where a warp has several owners: the
-// copy, and the SMs' change to another split of their memory between two
-// kernels of a small system, cost more (3,000 atoms, 20 steps: 6.64 ms without,
-// 7.02 with; the short rows gain 4 % at 98,304 atoms and nothing at 21,003).
+// 1.50, 1.39, with all three 2.13 (Sum2, in both since, adds 0.05).  Only where a
+// warp has several owners: the copy, and the SMs' change to another split of their
+// memory between two kernels of a small system, cost more (3,000 atoms, 20 steps:
+// 6.64 ms without, 7.02 with; the short rows gain 4 % at 98,304 atoms and nothing at
+// 21,003).
 constexpr int px_tables(bool ener) { return ener ? 2 : 1; }
 
 struct PxQueue {  // pairs put aside for their LJ term, per warp
@@ -763,24 +793,26 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64x(
   const unsigned eem = v.rae_on ? eemask : 0u;
   Acc64 a;
   acc_zero(a);
-  long long ie = 0, ivx = 0, ivy = 0, ivz = 0;  // this owner's row
+  Sum2 ie, ivx, ivy, ivz;  // this owner's row
   int nq = 0, nslow = 0;
   auto add = [&](int i, long long x, long long y, long long z) {
     atomicAdd(&ff[i], (unsigned long long)x);
     atomicAdd(&ff[(size_t)n + i], (unsigned long long)y);
     atomicAdd(&ff[2 * (size_t)n + i], (unsigned long long)z);
   };
-  auto virial = [&](long long x, long long y, long long z, I2 dx, I2 dy, I2 dz) {
-    ivx += mulhi2(split2(x), dx);
-    ivy += mulhi2(split2(y), dy);
-    ivz += mulhi2(split2(z), dz);
+  // g: to the nearest.  Forces take it floored: half a unit along each of an atom's
+  // pairs cancels, in a virial it adds up.
+  auto virial = [&](I2 g, I2 dx, I2 dy, I2 dz, long long cx, long long cy, long long cz) {
+    ivx.add(g, split2(sq4(dx, cx)));
+    ivy.add(g, split2(sq4(dy, cy)));
+    ivz.add(g, split2(sq4(dz, cz)));
   };
   // the last m (<= 32) pairs of the LJ queue: their LJ terms, then forces
   auto lj_batch = [&](int m) {
     __syncwarp();
     if (lane < m) {
       const int e = nq - m + lane;
-      const int tix = q.tix[e], i = q.i[e], j = q.j[e];
+      const int tix = ENER ? q.tix[e] >> 1 : q.tix[e], i = q.i[e], j = q.j[e];
       const double r = (double)px_eval(px.tab + PT_R2I * px.nbin, px_arg(px, q.r2[e]));
       // times 2^-s2 by the exponent
       const double R2I =
@@ -799,10 +831,13 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64x(
       }
       // 2^60: the sums of forces stay far below 2^63
       if ((__double_as_longlong(FL) & 0x7fffffffffffffffLL) < 0x43b0000000000000LL) {
-        const I2 g = split2(q.g[e] + __double2ll_rn(FL));
+        const long long G64 = q.g[e] + __double2ll_rn(FL);
+        const I2 g = split2(G64);
         const I2 dx = split2(q.x[e]), dy = split2(q.y[e]), dz = split2(q.z[e]);
         const long long gx = mulhi2(g, dx), gy = mulhi2(g, dy), gz = mulhi2(g, dz);
-        if (ENER) virial(gx, gy, gz, dx, dy, dz);
+        if (ENER)
+          virial(split2(G64 + (q.tix[e] & 1)), dx, dy, dz, sq_cross(dx), sq_cross(dy),
+                 sq_cross(dz));
         add(i, gx, gy, gz);
         add(j, -gx, -gy, -gz);
       } else {
@@ -857,11 +892,10 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64x(
       DY <<= px.s;
       DZ <<= px.s;
       const I2 dx = split2(DX), dy = split2(DY), dz = split2(DZ);
-      const long long cr = (long long)dx.h * dx.l + (long long)dy.h * dy.l +
-                           (long long)dz.h * dz.l + 0x40000000LL;
+      const long long cx = sq_cross(dx), cy = sq_cross(dy), cz = sq_cross(dz);
       const unsigned long long r2 =
           (unsigned long long)((long long)dx.h * dx.h + (long long)dy.h * dy.h +
-                               (long long)dz.h * dz.h + (cr >> 31));
+                               (long long)dz.h * dz.h + ((cx + cy + cz + 0x10000000LL) >> 31));
       PxArg p = px_arg(px, r2);
       const bool other = (SHORT && e < 0) || aj.y == ai.y || eei || ((eem >> aj.x) & 1u) ||
                          jp.w == IPOS_BAD || !in || (unsigned)p.bin >= (unsigned)px.nbin;
@@ -876,10 +910,12 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64x(
       }
       const I2 qq = split2(mulhi2(qi, split2(jp.w)));
       const I2 F = split2(px_eval(tab + PT_FORCE * px.nbin, p));
-      const long long g = (((long long)F.h * qq.h) << 4) + (cross2(F, qq) >> 28);
+      const long long cg = cross2(F, qq);
+      const long long g = (((long long)F.h * qq.h) << 4) + (cg >> 28);
+      const int up = (int)(cg >> 27) & 1;  // g + up: to the nearest
       if (ENER) {
-        const long long E = mulhi2(split2(px_eval(tab + PT_ENER * px.nbin, p)), qq);
-        if (fast) ie += E;
+        const I2 E = split2(px_eval(tab + PT_ENER * px.nbin, p));
+        if (fast) ie.add(E, qq);
       }
       if (SPLIT && fast)
         split_add(a, tc.mdx[ai.x][aj.x],
@@ -889,7 +925,7 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64x(
       if (fast && !lb) {
         const I2 G = split2(g);
         const long long gx = mulhi2(G, dx), gy = mulhi2(G, dy), gz = mulhi2(G, dz);
-        if (ENER) virial(gx, gy, gz, dx, dy, dz);
+        if (ENER) virial(split2(g + up), dx, dy, dz, cx, cy, cz);
         ax += gx;
         ay += gy;
         az += gz;
@@ -906,7 +942,8 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64x(
           q.g[s] = g;
           q.i[s] = i;
           q.j[s] = j;
-          q.tix[s] = ai.z * pc.nnbt + aj.z;
+          const int tix = ai.z * pc.nnbt + aj.z;
+          q.tix[s] = ENER ? 2 * tix + up : tix;
         }
         nq += __popc(ml);
         if (nq >= 32) lj_batch(32);
@@ -923,19 +960,18 @@ __global__ void __launch_bounds__(32 * PT_WARPS, 2) k_pair64x(
       atomicAdd(&ff[(size_t)k * n + i], (unsigned long long)(k == 0 ? ax : k == 1 ? ay : az));
     }
     if (ENER) {  // a row's sums stay below 2^63
-      a.e[A_EES] = fma((double)ie, px.uE, a.e[A_EES]);
-      a.e[A_VX] = fma((double)ivx, px.uV, a.e[A_VX]);
-      a.e[A_VY] = fma((double)ivy, px.uV, a.e[A_VY]);
-      a.e[A_VZ] = fma((double)ivz, px.uV, a.e[A_VZ]);
-      ie = ivx = ivy = ivz = 0;
+      a.e[A_EES] = fma(ie.take(), px.uE, a.e[A_EES]);
+      a.e[A_VX] = fma(ivx.take(), px.uV, a.e[A_VX]);
+      a.e[A_VY] = fma(ivy.take(), px.uV, a.e[A_VY]);
+      a.e[A_VZ] = fma(ivz.take(), px.uV, a.e[A_VZ]);
     }
   }
   if (nq) lj_batch(nq);
   if (nslow) slow_batch(nslow);
   if (ENER) {
-    a.e[A_VX] = fma((double)ivx, px.uV, a.e[A_VX]);
-    a.e[A_VY] = fma((double)ivy, px.uV, a.e[A_VY]);
-    a.e[A_VZ] = fma((double)ivz, px.uV, a.e[A_VZ]);
+    a.e[A_VX] = fma(ivx.take(), px.uV, a.e[A_VX]);
+    a.e[A_VY] = fma(ivy.take(), px.uV, a.e[A_VY]);
+    a.e[A_VZ] = fma(ivz.take(), px.uV, a.e[A_VZ]);
   }
   sweep_out<SPLIT, ENER>(a, dst, s_split, split);
 }
@@ -998,7 +1034,7 @@ Px px_args(const mdx_ctx *ctx, bool shrt) {
   x.uG = std::ldexp(cf, q2 - s[PT_FORCE]);
   x.iG = 6.0 * std::ldexp(1.0 / cf, s[PT_FORCE] - q2);  // 6: FSR R1 / 6
   x.du = std::ldexp(1.0, rho - 62);
-  x.uV = std::ldexp(x.uG, 4 + 2 * (rho - 62) + 124);
+  x.uV = std::ldexp(x.uG, 2 * (rho - 62) + 126);
   x.uE = std::ldexp(cf, q2 + 4 - s[PT_ENER]);
   x.uR = std::ldexp(cf, q2 + 4 - s[PT_R1I]);
   x.s2 = s[PT_R2I];
